@@ -187,6 +187,26 @@ def test_sgemm(M, N, K):
     assert torch.equal(out1[0], out[M - 1])
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 1), (15, 63, 17), (17, 65, 16), (64, 128, 50), (65, 129, 64), (200, 68, 33)])
+def test_sgemm_tiles(M, N, K):
+    """Every tile gives a sum over k in order: the same bits."""
+    from tgo_b200.kernels.build import load_library
+    x, w = rnd(M, K, seed=3), rnd(N, K, seed=4)
+    outs = []
+    try:
+        for tile in (1, 2, 3):
+            load_library("sgemm").tgo_sgemm_force_tile(tile)
+            outs.append(torch.full((M, N), float("nan"), device=DEV))
+            ops().sgemm_tn(x, w, outs[-1])
+    finally:
+        load_library("sgemm").tgo_sgemm_force_tile(0)
+    want = x.double() @ w.double().t()
+    # a chain of K roundings of at most K |x| |w| 2^-24 each
+    bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
+    assert ((outs[0].double() - want).abs() <= bound + 1e-30).all()
+    assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
 # ----------------------------------------------------------------------- attention
 
 
@@ -285,6 +305,26 @@ def test_attention_mixed_batch(H, Hkv, dh, ps, window, dtype):
     ops().attention_generic(case["q"], out2, H, Hkv, dh, case["kc"], case["vc"], ps, case["bt"],
                             case["seq"], case["pos"], scale, window)
     assert torch.allclose(out2.float().cpu(), want, **tol(dtype))
+
+
+@pytest.mark.parametrize("H,Hkv,dh,ps", [(4, 4, 8, 4), (6, 2, 36, 8), (16, 1, 256, 16), (5, 1, 132, 32), (16, 4, 128, 16)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_tiles(H, Hkv, dh, ps, dtype, monkeypatch):
+    """Keys through shared memory for a block of queries: the bits of a warp a query, with every
+    option, requests that meet inside a block, and a token that brings nothing."""
+    case = paged_case([33, 1, 7, 64], [0, 40, 31, 5], H, Hkv, dh, ps, dtype, seed=dh)
+    case["pos"][-1] = -1
+    T = case["q"].shape[0]
+    extra = dict(sinks=rnd(H, seed=1), softcap=3.0, dist_bias=rnd(50, H, seed=2), gate=rnd(T, H, seed=3).to(dtype))
+    for kw in ({}, extra):
+        outs = []
+        for start in (4, 10 ** 9):
+            monkeypatch.setattr(ops(), "GENERIC_TILES_FROM", start)
+            outs.append(torch.full_like(case["q"], 7.0))
+            ops().attention_generic(case["q"], outs[-1], H, Hkv, dh, case["kc"], case["vc"], ps, case["bt"],
+                                    case["seq"], case["pos"], dh ** -0.5, 0, **kw)
+        assert torch.equal(outs[0], outs[1]) and bool(torch.isfinite(outs[0].float()).all())
+        assert not outs[0][-1].any()
 
 
 @pytest.mark.parametrize("H,Hkv,dh,ps", SHAPES)

@@ -111,6 +111,216 @@ __global__ void attention_generic_kernel(
     }
 }
 
+// ------------------------------------------------------------- prompt portions, every earlier key
+// The same sums in the same order, for steps that bring several tokens a request and see every
+// earlier key (window 0: the keys are then cut into the same 32 for every query). A block takes
+// AGT_Q query rows (the heads of one kv head x consecutive tokens) and brings each 32 keys and
+// values into shared memory once for all of them; a warp owns AGT_R rows, a lane one key for the
+// scores and 4 NV channels for the sums. Bound by reads of shared memory (a 16-byte read of a key
+// row feeds 4 AGT_R FMA). Rows of another request in the block are walked after the first's.
+// The caller picks this kernel from four tokens a request on (bits do not depend on it): MEASURED
+// (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this about 140.
+#define AGT_WARPS 4
+#define AGT_R 4
+#define AGT_Q (AGT_WARPS * AGT_R)
+
+__device__ __forceinline__ float4 ag_load4(const float* p) { return *(const float4*)p; }
+__device__ __forceinline__ float4 ag_load4(const bf16* p) {
+    const uint2 v = *(const uint2*)p;
+    const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&v.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&v.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+}
+
+template <typename T, int NV>
+__global__ void __launch_bounds__(32 * AGT_WARPS)
+attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* __restrict__ out, long long out_stride,
+                               int Tn, int H, int Hkv, int dh, int dv, const T* __restrict__ k_cache,
+                               const T* __restrict__ v_cache, int page_size, const int* __restrict__ block_tables,
+                               int max_blocks, const int* __restrict__ seq_ids, const int* __restrict__ positions,
+                               float scale, const float* __restrict__ sinks, float softcap, int v_row,
+                               const float* __restrict__ dist_bias, int n_dist, const T* __restrict__ gate,
+                               long long gate_stride) {
+    extern __shared__ __align__(16) float agt_smem[];
+    const int ldk = dh + 4;                              // 16-byte reads of 8 rows hit 8 different places
+    float* ks = agt_smem;                                // [32][ldk]
+    float* vs = ks + 32 * ldk;                           // [32][dv]
+    float* qs = vs + 32 * dv;                            // [AGT_Q][dh]
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int G = H / Hkv, kvh = blockIdx.y;
+    const int nt = AGT_Q / G, nq = nt * G;               // tokens and rows of a block (G <= AGT_Q)
+    const int t0 = blockIdx.x * nt, t_end = t0 + nt < Tn ? t0 + nt : Tn;
+    for (int i = threadIdx.x; i < nq * dh; i += blockDim.x) {
+        const int r = i / dh, t = t0 + r / G;
+        qs[i] = t < t_end ? to_f32(q[(size_t)t * q_stride + (size_t)(kvh * G + r % G) * dh + i % dh]) : 0.f;
+    }
+    float m[AGT_R], l[AGT_R];
+    float4 acc[AGT_R][NV];
+    int tok[AGT_R], pos[AGT_R];
+#pragma unroll
+    for (int r = 0; r < AGT_R; ++r) {
+        const int row = warp * AGT_R + r;
+        m[r] = -INFINITY;
+        l[r] = 0.f;
+        tok[r] = row < nq ? t0 + row / G : t_end;
+        pos[r] = tok[r] < t_end ? positions[tok[r]] : -1;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) acc[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+    for (int ta = t0; ta < t_end;) {                     // a run of tokens of one request
+        int tb = ta + 1, p_last = positions[ta];
+        const int b = p_last >= 0 ? seq_ids[ta] : -1;
+        for (; tb < t_end; ++tb) {
+            const int p = positions[tb];
+            if ((p >= 0 ? seq_ids[tb] : -1) != b) break;
+            p_last = p > p_last ? p : p_last;
+        }
+        const int* bt = block_tables + (size_t)(b < 0 ? 0 : b) * max_blocks;
+        for (int k0 = 0; k0 <= p_last; k0 += 32) {
+            __syncthreads();                             // the last keys have been read
+            for (int i = threadIdx.x; i < 32 * (dh / 4); i += blockDim.x) {
+                const int r = i / (dh / 4), c = (i % (dh / 4)) * 4, j = k0 + r;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j <= p_last)
+                    v = ag_load4(k_cache + (((size_t)bt[j / page_size] * Hkv + kvh) * page_size + (j % page_size)) * dh + c);
+                *(float4*)(ks + r * ldk + c) = v;
+            }
+            for (int i = threadIdx.x; i < 32 * (dv / 4); i += blockDim.x) {
+                const int r = i / (dv / 4), c = (i % (dv / 4)) * 4, j = k0 + r;
+                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (j <= p_last)
+                    v = ag_load4(v_cache + (((size_t)bt[j / page_size] * Hkv + kvh) * page_size + (j % page_size)) * v_row + c);
+                *(float4*)(vs + r * dv + c) = v;
+            }
+            __syncthreads();
+            float a[AGT_R], w[AGT_R];
+#pragma unroll
+            for (int r = 0; r < AGT_R; ++r) a[r] = 0.f;
+#pragma unroll 4
+            for (int d = 0; d < dh; d += 4) {
+                const float4 k4 = *(const float4*)(ks + lane * ldk + d);
+#pragma unroll
+                for (int r = 0; r < AGT_R; ++r) {
+                    const float4 q4 = *(const float4*)(qs + (warp * AGT_R + r) * dh + d);
+                    a[r] = fmaf(q4.x, k4.x, a[r]);
+                    a[r] = fmaf(q4.y, k4.y, a[r]);
+                    a[r] = fmaf(q4.z, k4.z, a[r]);
+                    a[r] = fmaf(q4.w, k4.w, a[r]);
+                }
+            }
+            int most = 0;
+#pragma unroll
+            for (int r = 0; r < AGT_R; ++r) {
+                const bool mine = tok[r] >= ta && tok[r] < tb && k0 <= pos[r];
+                const int p = pos[r], j = k0 + lane;
+                w[r] = 0.f;
+                if (!mine) continue;                     // the same for the whole warp
+                float s = -INFINITY;
+                if (j <= p) {
+                    s = a[r] * scale;
+                    if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+                    if (dist_bias) s += dist_bias[(size_t)((p - j) < n_dist ? (p - j) : n_dist - 1) * H + kvh * G + (warp * AGT_R + r) % G];
+                }
+                const float m_new = fmaxf(m[r], warp_max(s));
+                const float corr = expf(m[r] - m_new);
+                w[r] = j <= p ? expf(s - m_new) : 0.f;
+                l[r] = l[r] * corr + warp_sum(w[r]);
+#pragma unroll
+                for (int i = 0; i < NV; ++i) {
+                    acc[r][i].x *= corr; acc[r][i].y *= corr; acc[r][i].z *= corr; acc[r][i].w *= corr;
+                }
+                m[r] = m_new;
+                const int n = p - k0 + 1 < 32 ? p - k0 + 1 : 32;
+                most = n > most ? n : most;
+            }
+            for (int jj = 0; jj < most; ++jj) {
+                float4 v4[NV];
+#pragma unroll
+                for (int i = 0; i < NV; ++i)
+                    v4[i] = (lane + 32 * i) * 4 < dv ? *(const float4*)(vs + jj * dv + (lane + 32 * i) * 4)
+                                                     : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int r = 0; r < AGT_R; ++r) {
+                    const float wj = __shfl_sync(0xffffffffu, w[r], jj);
+                    if (k0 + jj > pos[r]) continue;      // past this row's keys: nothing is added, not even 0 x NaN
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) {
+                        acc[r][i].x = fmaf(wj, v4[i].x, acc[r][i].x);
+                        acc[r][i].y = fmaf(wj, v4[i].y, acc[r][i].y);
+                        acc[r][i].z = fmaf(wj, v4[i].z, acc[r][i].z);
+                        acc[r][i].w = fmaf(wj, v4[i].w, acc[r][i].w);
+                    }
+                }
+            }
+        }
+        ta = tb;
+    }
+#pragma unroll
+    for (int r = 0; r < AGT_R; ++r) {
+        if (tok[r] >= t_end) continue;
+        const int h = kvh * G + (warp * AGT_R + r) % G;
+        if (sinks && pos[r] >= 0) {                      // the sink joins the denominator last
+            const float sk = sinks[h];
+            const float m_new = fmaxf(m[r], sk);
+            const float corr = expf(m[r] - m_new);
+            l[r] = l[r] * corr + expf(sk - m_new);
+#pragma unroll
+            for (int i = 0; i < NV; ++i) {
+                acc[r][i].x *= corr; acc[r][i].y *= corr; acc[r][i].z *= corr; acc[r][i].w *= corr;
+            }
+        }
+        float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+        if (gate) inv *= 1.f / (1.f + expf(-to_f32(gate[(size_t)tok[r] * gate_stride + h])));
+        T* o = out + (size_t)tok[r] * out_stride + (size_t)h * dv;
+#pragma unroll
+        for (int i = 0; i < NV; ++i) {
+            const int d = (lane + 32 * i) * 4;
+            if (d >= dv) continue;
+            o[d] = from_f32<T>(acc[r][i].x * inv);
+            o[d + 1] = from_f32<T>(acc[r][i].y * inv);
+            o[d + 2] = from_f32<T>(acc[r][i].z * inv);
+            o[d + 3] = from_f32<T>(acc[r][i].w * inv);
+        }
+    }
+}
+
+// 1 if the tiled kernel takes the step: heads of a group within a block's rows, widths of whole
+// 16-byte (8-byte in bfloat16) pieces up to 256.
+TGO_API int tgo_attention_generic_tiles_takes(int H, int Hkv, int dh, int dv, int v_row) {
+    return Hkv > 0 && H % Hkv == 0 && H / Hkv <= AGT_Q && dh > 0 && dh <= AG_MAX_DH && dh % 4 == 0 && dv > 0 &&
+           dv <= AG_MAX_DH && dv % 4 == 0 && v_row >= dv && v_row % 4 == 0;
+}
+
+TGO_API int tgo_attention_generic_tiles(const void* q, long long q_stride, void* out, long long out_stride, int dtype,
+                                        int T, int H, int Hkv, int dh, int dv, const void* k_cache,
+                                        const void* v_cache, int page_size, const int* block_tables, int max_blocks,
+                                        const int* seq_ids, const int* positions, float scale, const float* sinks,
+                                        float softcap, int v_row, const float* dist_bias, int n_dist,
+                                        const void* gate, long long gate_stride, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (v_row <= 0) v_row = dv;
+    if (!tgo_attention_generic_tiles_takes(H, Hkv, dh, dv, v_row) || Hkv > 65535 || page_size <= 0 || max_blocks <= 0 ||
+        !(softcap >= 0.f) || (dist_bias && n_dist <= 0) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15) ||
+        (dtype != TGO_BF16 && dtype != TGO_F32))
+        return TGO_E_BAD_ARG;
+    const int nt = AGT_Q / (H / Hkv);
+    const dim3 grid((T + nt - 1) / nt, Hkv);
+    const size_t smem = (size_t)(32 * (dh + 4) + 32 * dv + AGT_Q * dh) * sizeof(float);
+#define AGT_GO(TT, NV)                                                                                         \
+    do {                                                                                                        \
+        const cudaError_t e = cudaFuncSetAttribute(attention_generic_tiles_kernel<TT, NV>,                      \
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
+        if (e != cudaSuccess) return (int)e;                                                                    \
+        attention_generic_tiles_kernel<TT, NV><<<grid, 32 * AGT_WARPS, smem, stream>>>(                         \
+            (const TT*)q, q_stride, (TT*)out, out_stride, T, H, Hkv, dh, dv, (const TT*)k_cache,                \
+            (const TT*)v_cache, page_size, block_tables, max_blocks, seq_ids, positions, scale, sinks, softcap, \
+            v_row, dist_bias, n_dist, (const TT*)gate, gate_stride);                                            \
+    } while (0)
+    if (dtype == TGO_BF16) { if (dv > 128) AGT_GO(bf16, 2); else AGT_GO(bf16, 1); }
+    else { if (dv > 128) AGT_GO(float, 2); else AGT_GO(float, 1); }
+#undef AGT_GO
+    return launch_status();
+}
+
 TGO_API int tgo_attention_generic(const void* q, long long q_stride, void* out,
                                   long long out_stride, int dtype, int T, int H, int Hkv, int dh, int dv,
                                   const void* k_cache, const void* v_cache, int page_size,

@@ -196,6 +196,10 @@ def qk_norm_rope_cache(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[t
         "qk_norm_rope_cache", f"(head_dim={head_dim}, rotary_dim={rotary_dim})")
 
 
+GENERIC_TILES_FROM = 4      # tokens a request from which the generic attention's keys go through
+                            # shared memory, once for a block of queries (bits are the same)
+
+
 def attention_generic(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_heads: int,
                       head_dim: int, k_cache: torch.Tensor, v_cache: torch.Tensor, page_size: int,
                       block_tables: torch.Tensor, seq_ids: torch.Tensor, positions: torch.Tensor,
@@ -228,6 +232,20 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv
     assert block_tables.is_contiguous() and seq_ids.dtype == torch.int32
     assert positions.dtype == torch.int32
     lib = load_library("attention_generic")
+    if not window and T >= GENERIC_TILES_FROM * block_tables.shape[0] and \
+            k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and \
+            lib.tgo_attention_generic_tiles_takes(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
+                                                  c_int(value_dim or head_dim),
+                                                  c_int(value_row or value_dim or head_dim)):
+        _check(lib.tgo_attention_generic_tiles(
+            _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(dtype_code(q.dtype)), c_int(T),
+            c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim or head_dim), _ptr(k_cache),
+            _ptr(v_cache), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(seq_ids),
+            _ptr(positions), c_float(scale), _ptr(sinks), c_float(softcap or 0.0), c_int(value_row),
+            _ptr(dist_bias), c_int(dist_bias.shape[0] if dist_bias is not None else 0), _ptr(gate),
+            c_ll(gate.stride(0) if gate is not None else 0), _stream()), "attention_generic_tiles",
+            f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads})")
+        return
     _check(lib.tgo_attention_generic(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(dtype_code(q.dtype)),
         c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
