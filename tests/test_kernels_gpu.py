@@ -964,3 +964,35 @@ def test_attention_decode_beyond_the_on_chip_table(window):
                               n_splits=n_splits)
         assert torch.allclose(out.float().cpu(), want, **tol(torch.bfloat16)), n_splits
     assert ops().attention_decode_tma_error() == 0
+
+
+@pytest.mark.parametrize("H,Hkv,dh,ps", [(8, 2, 64, 16), (5, 1, 128, 8), (16, 1, 64, 32), (4, 4, 128, 64)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (130, 0), (140, 5), (300, 200)])
+@pytest.mark.parametrize("extra", ["sink", "cap", "bias", "all"])
+def test_attention_tc_options(H, Hkv, dh, ps, window, keep, extra):
+    """The tcgen05 attention with a sink, kept first keys, bounded scores, a bias by distance and a
+    gate, against the generic kernel's float32 arithmetic on the same stored values. P and the
+    result are rounded to bfloat16, as in the plain form."""
+    case = paged_case([150, 1, 40, 261], [333, 500, 0, 7], H, Hkv, dh, ps, torch.bfloat16, seed=dh + ps)
+    T = case["q"].shape[0]
+    kw = dict(softcap=2.0 if extra in ("cap", "all") else 0.0, keep_first=keep,
+              dist_bias=rnd(70, H, seed=1) if extra in ("bias", "all") else None,
+              sinks=rnd(H, seed=2) if extra in ("sink", "all") else None,
+              gate=rnd(T, H, seed=3).to(torch.bfloat16) if extra == "all" else None)
+    scale, o = dh ** -0.5, ops()
+    if keep:
+        # what lies between the kept keys and the window of every token of the step has gone back
+        for i in range(-(-keep // ps), max(0, 333 - window + 1) // ps):
+            case["bt"][0, i] = 0
+    t0, nt = attention_part().step_tiles(Ctx(case, False), 128 // (H // Hkv))
+    out = torch.full_like(case["q"], 9.0)
+    o.attention_tc_prefill(case["q"], out, H, Hkv, dh, case["kc"], case["vc"], ps, case["bt"], case["pos"],
+                           case["seq"], t0, nt, scale, window, own_counters=True, **kw)
+    want = torch.empty_like(case["q"].float())
+    if kw["gate"] is not None:
+        kw["gate"] = kw["gate"].float()
+    o.attention_generic(case["q"].float(), want, H, Hkv, dh, case["kc"].float(), case["vc"].float(), ps, case["bt"],
+                        case["seq"], case["pos"], scale, window, **kw)
+    assert o.attention_tc_error() == 0
+    assert bool(torch.isfinite(want).all())
+    assert torch.allclose(out.float(), want, **tol(torch.bfloat16))

@@ -1,4 +1,4 @@
-// Paged causal attention for prompt portions on the tcgen05 tensor cores (head size 128,
+// Paged causal attention for prompt portions on the tcgen05 tensor cores (head sizes 64 and 128,
 // bfloat16): S = Q K^T and O += P V are tcgen05.mma with the accumulators in tensor memory,
 // Q, K and V come in by TMA, and the softmax runs in registers between the two products.
 //
@@ -35,6 +35,11 @@
 // softmax threads a row, 32 keys each, sixteen softmax warps (68.5 us against 66.2, 651 against
 // 612 at 8192 tokens: nor do they lack warps to hide their own latency).
 //
+// The same kernel serves the attention that has a sink, first keys kept beside a window, bounded
+// scores, a bias by distance or a gate per head, at head sizes 64 and 128 (`ApExtra`); the kept
+// keys' tiles are walked before the window's. MEASURED, 2348 + 1611 tokens' worth of keys for 2048 +
+// 1536 queries of 16/4 heads of 128, window 1024, sink: 60 us; 390 us for the mma.sync tiles.
+//
 // Every wait has a time limit (about two seconds): it records a code, the CTA stops issuing,
 // frees its tensor memory and returns. No cluster, no multicast.
 #include <cuda.h>
@@ -46,14 +51,10 @@
 
 #define AT_BM 128
 #define AT_BN 128
-#define AT_DH 128
 #define AT_WAIT_CYCLES 4000000000ll
 #define AT_BLOCK_BYTES (128 * 64 * 2)          // 128 rows x 64 columns of bf16
 #define AT_TILE_BYTES (2 * AT_BLOCK_BYTES)     // a Q, K or V tile: two column halves
 #define AT_PAGES_CAP 1024
-#ifndef AP_PV_N
-#define AP_PV_N 128      // output columns of one P V product: 128, or 64 (two products a k-step)
-#endif
 #ifndef AP_LBO_BYTES
 #define AP_LBO_BYTES AT_BLOCK_BYTES
 #endif
@@ -134,7 +135,7 @@ __device__ __forceinline__ uint64_t at_desc(const void* tile) {
 // lies AP_LBO_BYTES after the first.
 __device__ __forceinline__ uint64_t at_desc_mn(const void* tile) {
     uint64_t d = (uint64_t)((at_smem(tile) & 0x3ffff) >> 4);
-    d |= (uint64_t)((AP_PV_N == 128 ? AP_LBO_BYTES : 1024) >> 4) << 16;
+    d |= (uint64_t)(AP_LBO_BYTES >> 4) << 16;
     d |= (uint64_t)(1024 >> 4) << 32;
     d |= (uint64_t)1 << 46;
     d |= (uint64_t)2 << 61;
@@ -208,15 +209,41 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
 struct ApItem {          // what warp 0 tells the others about an item
     int valid;           // 0: no more items
     int tok0, n_rows, p0, n_it, t_lo, key_lo, key_hi, seq, kvh;
-    int pad[6];
+    int n_kept;          // key tiles of kept first keys that lie before tile t_lo: walked first
+    int pad[5];
 };
 
 // The counter the CTAs draw items from, and the count of CTAs that have finished: the last
 // CTA of a launch to finish sets both back to zero for the next launch (every CTA reaches its
 // end, whatever its waits did).
-__device__ unsigned int ap_ticket = 0;
-__device__ unsigned int ap_finished = 0;
+// A caller may bring two zeroed counters of its own instead (launches that may overlap).
+__device__ unsigned int ap_counters[2];
 
+// What a call may ask beside plain windowed attention; null, 0 or 1 where it does not.
+struct ApExtra {
+    const float* sinks;          // [H]: exp(sink_h) joins the denominator
+    float cap_log2, scale_over_cap;      // soft cap c: c log2 e, scale / c; 0: none
+    int keep_first;              // first keys of a request seen beside the window
+    const float* dist_bias;      // [n_dist][H], added to the scaled score by distance
+    int n_dist;
+    const bf16* gate;            // [T, >= H]: head h's output times the logistic function of it
+    long long gate_stride;
+    unsigned int* ticket;        // two zeroed counters of this launch alone; null: the library's
+};
+
+// A raw product q . k as the exponent in base 2, bounded by the cap: c tanh(x / c) = C - 2 C /
+// (1 + 2^(2 log2(e) x / c)) with the hardware's exponential and reciprocal (an exponential that
+// overflows gives the bound itself).
+__device__ __forceinline__ float at_capped(float qk, float cap_log2, float scale_over_cap) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(qk * (scale_over_cap * 2.8853900817779268f)));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+    return fmaf(-2.f * cap_log2, r, cap_log2);
+}
+
+// DH: head size, 64 or 128. XF: the scores go through the cap or take the bias by distance before
+// the softmax (the plain form folds the scale into the exponential's argument).
+template <int DH, bool XF>
 __global__ void __launch_bounds__(AP_THREADS, 1)
 attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                const __grid_constant__ CUtensorMap map_q, bf16* __restrict__ out,
@@ -224,7 +251,10 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                                const int* __restrict__ block_tables, int max_blocks,
                                const int* __restrict__ positions, const int* __restrict__ seq_ids,
                                const int* __restrict__ tile_tok0, const int* __restrict__ tile_ntok,
-                               int n_tiles, int H, int Hkv, float scale_log2, int window) {
+                               int n_tiles, int H, int Hkv, float scale_log2, int window, const ApExtra ex) {
+    constexpr int NH = DH / 64;                                 // 64-column blocks of a row
+    constexpr int OC = DH / 2;                                  // output columns of a softmax thread
+    unsigned int* const ticket = ex.ticket ? ex.ticket : ap_counters;
     extern __shared__ unsigned char at_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)at_raw + 1023) & ~(uintptr_t)1023);
     unsigned char* sQ = base;                                   // [2][2 halves][128 rows][128 B]
@@ -281,9 +311,12 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
     const uint32_t tmem = *tmem_slot;
 
     // pages of key tile j that hold a key some row of the item may read: [first, last)
-    auto page_range = [&](int j, int key_lo, int key_hi, int& first, int& last) {
+    // (a tile with kept first keys starts with them; one that lies before the window holds no others)
+    auto page_range = [&](int j, bool kept, int key_lo, int key_hi, int& first, int& last) {
         first = j * pages_per_tile;
         last = first + pages_per_tile;
+        if (j * AT_BN < ex.keep_first) key_lo = j * AT_BN;
+        if (kept && ex.keep_first < key_hi) key_hi = ex.keep_first;
         while (first < last && (first + 1) * page_size <= key_lo) ++first;
         while (last > first && (last - 1) * page_size >= key_hi) --last;
     };
@@ -293,7 +326,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
         bool ok = true;
         auto draw = [&](int& item, int& tok0, int& ntok) {
             item = 0;
-            if (lane == 0) item = (int)atomicAdd(&ap_ticket, 1u);
+            if (lane == 0) item = (int)atomicAdd(ticket, 1u);
             item = __shfl_sync(0xffffffffu, item, 0);
             tok0 = ntok = 0;
             if (item < n_items) {
@@ -332,10 +365,13 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int key_lo = (window > 0 && p0 - window + 1 > 0) ? p0 - window + 1 : 0;
             const int key_hi = p_last + 1;
             const int t_lo = key_lo / AT_BN, t_hi = (key_hi + AT_BN - 1) / AT_BN;
-            const int n_it = p0 < 0 ? 0 : t_hi - t_lo;
+            int n_kept = ex.keep_first > 0 ? (ex.keep_first + AT_BN - 1) / AT_BN : 0;
+            if (n_kept > t_lo) n_kept = t_lo;
+            const int n_it = p0 < 0 ? 0 : n_kept + t_hi - t_lo;
             if (lane == 0) {
                 rec->valid = 1; rec->tok0 = q_tok0; rec->n_rows = n_rows; rec->p0 = p0; rec->n_it = n_it;
                 rec->t_lo = t_lo; rec->key_lo = key_lo; rec->key_hi = key_hi; rec->seq = seq; rec->kvh = kvh;
+                rec->n_kept = n_kept;
                 if (n_it > 0) {
                     // The item's Q rows by TMA: two boxes (the two 64-column halves of the head
                     // size) of G heads x the tile's tokens, which land in row order token * G +
@@ -346,9 +382,9 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     // took 8 us to arrive and those of later items 13 us, competing with the
                     // softmax warps for issue slots: measured with the global timer.)
                     unsigned char* dq = sQ + qb * AT_TILE_BYTES;
-                    at_expect_tx(&q_full[qb], 2u * (uint32_t)q_box_rows * 128u);
+                    at_expect_tx(&q_full[qb], (uint32_t)NH * (uint32_t)q_box_rows * 128u);
                     at_tma_4d(dq, &map_q, 0, 0, kvh * G, q_tok0, &q_full[qb]);
-                    at_tma_4d(dq + AT_BLOCK_BYTES, &map_q, 0, 1, kvh * G, q_tok0, &q_full[qb]);
+                    if (NH > 1) at_tma_4d(dq + AT_BLOCK_BYTES, &map_q, 0, 1, kvh * G, q_tok0, &q_full[qb]);
                 } else {
                     at_arrive(&q_full[qb]);
                 }
@@ -375,27 +411,30 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int* bt = block_tables + (size_t)rec.seq * max_blocks;
             const int pg_lo = rec.t_lo * pages_per_tile;
             if (rec.n_it > 0) {
-                int pg_hi = (rec.t_lo + rec.n_it) * pages_per_tile;
+                int pg_hi = (rec.t_lo + rec.n_it - rec.n_kept) * pages_per_tile;
                 if (pg_hi > max_blocks) pg_hi = max_blocks;
                 if (pg_hi - pg_lo > AT_PAGES_CAP) pg_hi = pg_lo + AT_PAGES_CAP;
                 for (int i = pg_lo + lane; i < pg_hi; i += 32) s_pages[i - pg_lo] = bt[i];
             }
             __syncwarp();
-            auto page_of = [&](int pi) { return pi - pg_lo < AT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi]; };
+            auto page_of = [&](int pi) {
+                return pi >= pg_lo && pi - pg_lo < AT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi];
+            };
             for (int it = 0; it < rec.n_it; ++it, ++g) {
                 const uint32_t s = g & 1u, ph = (g >> 1) & 1u;
-                const int j = rec.t_lo + it;
+                const bool kept = it < rec.n_kept;
+                const int j = kept ? it : rec.t_lo + it - rec.n_kept;
                 int first, last;
-                page_range(j, rec.key_lo, rec.key_hi, first, last);
+                page_range(j, kept, rec.key_lo, rec.key_hi, first, last);
                 ok = __all_sync(0xffffffffu, at_wait(&empty[s], ph ^ 1u, 1));
                 if (!ok) break;
-                if (lane == 0) at_expect_tx(&full[s], (uint32_t)(last - first) * (uint32_t)page_size * 256u);
+                if (lane == 0) at_expect_tx(&full[s], (uint32_t)(last - first) * (uint32_t)page_size * (uint32_t)(DH * 2));
                 __syncwarp();
                 for (int pi = first + lane; pi < last; pi += 32) {
                     const int row = (page_of(pi) * Hkv + rec.kvh) * page_size;
                     unsigned char* dst = tiles + s * AT_TILE_BYTES + (pi - j * pages_per_tile) * page_size * 128;
                     at_tma_2d(dst, map, 0, row, &full[s]);
-                    at_tma_2d(dst + AT_BLOCK_BYTES, map, 64, row, &full[s]);
+                    if (NH > 1) at_tma_2d(dst + AT_BLOCK_BYTES, map, 64, row, &full[s]);
                 }
             }
             __syncwarp();
@@ -426,8 +465,9 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     const uint64_t dk0 = at_desc(sK + s * AT_TILE_BYTES), dk1 = at_desc(sK + s * AT_TILE_BYTES + AT_BLOCK_BYTES);
 #pragma unroll
                     for (int k = 0; k < 4; ++k) at_mma_ss(tmem + 128u * s, dq0 + 2 * k, dk0 + 2 * k, idesc_qk, k > 0 ? 1u : 0u);
+                    if (NH > 1)
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) at_mma_ss(tmem + 128u * s, dq1 + 2 * k, dk1 + 2 * k, idesc_qk, 1u);
+                        for (int k = 0; k < 4; ++k) at_mma_ss(tmem + 128u * s, dq1 + 2 * k, dk1 + 2 * k, idesc_qk, 1u);
                     at_commit(&k_empty[s]);
                     at_commit(&s_full[s]);
                 }
@@ -438,7 +478,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
         // ---------------------------------------------------------- issuer of O += P V
         if (lane == 0) {
             const uint32_t idesc_pv = (1u << 4) | (1u << 7) | (1u << 10) | (1u << 16) |
-                                      ((uint32_t)(AP_PV_N >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+                                      ((uint32_t)(DH >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
             uint32_t g = 0;
             bool ok = true;
             for (uint32_t n = 0; ok; ++n) {
@@ -455,14 +495,11 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     ok = ok && at_wait(&p_full[s], ph, 2) && at_wait(&v_full[s], ph, 2);
                     if (!ok) break;
                     at_fence_after();
+                    const uint64_t dv = NH > 1 ? at_desc_mn(sV + s * AT_TILE_BYTES) : at_desc(sV + s * AT_TILE_BYTES);
 #pragma unroll
-                    for (int h = 0; h < 128 / AP_PV_N; ++h) {
-                        const uint64_t dv = at_desc_mn(sV + s * AT_TILE_BYTES + h * AT_BLOCK_BYTES);
-#pragma unroll
-                        for (int k = 0; k < 8; ++k)           // 16 keys = 2 groups of 8 rows = 2048 bytes
-                            at_mma_ts(tm_o + 64u * h, tmem + 128u * s + 8u * k, dv + (uint64_t)(128 * k), idesc_pv,
-                                      (it > 0 || k > 0) ? 1u : 0u);
-                    }
+                    for (int k = 0; k < 8; ++k)               // 16 keys = 2 groups of 8 rows = 2048 bytes
+                        at_mma_ts(tm_o, tmem + 128u * s + 8u * k, dv + (uint64_t)(128 * k), idesc_pv,
+                                  (it > 0 || k > 0) ? 1u : 0u);
                     at_commit(&v_empty[s]);
                     at_commit(&p_free[s]);
                     at_commit(o_done);
@@ -489,11 +526,11 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int n_rows = rec.n_rows, p0 = rec.p0, n_it = rec.n_it, key_lo = rec.key_lo, key_hi = rec.key_hi;
             const bool row_ok = row < n_rows;
             bf16* dst = out + (size_t)(rec.tok0 + (row_ok ? row : 0) / G) * out_stride +
-                        (size_t)(rec.kvh * G + (row_ok ? row : 0) % G) * AT_DH + 64 * half;
+                        (size_t)(rec.kvh * G + (row_ok ? row : 0) % G) * DH + OC * half;
             if (n_it == 0) {                       // a request that brings nothing: zeros out
                 if (row_ok) {
 #pragma unroll
-                    for (int i = 0; i < 8; ++i) *(uint4*)(dst + i * 8) = make_uint4(0u, 0u, 0u, 0u);
+                    for (int i = 0; i < OC / 8; ++i) *(uint4*)(dst + i * 8) = make_uint4(0u, 0u, 0u, 0u);
                 }
                 __syncwarp();
                 if (lane == 0) at_arrive(&o_free[ob]);
@@ -510,7 +547,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             for (int it = 0; it < n_it; ++it, ++g) {
                 const uint32_t s = g & 1u, ph = (g >> 1) & 1u;
                 const uint32_t tm_s = tmem + 128u * s;
-                const int tile_lo = (rec.t_lo + it) * AT_BN;
+                const int tile_lo = (it < rec.n_kept ? it : rec.t_lo + it - rec.n_kept) * AT_BN;
                 const int kbase = tile_lo + 64 * half;
                 if (ok) ok = at_wait(&s_full[s], ph, 3);
                 at_fence_after();
@@ -523,6 +560,22 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
 #pragma unroll
                     for (int i = 0; i < 32; ++i) { sc[i] = __uint_as_float(r0[i]); sc[32 + i] = __uint_as_float(r1[i]); }
                 }
+                if (XF) {
+                    // the exponents in base 2 themselves; further down the factor is 1
+#pragma unroll
+                    for (int i = 0; i < 64; ++i)
+                        sc[i] = ex.cap_log2 > 0.f ? at_capped(sc[i], ex.cap_log2, ex.scale_over_cap) : sc[i] * scale_log2;
+                    if (ex.dist_bias) {
+                        const float* col = ex.dist_bias + rec.kvh * G + (row_ok ? row : 0) % G;
+#pragma unroll
+                        for (int i = 0; i < 64; ++i) {
+                            int dist = pos - kbase - i;
+                            dist = dist < 0 ? 0 : dist < ex.n_dist ? dist : ex.n_dist - 1;    // below 0: masked
+                            sc[i] = fmaf(col[(size_t)dist * H], 1.4426950408889634f, sc[i]);
+                        }
+                    }
+                }
+                const float factor = XF ? 1.f : scale_log2;
                 const bool full = warp_rows_ok && kbase + 63 <= warp_pos_min && kbase >= warp_vis_max;
                 float mx4[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
                 if (full) {
@@ -532,11 +585,11 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
 #pragma unroll
                     for (int i = 0; i < 64; ++i) {
                         const int key = kbase + i;
-                        sc[i] = (key <= pos && key >= vis_lo) ? sc[i] : -INFINITY;
+                        sc[i] = (key <= pos && (key >= vis_lo || key < ex.keep_first)) ? sc[i] : -INFINITY;
                         mx4[i & 3] = fmaxf(mx4[i & 3], sc[i]);
                     }
                 }
-                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * scale_log2;
+                float mx = fmaxf(fmaxf(mx4[0], mx4[1]), fmaxf(mx4[2], mx4[3])) * factor;
                 float* xm = s_xm + (g & 1u) * 256;
                 xm[half * 128 + row] = mx;
                 // the barrier: both halves have read their S (P is written over it below), and
@@ -557,8 +610,8 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     uint32_t r[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i) {
-                        const float a = at_ex2(fmaf(sc[2 * i], scale_log2, -base_m));
-                        const float b = at_ex2(fmaf(sc[2 * i + 1], scale_log2, -base_m));
+                        const float a = at_ex2(fmaf(sc[2 * i], factor, -base_m));
+                        const float b = at_ex2(fmaf(sc[2 * i + 1], factor, -base_m));
                         sum4[i & 3] += a + b;
                         r[i] = at_pack(a, b);
                     }
@@ -568,10 +621,10 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                 if (tile_lo + AT_BN > key_hi || tile_lo < key_lo) {     // rows of V that nobody may read
                     if (ok) ok = at_wait(&v_full[s], ph, 3);
                     const int key = tile_lo + row;
-                    if (key >= key_hi || key < key_lo) {
-                        unsigned char* vrow = sV + s * AT_TILE_BYTES + half * AT_BLOCK_BYTES + row * 128;
+                    if (key >= key_hi || (key < key_lo && key >= ex.keep_first)) {
+                        unsigned char* vrow = sV + s * AT_TILE_BYTES + row * 128 + (NH > 1 ? half * AT_BLOCK_BYTES : half * 64);
 #pragma unroll
-                        for (int c = 0; c < 8; ++c) *(uint4*)(vrow + c * 16) = make_uint4(0u, 0u, 0u, 0u);
+                        for (int c = 0; c < 4 * NH; ++c) *(uint4*)(vrow + c * 16) = make_uint4(0u, 0u, 0u, 0u);
                     }
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 }
@@ -581,12 +634,12 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     if (rescale) {
                         uint32_t r[32];
 #pragma unroll
-                        for (int c = 0; c < 2; ++c) {
-                            at_tmem_ld32(tm_o + lane_base + 64u * half + 32u * c, r);
+                        for (int c = 0; c < NH; ++c) {
+                            at_tmem_ld32(tm_o + lane_base + (uint32_t)(OC * half) + 32u * c, r);
                             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
                             for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__uint_as_float(r[i]) * corr);
-                            at_tmem_st32(tm_o + lane_base + 64u * half + 32u * c, r);
+                            at_tmem_st32(tm_o + lane_base + (uint32_t)(OC * half) + 32u * c, r);
                         }
                     }
                 }
@@ -602,11 +655,21 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             if (at_bar_or(!ok)) break;
             l += s_xl[(half ^ 1) * 128 + row];
             {
-                const float inv = l > 0.f ? 1.f / l : 0.f;
+                const int head = rec.kvh * G + (row_ok ? row : 0) % G;
+                float corr = 1.f;
+                if (ex.sinks) {                    // the sink joins the denominator last
+                    const float sk = ex.sinks[head] * 1.4426950408889634f;
+                    const float mn = fmaxf(m_used, sk);
+                    corr = exp2f(m_used - mn);
+                    l = l * corr + exp2f(sk - mn);
+                }
+                float inv = l > 0.f ? corr / l : 0.f;
+                if (ex.gate && row_ok)
+                    inv *= 1.f / (1.f + __expf(-__bfloat162float(ex.gate[(size_t)(rec.tok0 + row / G) * ex.gate_stride + head])));
 #pragma unroll
-                for (int c = 0; c < 2; ++c) {
+                for (int c = 0; c < NH; ++c) {
                     uint32_t r[32];
-                    at_tmem_ld32(tm_o + lane_base + 64u * half + 32u * c, r);
+                    at_tmem_ld32(tm_o + lane_base + (uint32_t)(OC * half) + 32u * c, r);
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                     if (row_ok) {
 #pragma unroll
@@ -632,9 +695,9 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
         at_fence_after();
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
     }
-    if (tid == 0 && atomicAdd(&ap_finished, 1u) == gridDim.x - 1u) {
-        ap_ticket = 0;              // nobody draws any more: every CTA has seen the end of the items
-        ap_finished = 0;
+    if (tid == 0 && atomicAdd(ticket + 1, 1u) == gridDim.x - 1u) {
+        ticket[0] = 0;              // nobody draws any more: every CTA has seen the end of the items
+        ticket[1] = 0;
         __threadfence();
     }
 }
@@ -645,51 +708,19 @@ typedef CUresult (*AtEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, vo
                                CUtensorMapInterleave, CUtensorMapSwizzle, CUtensorMapL2promotion,
                                CUtensorMapFloatOOBfill);
 
-// The tensor map of one layer's K or V pages, [rows, 128] bf16 in boxes of page_size x 64;
+// The tensor map of one layer's K or V pages, [rows, head size] bf16 in boxes of page_size x 64;
 // made once per (address, rows, page size) and kept.
-static const CUtensorMap* at_map_of(const void* pages, long long rows, int page_size) {
-    static std::mutex lock;
-    static std::unordered_map<uint64_t, CUtensorMap> maps;
-    static AtEncodeFn encode = nullptr;
-    std::lock_guard<std::mutex> hold(lock);
-    if (!encode) {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult qr;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess ||
-            qr != cudaDriverEntryPointSuccess)
-            return nullptr;
-        encode = (AtEncodeFn)p;
-    }
-    const uint64_t key = (uint64_t)(uintptr_t)pages ^ ((uint64_t)rows * 0x9e3779b97f4a7c15ull) ^ ((uint64_t)page_size << 56);
-    auto it = maps.find(key);
-    if (it != maps.end()) return &it->second;
-    CUtensorMap map;
-    const cuuint64_t dims[2] = {AT_DH, (cuuint64_t)rows};
-    const cuuint64_t strides[1] = {AT_DH * 2};
-    const cuuint32_t box[2] = {64, (cuuint32_t)page_size};
-    const cuuint32_t elem[2] = {1, 1};
-    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pages), dims, strides, box, elem,
-               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
-        return nullptr;
-    return &maps.emplace(key, map).first->second;
-}
-
-// The tensor map of a step's query rows, q [tokens, >= H * 128] bf16 with a row stride, seen
-// as (64 columns, 2 halves, H heads, tokens): a box is one half of G heads of a tile's tokens.
-// Kept by (address, stride, tokens, heads, group): a step's activations come back to the same
-// addresses step after step.
-static const CUtensorMap* at_map_q(const void* q, long long q_stride, int tokens, int H, int G) {
+static const CUtensorMap* at_map_of(const void* pages, long long rows, int page_size, int dh) {
     struct Key {
-        const void* q; long long stride; int tokens, H, G;
+        const void* pages; long long rows; int page_size, dh;
         bool operator==(const Key& o) const {
-            return q == o.q && stride == o.stride && tokens == o.tokens && H == o.H && G == o.G;
+            return pages == o.pages && rows == o.rows && page_size == o.page_size && dh == o.dh;
         }
     };
     struct Hash {
         size_t operator()(const Key& k) const {
-            return (size_t)(uintptr_t)k.q * 0x9e3779b97f4a7c15ull ^ ((size_t)k.stride << 32) ^ ((size_t)k.tokens << 12) ^
-                   ((size_t)k.H << 6) ^ (size_t)k.G;
+            return (size_t)(uintptr_t)k.pages ^ ((size_t)k.rows * 0x9e3779b97f4a7c15ull) ^ ((size_t)k.page_size << 56) ^
+                   ((size_t)k.dh << 48);
         }
     };
     static std::mutex lock;
@@ -704,12 +735,56 @@ static const CUtensorMap* at_map_q(const void* q, long long q_stride, int tokens
             return nullptr;
         encode = (AtEncodeFn)p;
     }
-    const Key key{q, q_stride, tokens, H, G};
+    const Key key{pages, rows, page_size, dh};
     auto it = maps.find(key);
     if (it != maps.end()) return &it->second;
     CUtensorMap map;
-    const cuuint64_t dims[4] = {64, 2, (cuuint64_t)H, (cuuint64_t)tokens};
-    const cuuint64_t strides[3] = {128, 256, (cuuint64_t)q_stride * 2};
+    const cuuint64_t dims[2] = {(cuuint64_t)dh, (cuuint64_t)rows};
+    const cuuint64_t strides[1] = {(cuuint64_t)dh * 2};
+    const cuuint32_t box[2] = {64, (cuuint32_t)page_size};
+    const cuuint32_t elem[2] = {1, 1};
+    if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(pages), dims, strides, box, elem,
+               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+        return nullptr;
+    return &maps.emplace(key, map).first->second;
+}
+
+// The tensor map of a step's query rows, q [tokens, >= H * 128] bf16 with a row stride, seen
+// as (64 columns, 2 halves, H heads, tokens): a box is one half of G heads of a tile's tokens.
+// Kept by (address, stride, tokens, heads, group): a step's activations come back to the same
+// addresses step after step.
+static const CUtensorMap* at_map_q(const void* q, long long q_stride, int tokens, int H, int G, int dh) {
+    struct Key {
+        const void* q; long long stride; int tokens, H, G, dh;
+        bool operator==(const Key& o) const {
+            return q == o.q && stride == o.stride && tokens == o.tokens && H == o.H && G == o.G && dh == o.dh;
+        }
+    };
+    struct Hash {
+        size_t operator()(const Key& k) const {
+            return (size_t)(uintptr_t)k.q * 0x9e3779b97f4a7c15ull ^ ((size_t)k.stride << 32) ^ ((size_t)k.tokens << 12) ^
+                   ((size_t)k.H << 6) ^ (size_t)k.G ^ ((size_t)k.dh << 56);
+        }
+    };
+    static std::mutex lock;
+    static std::unordered_map<Key, CUtensorMap, Hash> maps;
+    static AtEncodeFn encode = nullptr;
+    std::lock_guard<std::mutex> hold(lock);
+    if (!encode) {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult qr;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &qr) != cudaSuccess ||
+            qr != cudaDriverEntryPointSuccess)
+            return nullptr;
+        encode = (AtEncodeFn)p;
+    }
+    const Key key{q, q_stride, tokens, H, G, dh};
+    auto it = maps.find(key);
+    if (it != maps.end()) return &it->second;
+    CUtensorMap map;
+    const cuuint64_t dims[4] = {64, (cuuint64_t)(dh / 64), (cuuint64_t)H, (cuuint64_t)tokens};
+    const cuuint64_t strides[3] = {128, (cuuint64_t)dh * 2, (cuuint64_t)q_stride * 2};
     const cuuint32_t box[4] = {64, 1, (cuuint32_t)G, (cuuint32_t)(AT_BM / G)};
     const cuuint32_t elem[4] = {1, 1, 1, 1};
     if (encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(q), dims, strides, box, elem,
@@ -720,12 +795,12 @@ static const CUtensorMap* at_map_q(const void* q, long long q_stride, int tokens
     return &maps.emplace(key, map).first->second;
 }
 
-// 1 if this kernel takes the shape: head size 128, up to 16 query heads a kv head (a tile then
-// holds 128 / group tokens, rounded down), pages of 8, 16, 32, 64 or 128 tokens.
+// 1 if this kernel takes the shape: head size 64 or 128, up to 16 query heads a kv head (a tile
+// then holds 128 / group tokens, rounded down), pages of 8, 16, 32, 64 or 128 tokens.
 TGO_API int tgo_attention_tc_supports(int dh, int group, int page_size) {
     const bool g_ok = group >= 1 && group <= 16;
     const bool p_ok = page_size == 8 || page_size == 16 || page_size == 32 || page_size == 64 || page_size == 128;
-    return dh == AT_DH && g_ok && p_ok;
+    return (dh == 64 || dh == 128) && g_ok && p_ok;
 }
 
 
@@ -734,53 +809,82 @@ TGO_API int tgo_attention_tc_error(int* value) {
     return (int)cudaMemcpyFromSymbol(value, at_error_flag, sizeof(int));
 }
 
+template <int DH, bool XF>
+static int at_go(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq, void* out, long long out_stride,
+                 int page_size, int shift, const int* block_tables, int max_blocks, const int* positions,
+                 const int* seq_ids, const int* tile_tok0, const int* tile_ntok, int n_tiles, int H, int Hkv,
+                 float scale_log2, int window, const ApExtra& ex, cudaStream_t stream) {
+    constexpr size_t smem = 1024 + 6 * (size_t)AT_TILE_BYTES + 22 * 8 + 4 * sizeof(ApItem) +
+                            768 * sizeof(float) + 2 * AT_PAGES_CAP * sizeof(int);
+    // per device: its SM count, and whether this kernel's attribute is set there
+    static int sms_of[64] = {};
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
+    if (!sms_of[dev]) {
+        e = cudaFuncSetAttribute(attention_tc_persistent_kernel<DH, XF>,
+                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+        if (e != cudaSuccess) return (int)e;
+        int n = 0;
+        if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
+        sms_of[dev] = n;
+    }
+    const int sms = sms_of[dev];
+    const int items = n_tiles * Hkv;
+    attention_tc_persistent_kernel<DH, XF><<<dim3(items < sms ? items : sms), AP_THREADS, smem, stream>>>(
+        mk, mv, mq, (bf16*)out, out_stride, page_size, shift, block_tables, max_blocks,
+        positions, seq_ids, tile_tok0, tile_ntok, n_tiles, H, Hkv, scale_log2, window, ex);
+    return launch_status();
+}
+
 // Prompt portions: tiles of up to 128 / group consecutive tokens of one request each
-// (tile_tok0, tile_ntok); q has n_tokens rows of q_stride elements, its first H * 128 columns
-// the heads. k_cache and v_cache: [n_pages, Hkv, page_size, 128] bf16.
+// (tile_tok0, tile_ntok); q has n_tokens rows of q_stride elements, its first H * dh columns
+// the heads. k_cache and v_cache: [n_pages, Hkv, page_size, dh] bf16; scale > 0.
 // One CTA per SM draws (tile, kv head) items from a counter.
+// sinks .. gate_stride as in ApExtra (softcap 0: none). counters: two ints that this launch alone
+// uses, zeroed here; null: the library's own pair, for callers whose launches do not overlap.
 TGO_API int tgo_attention_tc_prefill(const void* q, long long q_stride, int n_tokens, void* out, long long out_stride,
                                      const void* k_cache, const void* v_cache, int n_pages, int page_size,
                                      const int* block_tables, int max_blocks, const int* positions,
                                      const int* seq_ids, const int* tile_tok0, const int* tile_ntok,
                                      int n_tiles, int H, int Hkv, int dh, float scale, int window,
+                                     const float* sinks, float softcap, int keep_first, const float* dist_bias,
+                                     int n_dist, const void* gate, long long gate_stride, int* counters,
                                      cudaStream_t stream) {
     if (n_tiles <= 0) return 0;
     if (n_tokens <= 0 || H <= 0 || Hkv <= 0 || H % Hkv || !tgo_attention_tc_supports(dh, H / Hkv, page_size) || n_pages <= 0 ||
         max_blocks <= 0 || window < 0 || Hkv > 65535 || !tile_tok0 || !tile_ntok || q_stride % 8 ||
         out_stride % 8 || ((uintptr_t)q % 16) || ((uintptr_t)out % 16) || ((uintptr_t)k_cache % 128) ||
-        ((uintptr_t)v_cache % 128))
+        ((uintptr_t)v_cache % 128) || !(softcap >= 0.f) || keep_first < 0 || (dist_bias && n_dist <= 0))
         return TGO_E_BAD_ARG;
     const long long rows = (long long)n_pages * Hkv * page_size;
     if (rows > 0x7fffffffll || (long long)n_tiles * Hkv > 0x7fffffffll) return TGO_E_BAD_ARG;
-    const CUtensorMap* mk = at_map_of(k_cache, rows, page_size);
-    const CUtensorMap* mv = at_map_of(v_cache, rows, page_size);
-    const CUtensorMap* mq = at_map_q(q, q_stride, n_tokens, H, H / Hkv);
+    const CUtensorMap* mk = at_map_of(k_cache, rows, page_size, dh);
+    const CUtensorMap* mv = at_map_of(v_cache, rows, page_size, dh);
+    const CUtensorMap* mq = at_map_q(q, q_stride, n_tokens, H, H / Hkv, dh);
     if (!mk || !mv || !mq) return TGO_E_BAD_ARG;
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
-    const float scale_log2 = scale * 1.4426950408889634f;
-    {
-        constexpr size_t smem = 1024 + 6 * (size_t)AT_TILE_BYTES + 22 * 8 + 4 * sizeof(ApItem) +
-                                768 * sizeof(float) + 2 * AT_PAGES_CAP * sizeof(int);
-        // per device: its SM count, and whether this kernel's attribute is set there
-        static int sms_of[64] = {};
-        int dev = 0;
-        cudaError_t e = cudaGetDevice(&dev);
+    const float log2e = 1.4426950408889634f;
+    ApExtra ex = {};
+    ex.sinks = sinks;
+    ex.cap_log2 = softcap * log2e;
+    ex.scale_over_cap = softcap > 0.f ? scale / softcap : 0.f;
+    ex.keep_first = window > 0 ? keep_first : 0;
+    ex.dist_bias = dist_bias;
+    ex.n_dist = n_dist;
+    ex.gate = (const bf16*)gate;
+    ex.gate_stride = gate_stride;
+    ex.ticket = (unsigned int*)counters;
+    if (counters) {
+        const cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(int), stream);
         if (e != cudaSuccess) return (int)e;
-        if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
-        if (!sms_of[dev]) {
-            e = cudaFuncSetAttribute(attention_tc_persistent_kernel,
-                                     cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-            if (e != cudaSuccess) return (int)e;
-            int n = 0;
-            if ((e = cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return (int)e;
-            sms_of[dev] = n;
-        }
-        const int sms = sms_of[dev];
-        const int items = n_tiles * Hkv;
-        attention_tc_persistent_kernel<<<dim3(items < sms ? items : sms), AP_THREADS, smem, stream>>>(
-            *mk, *mv, *mq, (bf16*)out, out_stride, page_size, shift, block_tables, max_blocks,
-            positions, seq_ids, tile_tok0, tile_ntok, n_tiles, H, Hkv, scale_log2, window);
-        return launch_status();
     }
+#define AT_GO(DH, XF)                                                                                             \
+    return at_go<DH, XF>(*mk, *mv, *mq, out, out_stride, page_size, shift, block_tables, max_blocks, positions,    \
+                         seq_ids, tile_tok0, tile_ntok, n_tiles, H, Hkv, scale * log2e, window, ex, stream)
+    if (dh == 128) { if (softcap > 0.f || dist_bias) AT_GO(128, true); else AT_GO(128, false); }
+    if (softcap > 0.f || dist_bias) AT_GO(64, true); else AT_GO(64, false);
+#undef AT_GO
 }

@@ -1821,11 +1821,23 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
                          head_dim: int, k_cache: torch.Tensor, v_cache: torch.Tensor, page_size: int,
                          block_tables: torch.Tensor, positions: torch.Tensor, seq_ids: torch.Tensor,
                          tile_tok0: torch.Tensor, tile_ntok: torch.Tensor, scale: float,
-                         window: int) -> None:
+                         window: int, sinks: Optional[torch.Tensor] = None, softcap: float = 0.0,
+                         keep_first: int = 0, dist_bias: Optional[torch.Tensor] = None,
+                         gate: Optional[torch.Tensor] = None, own_counters: bool = False) -> None:
     """Paged causal attention of prompt portions on the tcgen05 tensor cores (bfloat16, head
-    size 128): tiles of 128 // group consecutive tokens of one request (tile_tok0, tile_ntok,
-    int32); K and V pages [n_pages, kv_heads, page_size, 128] come in by TMA."""
-    _need_cuda(q, out, k_cache, v_cache, block_tables, positions, seq_ids, tile_tok0, tile_ntok)
+    size 64 or 128): tiles of 128 // group consecutive tokens of one request (tile_tok0, tile_ntok,
+    int32); K and V pages [n_pages, kv_heads, page_size, head size] come in by TMA. `sinks`,
+    `softcap`, `keep_first`, `dist_bias` and `gate` as in `attention_generic` (the scale is
+    positive). Calls that may run beside others on the device bring counters of their own
+    (`own_counters`); the others share the library's."""
+    _need_cuda(q, out, k_cache, v_cache, block_tables, positions, seq_ids, tile_tok0, tile_ntok, sinks, dist_bias,
+               gate)
+    assert gate is None or (gate.dtype == q.dtype and gate.shape == (q.shape[0], num_heads) and
+                            (gate.stride(1) == 1 or num_heads == 1))
+    assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.dim() == 2 and
+                                 dist_bias.shape[1] == num_heads and dist_bias.is_contiguous())
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == num_heads and
+                             sinks.is_contiguous())
     assert q.dtype == torch.bfloat16 and out.dtype == torch.bfloat16 and k_cache.dtype == torch.bfloat16
     assert q.stride(1) == 1 and out.stride(1) == 1 and k_cache.is_contiguous() and v_cache.is_contiguous()
     assert k_cache.shape == v_cache.shape and k_cache.shape[1:] == (num_kv_heads, page_size, head_dim)
@@ -1836,6 +1848,10 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
         c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]),
         _ptr(positions), _ptr(seq_ids), _ptr(tile_tok0), _ptr(tile_ntok), c_int(tile_tok0.numel()),
         c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_float(scale), c_int(window),
+        _ptr(sinks), c_float(softcap or 0.0), c_int(keep_first), _ptr(dist_bias),
+        c_int(dist_bias.shape[0] if dist_bias is not None else 0), _ptr(gate),
+        c_ll(gate.stride(0) if gate is not None else 0),
+        _ptr(torch.empty(2, dtype=torch.int32, device=q.device) if own_counters else None),
         _stream()), "attention_tc_prefill",
         f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads}, page_size={page_size})")
 

@@ -195,6 +195,8 @@ class SinkAttention(Part):
                  "attention_generic"]
         if dtype == torch.bfloat16:
             names.append("attention_sink")
+            if self.dk == self.dv and self.dk in (64, 128):
+                names.append("attention_tc")
         return names
 
     def prepare_capture(self, ctx, cache) -> None:
@@ -259,6 +261,18 @@ class SinkAttention(Part):
 USE_TILE_KERNELS = True
 
 
+def tc_takes(out, H, Hkv, dk, dv, cache, scale, value_row) -> bool:
+    """Whether a step with prompt portions runs on the tcgen05 kernel: keys and values of their
+    own planes, both 64 or 128 wide, groups and pages it knows, views it can read by TMA. It has no
+    size where the mma.sync tiles beat it among the steps measured (a layer over 2048 + 1536 tokens
+    of 16/4 heads of 128 with a window of 1024: 171 us against 499)."""
+    return value_row == 0 and dk == dv and dk in (64, 128) and scale > 0 and \
+        ops.attention_tc_supports(dk, H // Hkv, cache.page_size) and \
+        cache.k.is_contiguous() and cache.v.is_contiguous() and \
+        cache.k.data_ptr() % 128 == 0 and cache.v.data_ptr() % 128 == 0 and \
+        out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
+
+
 def tile_form(H, Hkv, dk, dv, value_row, dtype):
     """Which tensor-core kernel takes an attention of these sizes, and how many tokens of one
     request a tile of its holds: ("tile", n) for key and value rows up to 128 wide, ("wide", n)
@@ -278,7 +292,8 @@ def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, sof
     [n, H]: added to the scores by distance; `gate` [T, H]: every head's output times the logistic
     function of its number. `softcap` bounds the scores; `value_row` > 0 says that a value is the first
     dv channels of its key row, `value_row` wide (one cache plane serves as keys and values).
-    Which kernel runs the attention of a step. bfloat16 at sizes a tensor-core kernel takes
+    Which kernel runs the attention of a step. bfloat16 with prompt portions at sizes the tcgen05
+    kernel takes (`tc_takes`): that one. bfloat16 at sizes an mma.sync kernel takes
     (`tile_form`): that kernel, over tiles of consecutive tokens for steps with prompt portions
     (single tokens beside them are tiles of one), a tile a token for steps of single tokens, whose
     keys may be cut over several blocks. float32,
@@ -297,6 +312,11 @@ def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, sof
             ops.attention_sink_wide(q, out, H, Hkv, dk, dv, cache.k, cache.page_size, cache.block_tables,
                                     ctx.seq_ids, ctx.positions, scale, window, sinks, tok0, ntok,
                                     n_splits=splits, softcap=softcap)
+            return
+        if not ctx.decode_only and tc_takes(out, H, Hkv, dk, dv, cache, scale, value_row):
+            ops.attention_tc_prefill(q, out, H, Hkv, dk, cache.k, v_cache, cache.page_size, cache.block_tables,
+                                     ctx.positions, ctx.seq_ids, tok0, ntok, scale, window, sinks, softcap,
+                                     keep_first, dist_bias, gate, own_counters=True)
             return
         splits = decode_splits(ctx, Hkv, window, q.device) if ctx.decode_only else 1
         ops.attention_sink_tile(q, out, H, Hkv, dk, dv, cache.k, v_cache, cache.page_size,
