@@ -996,3 +996,33 @@ def test_attention_tc_options(H, Hkv, dh, ps, window, keep, extra):
     assert o.attention_tc_error() == 0
     assert bool(torch.isfinite(want).all())
     assert torch.allclose(out.float(), want, **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("T,d,ff,E,top", [(127, 64, 32, 1, 1), (128, 72, 40, 1, 1), (129, 136, 264, 1, 1), (257, 200, 104, 2, 1),
+                                          (1, 2048, 520, 8, 3), (300, 520, 136, 5, 2), (700, 64, 776, 3, 2), (9, 8, 8, 4, 4)])
+@pytest.mark.parametrize("gated,activation", [(True, "silu"), (True, "gelu_tanh"), (False, "relu_squared"), (False, "silu")])
+def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
+    """Row tiles at and past 128 rows of one expert, column tiles and k-blocks cut short, experts
+    without tokens. Hidden rows are bfloat16 (2^-9 each, ff of them in a sum), sums float32."""
+    o = ops()
+    if activation not in o.PLAIN_ACTIVATIONS or (gated and activation not in o.ACTIVATIONS):
+        pytest.skip("not an activation of this form")
+    x = rnd(T, d, seed=1).to(torch.bfloat16)
+    wr = rnd(E, d, seed=2) * d ** -0.5
+    wg, wu = ((rnd(E, ff, d, seed=s) * d ** -0.5).to(torch.bfloat16) for s in (3, 4))
+    wd = (rnd(E, d, ff, seed=5) * ff ** -0.5).to(torch.bfloat16)
+    got = o.moe_feed_forward(x, wr, None, wg if gated else None, wu, wd, top, activation)
+    assert o.moe_error() == 0
+    fn = {"silu": torch.nn.functional.silu, "relu_squared": lambda v: torch.relu(v) ** 2, "relu": torch.relu,
+          "gelu_tanh": lambda v: torch.nn.functional.gelu(v, approximate="tanh")}[activation]
+    z = x.double() @ wr.double().t()
+    ids = torch.topk(z, top, -1).indices
+    wt = torch.softmax(torch.gather(z, 1, ids), -1)
+    want, size = torch.zeros(T, d, dtype=torch.float64, device=DEV), torch.zeros(T, d, dtype=torch.float64, device=DEV)
+    for e in range(E):
+        row, place = torch.nonzero(ids == e, as_tuple=True)
+        xe = x[row].double()
+        h = fn(xe @ wu[e].double().t()) if not gated else fn(xe @ wg[e].double().t()) * (xe @ wu[e].double().t())
+        want.index_add_(0, row, (h @ wd[e].double().t()) * wt[row, place][:, None])
+        size.index_add_(0, row, (h.abs() @ wd[e].double().abs().t()) * wt[row, place][:, None])
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()

@@ -13,9 +13,8 @@
 //   combine    out[t] = sum_j weight[t][j] y[t top + j] (+ extra[t]), j in order, all float32
 //
 // The products are tiled: float32 storage takes plain-FMA tiles with float32 sums over k in
-// order; bfloat16 storage takes mma.sync m16n8k16 tiles (float32 accumulators) fed by cp.async
-// through two shared-memory buffers, when the widths are multiples of 8 (16-byte chunks), and
-// the plain tiles otherwise. Either way a row's result does not depend on which tile or batch
+// order; bfloat16 storage runs on tcgen05 (float32 accumulators in tensor memory, operands by
+// TMA) when the widths are multiples of 8 (16-byte chunks), and takes the plain tiles otherwise. Either way a row's result does not depend on which tile or batch
 // it falls in.
 //
 // Variants, each a parameter: `score_mode` 1 takes the softmax over ALL router logits; the choice
@@ -30,9 +29,10 @@
 // router row after all experts (`gate_out`) gives a logistic gate per token that multiplies
 // `extra` in the combine. Experts without a gate matrix (wg null) are W_down act(W_up x);
 // activation 3 is the square of relu.
-#include "mma_sync.cuh"
+#include "tcgen.cuh"
 
-#define MOE_TM 64
+#define MOE_TM 64                // rows of a tile of the plain products
+#define MOE_TILE 128             // rows of one expert a planned tile holds at most
 #define MOE_TN 64
 #define MOE_TK 16
 
@@ -268,7 +268,7 @@ __device__ __forceinline__ void moe_plan(const int* counts, int E, int* __restri
     int c = 0, nt = 0;
     for (int e = e_lo; e < e_hi; ++e) {
         c += counts[e];
-        nt += (counts[e] + MOE_TM - 1) / MOE_TM;
+        nt += (counts[e] + MOE_TILE - 1) / MOE_TILE;
     }
     int at = c, tile = nt;                               // inclusive sums over the lanes
 #pragma unroll
@@ -286,11 +286,11 @@ __device__ __forceinline__ void moe_plan(const int* counts, int E, int* __restri
         const int n = counts[e];
         offsets[e] = at;
         fill[e] = 0;
-        for (int r = 0; r < n; r += MOE_TM, ++tile) {
+        for (int r = 0; r < n; r += MOE_TILE, ++tile) {
             if (tile >= max_tiles) break;
             tiles[3 * tile] = e;
             tiles[3 * tile + 1] = at + r;
-            tiles[3 * tile + 2] = n - r < MOE_TM ? n - r : MOE_TM;
+            tiles[3 * tile + 2] = n - r < MOE_TILE ? n - r : MOE_TILE;
         }
         at += n;
     }
@@ -373,7 +373,9 @@ moe_up_kernel(const T* __restrict__ x, long long x_stride, const T* __restrict__
     __shared__ int toks[MOE_TM];
     pdl_wait();
     if ((int)blockIdx.y >= tile_info[0]) return;
-    const int e = tiles[3 * blockIdx.y], r0 = tiles[3 * blockIdx.y + 1], rows = tiles[3 * blockIdx.y + 2];
+    const int e = tiles[3 * blockIdx.y], skip = MOE_TM * blockIdx.z;     // z: which half of the planned tile
+    const int r0 = tiles[3 * blockIdx.y + 1] + skip, rows = min(tiles[3 * blockIdx.y + 2] - skip, MOE_TM);
+    if (rows <= 0) return;
     const int n0 = blockIdx.x * MOE_TN;
     if (threadIdx.x < MOE_TM) toks[threadIdx.x] = threadIdx.x < rows ? perm[r0 + threadIdx.x] / top : -1;
     __syncthreads();
@@ -439,7 +441,9 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
     __shared__ float ws[MOE_TK][MOE_TN + 4];
     pdl_wait();
     if ((int)blockIdx.y >= tile_info[0]) return;
-    const int e = tiles[3 * blockIdx.y], r0 = tiles[3 * blockIdx.y + 1], rows = tiles[3 * blockIdx.y + 2];
+    const int e = tiles[3 * blockIdx.y], skip = MOE_TM * blockIdx.z;     // z: which half of the planned tile
+    const int r0 = tiles[3 * blockIdx.y + 1] + skip, rows = min(tiles[3 * blockIdx.y + 2] - skip, MOE_TM);
+    if (rows <= 0) return;
     const int n0 = blockIdx.x * MOE_TN;
     const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
     const T* wde = wd + (size_t)e * d * ff;
@@ -486,108 +490,254 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
 }
 
 // ------------------------------------------------------------- products on the tensor cores
-// A tile of up to 64 rows of one expert by 64 columns; four warps, warp w owns rows 16w..16w+15
-// and all 64 columns. UP: A rows are x rows gathered by token, B is Wg[e] and Wu[e] ([N, K]
-// each), the result act(gate) * up goes to hidden[place] in bfloat16. MODE 1 is that; MODE 2
-// is the form without a gate, B is Wu[e] alone and the result act(up). MODE 0: A rows are
+// Persistent: one CTA an SM walks (planned tile, column tile) items, columns fastest, so that the
+// tiles of one expert run at the same time and its matrices come from memory once. MODE 1: A rows
+// are x rows gathered by token, B is Wg[e] and Wu[e] side by side ([N, K] each, bn rows of both
+// make one operand of 2 bn columns), the result act(gate) * up goes to hidden[place] in bfloat16.
+// MODE 2: the form without a gate, B is Wu[e] alone and the result act(up). MODE 0: A rows are
 // hidden[place], B is Wd[e], the result goes to y[pair] in float32.
+//   warp 0      TMA into a ring of stages: lanes 0 and 1 the B boxes; A in boxes of 32 rows where its
+//               rows lie in place order, else a lane four rows (gather4); rows past the tile's are
+//               not fetched, their sums are never stored;
+//   warp 1      issues the products (a thread), 128 x n x 16 each, into two accumulators in turn;
+//   warps 2..5  accumulator -> activation -> staged, so that a store covers whole 64- or 128-byte
+//               pieces of rows, while the next item's products run.
+// Bound by the weights' way from memory for a few rows an expert (each read once; a stage is
+// 32 KB of them, four in flight an SM) and by the operands' way into the SM (about 70 bytes a
+// cycle) for full tiles. MEASURED (B200, 32 experts, top 4, ff 768 of width 2048, gated; mma.sync
+// tiles of 64 x 64 fed by cp.async before): 2048 tokens, up 91 us (250) and down 41 (135), 570 and
+// 620 TFLOP/s with the copy of x's rows before them 8 us; 64 tokens, 40 us (66) and 21 (25), 5.0
+// and 4.8 TB/s of weights.
 #define MT_BK 64
-#define MT_LD (MT_BK + 8)
-#define MT_STAGES 3
+#define MT_A_BYTES (MOE_TILE * MT_BK * 2)
+#define MT_RING (192 * 1024)
+#define MT_STAGE_OUT 4096                  // per epilogue warp: 32 rows x 128 bytes on their way out
+#define MT_SMEM (MT_RING + 4 * MT_STAGE_OUT + 1024 + 256)
+#define MT_THREADS 192
+
+__device__ int moe_error_flag = 0;
+
+// act of the products' results: the hardware's exponential and reciprocal for the sigmoid (relative
+// error about 2^-21; the result is rounded to bfloat16)
+__device__ __forceinline__ float moe_act_fast(float z, int act) {
+    return act == 0 ? __fdividef(z, 1.f + __expf(-z)) : moe_act(z, act);
+}
 
 template <int MODE>
-__global__ void __launch_bounds__(128)
-moe_tc_kernel(const bf16* __restrict__ a, long long a_stride, const bf16* __restrict__ w0,
-              const bf16* __restrict__ w1, bf16* __restrict__ hidden, float* __restrict__ y, int N,
-              int K, int top, int act, const int* __restrict__ perm,
+__global__ void __launch_bounds__(MT_THREADS, 1)
+moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
+              const __grid_constant__ CUtensorMap map_b1, bf16* __restrict__ hidden, float* __restrict__ y, int N,
+              int K, int bn, int top, int act, int gather, const int* __restrict__ perm,
               const int* __restrict__ tile_info, const int* __restrict__ tiles) {
-    extern __shared__ __align__(16) unsigned char moe_smem[];
-    typedef bf16 (*Tile)[MOE_TM][MT_LD];
-    Tile As = (Tile)moe_smem;                                        // [MT_STAGES][64][MT_LD]
-    Tile B0 = (Tile)(moe_smem + sizeof(bf16) * MT_STAGES * MOE_TM * MT_LD);
-    Tile B1 = (Tile)(moe_smem + sizeof(bf16) * 2 * MT_STAGES * MOE_TM * MT_LD);   // UP only
-    __shared__ int src_row[MOE_TM];
     constexpr bool UP = MODE != 0, GATED = MODE == 1;
-    pdl_wait();
-    if ((int)blockIdx.y >= tile_info[0]) return;
-    const int e = tiles[3 * blockIdx.y], r0 = tiles[3 * blockIdx.y + 1], rows = tiles[3 * blockIdx.y + 2];
-    const int n0 = blockIdx.x * MOE_TN;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    if (tid < MOE_TM) src_row[tid] = tid < rows ? (UP ? perm[r0 + tid] / top : r0 + tid) : -1;
-    __syncthreads();
-    const bf16* w0e = w0 + (size_t)e * N * K;
-    const bf16* w1e = GATED ? w1 + (size_t)e * N * K : nullptr;
-    auto load = [&](int k0, int buf) {
-        // 64 rows x 8 chunks of 8 per operand
-        for (int i = tid; i < MOE_TM * (MT_BK / 8); i += 128) {
-            const int r = i >> 3, c = i & 7;
-            const int k = k0 + c * 8;
-            const int sr = src_row[r];
-            const bool oka = sr >= 0 && k < K;
-            cp_async16(&As[buf][r][c * 8], oka ? a + (size_t)sr * a_stride + k : a, oka);
-            const bool okb = n0 + r < N && k < K;
-            cp_async16(&B0[buf][r][c * 8], okb ? w0e + (size_t)(n0 + r) * K + k : w0, okb);
-            if (GATED) cp_async16(&B1[buf][r][c * 8], okb ? w1e + (size_t)(n0 + r) * K + k : w0, okb);
-        }
-    };
-    float c0[MOE_TN / 8][4], c1[GATED ? MOE_TN / 8 : 1][4];
-#pragma unroll
-    for (int i = 0; i < MOE_TN / 8; ++i) c0[i][0] = c0[i][1] = c0[i][2] = c0[i][3] = 0.f;
-#pragma unroll
-    for (int i = 0; i < (GATED ? MOE_TN / 8 : 1); ++i) c1[i][0] = c1[i][1] = c1[i][2] = c1[i][3] = 0.f;
-    const int steps = (K + MT_BK - 1) / MT_BK;
-#pragma unroll
-    for (int p = 0; p < MT_STAGES - 1; ++p) {
-        if (p < steps) load(p * MT_BK, p);
-        cp_async_commit();
+    const int nm = GATED ? 2 * bn : bn;                        // columns of a product
+    const int stage_bytes = MT_A_BYTES + nm * MT_BK * 2;
+    const int stages = min(MT_RING / stage_bytes, 8);
+    extern __shared__ unsigned char moe_raw[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)moe_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* out_stage = base + MT_RING;                 // [4][MT_STAGE_OUT]
+    uint64_t* full = (uint64_t*)(out_stage + 4 * MT_STAGE_OUT);
+    uint64_t* empty = full + 8;
+    uint64_t* acc_full = empty + 8;                            // [2]
+    uint64_t* acc_empty = acc_full + 2;                        // [2]
+    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 8; ++i) { tg_init(&full[i], 1); tg_init(&empty[i], 1); }
+        for (int i = 0; i < 2; ++i) { tg_init(&acc_full[i], 1); tg_init(&acc_empty[i], 4); }
+        tg_init_done();
     }
-    const bool warp_active = warp * 16 < rows;
-    for (int st = 0; st < steps; ++st) {
-        const int buf = st % MT_STAGES;
-        cp_async_wait<MT_STAGES - 2>();                   // this step's tiles have landed
-        __syncthreads();                                  // and the buffer of step st - 1 is free
-        if (st + MT_STAGES - 1 < steps) load((st + MT_STAGES - 1) * MT_BK, (st + MT_STAGES - 1) % MT_STAGES);
-        cp_async_commit();
-        if (warp_active) {
+    if (warp == 1) tg_alloc512(tmem_slot);
+    tg_before();
+    __syncthreads();
+    tg_after();
+    const uint32_t tmem = *tmem_slot;
+    pdl_wait();
+    const int n_nt = (N + bn - 1) / bn, total = tile_info[0] * n_nt, kbs = (K + MT_BK - 1) / MT_BK;
+
+    if (warp == 0) {
+        uint32_t it = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
+            const int tile = w / n_nt, n0 = (w % n_nt) * bn;
+            const int e = tiles[3 * tile], r0 = tiles[3 * tile + 1], rows = tiles[3 * tile + 2];
+            int src[4] = {0, 0, 0, 0};
+            if (gather)
 #pragma unroll
-            for (int ks = 0; ks < MT_BK / 16; ++ks) {
-                uint32_t fa[4];
-                ldmatrix_x4(fa, &As[buf][warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8][ks * 16 + (lane >> 4) * 8]);
+                for (int j = 0; j < 4; ++j) src[j] = perm[r0 + min(4 * lane + j, rows - 1)] / top;
+            const int groups = gather ? (rows + 3) / 4 : (rows + 31) / 32, group_bytes = gather ? 512 : 4096;
+            for (int kb = 0; kb < kbs; ++kb, ++it) {
+                const int s = it % stages;
+                ok = __all_sync(0xffffffffu, tg_wait(&empty[s], ((it / stages) & 1) ^ 1, &moe_error_flag, 1));
+                if (!ok) break;
+                unsigned char* st = base + (size_t)s * stage_bytes;
+                if (lane == 0) tg_expect(&full[s], (uint32_t)(groups * group_bytes + nm * MT_BK * 2));
+                __syncwarp();
+                if (lane == 0) tg_load_2d(st + MT_A_BYTES, &map_b0, kb * MT_BK, e * N + n0, &full[s]);
+                if (GATED && lane == 1) tg_load_2d(st + MT_A_BYTES + bn * MT_BK * 2, &map_b1, kb * MT_BK, e * N + n0, &full[s]);
+                if (lane < groups && !gather) tg_load_2d(st + lane * 4096, &map_a, kb * MT_BK, r0 + 32 * lane, &full[s]);
+                if (lane < groups && gather) tg_gather4(st + lane * 512, &map_a, kb * MT_BK, src[0], src[1], src[2], src[3], &full[s]);
+            }
+        }
+    } else if (warp == 1) {
+        if (lane == 0) {
+            const uint32_t idesc = tg_idesc(nm);
+            uint32_t it = 0, n = 0;
+            bool ok = true;
+            for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++n) {
+                const uint32_t buf = n & 1u, d = tmem + 256u * buf;
+                ok = tg_wait(&acc_empty[buf], ((n >> 1) & 1u) ^ 1u, &moe_error_flag, 2);
+                if (!ok) break;
+                tg_after();
+                for (int kb = 0; kb < kbs; ++kb, ++it) {
+                    const int s = it % stages;
+                    ok = tg_wait(&full[s], (it / stages) & 1, &moe_error_flag, 3);
+                    if (!ok) break;
+                    tg_after();
+                    unsigned char* st = base + (size_t)s * stage_bytes;
+                    const uint64_t da = tg_desc(st), db = tg_desc(st + MT_A_BYTES);
 #pragma unroll
-                for (int np = 0; np < MOE_TN / 16; ++np) {
-                    uint32_t fb[4];
-                    ldmatrix_x4(fb, &B0[buf][np * 16 + (lane & 7) + (lane >> 4) * 8][ks * 16 + ((lane >> 3) & 1) * 8]);
-                    mma_bf16(c0[2 * np], fa, fb[0], fb[1]);
-                    mma_bf16(c0[2 * np + 1], fa, fb[2], fb[3]);
-                    if (GATED) {
-                        ldmatrix_x4(fb, &B1[buf][np * 16 + (lane & 7) + (lane >> 4) * 8][ks * 16 + ((lane >> 3) & 1) * 8]);
-                        mma_bf16(c1[2 * np], fa, fb[0], fb[1]);
-                        mma_bf16(c1[2 * np + 1], fa, fb[2], fb[3]);
+                    for (int k = 0; k < MT_BK / 16; ++k) tg_mma(d, da + 2 * k, db + 2 * k, idesc, (kb > 0 || k > 0) ? 1u : 0u);
+                    tg_commit(&empty[s]);
+                }
+                tg_commit(&acc_full[buf]);
+            }
+        }
+    } else {
+        const int quarter = warp & 3;                          // tensor-memory lanes this warp may read
+        const int row = quarter * 32 + lane;
+        const uint32_t lane_base = (uint32_t)(quarter * 32) << 16;
+        const uint32_t stage = tg_smem(out_stage + (warp - 2) * MT_STAGE_OUT);
+        uint32_t n = 0;
+        bool ok = true;
+        for (int w = blockIdx.x; w < total && ok; w += gridDim.x, ++n) {
+            const int tile = w / n_nt, n0 = (w % n_nt) * bn;
+            const int r0 = tiles[3 * tile + 1], rows = tiles[3 * tile + 2];
+            const int pair = !UP && row < rows ? perm[r0 + row] : 0;
+            const uint32_t buf = n & 1u, acc = tmem + 256u * buf + lane_base;
+            ok = __all_sync(0xffffffffu, tg_wait(&acc_full[buf], (n >> 1) & 1u, &moe_error_flag, 4));
+            tg_after();
+            const bool any = ok && quarter * 32 < rows;        // the same for the whole warp
+            for (int c = 0; any && c < bn && n0 + c < N; c += 32) {
+                uint32_t a[32];
+                tg_ld32(acc + c, a);
+                if (UP) {
+                    uint32_t u[GATED ? 32 : 1];
+                    if constexpr (GATED) tg_ld32(acc + bn + c, u);
+                    tg_wait_ld();
+                    float v[32];
+#pragma unroll
+                    for (int i = 0; i < 32; ++i)
+                        v[i] = moe_act_fast(__uint_as_float(a[i]), act) * (GATED ? __uint_as_float(u[GATED ? i : 0]) : 1.f);
+                    // 64 bytes a row, pieces of 16 shifted by row so that neither side meets a bank twice
+#pragma unroll
+                    for (int q = 0; q < 4; ++q)
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};"
+                                     ::"r"(stage + (uint32_t)(lane * 64 + ((q ^ ((lane >> 1) & 3)) << 4))),
+                                     "r"(tg_pack(v[8 * q], v[8 * q + 1])), "r"(tg_pack(v[8 * q + 2], v[8 * q + 3])),
+                                     "r"(tg_pack(v[8 * q + 4], v[8 * q + 5])), "r"(tg_pack(v[8 * q + 6], v[8 * q + 7])) : "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int r = i * 8 + (lane >> 2), q = lane & 3;
+                        uint4 x;
+                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
+                                     : "r"(stage + (uint32_t)(r * 64 + ((q ^ ((r >> 1) & 3)) << 4))) : "memory");
+                        if (quarter * 32 + r < rows && n0 + c + q * 8 < N)
+                            *(uint4*)(hidden + (size_t)(r0 + quarter * 32 + r) * N + n0 + c + q * 8) = x;
+                    }
+                } else {
+                    tg_wait_ld();
+#pragma unroll
+                    for (int q = 0; q < 8; ++q)
+                        asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(stage + (uint32_t)(lane * 128 + ((q ^ (lane & 7)) << 4))),
+                                     "r"(a[4 * q]), "r"(a[4 * q + 1]), "r"(a[4 * q + 2]), "r"(a[4 * q + 3]) : "memory");
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 8; ++i) {
+                        const int r = i * 4 + (lane >> 3), q = lane & 7;
+                        uint4 x;
+                        asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(x.x), "=r"(x.y), "=r"(x.z), "=r"(x.w)
+                                     : "r"(stage + (uint32_t)(r * 128 + ((q ^ (r & 7)) << 4))) : "memory");
+                        const int to = __shfl_sync(0xffffffffu, pair, r);
+                        if (quarter * 32 + r < rows && n0 + c + q * 4 < N) *(uint4*)(y + (size_t)to * N + n0 + c + q * 4) = x;
                     }
                 }
+                __syncwarp();
             }
+            tg_before();
+            __syncwarp();
+            if (lane == 0) tg_arrive(&acc_empty[buf]);
         }
     }
-    cp_async_wait<0>();
-    if (!warp_active) return;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int row = warp * 16 + (lane >> 2) + 8 * h;
-        if (row >= rows) continue;
-        const int pair = UP ? 0 : perm[r0 + row];
-#pragma unroll
-        for (int i = 0; i < MOE_TN / 8; ++i) {
-            const int col = n0 + i * 8 + (lane & 3) * 2;
-            if (col >= N) continue;                       // N is even: col + 1 < N too
-            if (UP) {
-                const float v0 = moe_act(c0[i][2 * h], act) * (GATED ? c1[GATED ? i : 0][2 * h] : 1.f);
-                const float v1 = moe_act(c0[i][2 * h + 1], act) * (GATED ? c1[GATED ? i : 0][2 * h + 1] : 1.f);
-                *(uint32_t*)(hidden + (size_t)(r0 + row) * N + col) = pack_bf16(v0, v1);
-            } else {
-                *(float2*)(y + (size_t)pair * N + col) = make_float2(c0[i][2 * h], c0[i][2 * h + 1]);
-            }
-        }
+    tg_before();
+    __syncthreads();
+    if (warp == 1) {
+        tg_after();
+        tg_free512(tmem);
     }
+}
+
+// xg[place] = x[token of the pair at `place`]: a block a place, 16 bytes a thread and turn.
+__global__ void __launch_bounds__(128)
+moe_gather_kernel(const bf16* __restrict__ x, long long x_stride, bf16* __restrict__ xg, int d, int top, int E,
+                  const int* __restrict__ perm, const int* __restrict__ offsets) {
+    pdl_wait();
+    if ((int)blockIdx.x >= offsets[E]) return;           // identity experts' pairs have no place
+    const uint4* src = (const uint4*)(x + (size_t)(perm[blockIdx.x] / top) * x_stride);
+    uint4* dst = (uint4*)(xg + (size_t)blockIdx.x * d);
+    for (int c = threadIdx.x; c < d / 8; c += 128) dst[c] = src[c];
+}
+
+static int moe_sms() {
+    static int cached[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
+    return cached[dev] > 0 ? cached[dev] : 148;
+}
+
+// The column tile: a round of items costs its k-blocks at the slower of their products (2 cycles a
+// column) and of their bytes (70 a cycle), and about 1500 cycles; the number of planned tiles is
+// the device's to know, `m_est` what evenly spread tokens would make.
+static int moe_tc_width(int N, int K, int E, int pairs, bool gated) {
+    const int sms = moe_sms(), per = pairs / E;
+    const double m_est = pairs <= E ? pairs : per < 128 ? E : E * ((per + 64) / 128 + 0.5);
+    const double a_bytes = (per < 1 ? 4.0 : per < 128 ? per : 128.0) * 128.0;
+    const int f = gated ? 2 : 1, kbs = (K + MT_BK - 1) / MT_BK;
+    double best = -1.0;
+    int bn = 32;
+    for (int w = 256 / f; w >= 32; w -= 32) {
+        const double items = m_est * ((N + w - 1) / w);
+        const double math = 2.0 * w * f, feed = (a_bytes + 128.0 * w * f) / 70.0;
+        const double rounds = items <= sms ? 1.0 : items > 4.0 * sms ? items / sms : (double)(long long)(items / sms + 0.999);
+        const double cost = rounds * (kbs * (math > feed ? math : feed) + 1500.0);
+        if (best < 0 || cost < best) { best = cost; bn = w; }
+    }
+    return bn;
+}
+
+template <int MODE>
+static int moe_tc_launch(const void* a, long long a_rows, long long a_stride, const void* b0, const void* b1, void* hidden,
+                         float* y, int N, int K, int E, int pairs, int top, int act, bool gather,
+                         const int* perm, const int* tile_info, const int* tiles, cudaStream_t stream) {
+    static bool sized[64] = {};                                // per device
+    int dev = 0;
+    cudaError_t err = cudaGetDevice(&dev);
+    if (err != cudaSuccess) return (int)err;
+    if (dev < 0 || dev >= 64 || (long long)E * N > 0x7fffffffll) return TGO_E_BAD_ARG;
+    if (!sized[dev]) {
+        err = cudaFuncSetAttribute(moe_tc_kernel<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, MT_SMEM);
+        if (err != cudaSuccess) return (int)err;
+        sized[dev] = true;
+    }
+    const int bn = moe_tc_width(N, K, E, pairs, MODE == 1);
+    CUtensorMap ma, m0, m1;
+    if (!tg_map(&ma, a, a_rows, K, a_stride, gather ? 1 : 32) || !tg_map(&m0, b0, (long long)E * N, K, K, bn) ||
+        !tg_map(&m1, b1 ? b1 : b0, (long long)E * N, K, K, bn))
+        return TGO_E_BAD_ARG;
+    return tgo_launch_pdl(moe_tc_kernel<MODE>, dim3(moe_sms()), dim3(MT_THREADS), MT_SMEM, stream, ma, m0, m1, (bf16*)hidden, y,
+                          N, K, bn, top, act, gather ? 1 : 0, perm, tile_info, tiles);
 }
 
 // out[t][c] = sum_j wts[t][j] y[t top + j][c] + extra_gate[t] * extra[t][c]; a pair whose
@@ -644,7 +794,10 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
     }
 }
 
-TGO_API int tgo_moe_tile_rows() { return MOE_TM; }
+TGO_API int tgo_moe_tile_rows() { return MOE_TILE; }
+
+// Reads (and waits for the device to reach) the code a wait that ran out left; 0: none did.
+TGO_API int tgo_moe_error(int* value) { return (int)cudaMemcpyFromSymbol(value, moe_error_flag, sizeof(int)); }
 
 // ids, place int32 [T top]; wts float32 [T top]; logits float32 [T, router rows]; counts, fill
 // int32 [E]; offsets int32 [E + 1]; perm int32 [T top]; tile_info int32 [1]; tiles int32
@@ -700,11 +853,12 @@ TGO_API int tgo_moe_route(const void* x, long long x_stride, int dtype, const fl
 }
 
 // x [T, d] rows (stride x_stride); wg, wu [E, ff, d]; wd [E, d, ff]; hidden [T top, ff] in the
-// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out float32 [T, d].
+// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out float32 [T, d]. xg: null, or
+// [T top, d] in the storage type, 16-byte aligned: room for the rows of x in place order.
 TGO_API int tgo_moe_experts(const void* x, long long x_stride, int dtype, const void* wg,
                             const void* wu, const void* wd, void* hidden, float* y,
                             const float* wts, const float* extra, float* out, int T, int d, int ff,
-                            int top, int act, const int* perm, const int* tile_info,
+                            int top, int act, const int* perm, const int* offsets, void* xg, const int* tile_info,
                             const int* tiles, int max_tiles, const int* ids, int E_real,
                             const float* extra_gate, const void* beside, int beside_dtype,
                             int accumulate, cudaStream_t stream) {
@@ -720,32 +874,25 @@ TGO_API int tgo_moe_experts(const void* x, long long x_stride, int dtype, const 
                    out, d, top, ids, E_real, (const TT*)x, x_stride, extra_gate, (const TB*)beside, accumulate,     \
                    comb_vec)
 #define MOE_COMBINE(TT) (beside && beside_dtype == TGO_BF16 ? MOE_COMBINE_OF(TT, bf16) : MOE_COMBINE_OF(TT, float))
-    const dim3 g1((ff + MOE_TN - 1) / MOE_TN, max_tiles), g2((d + MOE_TN - 1) / MOE_TN, max_tiles);
+    const dim3 g1((ff + MOE_TN - 1) / MOE_TN, max_tiles, MOE_TILE / MOE_TM), g2((d + MOE_TN - 1) / MOE_TN, max_tiles, MOE_TILE / MOE_TM);
     int rc;
     const bool chunks = d % 8 == 0 && ff % 8 == 0 && x_stride % 8 == 0 && (uintptr_t)x % 16 == 0 &&
                         (uintptr_t)wg % 16 == 0 && (uintptr_t)wu % 16 == 0 && (uintptr_t)wd % 16 == 0 &&
-                        (uintptr_t)hidden % 16 == 0 && (uintptr_t)y % 8 == 0;
+                        (uintptr_t)hidden % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)xg % 16 == 0 && E_real > 0;
     if (dtype == TGO_BF16 && chunks) {
-        const size_t tile = sizeof(bf16) * MT_STAGES * MOE_TM * MT_LD;
-        static bool asked = false;
-        if (!asked) {
-            cudaFuncSetAttribute(moe_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(3 * tile));
-            cudaFuncSetAttribute(moe_tc_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile));
-            cudaFuncSetAttribute(moe_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(2 * tile));
-            asked = true;
+        const int pairs = T * top;
+        const void* a = x;
+        long long a_rows = T, a_stride = x_stride;
+        if (xg) {
+            rc = tgo_launch_pdl(moe_gather_kernel, dim3(pairs), dim3(128), 0, stream, (const bf16*)x, x_stride, (bf16*)xg, d,
+                                top, E_real, perm, offsets);
+            if (rc) return rc;
+            a = xg; a_rows = pairs; a_stride = d;
         }
-        if (wg)
-            rc = tgo_launch_pdl(moe_tc_kernel<1>, g1, dim3(128), 3 * tile, stream, (const bf16*)x, x_stride,
-                                (const bf16*)wg, (const bf16*)wu, (bf16*)hidden, (float*)nullptr, ff, d, top, act,
-                                perm, tile_info, tiles);
-        else
-            rc = tgo_launch_pdl(moe_tc_kernel<2>, g1, dim3(128), 2 * tile, stream, (const bf16*)x, x_stride,
-                                (const bf16*)wu, (const bf16*)nullptr, (bf16*)hidden, (float*)nullptr, ff, d, top,
-                                act, perm, tile_info, tiles);
+        rc = wg ? moe_tc_launch<1>(a, a_rows, a_stride, wg, wu, hidden, nullptr, ff, d, E_real, pairs, top, act, !xg, perm, tile_info, tiles, stream)
+                : moe_tc_launch<2>(a, a_rows, a_stride, wu, nullptr, hidden, nullptr, ff, d, E_real, pairs, top, act, !xg, perm, tile_info, tiles, stream);
         if (rc) return rc;
-        rc = tgo_launch_pdl(moe_tc_kernel<0>, g2, dim3(128), 2 * tile, stream, (const bf16*)hidden, (long long)ff,
-                            (const bf16*)wd, (const bf16*)nullptr, (bf16*)nullptr, y, d, ff, top, act, perm,
-                            tile_info, tiles);
+        rc = moe_tc_launch<0>(hidden, pairs, ff, wd, nullptr, nullptr, y, d, ff, E_real, pairs, top, act, false, perm, tile_info, tiles, stream);
         if (rc) return rc;
         return MOE_COMBINE(bf16);
     }

@@ -1159,6 +1159,20 @@ def moe_tile_rows() -> int:
     return int(load_library("moe").tgo_moe_tile_rows())
 
 
+# Rows an expert on average from which the routed products read copies of x's rows in place order:
+# a TMA gather of four rows takes about 100 cycles, so a tile of 128 gathered rows is fed at a
+# quarter of the rate of boxes of 32 rows (2048 tokens, 32 experts, top 4, width 2048: the up product
+# took 220 us so); below it the copy's launch costs more.
+MOE_GATHER_ROWS = 24
+
+
+def moe_error() -> int:
+    """The code a wait of the routed products left when it ran out, or 0. Synchronises."""
+    value = ctypes.c_int(0)
+    _check(load_library("moe").tgo_moe_error(ctypes.byref(value)), "moe_error")
+    return int(value.value)
+
+
 def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional[torch.Tensor],
                      w_gate: Optional[torch.Tensor], w_up: torch.Tensor, w_down: torch.Tensor, top: int,
                      activation: str, extra: Optional[torch.Tensor] = None,
@@ -1224,6 +1238,8 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     gate = torch.empty(T, dtype=torch.float32, device=dev) if extra_gated else None
     hidden = torch.empty((pairs, ff), dtype=x.dtype, device=dev)
     y = torch.empty((pairs, d), dtype=torch.float32, device=dev)
+    xg = torch.empty((pairs, d), dtype=x.dtype, device=dev) \
+        if x.dtype == torch.bfloat16 and pairs >= MOE_GATHER_ROWS * E else None
     out = residual if residual is not None else torch.empty((T, d), dtype=torch.float32, device=dev)
     lib = load_library("moe")
     _check(lib.tgo_moe_route(
@@ -1236,7 +1252,7 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     _check(lib.tgo_moe_experts(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w_gate), _ptr(w_up),
         _ptr(w_down), _ptr(hidden), _ptr(y), _ptr(wts), _ptr(extra), _ptr(out), c_int(T), c_int(d),
-        c_int(ff), c_int(top), c_int(PLAIN_ACTIVATIONS[activation]), _ptr(perm), _ptr(tile_info),
+        c_int(ff), c_int(top), c_int(PLAIN_ACTIVATIONS[activation]), _ptr(perm), _ptr(offsets), _ptr(xg), _ptr(tile_info),
         _ptr(tiles), c_int(max_tiles), _ptr(ids if identity else None), c_int(E), _ptr(gate),
         _ptr(beside), c_int(dtype_code(beside.dtype) if beside is not None else 0),
         c_int(1 if residual is not None else 0), _stream()), "moe_experts", f"(d={d}, ff={ff})")
@@ -2020,6 +2036,10 @@ def kernel_wait_errors() -> dict:
         code = attention_decode_tma_error()
         if code:
             out["attention_decode_tma"] = code
+    if "moe" in _loaded:
+        code = moe_error()
+        if code:
+            out["moe"] = code
     for key, flag in _tc_err.items():
         code = int(flag.item())
         if code:
