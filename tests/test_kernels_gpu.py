@@ -1026,3 +1026,52 @@ def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
         want.index_add_(0, row, (h @ wd[e].double().t()) * wt[row, place][:, None])
         size.index_add_(0, row, (h.abs() @ wd[e].double().abs().t()) * wt[row, place][:, None])
     assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
+
+
+@pytest.mark.parametrize("dk,dv,rot,act", [(64, 8, 0, 0), (64, 128, 32, 1), (128, 136, 128, 0), (128, 256, 64, 1)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
+    """Heads the register-tiled kernels take, requests that end before, on and after a chunk, against
+    the recurrence in 64 bits: sums of at most dk + 64 float32 terms behind at most ten chunks."""
+    o, H, lens = ops(), 3, [1, 63, 64, 65, 200, 577]
+    T, B = sum(lens), len(lens)
+    z = (rnd(T, H * (2 * dk + dv), seed=dk + dv) * 0.5).to(dtype)
+    q, k, v = z[:, :H * dk], z[:, H * dk:2 * H * dk], z[:, 2 * H * dk:]
+    decay = torch.tensor([0.5, 0.97, 1.0], device=DEV)
+    rope = torch.randn(T, rot, device=DEV) if rot else None
+    state = rnd(B + 2, H, dk, dv, seed=1)
+    before, slots = state.clone(), [3, 0, 5, 1, 7, 2]
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    C, t0, nt, first = o.retention_chunk_tokens(), [], [], []
+    for s, n in zip(starts, lens):
+        first.append(len(t0))
+        t0 += range(s, s + n, C)
+        nt += [min(C, n - a) for a in range(0, n, C)]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    out = torch.full((T, H * dv), float("nan"), device=DEV)
+    o.retention_chunked(q, k, v, out, B, H, dk, dv, decay, dk ** -0.5, rope, rot, i32(starts), i32(slots), state,
+                        i32(t0), i32(nt), i32(first), act=act)
+
+    def taken(x, w, turned):
+        x = x.double().view(T, H, w)
+        if act:
+            x = torch.nn.functional.silu(x)
+        if not turned or not rot:
+            return x
+        c, s = rope.double()[:, None, :rot // 2], rope.double()[:, None, rot // 2:]
+        a, b = x[..., :rot // 2], x[..., rot // 2:rot]
+        return torch.cat([a * c - b * s, b * c + a * s, x[..., rot:]], -1)
+    qq, kk, vv = taken(q, dk, True), taken(k, dk, True) * dk ** -0.5, taken(v, dv, False)
+    for b, n in enumerate(lens):
+        S = before[slots[b]].double()
+        want = torch.empty(n, H, dv, dtype=torch.float64, device=DEV)
+        for i in range(n):
+            t = starts[b] + i
+            S = decay.double()[:, None, None] * S + kk[t][:, :, None] * vv[t][:, None]
+            want[i] = torch.einsum("hkv,hk->hv", S, qq[t])
+        got = out[starts[b]:starts[b + 1]].view(n, H, dv).double()
+        assert (got - want).norm() <= 3e-6 * want.norm() and (state[slots[b]].double() - S).norm() <= 3e-6 * S.norm()
+    untouched = [i for i in range(B + 2) if i not in slots]
+    assert torch.equal(state[untouched], before[untouched])

@@ -15,7 +15,7 @@
 // The columns of S are independent, so a block owns a slice of dv columns of one
 // (request, head): grid (requests, heads, slices). The powers of the decay come from a table
 // made by repeated multiplication.
-#include "common.cuh"
+#include "fma_tile.cuh"
 
 #define RT_CHUNK 32
 #define RT_THREADS 256
@@ -484,6 +484,304 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
     }
 }
 
+// ------------------------------------------------ the same, for heads of 64 or 128 key channels
+// Register tiles of 8 x 8 and 4 x 8 outputs (fma_tile.cuh) instead of 4 x 4; what a product sums
+// over is the slow axis of both of its operands in shared memory. Bound by the FMA pipes; a true
+// 32-bit product has no faster unit. MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16
+// rows; the kernels above in brackets): summaries 140 us (255), scan 40 (139), outputs 312 (879).
+//   summaries   a block makes U for 128 columns of V: K (scaled rows) and V as they lie;
+//   scan        four neighbouring elements a thread, eight summaries asked for while the eight before
+//               them are used: bound by memory (every summary read once, every state written once);
+//   outputs     a block takes a chunk's 64 rows and, 128 columns at a time, decay^(i+1) Q P + A V:
+//               Q and K are laid down channel-major once, A token-major; P comes 16 channels at a
+//               time, two turns ahead. The columns are shared out over blocks when there are few
+//               chunks.
+#define RF_SLICE 128
+#define RF_LDN (RC_CHUNK + 4)         // rows of a channel-major tile
+#define RF_LDS (RF_SLICE + 4)
+#define RF_PK 16                      // channels of P a turn
+#define RF_PSTAGES 3
+
+// Eight channels' values of a row, after the activation.
+template <typename T>
+__device__ __forceinline__ void taken8(const T* __restrict__ x, int act, float (&f)[8]);
+template <>
+__device__ __forceinline__ void taken8<bf16>(const bf16* __restrict__ x, int act, float (&f)[8]) {
+    const uint4 u = *(const uint4*)x;
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const float2 v = __bfloat1622float2(*(const __nv_bfloat162*)&w[i]);
+        f[2 * i] = v.x;
+        f[2 * i + 1] = v.y;
+    }
+    if (act == 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.f + expf(-f[i]));
+}
+template <>
+__device__ __forceinline__ void taken8<float>(const float* __restrict__ x, int act, float (&f)[8]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+        const float4 v = ((const float4*)x)[i];
+        f[4 * i] = v.x; f[4 * i + 1] = v.y; f[4 * i + 2] = v.z; f[4 * i + 3] = v.w;
+    }
+    if (act == 1)
+#pragma unroll
+        for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.f + expf(-f[i]));
+}
+
+// Eight neighbouring channels d0 .. d0 + 7 of a row, rotated: d0 and rot / 2 are multiples of 8.
+template <typename T>
+__device__ __forceinline__ void rotated8(const T* __restrict__ x, const float* __restrict__ cs, int d0, int rot, int act,
+                                         float (&f)[8]) {
+    taken8(x + d0, act, f);
+    if (!cs || d0 >= rot) return;
+    const int half = rot >> 1;
+    const bool low = d0 < half;
+    const int p0 = low ? d0 : d0 - half;
+    float g[8];
+    taken8(x + (low ? d0 + half : p0), act, g);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+        const float c = cs[p0 + i], s = cs[half + p0 + i];
+        f[i] = low ? f[i] * c - g[i] * s : f[i] * c + g[i] * s;
+    }
+}
+
+// The powers of the decay, 0 .. RC_CHUNK, by repeated multiplication.
+__device__ __forceinline__ void rf_powers(float* pw, float g) {
+    if (threadIdx.x == 0) {
+        float x = 1.f;
+        for (int i = 0; i <= RC_CHUNK; ++i) { pw[i] = x; x *= g; }
+    }
+}
+
+// Columns c0 .. c0 + RF_SLICE - 1 of the chunk's values, rows past n and columns past dv zero.
+template <typename T>
+__device__ __forceinline__ void rf_load_v(float* Vs, const T* __restrict__ v, long long v_stride, int h, int dv, int c0,
+                                          int tok0, int n, int act) {
+    for (int i = threadIdx.x; i < RC_CHUNK * (RF_SLICE / 8); i += RC_THREADS) {
+        const int r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (r < n && c0 + c < dv) taken8(v + (size_t)(tok0 + r) * v_stride + (size_t)h * dv + c0 + c, act, f);
+        *(float4*)(Vs + r * RF_LDS + c) = make_float4(f[0], f[1], f[2], f[3]);
+        *(float4*)(Vs + r * RF_LDS + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+}
+
+template <typename T, int DK>
+__global__ void __launch_bounds__(RC_THREADS, 2)
+retention_summaries_tiled_kernel(const T* __restrict__ k, long long k_stride, const T* __restrict__ v, long long v_stride,
+                                 int H, int dv, const float* __restrict__ decay, float k_scale, int act,
+                                 const float* __restrict__ rope, int rot, const int* __restrict__ chunk_tok0,
+                                 const int* __restrict__ chunk_ntok, float* __restrict__ U) {
+    extern __shared__ __align__(16) float smem[];
+    float* Ks = smem;                                    // [RC_CHUNK][DK + 4]
+    float* Vs = Ks + RC_CHUNK * (DK + 4);                // [RC_CHUNK][RF_LDS]
+    __shared__ float pw[RC_CHUNK + 1];
+    pdl_wait();
+    const int ci = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * RF_SLICE;
+    const int tok0 = chunk_tok0[ci], n = chunk_ntok[ci];
+    rf_powers(pw, decay[h]);
+    __syncthreads();
+    for (int i = threadIdx.x; i < RC_CHUNK * (DK / 8); i += RC_THREADS) {
+        const int r = i / (DK / 8), d = (i % (DK / 8)) * 8;
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (r < n) {
+            const size_t t = (size_t)(tok0 + r);
+            rotated8(k + t * k_stride + (size_t)h * DK, rope ? rope + t * rot : nullptr, d, rot, act, f);
+            const float w = pw[n - 1 - r];
+#pragma unroll
+            for (int x = 0; x < 8; ++x) f[x] = f[x] * k_scale * w;
+        }
+        *(float4*)(Ks + r * (DK + 4) + d) = make_float4(f[0], f[1], f[2], f[3]);
+        *(float4*)(Ks + r * (DK + 4) + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+    }
+    rf_load_v(Vs, v, v_stride, h, dv, c0, tok0, n, act);
+    __syncthreads();
+    FmaTile<DK / 64, 2, 16, 16> t;
+    t.ty = threadIdx.x / 16;
+    t.tx = threadIdx.x % 16;
+    t.clear();
+    t.add(Ks, DK + 4, Vs, RF_LDS, n);
+    float* Uo = U + ((size_t)ci * H + h) * DK * dv;
+#pragma unroll
+    for (int i = 0; i < DK / 16; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c)
+            if (c0 + t.col(c) < dv) *(float4*)(Uo + (size_t)t.row(i) * dv + c0 + t.col(c)) = t.get(i, c);
+}
+
+// grid (requests, heads, ceil(dk dv / 1024)): a thread four neighbouring elements of the state
+__global__ void __launch_bounds__(256)
+retention_scan4_kernel(int H, int dkdv, const float* __restrict__ decay, const int* __restrict__ q_start,
+                       const int* __restrict__ state_slots, const int* __restrict__ chunk_first, float* __restrict__ U,
+                       float* __restrict__ state) {
+    pdl_wait();
+    const int b = blockIdx.x, h = blockIdx.y;
+    const int e = 4 * (blockIdx.z * blockDim.x + threadIdx.x);
+    const int n_tok = q_start[b + 1] - q_start[b];
+    if (e >= dkdv || n_tok <= 0) return;
+    const int chunks = (n_tok + RC_CHUNK - 1) / RC_CHUNK, last = n_tok - (chunks - 1) * RC_CHUNK;
+    const float g = decay[h];
+    float gfull = 1.f, glast = 1.f;
+    for (int i = 0; i < RC_CHUNK; ++i) {
+        gfull *= g;
+        if (i < last) glast *= g;
+    }
+    float4* sp = (float4*)(state + ((size_t)state_slots[b] * H + h) * dkdv + e);
+    float4 s = *sp;
+    const size_t step = (size_t)H * dkdv / 4;
+    float4* ub = (float4*)(U + ((size_t)chunk_first[b] * H + h) * dkdv + e);
+    constexpr int N = 8;
+    float4 u[N], w[N];
+#pragma unroll
+    for (int x = 0; x < N; ++x) u[x] = x < chunks ? ub[(size_t)x * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int cb = 0; cb < chunks; cb += N) {
+#pragma unroll
+        for (int x = 0; x < N; ++x)
+            w[x] = cb + N + x < chunks ? ub[(size_t)(cb + N + x) * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int x = 0; x < N; ++x) {
+            const int c = cb + x;
+            if (c >= chunks) break;
+            ub[(size_t)c * step] = s;
+            const float gn = c == chunks - 1 ? glast : gfull;
+            s.x = gn * s.x + u[x].x; s.y = gn * s.y + u[x].y; s.z = gn * s.z + u[x].z; s.w = gn * s.w + u[x].w;
+        }
+#pragma unroll
+        for (int x = 0; x < N; ++x) u[x] = w[x];
+    }
+    *sp = s;
+}
+
+template <typename T, int DK>
+__global__ void __launch_bounds__(RC_THREADS, 2)
+retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, const T* __restrict__ k, long long k_stride,
+                               const T* __restrict__ v, long long v_stride, float* __restrict__ out, int H, int dv,
+                               const float* __restrict__ decay, float k_scale, int act, const float* __restrict__ rope,
+                               int rot, const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_ntok,
+                               const float* __restrict__ P) {
+    extern __shared__ __align__(16) float smem[];
+    float* Qt = smem;                                    // [DK][RF_LDN]
+    float* At = Qt + DK * RF_LDN;                        // [RC_CHUNK][RF_LDN], token j major
+    float* Ps = At + RC_CHUNK * RF_LDN;                  // [RF_PSTAGES][RF_PK][RF_LDS]
+    float* KV = Ps + RF_PSTAGES * RF_PK * RF_LDS;        // K [DK][RF_LDN], later V [RC_CHUNK][RF_LDS]
+    __shared__ float pw[RC_CHUNK + 1];
+    pdl_wait();
+    const int ci = blockIdx.x, h = blockIdx.y;
+    const int tok0 = chunk_tok0[ci], n = chunk_ntok[ci];
+    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
+    rf_powers(pw, decay[h]);
+    // a lane a row: the stores of a warp hit 32 neighbouring places, a row's line is read from L1
+    for (int i = threadIdx.x; i < 2 * RC_CHUNK * (DK / 8); i += RC_THREADS) {
+        const int which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
+        const int r = j % RC_CHUNK, d = (j / RC_CHUNK) * 8;
+        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+        if (r < n) {
+            const size_t t = (size_t)(tok0 + r);
+            rotated8(which ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
+                     rope ? rope + t * rot : nullptr, d, rot, act, f);
+        }
+        float* dst = (which ? KV : Qt) + d * RF_LDN + r;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) dst[x * RF_LDN] = which ? f[x] * k_scale : f[x];
+    }
+    __syncthreads();
+    {
+        FmaTile<1, 1, 16, 16> a;                         // A[i][j], 64 x 64
+        a.ty = ty;
+        a.tx = tx;
+        a.clear();
+        if (4 * tx <= 4 * ty + 3) a.add(Qt, RF_LDN, KV, RF_LDN, DK);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 r = a.get(i, 0);
+            const float x[4] = {r.x, r.y, r.z, r.w};
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int gap = 4 * ty + i - (4 * tx + j);
+                At[(4 * tx + j) * RF_LDN + 4 * ty + i] = gap >= 0 ? x[j] * pw[gap >= 0 ? gap : 0] : 0.f;
+            }
+        }
+    }
+    const float* Pc = P + ((size_t)ci * H + h) * DK * dv;
+    // the warp's rows end at 4 ty + 3 of its upper half: later tokens of the chunk are zeros of A
+    const int j_end = min(n, 4 * (ty | 1) + 4);
+    for (int c0 = blockIdx.z * RF_SLICE; c0 < dv; c0 += gridDim.z * RF_SLICE) {
+        auto load_p = [&](int turn) {
+            if (turn < DK / RF_PK) {
+                float* dst = Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS;
+                for (int i = threadIdx.x; i < RF_PK * (RF_SLICE / 4); i += RC_THREADS) {
+                    const int d = i / (RF_SLICE / 4), c = (i % (RF_SLICE / 4)) * 4;
+                    const bool ok = c0 + c < dv;
+                    ft_copy16(dst + d * RF_LDS + c, ok ? Pc + (size_t)(turn * RF_PK + d) * dv + c0 + c : Pc, ok);
+                }
+            }
+            ft_commit();
+        };
+        __syncthreads();                                 // K (or the last slice's V) and P have been read
+#pragma unroll
+        for (int s = 0; s < RF_PSTAGES - 1; ++s) load_p(s);
+        rf_load_v(KV, v, v_stride, h, dv, c0, tok0, n, act);
+        FmaTile<1, 2, 16, 16> o;                         // 64 x 128
+        o.ty = ty;
+        o.tx = tx;
+        o.clear();
+        for (int turn = 0; turn < DK / RF_PK; ++turn) {
+            ft_wait<RF_PSTAGES - 2>();
+            __syncthreads();
+            load_p(turn + RF_PSTAGES - 1);
+            o.add(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS, RF_PK);
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) o.scale_row(i, pw[4 * ty + i + 1]);
+        o.add(At, RF_LDN, KV, RF_LDS, j_end);
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+            if (4 * ty + i < n)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    if (c0 + o.col(c) < dv)
+                        *(float4*)(out + ((size_t)(tok0 + 4 * ty + i) * H + h) * dv + c0 + o.col(c)) = o.get(i, c);
+    }
+}
+
+template <typename T, int DK>
+static int retention_tiled(const T* q, long long q_stride, const T* k, long long k_stride, const T* v, long long v_stride,
+                           float* out, int B, int H, int dv, const float* decay, float k_scale, int act,
+                           const float* rope, int rot, const int* q_start, const int* state_slots, float* state,
+                           int chunks, const int* chunk_tok0, const int* chunk_ntok, const int* chunk_first,
+                           float* scratch, cudaStream_t stream) {
+    constexpr size_t s1 = (size_t)RC_CHUNK * (DK + 4 + RF_LDS) * sizeof(float);
+    constexpr size_t kv = (size_t)(DK * RF_LDN > RC_CHUNK * RF_LDS ? DK * RF_LDN : RC_CHUNK * RF_LDS);
+    constexpr size_t s3 = ((size_t)(DK + RC_CHUNK) * RF_LDN + RF_PSTAGES * RF_PK * RF_LDS + kv) * sizeof(float);
+    auto k1 = retention_summaries_tiled_kernel<T, DK>;
+    auto k3 = retention_outputs_tiled_kernel<T, DK>;
+    static bool sized[64] = {};                          // per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
+    if (!sized[dev]) {
+        if ((e = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1)) != cudaSuccess) return (int)e;
+        if ((e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
+        sized[dev] = true;
+    }
+    const int slices = (dv + RF_SLICE - 1) / RF_SLICE;
+    int rc = tgo_launch_pdl(k1, dim3(chunks, H, slices), dim3(RC_THREADS), s1, stream, k, k_stride, v, v_stride, H, dv,
+                            decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, scratch);
+    if (rc) return rc;
+    rc = tgo_launch_pdl(retention_scan4_kernel, dim3(B, H, (DK * dv / 4 + 255) / 256), dim3(256), 0, stream, H, DK * dv,
+                        decay, q_start, state_slots, chunk_first, scratch, state);
+    if (rc) return rc;
+    // two blocks an SM: with fewer (chunk, head) pairs than twice that a block takes one slice
+    const int z = (long long)chunks * H < 592 ? slices : 1;
+    return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RC_THREADS), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
+                          H, dv, decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, (const float*)scratch);
+}
+
 static inline size_t summaries_smem(int dk) {
     return ((size_t)RC_CHUNK * (dk + 1) + (size_t)RC_CHUNK * RC_VS + RC_CHUNK + 1) * sizeof(float);
 }
@@ -511,6 +809,17 @@ static int retention_chunked(const T* q, long long q_stride, const T* k, long lo
         return tgo_launch_pdl(retention_decode_kernel<T>, dim3(B, H, (dv + 31) / 32), dim3(RD_THREADS), smem,
                               stream, q, q_stride, k, k_stride, v, v_stride, out, H, dk, dv, decay, k_scale, act,
                               rope, rot, state_slots, state);
+    }
+    // rows that can be read eight channels at a time, rotated halves of whole eights
+    auto whole = [&](const void* p, long long stride) { return (uintptr_t)p % 16 == 0 && stride * sizeof(T) % 16 == 0; };
+    if ((dk == 64 || dk == 128) && dv % 8 == 0 && rot % 16 == 0 && whole(q, q_stride) && whole(k, k_stride) &&
+        whole(v, v_stride) && (uintptr_t)out % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)scratch % 16 == 0) {
+#define RF_GO(DK)                                                                                                    \
+    return retention_tiled<T, DK>(q, q_stride, k, k_stride, v, v_stride, out, B, H, dv, decay, k_scale, act, rope,    \
+                                  rot, q_start, state_slots, state, chunks, chunk_tok0, chunk_ntok, chunk_first, scratch, stream)
+        if (dk == 128) RF_GO(128);
+        RF_GO(64);
+#undef RF_GO
     }
     const size_t s1 = summaries_smem(dk), s3 = outputs_smem(dk);
     auto k1 = retention_summaries_kernel<T>;
