@@ -1075,3 +1075,45 @@ def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
         assert (got - want).norm() <= 3e-6 * want.norm() and (state[slots[b]].double() - S).norm() <= 3e-6 * S.norm()
     untouched = [i for i in range(B + 2) if i not in slots]
     assert torch.equal(state[untouched], before[untouched])
+
+
+@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 3, 64, 128), (2, 2, 128, 128)])
+@pytest.mark.parametrize("lens", [[128], [1, 63, 64, 65, 200, 3], [700, 129]])
+def test_selective_scan_by_chunks(H, G, N, P, lens, monkeypatch):
+    """Requests that end before, on and after a chunk, fast and slow decays, against the recurrence
+    in 64 bits: sums of at most N + 64 float32 terms behind at most eleven chunks."""
+    o, T, B = ops(), sum(lens), len(lens)
+    C = H * P + 2 * G * N
+    xbc = rnd(T, C, seed=N + P)
+    dt_raw = rnd(T, H + 2, seed=3).to(torch.bfloat16)[:, 1:H + 1]
+    dt_bias, a_log, d = rnd(H, seed=4) - 2.0, torch.linspace(-3.0, 3.0, H, device=DEV), rnd(H, seed=5)
+    floats = 8 + H * N * P + 12
+    state = rnd(B + 2, floats, seed=6)
+    before, slots = state.clone(), [5, 0, 3, 1, 7, 2][:B] if B > 2 else [2, 0][:B]
+    starts = [0]
+    for n in lens:
+        starts.append(starts[-1] + n)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    y = torch.full((T, H * P), float("nan"), device=DEV)
+    monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1)
+    launches = o.LAUNCHES[0]
+    o.selective_scan(xbc, dt_raw, dt_bias, a_log, d, y, B, H, G, N, P, i32(starts), i32(slots), state, 8)
+    assert o.LAUNCHES[0] == launches + 4                 # the chunked form ran
+    x = xbc.double()
+    u, bm, cm = x[:, :H * P].view(T, H, P), x[:, H * P:H * P + G * N].view(T, G, N), x[:, H * P + G * N:].view(T, G, N)
+    bm, cm = (m.repeat_interleave(H // G, 1) for m in (bm, cm))
+    dt = torch.nn.functional.softplus(dt_raw.double() + dt_bias.double())
+    a = torch.exp(-torch.exp(a_log.double()) * dt)
+    for b, n in enumerate(lens):
+        S = before[slots[b], 8:8 + H * N * P].view(H, N, P).double()
+        want = torch.empty(n, H, P, dtype=torch.float64, device=DEV)
+        for i in range(n):
+            t = starts[b] + i
+            S = a[t][:, None, None] * S + bm[t][:, :, None] * (dt[t][:, None] * u[t])[:, None]
+            want[i] = torch.einsum("hnp,hn->hp", S, cm[t]) + d.double()[:, None] * u[t]
+        got = y[starts[b]:starts[b + 1]].view(n, H, P).double()
+        assert (got - want).norm() <= 3e-6 * want.norm()
+        assert (state[slots[b], 8:8 + H * N * P].view(H, N, P).double() - S).norm() <= 3e-6 * S.norm()
+    after = state.clone()
+    after[slots, 8:8 + H * N * P] = before[slots, 8:8 + H * N * P]
+    assert torch.equal(after, before)

@@ -19,7 +19,7 @@
 // A request's state row (float32, `state_stride` floats apart) holds the scan's state
 // [H][N][P] (or [channels][N]) at `ssm_offset` and the convolution's last taps - 1 inputs [taps - 1][C] (oldest
 // first) at `conv_offset`.
-#include "common.cuh"
+#include "fma_tile.cuh"
 
 // ------------------------------------------------------------------------- convolution
 // y[t][c] = silu(bias[c] + sum_j w[c][j] x[t - (taps - 1 - j)][c]); inputs before the step's
@@ -401,6 +401,355 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
         return scan_by_size<float>(xbc, C, (const float*)dt_raw, dt_stride, dt_bias, A_log, D, y, B, H, G, N,
                                    P, q_start, state_slots, state, state_stride, ssm_offset, stream);
     return TGO_E_BAD_ARG;
+}
+
+// ------------------------------------------------------------------- scan over prompt portions
+// The recurrence written out over chunks of up to SD_CHUNK tokens of one request, so that chunks of
+// every head run side by side. With L_i the logarithm of the product of the decays up to and with
+// token i of the chunk (n tokens), v_j = dt_j x_j:
+//
+//   y_i = exp(L_i) S^T C_i + sum_{j<=i} exp(L_i - L_j) (C_i . B_j) v_j + D x_i
+//   S  <- exp(L_n) S + sum_j exp(L_n - L_j) B_j v_j^T
+//
+// Four launches: steps (dt and L of every token; L in 64 bits, so that the differences of large
+// sums lose nothing), summaries (the sum of S's line), a scan over the chunks, which leaves the
+// state before each chunk in its summary's place, and outputs. Float32 products in register tiles
+// (fma_tile.cuh), bound by the FMA pipes. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128): 711 us
+// by the walk above, 263 so (summaries 54, scan over the chunks 32, outputs 173); error against 64 bits
+// 1.2e-7 (1.9e-7 by the walk).
+// The walk stays for the float32 engine, whose sums do not depend on how a prompt is cut, for
+// steps of few tokens a request, and for other sizes.
+#define SD_CHUNK 64
+#define SD_LD (SD_CHUNK + 4)
+
+// The request and tokens of chunk `ci` (chunks are numbered request after request): false past the
+// last. One warp.
+__device__ __forceinline__ bool sd_find(const int* __restrict__ q_start, int B, int ci, int& b, int& tok0, int& n, int& nth) {
+    const int lane = threadIdx.x & 31;
+    int before = 0;
+    for (int b0 = 0; b0 < B; b0 += 32) {
+        const int r = b0 + lane;
+        const int s = r < B ? q_start[r] : 0, len = r < B ? q_start[r + 1] - s : 0;
+        const int c = (len + SD_CHUNK - 1) / SD_CHUNK;
+        int incl = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int a = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += a;
+        }
+        const unsigned hit = __ballot_sync(0xffffffffu, ci < before + incl);
+        if (hit) {
+            const int src = __ffs(hit) - 1;
+            nth = ci - before - __shfl_sync(0xffffffffu, incl - c, src);
+            const int start = __shfl_sync(0xffffffffu, s, src), all = __shfl_sync(0xffffffffu, len, src);
+            b = b0 + src;
+            tok0 = start + nth * SD_CHUNK;
+            n = all - nth * SD_CHUNK < SD_CHUNK ? all - nth * SD_CHUNK : SD_CHUNK;
+            return true;
+        }
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    return false;
+}
+
+// chunks [chunks][4]: first token, tokens, request, place among the request's chunks (tokens 0: none).
+// dts, cum [chunks][H][SD_CHUNK].
+template <typename T>
+__global__ void __launch_bounds__(256)
+ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float* __restrict__ dt_bias,
+                 const float* __restrict__ A_log, int H, const int* __restrict__ q_start, int B,
+                 int4* __restrict__ chunks, float* __restrict__ dts, double* __restrict__ cum) {
+    pdl_wait();
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, ci = blockIdx.x;
+    int b = 0, tok0 = 0, n = 0, nth = 0;
+    if (!sd_find(q_start, B, ci, b, tok0, n, nth)) n = 0;
+    if (blockIdx.y == 0 && threadIdx.x == 0) chunks[ci] = make_int4(tok0, n, b, nth);
+    const int h = blockIdx.y * 8 + warp;
+    if (n == 0 || h >= H) return;
+    const float A = expf(A_log[h]), bias = dt_bias ? dt_bias[h] : 0.f;
+    double l[2];
+    float dt[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {                        // tokens 2 lane, 2 lane + 1
+        const int t = 2 * lane + i;
+        dt[i] = 0.f;
+        if (t < n) {
+            const float z = to_f32(dt_raw[(size_t)(tok0 + t) * dt_stride + h]) + bias;
+            dt[i] = z > 20.f ? z : log1pf(expf(z));
+        }
+        l[i] = -(double)A * (double)dt[i];
+    }
+    double incl = l[0] + l[1];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double a = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += a;
+    }
+    const size_t at = ((size_t)ci * H + h) * SD_CHUNK + 2 * lane;
+    *(float2*)(dts + at) = make_float2(dt[0], dt[1]);
+    *(double2*)(cum + at) = make_double2(incl - l[1], incl);
+}
+
+template <int N, int P>
+__global__ void __launch_bounds__(N * P / 64, 512 / (N * P / 64))
+ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, const int4* __restrict__ chunks,
+                     const float* __restrict__ dts, const double* __restrict__ cum, float* __restrict__ U) {
+    constexpr int THREADS = N * P / 64;
+    extern __shared__ __align__(16) float smem[];
+    float* Bs = smem;                                    // [SD_CHUNK][N + 4]
+    float* Vs = Bs + SD_CHUNK * (N + 4);                 // [SD_CHUNK][P + 4], rows times dt exp(L_n - L_j)
+    __shared__ float ws[SD_CHUNK];
+    pdl_wait();
+    const int4 ch = chunks[blockIdx.x];
+    const int h = blockIdx.y, n = ch.y;
+    if (n == 0) return;
+    const float* rows = xbc + (size_t)ch.x * C;
+    const size_t at = ((size_t)blockIdx.x * H + h) * SD_CHUNK;
+    for (int i = threadIdx.x; i < n * (N / 4); i += THREADS) {
+        const int r = i / (N / 4), c = (i % (N / 4)) * 4;
+        ft_copy16(Bs + r * (N + 4) + c, rows + (size_t)r * C + H * P + (h / (H / G)) * N + c, true);
+    }
+    ft_commit();
+    for (int i = threadIdx.x; i < n; i += THREADS) ws[i] = dts[at + i] * expf((float)(cum[at + n - 1] - cum[at + i]));
+    __syncthreads();
+    for (int i = threadIdx.x; i < n * (P / 4); i += THREADS) {
+        const int r = i / (P / 4), c = (i % (P / 4)) * 4;
+        float4 v = *(const float4*)(rows + (size_t)r * C + h * P + c);
+        const float w = ws[r];
+        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
+        *(float4*)(Vs + r * (P + 4) + c) = v;
+    }
+    ft_wait<0>();
+    __syncthreads();
+    FmaTile<2, 2, N / 8, P / 8> t;
+    t.ty = threadIdx.x / (P / 8);
+    t.tx = threadIdx.x % (P / 8);
+    t.clear();
+    t.add(Bs, N + 4, Vs, P + 4, n);
+    float* Uo = U + ((size_t)blockIdx.x * H + h) * N * P;
+#pragma unroll
+    for (int i = 0; i < 8; ++i)
+#pragma unroll
+        for (int c = 0; c < 2; ++c) *(float4*)(Uo + (size_t)t.row(i) * P + t.col(c)) = t.get(i, c);
+}
+
+// grid (requests, heads, ceil(N P / 1024)): a thread four neighbouring elements of the state
+__global__ void __launch_bounds__(256)
+ssd_scan_kernel(int H, int NP, const int* __restrict__ q_start, const int* __restrict__ state_slots,
+                const double* __restrict__ cum, float* __restrict__ U, float* __restrict__ state, long long state_stride,
+                long long offset) {
+    pdl_wait();
+    const int b = blockIdx.x, h = blockIdx.y;
+    const int e = 4 * (blockIdx.z * blockDim.x + threadIdx.x);
+    const int n_tok = q_start[b + 1] - q_start[b];
+    __shared__ int s_first;
+    if (threadIdx.x < 32) {                              // chunks of the requests before this one
+        int first = 0;
+        for (int r = threadIdx.x; r < b; r += 32) first += (q_start[r + 1] - q_start[r] + SD_CHUNK - 1) / SD_CHUNK;
+        first = __reduce_add_sync(0xffffffffu, first);
+        if (threadIdx.x == 0) s_first = first;
+    }
+    __syncthreads();
+    if (e >= NP || n_tok <= 0) return;
+    const int chunks = (n_tok + SD_CHUNK - 1) / SD_CHUNK;
+    const size_t first = ((size_t)s_first * H + h);
+    float4* sp = (float4*)(state + (size_t)state_slots[b] * state_stride + offset + (size_t)h * NP + e);
+    float4 s = *sp;
+    const size_t step = (size_t)H * NP / 4;
+    float4* ub = (float4*)(U + first * NP + e);
+    const double* total = cum + first * SD_CHUNK;        // a chunk's whole decay stands at its last token
+    constexpr int X = 8;
+    float4 u[X], w[X];
+#pragma unroll
+    for (int x = 0; x < X; ++x) u[x] = x < chunks ? ub[(size_t)x * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int cb = 0; cb < chunks; cb += X) {
+#pragma unroll
+        for (int x = 0; x < X; ++x)
+            w[x] = cb + X + x < chunks ? ub[(size_t)(cb + X + x) * step] : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int x = 0; x < X; ++x) {
+            const int c = cb + x;
+            if (c >= chunks) break;
+            ub[(size_t)c * step] = s;
+            const int last = c == chunks - 1 ? n_tok - 1 - c * SD_CHUNK : SD_CHUNK - 1;
+            const float g = expf((float)total[(size_t)c * H * SD_CHUNK + last]);
+            s.x = fmaf(g, s.x, u[x].x); s.y = fmaf(g, s.y, u[x].y); s.z = fmaf(g, s.z, u[x].z); s.w = fmaf(g, s.w, u[x].w);
+        }
+#pragma unroll
+        for (int x = 0; x < X; ++x) u[x] = w[x];
+    }
+    *sp = s;
+}
+
+// A block: a chunk's rows of one head. B, C and the state come 64 of the N states at a time; C . B
+// and S^T C grow side by side in registers, then A times v is added.
+template <int N, int P>
+__global__ void __launch_bounds__(2 * P, 512 / (2 * P))
+ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const float* __restrict__ D,
+                   const int4* __restrict__ chunks, const float* __restrict__ dts, const double* __restrict__ cum,
+                   const float* __restrict__ U, float* __restrict__ y) {
+    constexpr int THREADS = 2 * P, TX = P / 8;           // 16 x TX threads, 4 x 8 outputs each
+    constexpr int GN = SD_CHUNK / (4 * TX);              // columns of C . B a thread owns, in fours
+    extern __shared__ __align__(16) float smem[];
+    float* Ct = smem;                                    // [64][SD_LD] state-major; later A [SD_CHUNK][SD_LD] token-j-major
+    float* Bt = Ct + 64 * SD_LD;                         // [64][SD_LD]; later v [SD_CHUNK][P + 4]
+    float* Ss = Bt + (64 * SD_LD > SD_CHUNK * (P + 4) ? 64 * SD_LD : SD_CHUNK * (P + 4));      // [64][P + 4]
+    __shared__ double ls[SD_CHUNK];
+    __shared__ float ds[SD_CHUNK];
+    pdl_wait();
+    const int4 ch = chunks[blockIdx.x];
+    const int h = blockIdx.y, n = ch.y;
+    if (n == 0) return;
+    const float* rows = xbc + (size_t)ch.x * C;
+    const float* brow = rows + H * P + (h / (H / G)) * N;
+    const float* crow = brow + (size_t)G * N;
+    const size_t at = ((size_t)blockIdx.x * H + h) * SD_CHUNK;
+    const float* Sc = U + ((size_t)blockIdx.x * H + h) * N * P;
+    for (int i = threadIdx.x; i < SD_CHUNK; i += THREADS) {
+        ls[i] = cum[at + i];
+        ds[i] = dts[at + i];
+    }
+    FmaTile<1, GN, 16, TX> g;
+    FmaTile<1, 2, 16, TX> o;
+    g.ty = o.ty = threadIdx.x / TX;
+    g.tx = o.tx = threadIdx.x % TX;
+    g.clear();
+    o.clear();
+    const bool busy = 4 * (o.ty & ~(32 / TX - 1)) < n;   // the warp's first row exists
+    for (int n0 = 0; n0 < N; n0 += 64) {
+        if (n0) __syncthreads();
+        for (int i = threadIdx.x; i < 64 * (P / 4); i += THREADS) {
+            const int r = i / (P / 4), c = (i % (P / 4)) * 4;
+            ft_copy16(Ss + r * (P + 4) + c, Sc + (size_t)(n0 + r) * P + c, true);
+        }
+        ft_commit();
+        // a lane a row: the stores of a warp hit 32 neighbouring places
+        for (int i = threadIdx.x; i < 2 * SD_CHUNK * 16; i += THREADS) {
+            const int r = i % SD_CHUNK, c = ((i / SD_CHUNK) % 16) * 4, which = i / (SD_CHUNK * 16);
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (r < n) v = *(const float4*)((which ? brow : crow) + (size_t)r * C + n0 + c);
+            float* dst = (which ? Bt : Ct) + c * SD_LD + r;
+            dst[0] = v.x; dst[SD_LD] = v.y; dst[2 * SD_LD] = v.z; dst[3 * SD_LD] = v.w;
+        }
+        ft_wait<0>();
+        __syncthreads();
+        if (busy) {
+            g.add(Ct, SD_LD, Bt, SD_LD, 64);
+            o.add(Ct, SD_LD, Ss, P + 4, 64);
+        }
+    }
+    __syncthreads();
+    // A over C, v over B
+    if (busy)
+#pragma unroll
+        for (int c = 0; c < GN; ++c)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int cj = g.col(c) + j;
+                float a[4];
+#pragma unroll
+                for (int i = 0; i < 4; ++i) {
+                    const int ri = 4 * g.ty + i;
+                    const float4 x = g.get(i, c);
+                    const float z = j == 0 ? x.x : j == 1 ? x.y : j == 2 ? x.z : x.w;
+                    a[i] = cj <= ri ? z * expf((float)(ls[ri] - ls[cj])) : 0.f;
+                }
+                *(float4*)(Ct + cj * SD_LD + 4 * g.ty) = make_float4(a[0], a[1], a[2], a[3]);
+            }
+    for (int i = threadIdx.x; i < SD_CHUNK * (P / 4); i += THREADS) {
+        const int r = i / (P / 4), c = (i % (P / 4)) * 4;
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (r < n) v = *(const float4*)(rows + (size_t)r * C + h * P + c);
+        const float w = ds[r];
+        *(float4*)(Bt + r * (P + 4) + c) = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+    }
+    __syncthreads();
+    if (!busy) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) o.scale_row(i, expf((float)ls[4 * o.ty + i]));
+    o.add(Ct, SD_LD, Bt, P + 4, min(n, 4 * (o.ty | (32 / TX - 1)) + 4));
+    const float Dh = D ? D[h] : 0.f;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        const int r = 4 * o.ty + i;
+        if (r >= n) break;
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+            const float4 x = *(const float4*)(rows + (size_t)r * C + h * P + o.col(c));
+            float4 v = o.get(i, c);
+            v.x = fmaf(Dh, x.x, v.x); v.y = fmaf(Dh, x.y, v.y); v.z = fmaf(Dh, x.z, v.z); v.w = fmaf(Dh, x.w, v.w);
+            *(float4*)(y + (size_t)(ch.x + r) * H * P + h * P + o.col(c)) = v;
+        }
+    }
+}
+
+TGO_API int tgo_ssd_chunk_tokens() { return SD_CHUNK; }
+// Floats of workspace for T tokens of B requests: a summary, the steps' sizes and logarithms, and
+// what each chunk is.
+TGO_API long long tgo_ssd_floats(int T, int B, int H, int N, int P) {
+    const long long chunks = T / SD_CHUNK + B;
+    return chunks * (H * ((long long)N * P + 3 * SD_CHUNK) + 4);
+}
+
+template <int N, int P>
+static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stride, const float* dt_bias, const float* A_log,
+                  const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
+                  float* state, long long state_stride, long long offset, float* ws, cudaStream_t stream) {
+    constexpr size_t s1 = (size_t)SD_CHUNK * (N + 4 + P + 4) * sizeof(float);
+    constexpr size_t vb = 64 * SD_LD > SD_CHUNK * (P + 4) ? 64 * SD_LD : SD_CHUNK * (P + 4);
+    constexpr size_t s3 = ((size_t)64 * SD_LD + vb + 64 * (P + 4)) * sizeof(float);
+    static bool sized[64] = {};                          // per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
+    if (!sized[dev]) {
+        if ((e = cudaFuncSetAttribute(ssd_summaries_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1)) != cudaSuccess) return (int)e;
+        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
+        sized[dev] = true;
+    }
+    const int n_chunks = T / SD_CHUNK + B;               // at least as many as there are
+    float* U = ws;
+    double* cum = (double*)(U + (size_t)n_chunks * H * N * P);
+    float* dts = (float*)(cum + (size_t)n_chunks * H * SD_CHUNK);
+    int4* chunks = (int4*)(dts + (size_t)n_chunks * H * SD_CHUNK);
+    int rc = tgo_launch_pdl(ssd_steps_kernel<bf16>, dim3(n_chunks, (H + 7) / 8), dim3(256), 0, stream, dt_raw, dt_stride, dt_bias,
+                            A_log, H, q_start, B, chunks, dts, cum);
+    if (rc) return rc;
+    rc = tgo_launch_pdl(ssd_summaries_kernel<N, P>, dim3(n_chunks, H), dim3(N * P / 64), s1, stream, xbc, C, H, G,
+                        (const int4*)chunks, (const float*)dts, (const double*)cum, U);
+    if (rc) return rc;
+    rc = tgo_launch_pdl(ssd_scan_kernel, dim3(B, H, (N * P / 4 + 255) / 256), dim3(256), 0, stream, H, N * P, q_start,
+                        state_slots, (const double*)cum, U, state, state_stride, offset);
+    if (rc) return rc;
+    return tgo_launch_pdl(ssd_outputs_kernel<N, P>, dim3(n_chunks, H), dim3(2 * P), s3, stream, xbc, C, H, G, D,
+                          (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+}
+
+// 1 if the chunked scan takes these sizes and places; bfloat16 engine only.
+TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, long long state_stride, long long offset, int H,
+                          int G, int N, int P) {
+    return H > 0 && H <= 65535 && G > 0 && H % G == 0 && (N == 64 || N == 128) && (P == 64 || P == 128) &&
+           (uintptr_t)xbc % 16 == 0 && (uintptr_t)y % 16 == 0 && (uintptr_t)state % 16 == 0 && state_stride % 4 == 0 &&
+           offset % 4 == 0;
+}
+
+// As tgo_selective_scan with dt_raw in bfloat16; ws: tgo_ssd_floats(T, B, H, N, P) floats, 16-byte aligned.
+TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long dt_stride, const float* dt_bias,
+                         const float* A_log, const float* D, float* y, int T, int B, int H, int G, int N, int P,
+                         const int* q_start, const int* state_slots, float* state, long long state_stride,
+                         long long ssm_offset, float* ws, cudaStream_t stream) {
+    if (B <= 0 || T <= 0) return 0;
+    if (!tgo_ssd_takes(xbc, y, state, state_stride, ssm_offset, H, G, N, P) || C != H * P + 2 * G * N ||
+        state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16)
+        return TGO_E_BAD_ARG;
+#define SD_GO(N, P)                                                                                                    \
+    return ssd_go<N, P>(xbc, C, (const bf16*)dt_raw, dt_stride, dt_bias, A_log, D, y, T, B, H, G, q_start, state_slots, state, \
+                        state_stride, ssm_offset, ws, stream)
+    if (N == 128) { if (P == 64) SD_GO(128, 64); SD_GO(128, 128); }
+    if (P == 64) SD_GO(64, 64);
+    SD_GO(64, 128);
+#undef SD_GO
 }
 
 // ---------------------------------------------------------------------- scan per channel

@@ -976,6 +976,14 @@ def causal_conv_act(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
         LAUNCHES[0] += 1
 
 
+# Steps of at least so many tokens, and so many a request on average, run the selective scan by
+# chunks in the bfloat16 engine (64 heads of 64 x 128, a call's wall time, walk against chunks: 64
+# tokens 28 against 36 us, 128 47 / 47, 256 90 / 60; 16 requests of 128 359 / 288; 256 tokens beside 31
+# single ones 198 / 226, 32 requests of 16 114 / 208: a chunk costs its two state-sized rows)
+SSD_MIN_TOKENS = 160
+SSD_TOKENS_A_REQUEST = 64
+
+
 def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[torch.Tensor],
                    a_log: torch.Tensor, d_skip: Optional[torch.Tensor], y: torch.Tensor,
                    num_seqs: int, heads: int, groups: int, state_dim: int, value_dim: int,
@@ -997,6 +1005,19 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
     assert q_start.dtype == state_slots.dtype == torch.int32
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
     lib = load_library("state_space")
+    if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and \
+            lib.tgo_ssd_takes(_ptr(xbc), _ptr(y), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(heads),
+                              c_int(groups), c_int(state_dim), c_int(value_dim)):
+        lib.tgo_ssd_floats.restype = c_ll
+        floats = lib.tgo_ssd_floats(c_int(T), c_int(num_seqs), c_int(heads), c_int(state_dim), c_int(value_dim))
+        ws = torch.empty(floats, dtype=torch.float32, device=xbc.device)
+        _check(lib.tgo_ssd_scan(
+            _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y),
+            c_int(T), c_int(num_seqs), c_int(heads), c_int(groups), c_int(state_dim), c_int(value_dim), _ptr(q_start),
+            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), _ptr(ws), _stream()), "ssd_scan",
+            f"(heads={heads}, groups={groups}, state={state_dim}, vdim={value_dim})")
+        LAUNCHES[0] += 3
+        return
     _check(lib.tgo_selective_scan(
         _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), c_int(dtype_code(dt_raw.dtype)),
         _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y), c_int(num_seqs), c_int(heads),
