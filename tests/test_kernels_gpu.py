@@ -1117,3 +1117,22 @@ def test_selective_scan_by_chunks(H, G, N, P, lens, monkeypatch):
     after = state.clone()
     after[slots, 8:8 + H * N * P] = before[slots, 8:8 + H * N * P]
     assert torch.equal(after, before)
+
+
+@pytest.mark.parametrize("n,groups", [(4, 3), (124, 2), (128, 16), (132, 1), (256, 5), (300, 2), (512, 8)])
+@pytest.mark.parametrize("act,first", [(None, False), ("silu", True), ("sigmoid", False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_group_norm_in_fours(n, groups, act, first, dtype):
+    """Groups read four channels at a time: whole and cut turns of 128, strided gates."""
+    T, W = 37, n * groups
+    o, gain = rnd(T, W, seed=n), rnd(W, seed=2)
+    gate = rnd(T, W + 8, seed=3).to(dtype)[:, 4:W + 4] if act else None
+    out = torch.empty(T, W, dtype=dtype, device=DEV)
+    ops().gated_group_norm(o, gate, gain, out, groups, 1e-5, act, first)
+    z = {None: 1.0, "silu": None, "sigmoid": None}[act]
+    if act:
+        z = gate.double() * torch.sigmoid(gate.double()) if act == "silu" else torch.sigmoid(gate.double())
+    x = o.double() * (z if first else 1.0)
+    want = (x.view(T, groups, n) * torch.rsqrt((x.view(T, groups, n) ** 2).mean(-1, keepdim=True) + 1e-5)).view(T, W)
+    want = want * gain.double() * (1.0 if first else z)
+    assert torch.allclose(out.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5, atol=1e-6)
