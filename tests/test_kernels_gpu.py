@@ -1136,3 +1136,32 @@ def test_gated_group_norm_in_fours(n, groups, act, first, dtype):
     want = (x.view(T, groups, n) * torch.rsqrt((x.view(T, groups, n) ** 2).mean(-1, keepdim=True) + 1e-5)).view(T, W)
     want = want * gain.double() * (1.0 if first else z)
     assert torch.allclose(out.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5, atol=1e-6)
+
+
+@pytest.mark.parametrize("H,dk,dv,ps", [(16, 576, 512, 16), (5, 576, 512, 8), (128, 264, 256, 64), (24, 200, 64, 32), (3, 448, 320, 128)])
+@pytest.mark.parametrize("window,sink", [(0, False), (130, True), (300, False)])
+def test_attention_latent_tc(H, dk, dv, ps, window, sink):
+    """One wide row a token whose first channels are the values, on tcgen05: tiles of one to 42 tokens,
+    one and two parts of the values, rows with a cut last block, pages inside and around a slot of 32
+    keys, NaN in what nobody may read; against the generic kernel's float32 arithmetic. P and the
+    result are rounded to bfloat16."""
+    o, scale = ops(), dk ** -0.5
+    assert o.attention_latent_tc_supports(H, dk, dv, ps)
+    case = paged_case([150, 1, 40, 261], [333, 500, 0, 7], H, 1, dk, ps, torch.bfloat16, seed=dk + ps)
+    if window:                                           # what lies before every window has gone back
+        for b, f in enumerate(case["firsts"]):
+            for i in range(max(0, f - window + 1) // ps):
+                case["bt"][b, i] = 0
+    sinks = rnd(H, seed=2) if sink else None
+    t0, nt = attention_part().step_tiles(Ctx(case, False), 128 // H)
+    T = case["q"].shape[0]
+    out = torch.full((T, H * dv), 9.0, dtype=torch.bfloat16, device=DEV)
+    o.attention_latent_tc(case["q"], out, H, dk, dv, case["kc"], ps, case["bt"], case["seq"], case["pos"], scale, window,
+                          sinks, t0, nt)
+    want = torch.empty(T, H * dv, device=DEV)
+    kc = case["kc"].float()
+    o.attention_generic(case["q"].float(), want, H, 1, dk, kc, kc, ps, case["bt"], case["seq"], case["pos"], scale, window,
+                        value_dim=dv, sinks=sinks, value_row=dk)
+    assert o.attention_latent_tc_error() == 0
+    assert bool(torch.isfinite(want).all())
+    assert torch.allclose(out.float(), want, **tol(torch.bfloat16))

@@ -136,23 +136,40 @@ __device__ __forceinline__ uint32_t tg_pack(float lo, float hi) {
 typedef CUresult (*TgEncodeFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-// The map of a bfloat16 matrix [rows, cols] whose rows lie `stride` elements apart, in boxes of
-// box_rows x 64 columns. False: the driver refused it.
-static inline bool tg_map(CUtensorMap* map, const void* ptr, long long rows, long long cols, long long stride, int box_rows) {
+static inline TgEncodeFn tg_encode() {
     static TgEncodeFn encode = nullptr;
     if (!encode) {
         void* p = nullptr;
         cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess)
-            return false;
-        encode = (TgEncodeFn)p;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) == cudaSuccess &&
+            q == cudaDriverEntryPointSuccess)
+            encode = (TgEncodeFn)p;
     }
+    return encode;
+}
+// The map of a bfloat16 matrix [rows, cols] whose rows lie `stride` elements apart, in boxes of
+// box_rows x 64 columns. False: the driver refused it.
+static inline bool tg_map(CUtensorMap* map, const void* ptr, long long rows, long long cols, long long stride, int box_rows) {
+    const TgEncodeFn encode = tg_encode();
+    if (!encode) return false;
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)stride * 2};
     const cuuint32_t box[2] = {64, (cuuint32_t)box_rows};
     const cuuint32_t elem[2] = {1, 1};
     return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, elem,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+// The map of query rows, `tokens` of them `stride` elements apart, H heads of `width` channels each: boxes
+// of 64 channels of all the heads of box_tokens tokens. Channels past a head's width are zeros.
+static inline bool tg_map_heads(CUtensorMap* map, const void* ptr, int tokens, int H, int width, long long stride, int box_tokens) {
+    const TgEncodeFn encode = tg_encode();
+    if (!encode) return false;
+    const cuuint64_t dims[3] = {(cuuint64_t)width, (cuuint64_t)H, (cuuint64_t)tokens};
+    const cuuint64_t strides[2] = {(cuuint64_t)width * 2, (cuuint64_t)stride * 2};
+    const cuuint32_t box[3] = {64, (cuuint32_t)H, (cuuint32_t)box_tokens};
+    const cuuint32_t elem[3] = {1, 1, 1};
+    return encode(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(ptr), dims, strides, box, elem,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }

@@ -41,6 +41,7 @@ LIBRARIES = {
     "moe": (["moe.cu"], []),
     "attention_flash": (["attention_flash.cu"], []),
     "attention_tc": (["attention_tc.cu"], []),
+    "attention_latent_tc": (["attention_latent_tc.cu"], []),
     "attention_decode_tma": (["attention_decode_tma.cu"], []),
     "sgemm": (["sgemm.cu"], []),
     "gemm_skinny": (["gemm_skinny.cu"], []),

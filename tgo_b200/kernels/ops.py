@@ -558,6 +558,42 @@ def attention_sink_wide(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_
         LAUNCHES[0] += 1
 
 
+def attention_latent_tc_supports(num_heads: int, key_dim: int, value_dim: int, page_size: int) -> bool:
+    """Whether the tcgen05 kernel for one wide row a token takes these sizes."""
+    return bool(load_library("attention_latent_tc").tgo_attention_latent_tc_supports(
+        c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(page_size)))
+
+
+def attention_latent_tc_error() -> int:
+    """The code a wait of that kernel left when it ran out, or 0. Synchronises."""
+    value = ctypes.c_int(0)
+    _check(load_library("attention_latent_tc").tgo_attention_latent_tc_error(ctypes.byref(value)),
+           "attention_latent_tc_error")
+    return int(value.value)
+
+
+def attention_latent_tc(q: torch.Tensor, out: torch.Tensor, num_heads: int, key_dim: int, value_dim: int,
+                        cache: torch.Tensor, page_size: int, block_tables: torch.Tensor, seq_ids: torch.Tensor,
+                        positions: torch.Tensor, scale: float, window: int, sinks: Optional[torch.Tensor],
+                        tile_tok0: torch.Tensor, tile_ntok: torch.Tensor) -> None:
+    """`attention_sink_wide` for prompt portions with one key/value head on the tcgen05 tensor cores:
+    tiles of 128 // num_heads consecutive tokens of one request; cache [pages, 1, page_size, key_dim]."""
+    _need_cuda(q, out, cache, block_tables, seq_ids, positions, sinks, tile_tok0, tile_ntok)
+    assert q.dtype == out.dtype == cache.dtype == torch.bfloat16
+    assert q.stride(1) == 1 and out.stride(1) == 1 and cache.is_contiguous()
+    assert cache.shape[1:] == (1, page_size, key_dim)
+    assert block_tables.is_contiguous() and block_tables.dtype == torch.int32 and block_tables.dim() == 2
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == num_heads)
+    assert tile_tok0.dtype == tile_ntok.dtype == torch.int32
+    _check(load_library("attention_latent_tc").tgo_attention_latent_tc(
+        _ptr(q), c_ll(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_ll(out.stride(0)), _ptr(cache),
+        c_int(cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
+        _ptr(seq_ids), _ptr(tile_tok0), _ptr(tile_ntok), c_int(tile_tok0.numel()), c_int(num_heads), c_int(key_dim),
+        c_int(value_dim), c_float(scale), c_int(window), _ptr(sinks),
+        _ptr(torch.empty(1, dtype=torch.int32, device=q.device)), _stream()), "attention_latent_tc",
+        f"(heads={num_heads}, dk={key_dim}, dv={value_dim})")
+
+
 GATE_ACTIVATIONS = {None: 0, "silu": 1, "sigmoid": 2}
 
 
@@ -2057,6 +2093,10 @@ def kernel_wait_errors() -> dict:
         code = attention_decode_tma_error()
         if code:
             out["attention_decode_tma"] = code
+    if "attention_latent_tc" in _loaded:
+        code = attention_latent_tc_error()
+        if code:
+            out["attention_latent_tc"] = code
     if "moe" in _loaded:
         code = moe_error()
         if code:

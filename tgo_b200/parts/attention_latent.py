@@ -133,13 +133,15 @@ class LatentAttention(Part):
         names = ["sgemm" if dtype == torch.float32 else "gemm_skinny", "elementwise", "layer_ops",
                  "latent", "attention_generic"]
         if dtype == torch.bfloat16:
-            names.append("attention_sink")
+            names += ["attention_sink", "attention_latent_tc"]
         return names
 
     def prepare_capture(self, ctx, cache) -> None:
         form, tokens = tile_form(self.H, 1, self.row, self.rank, self.row, ctx.act_dtype)
         if not ctx.decode_only and cache is not None and form is not None:
             step_tiles(ctx, tokens)
+            if form == "wide" and 0 < self.H <= 128:
+                step_tiles(ctx, 128 // self.H)
 
     def flops(self, extents, first_positions, writes_cache: bool = True) -> float:
         n, H, d = sum(extents), self.H, self.hidden

@@ -261,11 +261,15 @@ class SinkAttention(Part):
 USE_TILE_KERNELS = True
 
 
+# Steps whose longest context is shorter stay on the mma.sync tiles (2 tokens with bounded scores 27 us
+# a layer against 28; from 8 tokens on the tcgen05 kernel is ahead, 33 against 29).
+TC_CONTEXT = 8
+
+
 def tc_takes(out, H, Hkv, dk, dv, cache, scale, value_row) -> bool:
     """Whether a step with prompt portions runs on the tcgen05 kernel: keys and values of their
-    own planes, both 64 or 128 wide, groups and pages it knows, views it can read by TMA. It has no
-    size where the mma.sync tiles beat it among the steps measured (a layer over 2048 + 1536 tokens
-    of 16/4 heads of 128 with a window of 1024: 171 us against 499)."""
+    own planes, both 64 or 128 wide, groups and pages it knows, views it can read by TMA (a layer
+    over 2048 + 1536 tokens of 16/4 heads of 128 with a window of 1024: 171 us against 499)."""
     return value_row == 0 and dk == dv and dk in (64, 128) and scale > 0 and \
         ops.attention_tc_supports(dk, H // Hkv, cache.page_size) and \
         cache.k.is_contiguous() and cache.v.is_contiguous() and \
@@ -286,6 +290,18 @@ def tile_form(H, Hkv, dk, dv, value_row, dtype):
     return None, 0
 
 
+# Contexts up to this stay on the mma.sync tiles of wide rows (a layer over 2, 20 and 64 new tokens: 35,
+# 46 and 52 us against 41, 50 and 53; 200 tokens 77 against 64, 20 tokens after 1500 236 against 93).
+LATENT_TC_CONTEXT = 64
+
+
+def latent_tc_takes(out, H, Hkv, dk, dv, cache, scale) -> bool:
+    """Whether a step with prompt portions over wide rows runs on the tcgen05 kernel for them."""
+    return Hkv == 1 and scale > 0 and ops.attention_latent_tc_supports(H, dk, dv, cache.page_size) and \
+        cache.k.is_contiguous() and cache.k.data_ptr() % 16 == 0 and \
+        out.stride(0) % 8 == 0 and out.data_ptr() % 16 == 0
+
+
 def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, softcap=0.0,
                    value_row=0, keep_first=0, dist_bias=None, gate=None) -> None:
     """`keep_first`: the first keys of a request that stay visible beside the window; `dist_bias`
@@ -302,6 +318,13 @@ def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, sof
     form, tokens = tile_form(H, Hkv, dk, dv, value_row, q.dtype)
     if form == "wide" and (keep_first or dist_bias is not None or gate is not None):
         form = None                     # the kernel for wide rows knows none of them
+    if not ctx.decode_only and form == "wide" and not softcap and ctx.max_context > LATENT_TC_CONTEXT and \
+            ops.attention_sink_takes(q, out) and \
+            latent_tc_takes(out, H, Hkv, dk, dv, cache, scale):
+        tok0, ntok = step_tiles(ctx, 128 // H)
+        ops.attention_latent_tc(q, out, H, dk, dv, cache.k, cache.page_size, cache.block_tables, ctx.seq_ids,
+                                ctx.positions, scale, window, sinks, tok0, ntok)
+        return
     if form is not None and ops.attention_sink_takes(q, out):
         tok0, ntok = (None, None) if ctx.decode_only else step_tiles(ctx, tokens)
         if form == "wide":
@@ -313,7 +336,7 @@ def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, sof
                                     ctx.seq_ids, ctx.positions, scale, window, sinks, tok0, ntok,
                                     n_splits=splits, softcap=softcap)
             return
-        if not ctx.decode_only and tc_takes(out, H, Hkv, dk, dv, cache, scale, value_row):
+        if not ctx.decode_only and ctx.max_context >= TC_CONTEXT and tc_takes(out, H, Hkv, dk, dv, cache, scale, value_row):
             ops.attention_tc_prefill(q, out, H, Hkv, dk, cache.k, v_cache, cache.page_size, cache.block_tables,
                                      ctx.positions, ctx.seq_ids, tok0, ntok, scale, window, sinks, softcap,
                                      keep_first, dist_bias, gate, own_counters=True)
