@@ -1165,3 +1165,34 @@ def test_attention_latent_tc(H, dk, dv, ps, window, sink):
     assert o.attention_latent_tc_error() == 0
     assert bool(torch.isfinite(want).all())
     assert torch.allclose(out.float(), want, **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("H,Hkv,ps", [(16, 4, 16), (5, 1, 8), (12, 1, 32), (16, 2, 64)])
+@pytest.mark.parametrize("window,keep", [(0, 0), (130, 0), (140, 5), (300, 200)])
+@pytest.mark.parametrize("extra", ["sink", "cap", "bias", "all"])
+def test_attention_sink_decode_tma(H, Hkv, ps, window, keep, extra):
+    """Single tokens with a sink, kept first keys, bounded scores, a bias by distance and a gate, keys
+    whole and cut in shares (some empty), against the generic kernel's float32 arithmetic."""
+    dh, o = 128, ops()
+    case = paged_case([1, 1, 1, 1, 1], [0, 63, 64, 700, 333], H, Hkv, dh, ps, torch.bfloat16, seed=ps)
+    case["pos"][0] = -1                                   # a request that brings nothing
+    T = case["q"].shape[0]
+    if keep:                                              # what lies between has gone back
+        for b, f in enumerate(case["firsts"]):
+            for i in range(-(-keep // ps), max(0, f - window + 1) // ps):
+                case["bt"][b, i] = 0
+    kw = dict(softcap=2.0 if extra in ("cap", "all") else 0.0, keep_first=keep,
+              dist_bias=rnd(70, H, seed=1) if extra in ("bias", "all") else None,
+              gate=rnd(T, H, seed=3).to(torch.bfloat16) if extra == "all" else None)
+    sinks = rnd(H, seed=2) if extra in ("sink", "all") else None
+    want = torch.empty_like(case["q"].float())
+    kw32 = dict(kw, gate=kw["gate"].float() if kw["gate"] is not None else None)
+    o.attention_generic(case["q"].float(), want, H, Hkv, dh, case["kc"].float(), case["vc"].float(), ps, case["bt"],
+                        case["seq"], case["pos"], dh ** -0.5, window, sinks=sinks, **kw32)
+    assert bool(torch.isfinite(want).all())
+    for splits in (1, 3, 16):
+        out = torch.full_like(case["q"], 9.0)
+        o.attention_sink_decode_tma(case["q"], out, H, Hkv, dh, case["kc"], case["vc"], ps, case["bt"], case["seq"],
+                                    case["pos"], dh ** -0.5, window, sinks, splits, **kw)
+        assert o.attention_decode_tma_error() == 0
+        assert torch.allclose(out.float(), want, **tol(torch.bfloat16)), splits

@@ -19,6 +19,11 @@
 // that TMA brought (a stale row of the page). The arithmetic is that of
 // qk_norm_rope_cache_dh128_kernel, operation for operation, so both ways give the same bits.
 //
+// The EX instances serve the attention that has a sink, kept first keys, bounded scores, a bias by
+// distance or a gate (DtExtra). MEASURED (B200, a layer of 16/4 heads, its products among it; the
+// kernel of attention_sink.cu, whose blocks copy with cp.async, in brackets): 64 requests of about 2800
+// keys 96 us (182), of 850 43 us (76), 8 of 850 23 us (29), one of 100 17 us (21).
+//
 // Every mbarrier wait has a time limit (about two seconds), after which a flag is set and the
 // CTA runs to its end without waiting again.
 #include <cuda.h>
@@ -90,6 +95,37 @@ struct DtFuse {
     bf16* v_cache;
 };
 
+// What a call may ask beside plain windowed attention (the EX instances): exp(sink_h) in the
+// denominator, scores bounded by a soft cap c (cap_log2 = c log2 e, scale_over_cap = scale / c), first
+// keys seen beside the window, a bias by distance [n_dist][H], a logistic gate per head. Sink and gate
+// are applied here when the keys are not cut, else by the kernel that joins the shares.
+struct DtExtra {
+    const float* sinks;
+    float cap_log2, scale_over_cap;
+    int keep_first;
+    const float* dist_bias;
+    int n_dist;
+    const bf16* gate;
+    long long gate_stride;
+};
+
+// A raw product as the exponent in base 2: scaled, bounded (c tanh(x / c) by the hardware's
+// exponential and reciprocal), with the bias of its distance.
+__device__ __forceinline__ float dt_scored(float qk, float scale_log2, const DtExtra& ex, int dist, int head, int H) {
+    float sc = qk * scale_log2;
+    if (ex.cap_log2 > 0.f) {
+        float e, r;
+        asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(qk * (ex.scale_over_cap * 2.8853900817779268f)));
+        asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.f + e));
+        sc = fmaf(-2.f * ex.cap_log2, r, ex.cap_log2);
+    }
+    if (ex.dist_bias) {
+        const int d = dist < 0 ? 0 : dist < ex.n_dist ? dist : ex.n_dist - 1;        // below 0: masked
+        sc = fmaf(ex.dist_bias[(size_t)d * H + head], 1.4426950408889634f, sc);
+    }
+    return sc;
+}
+
 // One head vector of 128 channels by a warp, lane l holding channels 4l .. 4l+3: RMSNorm with
 // `gain` (if given), then the half-split rotation by the token's cosines and sines (if given),
 // the partner channel i +- 64 sitting 16 lanes away. Returns the four values as bfloat16.
@@ -124,7 +160,7 @@ __device__ __forceinline__ uint2 dt_norm_rope(const bf16* __restrict__ vec, cons
     return out;
 }
 
-template <bool KEYS_ON_M>
+template <bool KEYS_ON_M, bool EX>
 __global__ void __launch_bounds__(DT_THREADS, DT_MIN_BLOCKS)
 flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                         const bf16* __restrict__ q, long long q_stride, bf16* __restrict__ out,
@@ -133,7 +169,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                         const int* __restrict__ positions, const int* __restrict__ seq_ids, int H,
                         int Hkv, float scale_log2, int window, int n_splits,
                         float* __restrict__ part_o, float* __restrict__ part_ml,
-                        const int* __restrict__ tok_list, const DtFuse fz) {
+                        const int* __restrict__ tok_list, const DtFuse fz, const DtExtra ex) {
     constexpr int DH = DT_DH, KS = DH / 16, CH = DH / 8, LDQ = DH + 8;
     extern __shared__ unsigned char dt_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)dt_raw + 1023) & ~(uintptr_t)1023);
@@ -168,13 +204,20 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     const int key_lo = (window > 0 && p - window + 1 > 0) ? p - window + 1 : 0;
     const int key_hi = p + 1;
     const int t_first = key_lo / DT_BN, t_end = (key_hi + DT_BN - 1) / DT_BN;
-    int t_lo = t_first, t_hi = t_end;
+    // the walk: tiles of kept first keys that lie before the window (EX), then the window's; a CTA takes
+    // places [w_lo, w_hi) of it. t_lo, t_hi: the window tiles among them.
+    const int keep = EX ? ex.keep_first : 0;
+    int n_kept = (keep + DT_BN - 1) / DT_BN;
+    if (n_kept > t_first) n_kept = t_first;
+    int w_lo = 0, w_hi = n_kept + t_end - t_first;
     if (n_splits > 1) {
-        const int per = (t_end - t_first + n_splits - 1) / n_splits;
-        t_lo = t_first + split * per;
-        t_hi = t_lo + per < t_end ? t_lo + per : t_end;
+        const int per = (w_hi + n_splits - 1) / n_splits;
+        w_lo = split * per;
+        w_hi = w_lo + per < w_hi ? w_lo + per : w_hi;
     }
-    const int n_it = t_hi > t_lo ? t_hi - t_lo : 0;
+    const int n_it = w_hi > w_lo ? w_hi - w_lo : 0;
+    const int t_lo = t_first + (w_lo > n_kept ? w_lo - n_kept : 0), t_hi = t_first + (w_hi > n_kept ? w_hi - n_kept : 0);
+    auto tile_of = [&](int it) { return EX && w_lo + it < n_kept ? w_lo + it : t_first + w_lo + it - n_kept; };
     const int pages_per_tile = DT_BN >> page_shift;
     const int pg_lo = t_lo * pages_per_tile;
     {
@@ -245,15 +288,17 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 
     if (warp == 4) {
         // ------------------------------------------------------------- producer
-        auto page_of = [&](int pi) { return pi - pg_lo < DT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi]; };
+        auto page_of = [&](int pi) { return (!EX || pi >= pg_lo) && pi - pg_lo < DT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi]; };
         bool ok = true;
         for (int it = 0; it < n_it; ++it) {
             const int s = it % DT_STAGES;
             const uint32_t ph = (uint32_t)(it / DT_STAGES) & 1u;
-            const int j = t_lo + it;
+            const int j = tile_of(it);
             int first = j * pages_per_tile, last = first + pages_per_tile;      // pages with a readable key
-            while (first < last && (first + 1) * page_size <= key_lo) ++first;
-            while (last > first && (last - 1) * page_size >= key_hi) --last;
+            const int lo = EX && j * DT_BN < keep ? j * DT_BN : key_lo;
+            const int hi = EX && w_lo + it < n_kept && keep < key_hi ? keep : key_hi;
+            while (first < last && (first + 1) * page_size <= lo) ++first;
+            while (last > first && (last - 1) * page_size >= hi) --last;
             ok = __all_sync(0xffffffffu, ok && dt_wait(smem_u32(&bars[DT_STAGES + s]), ph ^ 1u));
             if (!ok) break;
             // K and V of a tile have a barrier each: Q K^T starts when K is there
@@ -305,7 +350,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         for (int it = 0; it < n_it; ++it) {
             const int s = it % DT_STAGES;
             const uint32_t ph = (uint32_t)(it / DT_STAGES) & 1u;
-            const int tile = t_lo + it;
+            const int tile = tile_of(it);
             if (ok) ok = dt_wait(smem_u32(&bars[s]), ph);           // K
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -323,11 +368,16 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 mma_bf16(sc, ka, qb[ks >> 1][(ks & 1) * 2], qb[ks >> 1][(ks & 1) * 2 + 1]);
             }
             const int key_a = my_key0 + g, key_b = key_a + 8;
-            const bool vis_a = key_a >= key_lo && key_a < key_hi, vis_b = key_b >= key_lo && key_b < key_hi;
-            sc[0] = (vis_a && q0_ok) ? sc[0] * scale_log2 : -INFINITY;
-            sc[1] = (vis_a && q1_ok) ? sc[1] * scale_log2 : -INFINITY;
-            sc[2] = (vis_b && q0_ok) ? sc[2] * scale_log2 : -INFINITY;
-            sc[3] = (vis_b && q1_ok) ? sc[3] * scale_log2 : -INFINITY;
+            const bool vis_a = (key_a >= key_lo || (EX && key_a < keep)) && key_a < key_hi;
+            const bool vis_b = (key_b >= key_lo || (EX && key_b < keep)) && key_b < key_hi;
+            auto scored = [&](float v, int key, int r) {
+                if constexpr (EX) return dt_scored(v, scale_log2, ex, p - key, kvh * G + r, H);
+                else return v * scale_log2;
+            };
+            sc[0] = (vis_a && q0_ok) ? scored(sc[0], key_a, 2 * t) : -INFINITY;
+            sc[1] = (vis_a && q1_ok) ? scored(sc[1], key_a, 2 * t + 1) : -INFINITY;
+            sc[2] = (vis_b && q0_ok) ? scored(sc[2], key_b, 2 * t) : -INFINITY;
+            sc[3] = (vis_b && q1_ok) ? scored(sc[3], key_b, 2 * t + 1) : -INFINITY;
             float mx0 = fmaxf(sc[0], sc[2]), mx1 = fmaxf(sc[1], sc[3]);
 #pragma unroll
             for (int off = 4; off <= 16; off <<= 1) {             // over the keys: lanes of equal t
@@ -351,7 +401,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 for (int i = lane; i < 16 * 16; i += 32) {
                     const int r = i >> 4, c = i & 15;
                     const int key = my_key0 + r;
-                    if (key >= key_hi || key < key_lo)
+                    if (key >= key_hi || (key < key_lo && (!EX || key >= keep)))
                         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(vt + dt_at(warp * 16 + r, c)), "r"(0u) : "memory");
                 }
                 __syncwarp();
@@ -387,7 +437,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         for (int it = 0; it < n_it; ++it) {
             const int s = it % DT_STAGES;
             const uint32_t ph = (uint32_t)(it / DT_STAGES) & 1u;
-            const int t = t_lo + it;
+            const int t = tile_of(it);
             if (ok) ok = dt_wait(smem_u32(&bars[s]), ph) && dt_wait(smem_u32(&bars[2 * DT_STAGES + s]), ph);
             ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
@@ -403,7 +453,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
                 for (int i = lane; i < 16 * 16; i += 32) {
                     const int r = i >> 4, c = i & 15;
                     const int key = my_key0 + r;
-                    if (key >= key_hi || key < key_lo)
+                    if (key >= key_hi || (key < key_lo && (!EX || key >= keep)))
                         asm volatile("st.shared.v4.u32 [%0], {%1, %1, %1, %1};" ::"r"(vt + dt_at(warp * 16 + r, c)), "r"(0u) : "memory");
                 }
                 __syncwarp();
@@ -427,9 +477,13 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
 #pragma unroll
                 for (int e = 0; e < 2; ++e) {
                     const int j = kbase + i * 8 + e;
-                    const bool vis = j >= key_lo && j < key_hi;
-                    sc[i][e] = (vis && row_lo_ok) ? sc[i][e] * scale_log2 : -INFINITY;
-                    sc[i][2 + e] = (vis && row_hi_ok) ? sc[i][2 + e] * scale_log2 : -INFINITY;
+                    const bool vis = (j >= key_lo || (EX && j < keep)) && j < key_hi;
+                    auto scored = [&](float v, int r) {
+                        if constexpr (EX) return dt_scored(v, scale_log2, ex, p - j, kvh * G + r, H);
+                        else return v * scale_log2;
+                    };
+                    sc[i][e] = (vis && row_lo_ok) ? scored(sc[i][e], r_lo) : -INFINITY;
+                    sc[i][2 + e] = (vis && row_hi_ok) ? scored(sc[i][2 + e], r_hi) : -INFINITY;
                     mx_lo = fmaxf(mx_lo, sc[i][e]);
                     mx_hi = fmaxf(mx_hi, sc[i][2 + e]);
                 }
@@ -540,7 +594,16 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
         }
         const int head = kvh * G + r;
         if (n_splits == 1) {
-            out[(size_t)tok * out_stride + (size_t)head * DH + d] = __float2bfloat16_rn(l > 0.f ? acc / l : 0.f);
+            float f = 1.f;
+            if constexpr (EX) {
+                if (ex.sinks) {                // the sink joins the denominator last
+                    const float sk = ex.sinks[head] * 1.4426950408889634f, mn = fmaxf(m, sk);
+                    f = exp2f(m - mn);
+                    l = l * f + exp2f(sk - mn);
+                }
+                if (ex.gate) f *= 1.f / (1.f + __expf(-__bfloat162float(ex.gate[(size_t)tok * ex.gate_stride + head])));
+            }
+            out[(size_t)tok * out_stride + (size_t)head * DH + d] = __float2bfloat16_rn(l > 0.f ? (EX ? acc * f : acc) / l : 0.f);
         } else {
             const size_t at = ((size_t)slot * H + head) * n_splits + split;
             part_o[at * DH + d] = acc;
@@ -607,7 +670,7 @@ static int dt_launch(const void* q, long long q_stride, void* out, long long out
                      const int* block_tables, int max_blocks, const int* positions,
                      const int* seq_ids, int T, int H, int Hkv, int dh, float scale,
                      int window, int n_splits, float* part_o, float* part_ml,
-                     const int* tok_list, const DtFuse& fz, cudaStream_t stream) {
+                     const int* tok_list, const DtFuse& fz, const DtExtra* ex, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (H <= 0 || Hkv <= 0 || H % Hkv || !tgo_attention_decode_tma_supports(dh, H / Hkv, page_size) ||
         n_pages <= 0 || max_blocks <= 0 || window < 0 || n_splits < 1 || n_splits > 65535 || Hkv > 65535 ||
@@ -623,25 +686,25 @@ static int dt_launch(const void* q, long long q_stride, void* out, long long out
     static_assert(ring >= (size_t)4 * 16 * DT_DH * sizeof(float), "the join of the four warps reuses the ring");
     constexpr size_t smem = 1024 + ring + 3 * DT_STAGES * 8 + 16 * (DT_DH + 8) * sizeof(bf16) +
                             4 * 16 * 2 * sizeof(float) + DT_PAGES_CAP * sizeof(int);
-    static bool once = false;
-    if (!once) {
-        cudaError_t e = cudaFuncSetAttribute(flash_decode_tma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e == cudaSuccess)
-            e = cudaFuncSetAttribute(flash_decode_tma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return (int)e;
-        once = true;
+    static bool once[64] = {};                 // per device
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
+    if (!once[dev]) {
+        for (auto kern : {flash_decode_tma_kernel<true, false>, flash_decode_tma_kernel<false, false>,
+                          flash_decode_tma_kernel<true, true>, flash_decode_tma_kernel<false, true>})
+            if ((e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)) != cudaSuccess) return (int)e;
+        once[dev] = true;
     }
     int shift = 0;
     while ((1 << shift) < page_size) ++shift;
-    if (H / Hkv <= DT_KEYS_ON_M_MAX_GROUP)
-        return tgo_launch_pdl(flash_decode_tma_kernel<true>, dim3(T, Hkv, n_splits), dim3(DT_THREADS), smem, stream,
-                              *mk, *mv, (const bf16*)q, q_stride, (bf16*)out, out_stride, page_size, shift,
-                              block_tables, max_blocks, positions, seq_ids, H, Hkv, scale * 1.4426950408889634f,
-                              window, n_splits, part_o, part_ml, tok_list, fz);
-    return tgo_launch_pdl(flash_decode_tma_kernel<false>, dim3(T, Hkv, n_splits), dim3(DT_THREADS), smem, stream,
-                          *mk, *mv, (const bf16*)q, q_stride, (bf16*)out, out_stride, page_size, shift,
-                          block_tables, max_blocks, positions, seq_ids, H, Hkv, scale * 1.4426950408889634f,
-                          window, n_splits, part_o, part_ml, tok_list, fz);
+    const bool on_m = H / Hkv <= DT_KEYS_ON_M_MAX_GROUP;
+    auto kern = ex ? (on_m ? flash_decode_tma_kernel<true, true> : flash_decode_tma_kernel<false, true>)
+                   : (on_m ? flash_decode_tma_kernel<true, false> : flash_decode_tma_kernel<false, false>);
+    return tgo_launch_pdl(kern, dim3(T, Hkv, n_splits), dim3(DT_THREADS), smem, stream, *mk, *mv, (const bf16*)q, q_stride,
+                          (bf16*)out, out_stride, page_size, shift, block_tables, max_blocks, positions, seq_ids, H, Hkv,
+                          scale * 1.4426950408889634f, window, n_splits, part_o, part_ml, tok_list, fz, ex ? *ex : DtExtra{});
 }
 
 TGO_API int tgo_attention_decode_tma(const void* q, long long q_stride, void* out, long long out_stride,
@@ -653,7 +716,33 @@ TGO_API int tgo_attention_decode_tma(const void* q, long long q_stride, void* ou
     DtFuse none = {};
     return dt_launch(q, q_stride, out, out_stride, k_cache, v_cache, n_pages, page_size, block_tables,
                      max_blocks, positions, seq_ids, T, H, Hkv, dh, scale, window, n_splits, part_o,
-                     part_ml, tok_list, none, stream);
+                     part_ml, tok_list, none, nullptr, stream);
+}
+
+// The form with a sink, a soft cap (0: none), first keys kept beside a window, a bias by distance and a
+// gate per head (DtExtra): every token of the step. With n_splits > 1 the shares are left in part_o and
+// part_ml for the join that applies the sink and the gate.
+TGO_API int tgo_attention_decode_tma_extra(const void* q, long long q_stride, void* out, long long out_stride,
+                                           const void* k_cache, const void* v_cache, int n_pages, int page_size,
+                                           const int* block_tables, int max_blocks, const int* positions,
+                                           const int* seq_ids, int T, int H, int Hkv, int dh, float scale, int window,
+                                           int n_splits, float* part_o, float* part_ml, const float* sinks, float softcap,
+                                           int keep_first, const float* dist_bias, int n_dist, const void* gate,
+                                           long long gate_stride, cudaStream_t stream) {
+    if (!(softcap >= 0.f) || keep_first < 0 || (dist_bias && n_dist <= 0)) return TGO_E_BAD_ARG;
+    DtFuse none = {};
+    DtExtra ex = {};
+    ex.sinks = sinks;
+    ex.cap_log2 = softcap * 1.4426950408889634f;
+    ex.scale_over_cap = softcap > 0.f ? scale / softcap : 0.f;
+    ex.keep_first = window > 0 ? keep_first : 0;
+    ex.dist_bias = dist_bias;
+    ex.n_dist = n_dist;
+    ex.gate = (const bf16*)gate;
+    ex.gate_stride = gate_stride;
+    return dt_launch(q, q_stride, out, out_stride, k_cache, v_cache, n_pages, page_size, block_tables,
+                     max_blocks, positions, seq_ids, T, H, Hkv, dh, scale, window, n_splits, part_o,
+                     part_ml, nullptr, none, &ex, stream);
 }
 
 // The fused form: q holds the raw query rows of the step's T tokens (every token, no list);
@@ -682,5 +771,5 @@ TGO_API int tgo_attention_decode_tma_fused(const void* q, long long q_stride, vo
     fz.k_cache = (bf16*)k_cache; fz.v_cache = (bf16*)v_cache;
     return dt_launch(q, q_stride, out, out_stride, k_cache, v_cache, n_pages, page_size, block_tables,
                      max_blocks, positions, seq_ids, T, H, Hkv, dh, scale, window, n_splits, part_o,
-                     part_ml, nullptr, fz, stream);
+                     part_ml, nullptr, fz, nullptr, stream);
 }

@@ -1093,6 +1093,17 @@ attention_sink_join_kernel(const float* __restrict__ part_o, const float* __rest
     }
 }
 
+// The shares that a step of single tokens left in part_o [T, H, n_splits, dv] and part_ml [T, H, n_splits, 2]
+// joined, with the sink and the gate.
+TGO_API int tgo_attention_sink_join(const float* part_o, const float* part_ml, const int* positions, const float* sinks,
+                                    void* out, long long out_stride, int T, int H, int dv, int n_splits, const void* gate,
+                                    long long gate_stride, cudaStream_t stream) {
+    if (T <= 0) return 0;
+    if (H <= 0 || H > 65535 || dv <= 0 || n_splits < 1 || !part_o || !part_ml) return TGO_E_BAD_ARG;
+    return tgo_launch_pdl(attention_sink_join_kernel, dim3(T, H), dim3(128), 0, stream, part_o, part_ml, positions, sinks,
+                          (bf16*)out, out_stride, H, dv, n_splits, (const bf16*)gate, gate_stride);
+}
+
 TGO_API int tgo_attention_sink_supports(int H, int Hkv, int dk, int dv) {
     return (H > 0 && Hkv > 0 && H % Hkv == 0 && H / Hkv <= AS_BM && dk > 0 && dv > 0 && dk % 8 == 0 &&
             dv % 8 == 0 && dk <= 128 && dv <= 128) ? 1 : 0;

@@ -558,6 +558,44 @@ def attention_sink_wide(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_
         LAUNCHES[0] += 1
 
 
+def attention_sink_decode_tma(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_heads: int, head_dim: int,
+                              k_cache: torch.Tensor, v_cache: torch.Tensor, page_size: int, block_tables: torch.Tensor,
+                              seq_ids: torch.Tensor, positions: torch.Tensor, scale: float, window: int,
+                              sinks: Optional[torch.Tensor], n_splits: int = 1, softcap: float = 0.0, keep_first: int = 0,
+                              dist_bias: Optional[torch.Tensor] = None, gate: Optional[torch.Tensor] = None) -> None:
+    """`attention_sink_tile` for a step of single tokens with keys and values of 128 in planes of their
+    own: the pages come in by TMA."""
+    _need_cuda(q, out, k_cache, v_cache, block_tables, seq_ids, positions, sinks, dist_bias, gate)
+    T = q.shape[0]
+    assert q.dtype == out.dtype == k_cache.dtype == v_cache.dtype == torch.bfloat16
+    assert q.stride(1) == 1 and out.stride(1) == 1 and k_cache.is_contiguous() and v_cache.is_contiguous()
+    assert k_cache.shape == v_cache.shape and k_cache.shape[1:] == (num_kv_heads, page_size, head_dim)
+    assert block_tables.dtype == torch.int32 and block_tables.is_contiguous() and block_tables.dim() == 2
+    assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == num_heads and sinks.is_contiguous())
+    assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.dim() == 2 and
+                                 dist_bias.shape[1] == num_heads and dist_bias.is_contiguous())
+    assert gate is None or (gate.dtype == q.dtype and gate.shape == (T, num_heads) and
+                            (gate.stride(1) == 1 or num_heads == 1))
+    part_o = part_ml = None
+    if n_splits > 1:
+        part_o = torch.empty((T, num_heads, n_splits, head_dim), dtype=torch.float32, device=q.device)
+        part_ml = torch.empty((T, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
+    gate_stride = c_ll(gate.stride(0) if gate is not None else 0)
+    _check(load_library("attention_decode_tma").tgo_attention_decode_tma_extra(
+        _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
+        c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
+        _ptr(seq_ids), c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_float(scale), c_int(window),
+        c_int(n_splits), _ptr(part_o), _ptr(part_ml), _ptr(sinks), c_float(softcap or 0.0), c_int(keep_first),
+        _ptr(dist_bias), c_int(dist_bias.shape[0] if dist_bias is not None else 0), _ptr(gate), gate_stride,
+        _stream()), "attention_decode_tma_extra",
+        f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads}, page_size={page_size})")
+    if n_splits > 1:
+        _check(load_library("attention_sink").tgo_attention_sink_join(
+            _ptr(part_o), _ptr(part_ml), _ptr(positions), _ptr(sinks), _ptr(out), c_ll(out.stride(0)), c_int(T),
+            c_int(num_heads), c_int(head_dim), c_int(n_splits), _ptr(gate), gate_stride, _stream()),
+            "attention_sink_join")
+
+
 def attention_latent_tc_supports(num_heads: int, key_dim: int, value_dim: int, page_size: int) -> bool:
     """Whether the tcgen05 kernel for one wide row a token takes these sizes."""
     return bool(load_library("attention_latent_tc").tgo_attention_latent_tc_supports(

@@ -196,7 +196,7 @@ class SinkAttention(Part):
         if dtype == torch.bfloat16:
             names.append("attention_sink")
             if self.dk == self.dv and self.dk in (64, 128):
-                names.append("attention_tc")
+                names += ["attention_tc"] + (["attention_decode_tma"] if self.dk == 128 else [])
         return names
 
     def prepare_capture(self, ctx, cache) -> None:
@@ -290,6 +290,13 @@ def tile_form(H, Hkv, dk, dv, value_row, dtype):
     return None, 0
 
 
+def decode_tma_takes(H, Hkv, dk, dv, cache, value_row) -> bool:
+    """Whether a step of single tokens runs on the decode kernel whose pages come in by TMA."""
+    return value_row == 0 and dk == dv and ops.attention_decode_tma_supports(dk, H // Hkv, cache.page_size) and \
+        cache.k.is_contiguous() and cache.v.is_contiguous() and \
+        cache.k.data_ptr() % 128 == 0 and cache.v.data_ptr() % 128 == 0
+
+
 # Contexts up to this stay on the mma.sync tiles of wide rows (a layer over 2, 20 and 64 new tokens: 35,
 # 46 and 52 us against 41, 50 and 53; 200 tokens 77 against 64, 20 tokens after 1500 236 against 93).
 LATENT_TC_CONTEXT = 64
@@ -342,6 +349,11 @@ def sink_attention(q, out, H, Hkv, dk, dv, cache, ctx, scale, window, sinks, sof
                                      keep_first, dist_bias, gate, own_counters=True)
             return
         splits = decode_splits(ctx, Hkv, window, q.device) if ctx.decode_only else 1
+        if ctx.decode_only and decode_tma_takes(H, Hkv, dk, dv, cache, value_row):
+            ops.attention_sink_decode_tma(q, out, H, Hkv, dk, cache.k, v_cache, cache.page_size, cache.block_tables,
+                                          ctx.seq_ids, ctx.positions, scale, window, sinks, splits, softcap, keep_first,
+                                          dist_bias, gate)
+            return
         ops.attention_sink_tile(q, out, H, Hkv, dk, dv, cache.k, v_cache, cache.page_size,
                                 cache.block_tables, ctx.seq_ids, ctx.positions, scale, window, sinks,
                                 tok0, ntok, n_splits=splits, softcap=softcap, value_row=value_row,
