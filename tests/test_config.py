@@ -136,3 +136,37 @@ def test_build_folder_is_one_for_all_threads():
     # and the host library, which needs no CUDA compiler, builds and loads
     lib = kb.load_library("host_runtime")
     assert lib.tgo_cache_create
+
+
+def test_entry_points_hand_over_what_ctypes_does(tmp_path):
+    """Whole numbers of every width, singles and doubles in any order and number, against ctypes."""
+    import ctypes
+    import subprocess
+
+    from tgo_b200.kernels import build as kb
+    if kb.find_host_compiler() is None:
+        pytest.skip("no host compiler")
+    src = tmp_path / "probe.cpp"
+    src.write_text("""
+extern "C" int many(int a, float b, long long c, double d, const void* e, short f, int g, int h, float i, long long j,
+                    int k, int l, int m, int n, float o, const void* p) {
+    return (a == -1) + 2 * (b == 0.1f) + 4 * (c == -(1ll << 40)) + 8 * (d == 0.1) + 16 * (e == (void*)0xffff800000000010ull) +
+           32 * (f == -7) + 64 * (g == 5) + 128 * (h == 1) + 256 * (i == -2.5f) + 512 * (j == (1ll << 62)) + 1024 * (k == 0) +
+           2048 * (l == 11) + 4096 * (m == 12) + 8192 * (n == -13) + 16384 * (o == 3.0f) + 32768 * (p == 0);
+}
+extern "C" int negative() { return -3; }
+""")
+    so = tmp_path / "probe.so"
+    subprocess.run([kb.find_host_compiler(), "-shared", "-fPIC", "-o", str(so), str(src)], check=True)
+    lib = ctypes.CDLL(str(so))
+    args = (-1, 0.1, -(1 << 40), (0.1,), 0xffff800000000010, -7, 5, True, -2.5, 1 << 62, 0, 11, 12, -13, 3.0, 0)
+    for bind in (kb._find_binder(), kb._bind_ctypes):
+        entries = kb._Entries(lib, bind)
+        assert entries.many(*args) == 65535 and entries.negative() == -3
+    fast = kb._Entries(lib, kb._find_binder()).many
+    if kb._find_binder() is not kb._bind_ctypes:
+        for bad in ("x", None, b"y", (1.0, 2.0), 1 << 70):
+            with pytest.raises((TypeError, OverflowError)):
+                fast(bad)
+        with pytest.raises(TypeError):
+            fast(*([0] * 49))

@@ -684,13 +684,6 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const flo
 }
 
 TGO_API int tgo_ssd_chunk_tokens() { return SD_CHUNK; }
-// Floats of workspace for T tokens of B requests: a summary, the steps' sizes and logarithms, and
-// what each chunk is.
-TGO_API long long tgo_ssd_floats(int T, int B, int H, int N, int P) {
-    const long long chunks = T / SD_CHUNK + B;
-    return chunks * (H * ((long long)N * P + 3 * SD_CHUNK) + 4);
-}
-
 template <int N, int P>
 static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stride, const float* dt_bias, const float* A_log,
                   const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
@@ -726,7 +719,7 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
                           (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
 }
 
-// 1 if the chunked scan takes these sizes and places; bfloat16 engine only.
+// 1 if the chunked scan takes these sizes and places (places as addresses); bfloat16 engine only.
 TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, long long state_stride, long long offset, int H,
                           int G, int N, int P) {
     return H > 0 && H <= 65535 && G > 0 && H % G == 0 && (N == 64 || N == 128) && (P == 64 || P == 128) &&
@@ -734,7 +727,9 @@ TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, lon
            offset % 4 == 0;
 }
 
-// As tgo_selective_scan with dt_raw in bfloat16; ws: tgo_ssd_floats(T, B, H, N, P) floats, 16-byte aligned.
+// As tgo_selective_scan with dt_raw in bfloat16; ws: (T / tgo_ssd_chunk_tokens() + B) times (H (N P + 3
+// tgo_ssd_chunk_tokens()) + 4) floats, 16-byte aligned: a summary, the steps' sizes and logarithms, and
+// what each chunk is.
 TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long dt_stride, const float* dt_bias,
                          const float* A_log, const float* D, float* y, int T, int B, int H, int G, int N, int P,
                          const int* q_start, const int* state_slots, float* state, long long state_stride,

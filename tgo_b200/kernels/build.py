@@ -17,6 +17,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 import tempfile
 import threading
 import time
@@ -49,8 +50,11 @@ LIBRARIES = {
     "sampling": (["sampling.cu"], []),
     # host code only (no kernel): the cache books and the packing of a step
     "host_runtime": (["host_runtime.cpp"], []),
+    # calls of the other libraries' entry points (a Python extension; see `entry_points`)
+    "fastcall": (["fastcall.cpp"], []),
 }
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
+PYTHON_INCLUDE = sysconfig.get_paths()["include"]
 
 _loaded = {}
 _lock = threading.Lock()
@@ -147,12 +151,12 @@ def compile_library(name: str, verbose: bool = True, ptxas_info: bool = False) -
     host_only = all(src.endswith(".cpp") for src in sources)
     cxx = find_host_compiler() if host_only else None
     if cxx:
-        cmd = [cxx] + HOST_FLAGS + ["-I", CSRC, "-o", tmp] + \
+        cmd = [cxx] + HOST_FLAGS + ["-I", CSRC, "-I", PYTHON_INCLUDE, "-o", tmp] + \
             [os.path.join(CSRC, s) for s in sources] + list(link_flags)
     else:
         nvcc = find_nvcc()
         cmd = [nvcc] + ARCH_FLAGS + NVCC_FLAGS + (["-Xptxas", "-v"] if ptxas_info else []) + \
-            ["-I", CSRC, "-o", tmp] + [os.path.join(CSRC, s) for s in sources] + list(link_flags)
+            ["-I", CSRC, "-I", PYTHON_INCLUDE, "-o", tmp] + [os.path.join(CSRC, s) for s in sources] + list(link_flags)
     if verbose:
         _say(f"[tgo_b200] compiling {name} ({', '.join(sources)})"
              f"{' for the host' if host_only else ' for sm_100a'} ...")
@@ -204,6 +208,58 @@ def load_library(name: str) -> ctypes.CDLL:
                 raise KernelBuildError(f"{path} was built and does not load: {e}") from None
             _loaded[name] = lib
     return lib
+
+
+class _Entries:
+    """The C entry points of a library, each bound when it is first asked for."""
+
+    def __init__(self, lib: ctypes.CDLL, bind):
+        self._lib, self._bind = lib, bind
+
+    def __getattr__(self, name: str):
+        fn = self._bind(getattr(self._lib, name))
+        setattr(self, name, fn)
+        return fn
+
+
+def _bind_ctypes(fn):
+    """Where the Python headers or the calling convention are missing: the same calls by ctypes."""
+    def call(*args):
+        return fn(*[ctypes.c_float(a) if isinstance(a, float) else ctypes.c_double(a[0]) if isinstance(a, tuple)
+                    else ctypes.c_longlong(a if a < 1 << 63 else a - (1 << 64)) for a in args])
+    return call
+
+
+_binder = None
+_entries = {}
+
+
+def _find_binder():
+    import platform
+    if platform.machine() != "x86_64" or not sys.platform.startswith("linux") or \
+            not os.path.exists(os.path.join(PYTHON_INCLUDE, "Python.h")):
+        return _bind_ctypes
+    import importlib.machinery
+    import importlib.util
+    path = compile_library("fastcall")
+    loader = importlib.machinery.ExtensionFileLoader("tgo_fastcall", path)
+    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("tgo_fastcall", loader))
+    loader.exec_module(module)
+    return lambda fn: module.bind(ctypes.cast(fn, ctypes.c_void_p).value)
+
+
+def entry_points(name: str):
+    """The library's entry points as callables that take plain numbers (whole numbers and addresses,
+    floats for single precision, a one-element tuple for a double) and return the function's int."""
+    global _binder
+    got = _entries.get(name)
+    if got is None:
+        lib = load_library(name)
+        with _lock:
+            if _binder is None:
+                _binder = _find_binder()
+            got = _entries.setdefault(name, _Entries(lib, _binder))
+    return got
 
 
 def compile_together(names, verbose: bool = True) -> None:

@@ -7,17 +7,21 @@ nothing falls back to it. A refused size raises with the kernel's name in the me
 from __future__ import annotations
 
 import ctypes
+from operator import index
 from typing import Optional
 
 import torch
 
-from .build import load_library
+from .build import entry_points, load_library
 
 F32, BF16 = 0, 1
 _CODES = {torch.float32: F32, torch.bfloat16: BF16}
 E_BAD_ARG = 1000
 
-c_int, c_ll, c_float, c_void = ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctypes.c_void_p
+# What an entry point is handed (`entry_points`): whole numbers as they are (anything else refused),
+# single-precision numbers as floats, addresses as whole numbers.
+c_int = c_ll = index
+c_float = float
 
 
 class KernelError(RuntimeError):
@@ -32,11 +36,11 @@ def dtype_code(dt: torch.dtype) -> int:
 
 
 def _ptr(t: Optional[torch.Tensor]):
-    return c_void(0) if t is None else c_void(t.data_ptr())
+    return 0 if t is None else t.data_ptr()
 
 
 def _stream():
-    return c_void(torch.cuda.current_stream().cuda_stream)
+    return torch._C._cuda_getCurrentRawStream(torch._C._cuda_getDevice())
 
 
 def _need_cuda(*tensors) -> None:
@@ -63,7 +67,7 @@ def embed(table: torch.Tensor, ids: torch.Tensor, out: torch.Tensor, scale: floa
     _need_cuda(table, ids, out)
     T, d = out.shape
     assert ids.dtype == torch.int32 and out.dtype == torch.float32 and table.is_contiguous()
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_embed(_ptr(table), c_int(dtype_code(table.dtype)), _ptr(ids), _ptr(out),
                          c_int(T), c_int(d), c_int(table.shape[0]), c_float(scale), _stream()), "embed")
 
@@ -76,7 +80,7 @@ def embed_rmsnorm(table: torch.Tensor, ids: torch.Tensor, gain: torch.Tensor, ep
     assert ids.dtype == torch.int32 and ids.numel() == T and table.is_contiguous() and table.shape[1] == d
     assert out.dtype == gain.dtype == torch.float32 and out.is_contiguous() and gain.numel() == d
     assert copy is None or (copy.dtype == torch.float32 and copy.shape == out.shape and copy.is_contiguous())
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_embed_rmsnorm(_ptr(table), c_int(dtype_code(table.dtype)), _ptr(ids), _ptr(gain),
                                  c_float(eps), _ptr(out), _ptr(copy), c_int(T), c_int(d),
                                  c_int(table.shape[0]), c_float(scale), _stream()), "embed_rmsnorm")
@@ -96,7 +100,7 @@ def add_rmsnorm(h: torch.Tensor, delta: Optional[torch.Tensor], gain: torch.Tens
         assert rows.dtype == torch.int32 and rows.numel() == n
     else:
         assert h.shape[0] == n
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_add_rmsnorm(_ptr(h), _ptr(delta),
                                c_int(dtype_code(delta.dtype) if delta is not None else 0),
                                _ptr(gain), c_float(eps), _ptr(out), c_int(dtype_code(out.dtype)),
@@ -119,7 +123,7 @@ def add_layernorm(h: torch.Tensor, delta: Optional[torch.Tensor], gain: torch.Te
         assert rows.dtype == torch.int32 and rows.numel() == n
     else:
         assert h.shape[0] == n
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_add_layernorm(_ptr(h), _ptr(delta),
                                  c_int(dtype_code(delta.dtype) if delta is not None else 0),
                                  _ptr(gain), _ptr(bias), c_float(eps), _ptr(out),
@@ -132,7 +136,7 @@ def residual_add(h: torch.Tensor, delta: torch.Tensor) -> None:
     _need_cuda(h, delta)
     assert h.dtype == torch.float32 and h.is_contiguous() and delta.is_contiguous()
     assert h.shape == delta.shape
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_residual_add(_ptr(h), _ptr(delta), c_int(dtype_code(delta.dtype)),
                                 c_ll(h.numel()), _stream()), "residual_add")
 
@@ -144,7 +148,7 @@ def swiglu(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool = False) 
     T, f = out.shape
     assert gate_up.shape == (T, 2 * f) and gate_up.is_contiguous() and out.is_contiguous()
     assert gate_up.dtype == out.dtype
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_swiglu(_ptr(gate_up), _ptr(out), c_int(dtype_code(out.dtype)), c_int(T),
                           c_int(f), c_int(1 if interleaved else 0), _stream()), "swiglu",
            f"(T={T}, f={f})")
@@ -157,9 +161,9 @@ def rope_table(positions: torch.Tensor, inv_freq: torch.Tensor, mag: float = 1.0
     assert positions.dtype == torch.int32 and inv_freq.dtype == torch.float64
     T, half = positions.numel(), inv_freq.numel()
     table = torch.empty((T, 2 * half), dtype=torch.float32, device=positions.device)
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_rope_table(_ptr(positions), _ptr(inv_freq), _ptr(table), c_int(T),
-                              c_int(half), ctypes.c_double(mag), _stream()), "rope_table")
+                              c_int(half), (float(mag),), _stream()), "rope_table")
     return table
 
 
@@ -186,7 +190,7 @@ def qk_norm_rope_cache(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[t
         assert (v is None and v_cache is None) or \
             (v_cache.dtype == q.dtype and v_cache.is_contiguous())
         assert slots.dtype == torch.int32 and slots.numel() == T
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_qk_norm_rope_cache(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0) if k is not None else 0),
         _ptr(v), c_ll(v.stride(0) if v is not None else 0), c_int(dtype_code(q.dtype)), c_int(T),
@@ -231,7 +235,7 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv
     assert block_tables.dtype == torch.int32 and block_tables.dim() == 2
     assert block_tables.is_contiguous() and seq_ids.dtype == torch.int32
     assert positions.dtype == torch.int32
-    lib = load_library("attention_generic")
+    lib = entry_points("attention_generic")
     if not window and T >= GENERIC_TILES_FROM * block_tables.shape[0] and \
             k_cache.data_ptr() % 16 == 0 and v_cache.data_ptr() % 16 == 0 and \
             lib.tgo_attention_generic_tiles_takes(c_int(num_heads), c_int(num_kv_heads), c_int(head_dim),
@@ -263,7 +267,7 @@ def cast_rows(h: torch.Tensor, out: torch.Tensor) -> None:
     _need_cuda(h, out)
     assert h.dtype == torch.float32 and h.is_contiguous() and out.is_contiguous()
     assert h.shape == out.shape
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_cast_rows(_ptr(h), _ptr(out), c_int(dtype_code(out.dtype)), c_ll(h.numel()),
                              _stream()), "cast_rows")
 
@@ -280,7 +284,7 @@ def group_norm_scale_add(h: torch.Tensor, y: torch.Tensor, gain: torch.Tensor,
     assert y.shape == h.shape and gain.dtype == torch.float32 and gain.numel() == d
     assert scale is None or (scale.dtype == torch.float32 and scale.numel() == d)
     assert act is None or (act.shape == h.shape and act.is_contiguous())
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_group_norm_scale_add(
         _ptr(h), _ptr(y), c_int(dtype_code(y.dtype)), _ptr(gain), _ptr(scale), c_float(eps),
         c_int(groups), _ptr(act), c_int(dtype_code(act.dtype) if act is not None else 0),
@@ -298,7 +302,7 @@ def norm_add_norm(h: torch.Tensor, y: torch.Tensor, gain_y: torch.Tensor, eps_y:
     assert y.shape == out.shape == h.shape and gain_y.numel() == gain.numel() == d
     assert all(t.is_contiguous() for t in (h, y, gain_y, gain, out))
     assert extra is None or (extra.dtype == torch.float32 and extra.shape == h.shape and extra.is_contiguous())
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_norm_add_norm(_ptr(h), _ptr(y), _ptr(gain_y), c_float(eps_y), _ptr(extra), _ptr(gain),
                                  c_float(eps), _ptr(out), c_int(dtype_code(out.dtype)), c_int(T), c_int(d),
                                  _stream()), "norm_add_norm", f"(d={d})")
@@ -312,7 +316,7 @@ def group_norm_rows(h: torch.Tensor, rows: Optional[torch.Tensor], gain: torch.T
     assert h.dtype == torch.float32 and h.is_contiguous() and out.is_contiguous()
     assert h.shape[1] == d and gain.dtype == torch.float32 and gain.numel() == d
     assert (rows is None and h.shape[0] == n) or (rows.dtype == torch.int32 and rows.numel() == n)
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_group_norm_rows(_ptr(h), _ptr(rows), _ptr(gain), c_float(eps), c_int(groups),
                                    _ptr(out), c_int(dtype_code(out.dtype)), c_int(n), c_int(d),
                                    _stream()), "group_norm_rows", f"(d={d}, groups={groups})")
@@ -322,7 +326,7 @@ def softcap(x: torch.Tensor, cap: float) -> None:
     """x <- cap * tanh(x / cap) in place, float32."""
     _need_cuda(x)
     assert x.dtype == torch.float32 and x.is_contiguous()
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_softcap(_ptr(x), c_ll(x.numel()), c_float(cap), _stream()), "softcap")
 
 
@@ -341,7 +345,7 @@ def gated_act(gate_up: torch.Tensor, out: torch.Tensor, interleaved: bool, activ
     assert gate_up.dtype == out.dtype
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == 2 * f and
                             bias.is_contiguous())
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_gated_act(_ptr(gate_up), _ptr(out), c_int(dtype_code(out.dtype)), c_int(T),
                              c_int(f), c_int(1 if interleaved else 0),
                              c_int(ACTIVATIONS[activation]), _ptr(bias), _stream()), "gated_act",
@@ -359,7 +363,7 @@ def scaled_add_norm(h: torch.Tensor, y: torch.Tensor, bias: Optional[torch.Tenso
     assert bias is None or (bias.dtype == torch.float32 and bias.numel() == d)
     assert act is None or (act.dtype == torch.bfloat16 and act.shape == h.shape and
                            act.is_contiguous())
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_scaled_add_norm(_ptr(h), _ptr(y), c_int(dtype_code(y.dtype)), _ptr(bias),
                                    c_float(alpha), _ptr(gain), c_float(eps), _ptr(act), c_int(T),
                                    c_int(d), _stream()), "scaled_add_norm", f"(d={d})")
@@ -370,7 +374,7 @@ def add_bias(y: torch.Tensor, bias: torch.Tensor) -> None:
     _need_cuda(y, bias)
     T, d = y.shape
     assert y.is_contiguous() and bias.dtype == torch.float32 and bias.numel() == d
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_add_bias(_ptr(y), c_int(dtype_code(y.dtype)), _ptr(bias), c_int(T), c_int(d),
                             _stream()), "add_bias")
 
@@ -392,7 +396,7 @@ def value_norm_share_cache(v: torch.Tensor, num_kv_heads: int, value_dim: int, n
         assert shared.shape == (T, num_kv_heads * value_dim)
     if mode == 2:
         assert blend.dtype == torch.float32 and blend.numel() == 1
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_value_norm_share_cache(
         _ptr(v), c_ll(v.stride(0)), c_int(dtype_code(v.dtype)), c_int(T), c_int(num_kv_heads),
         c_int(value_dim), c_int(1 if norm else 0), c_float(eps), _ptr(blend), _ptr(shared),
@@ -409,7 +413,7 @@ def head_norm_gate(o: torch.Tensor, gate: Optional[torch.Tensor], out: torch.Ten
     assert o.dtype == torch.float32 and o.is_contiguous() and out.is_contiguous()
     assert o.shape == out.shape == (T, heads * value_dim)
     assert gate is None or (gate.stride(1) == 1 and gate.dtype == out.dtype)
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_head_norm_gate(_ptr(o), _ptr(gate), c_ll(gate.stride(0) if gate is not None else 0),
                                   _ptr(out), c_int(dtype_code(out.dtype)), c_int(T), c_int(heads),
                                   c_int(value_dim), c_float(eps), _stream()), "head_norm_gate")
@@ -421,7 +425,7 @@ def weighted_sum(parts, scales, out: torch.Tensor) -> None:
     assert parts and len(parts) == len(scales) and out.dtype == torch.float32 and out.is_contiguous()
     for p in parts:
         assert p.shape == out.shape and p.is_contiguous() and p.dtype == parts[0].dtype
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     code = dtype_code(parts[0].dtype)
     if len(parts) == 1:
         _check(lib.tgo_scaled_sum(_ptr(parts[0]), c_float(scales[0]), _ptr(None), c_float(0.0),
@@ -439,14 +443,14 @@ def weighted_sum(parts, scales, out: torch.Tensor) -> None:
 def attention_sink_supports(num_heads: int, num_kv_heads: int, key_dim: int, value_dim: int) -> bool:
     """Whether the tensor-core kernel of the windowed attention with a sink takes these sizes
     (bfloat16; widths that are multiples of 8 up to 128)."""
-    return bool(load_library("attention_sink").tgo_attention_sink_supports(
+    return bool(entry_points("attention_sink").tgo_attention_sink_supports(
         c_int(num_heads), c_int(num_kv_heads), c_int(key_dim), c_int(value_dim)))
 
 
 def attention_sink_tile_tokens(group: int) -> int:
     """Tokens of one request a tile of that kernel holds at most, for `group` query heads a
     kv head."""
-    return max(1, int(load_library("attention_sink").tgo_attention_sink_tile_rows()) // group)
+    return max(1, int(entry_points("attention_sink").tgo_attention_sink_tile_rows()) // group)
 
 
 def attention_sink_takes(q: torch.Tensor, out: torch.Tensor) -> bool:
@@ -492,7 +496,7 @@ def attention_sink_tile(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_
     if n_splits > 1:
         part_o = torch.empty((n_tiles, num_heads, n_splits, value_dim), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n_tiles, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
-    lib = load_library("attention_sink")
+    lib = entry_points("attention_sink")
     _check(lib.tgo_attention_sink(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
         c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
@@ -510,14 +514,14 @@ def attention_sink_tile(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_
 def attention_sink_wide_supports(num_heads: int, num_kv_heads: int, key_dim: int, value_dim: int) -> bool:
     """Whether the tensor-core kernel for wide key rows whose first `value_dim` channels are the
     values takes these sizes (bfloat16; multiples of 8, keys up to 576, values up to 512)."""
-    return bool(load_library("attention_sink").tgo_attention_sink_wide_supports(
+    return bool(entry_points("attention_sink").tgo_attention_sink_wide_supports(
         c_int(num_heads), c_int(num_kv_heads), c_int(key_dim), c_int(value_dim)))
 
 
 def attention_sink_wide_tile_tokens(group: int) -> int:
     """Tokens of one request a tile of that kernel holds at most, for `group` query heads a
     kv head."""
-    return int(load_library("attention_sink").tgo_attention_sink_wide_tile_tokens(c_int(group)))
+    return int(entry_points("attention_sink").tgo_attention_sink_wide_tile_tokens(c_int(group)))
 
 
 def attention_sink_wide(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_heads: int,
@@ -546,7 +550,7 @@ def attention_sink_wide(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_
     if n_splits > 1:
         part_o = torch.empty((n_tiles, num_heads, n_splits, value_dim), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((n_tiles, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
-    lib = load_library("attention_sink")
+    lib = entry_points("attention_sink")
     _check(lib.tgo_attention_sink_wide(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), c_int(page_size),
         _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions), _ptr(seq_ids),
@@ -581,7 +585,7 @@ def attention_sink_decode_tma(q: torch.Tensor, out: torch.Tensor, num_heads: int
         part_o = torch.empty((T, num_heads, n_splits, head_dim), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((T, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
     gate_stride = c_ll(gate.stride(0) if gate is not None else 0)
-    _check(load_library("attention_decode_tma").tgo_attention_decode_tma_extra(
+    _check(entry_points("attention_decode_tma").tgo_attention_decode_tma_extra(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
         c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
         _ptr(seq_ids), c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_float(scale), c_int(window),
@@ -590,7 +594,7 @@ def attention_sink_decode_tma(q: torch.Tensor, out: torch.Tensor, num_heads: int
         _stream()), "attention_decode_tma_extra",
         f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads}, page_size={page_size})")
     if n_splits > 1:
-        _check(load_library("attention_sink").tgo_attention_sink_join(
+        _check(entry_points("attention_sink").tgo_attention_sink_join(
             _ptr(part_o), _ptr(part_ml), _ptr(positions), _ptr(sinks), _ptr(out), c_ll(out.stride(0)), c_int(T),
             c_int(num_heads), c_int(head_dim), c_int(n_splits), _ptr(gate), gate_stride, _stream()),
             "attention_sink_join")
@@ -598,14 +602,14 @@ def attention_sink_decode_tma(q: torch.Tensor, out: torch.Tensor, num_heads: int
 
 def attention_latent_tc_supports(num_heads: int, key_dim: int, value_dim: int, page_size: int) -> bool:
     """Whether the tcgen05 kernel for one wide row a token takes these sizes."""
-    return bool(load_library("attention_latent_tc").tgo_attention_latent_tc_supports(
+    return bool(entry_points("attention_latent_tc").tgo_attention_latent_tc_supports(
         c_int(num_heads), c_int(key_dim), c_int(value_dim), c_int(page_size)))
 
 
 def attention_latent_tc_error() -> int:
     """The code a wait of that kernel left when it ran out, or 0. Synchronises."""
     value = ctypes.c_int(0)
-    _check(load_library("attention_latent_tc").tgo_attention_latent_tc_error(ctypes.byref(value)),
+    _check(entry_points("attention_latent_tc").tgo_attention_latent_tc_error(ctypes.addressof(value)),
            "attention_latent_tc_error")
     return int(value.value)
 
@@ -623,7 +627,7 @@ def attention_latent_tc(q: torch.Tensor, out: torch.Tensor, num_heads: int, key_
     assert block_tables.is_contiguous() and block_tables.dtype == torch.int32 and block_tables.dim() == 2
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == num_heads)
     assert tile_tok0.dtype == tile_ntok.dtype == torch.int32
-    _check(load_library("attention_latent_tc").tgo_attention_latent_tc(
+    _check(entry_points("attention_latent_tc").tgo_attention_latent_tc(
         _ptr(q), c_ll(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_ll(out.stride(0)), _ptr(cache),
         c_int(cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
         _ptr(seq_ids), _ptr(tile_tok0), _ptr(tile_ntok), c_int(tile_tok0.numel()), c_int(num_heads), c_int(key_dim),
@@ -648,7 +652,7 @@ def gated_group_norm(o: torch.Tensor, gate: Optional[torch.Tensor], gain: Option
     assert out.shape == (T, W)
     assert gate is None or (gate.stride(1) == 1 and gate.dtype == out.dtype and gate.shape == (T, W))
     assert gain is None or (gain.dtype == torch.float32 and gain.numel() == W)
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_gated_group_norm(
         _ptr(o), _ptr(gate), c_ll(gate.stride(0) if gate is not None else 0), _ptr(gain), _ptr(out),
         c_int(dtype_code(out.dtype)), c_int(T), c_int(W), c_int(groups), c_float(eps),
@@ -683,7 +687,7 @@ def qkv_bias_rope_cache(q: torch.Tensor, k: Optional[torch.Tensor], v: Optional[
         assert slots.dtype == torch.int32 and slots.numel() == T
     if v is not None:
         assert v_cache is not None and v_cache.dtype == q.dtype and v_cache.is_contiguous()
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_qkv_bias_rope_cache(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0) if k is not None else 0),
         _ptr(v), c_ll(v.stride(0) if v is not None else 0), c_int(dtype_code(q.dtype)), c_int(T),
@@ -724,7 +728,7 @@ def qk_rownorm_rope_cache(q: torch.Tensor, k: Optional[torch.Tensor], v: Optiona
         assert slots.dtype == torch.int32 and slots.numel() == T
     if v is not None:
         assert v_cache is not None and v_cache.dtype == q.dtype and v_cache.is_contiguous()
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     _check(lib.tgo_qk_rownorm_rope_cache(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0) if k is not None else 0),
         _ptr(v), c_ll(v.stride(0) if v is not None else 0), c_int(dtype_code(q.dtype)), c_int(T),
@@ -769,7 +773,7 @@ def qkv_conv_rope_norm_cache(qkv: torch.Tensor, q_out: torch.Tensor, num_heads: 
                 state.stride(1) == 1
     if rope is not None:
         assert rope.dtype == torch.float32 and rope.shape == (T, rotary_dim) and rope.is_contiguous()
-    lib = load_library("elementwise")
+    lib = entry_points("elementwise")
     has_state = taps > 1
     _check(lib.tgo_qkv_conv_rope_norm_cache(
         _ptr(qkv), c_ll(qkv.stride(0)), _ptr(q_out), c_ll(q_out.stride(0)),
@@ -796,7 +800,7 @@ def stream_spread(h: torch.Tensor, x: torch.Tensor) -> None:
     _need_cuda(h, x)
     assert h.dtype == x.dtype == torch.float32 and h.is_contiguous() and x.is_contiguous()
     assert x.shape[1:] == h.shape
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_stream_spread(_ptr(h), _ptr(x), c_ll(h.numel()), c_int(x.shape[0]), _stream()),
            "stream_spread", f"(streams={x.shape[0]})")
 
@@ -809,7 +813,7 @@ def stream_read_norm(x: torch.Tensor, cin: torch.Tensor, gain: torch.Tensor, eps
     S, T, d = x.shape
     assert x.dtype == torch.float32 and x.is_contiguous() and out.is_contiguous() and out.shape == (T, d)
     assert cin.dtype == gain.dtype == torch.float32 and cin.numel() == S and gain.numel() == d
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_stream_read_norm(_ptr(x), c_int(S), c_int(T), c_int(d), _ptr(cin), _ptr(gain),
                                     c_float(eps), _ptr(out), c_int(dtype_code(out.dtype)), _stream()),
            "stream_read_norm", f"(streams={S}, d={d})")
@@ -834,7 +838,7 @@ def stream_write(x: torch.Tensor, y: torch.Tensor, mix: torch.Tensor, cout: torc
         assert next_in.numel() == S and next_gain.numel() == d
     assert sum_out is None or (sum_out.dtype == torch.float32 and sum_out.shape == (T, d) and
                                sum_out.is_contiguous())
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_stream_write(
         _ptr(x), c_int(S), c_int(T), c_int(d), _ptr(y), c_int(dtype_code(y.dtype)), _ptr(mix),
         _ptr(cout), _ptr(next_in), _ptr(next_gain), c_float(eps), _ptr(next_out),
@@ -846,7 +850,7 @@ def act_rows(x: torch.Tensor, activation: str) -> None:
     """x <- activation(x) in place: the hidden rows of a feed-forward without a gate."""
     _need_cuda(x)
     assert x.is_contiguous()
-    lib = load_library("layer_ops")
+    lib = entry_points("layer_ops")
     _check(lib.tgo_act_rows(_ptr(x), c_int(dtype_code(x.dtype)), c_ll(x.numel()),
                             c_int(PLAIN_ACTIVATIONS[activation]), _stream()), "act_rows", activation)
 
@@ -879,7 +883,7 @@ def mlstm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_i: torch.Tenso
     assert q_start.dtype == torch.int32 and state_slots.dtype == torch.int32
     rec = torch.empty((T, num_heads, 4), dtype=torch.float32, device=q.device)
     m_first = torch.empty((num_seqs, num_heads), dtype=torch.float32, device=q.device)
-    lib = load_library("mlstm")
+    lib = entry_points("mlstm")
     _check(lib.tgo_mlstm(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0)), _ptr(v), c_ll(v.stride(0)),
         c_int(dtype_code(q.dtype)), _ptr(gate_i), _ptr(gate_f), c_ll(gate_i.stride(0)), _ptr(bias_i),
@@ -892,11 +896,11 @@ def mlstm(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_i: torch.Tenso
 
 def mlstm_chunk_tokens() -> int:
     """Tokens of one request a chunk of the chunked matrix-memory kernels holds at most."""
-    return int(load_library("mlstm").tgo_mlstm_chunk_tokens())
+    return int(entry_points("mlstm").tgo_mlstm_chunk_tokens())
 
 
 def mlstm_chunked_supports(num_heads: int, key_dim: int, value_dim: int) -> bool:
-    return bool(load_library("mlstm").tgo_mlstm_chunked_supports(
+    return bool(entry_points("mlstm").tgo_mlstm_chunked_supports(
         c_int(num_heads), c_int(key_dim), c_int(value_dim)))
 
 
@@ -936,7 +940,7 @@ def mlstm_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate_i: tor
         scratch = torch.empty((chunks, num_heads, key_dim * value_dim + key_dim + 4),
                               dtype=torch.float32, device=q.device)
         m_last = torch.empty((num_seqs, num_heads), dtype=torch.float32, device=q.device)
-    lib = load_library("mlstm")
+    lib = entry_points("mlstm")
     _check(lib.tgo_mlstm_chunked(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0)), _ptr(v), c_ll(v.stride(0)),
         c_int(dtype_code(q.dtype)), _ptr(gate_i), _ptr(gate_f), c_ll(gate_i.stride(0)), _ptr(bias_i),
@@ -962,7 +966,7 @@ def latent_row_cache(kv: torch.Tensor, rank: int, width: int, gain: torch.Tensor
     assert gain.dtype == torch.float32 and gain.numel() == rank and slots.dtype == torch.int32
     if rope is not None:
         assert rope.dtype == torch.float32 and rope.shape == (T, rotary_dim) and rope.is_contiguous()
-    lib = load_library("latent")
+    lib = entry_points("latent")
     _check(lib.tgo_latent_row_cache(
         _ptr(kv), c_ll(kv.stride(0)), c_int(dtype_code(kv.dtype)), c_int(T), c_int(rank), c_int(width),
         _ptr(gain), c_float(eps), _ptr(rope), c_int(rotary_dim if rope is not None else 0),
@@ -980,7 +984,7 @@ def rope_slice(src: torch.Tensor, src_head: int, src_off: int, dst: torch.Tensor
     assert src.stride(1) == 1 and dst.stride(1) == 1 and src.dtype == dst.dtype and dst.shape[0] == T
     if rope is not None:
         assert rope.dtype == torch.float32 and rope.shape == (T, rotary_dim) and rope.is_contiguous()
-    lib = load_library("latent")
+    lib = entry_points("latent")
     _check(lib.tgo_rope_slice(
         _ptr(src), c_ll(src.stride(0)), c_int(src_head), c_int(src_off), _ptr(dst),
         c_ll(dst.stride(0)), c_int(dst_head), c_int(dst_off), c_int(dtype_code(src.dtype)), c_int(T),
@@ -1006,7 +1010,7 @@ def head_linear(x: torch.Tensor, x_head: int, w: torch.Tensor, y: torch.Tensor, 
     if x.dtype == torch.bfloat16:
         xv = torch.as_strided(x, (H, T, K), (x_head, x.stride(0), 1))
         if gate is not None:
-            lib = load_library("latent")
+            lib = entry_points("latent")
             by_head = torch.bmm(xv, w.transpose(1, 2))
             _check(lib.tgo_head_rows_gate(_ptr(by_head), _ptr(y), c_ll(y.stride(0)), c_int(y_head),
                                           c_int(dtype_code(y.dtype)), c_int(T), c_int(H), c_int(N),
@@ -1014,7 +1018,7 @@ def head_linear(x: torch.Tensor, x_head: int, w: torch.Tensor, y: torch.Tensor, 
             return
         torch.bmm(xv, w.transpose(1, 2), out=torch.as_strided(y, (H, T, N), (y_head, y.stride(0), 1)))
         return
-    lib = load_library("latent")
+    lib = entry_points("latent")
     _check(lib.tgo_head_linear(_ptr(x), c_ll(x.stride(0)), c_int(x_head), _ptr(w), _ptr(y),
                                c_ll(y.stride(0)), c_int(y_head), c_int(dtype_code(x.dtype)), c_int(T),
                                c_int(H), c_int(N), c_int(K), _ptr(gate),
@@ -1040,7 +1044,7 @@ def causal_conv_act(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
     assert state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
     assert seq_ids.dtype == q_start.dtype == state_slots.dtype == torch.int32
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
-    lib = load_library("state_space")
+    lib = entry_points("state_space")
     _check(lib.tgo_causal_conv_act(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w), _ptr(bias), _ptr(y),
         c_int(dtype_code(y.dtype)), c_int(T), c_int(num_seqs), c_int(C), c_int(taps), _ptr(seq_ids), _ptr(q_start),
@@ -1078,12 +1082,11 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
     assert state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1
     assert q_start.dtype == state_slots.dtype == torch.int32
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
-    lib = load_library("state_space")
+    lib = entry_points("state_space")
     if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and \
             lib.tgo_ssd_takes(_ptr(xbc), _ptr(y), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(heads),
                               c_int(groups), c_int(state_dim), c_int(value_dim)):
-        lib.tgo_ssd_floats.restype = c_ll
-        floats = lib.tgo_ssd_floats(c_int(T), c_int(num_seqs), c_int(heads), c_int(state_dim), c_int(value_dim))
+        floats = (T // 64 + num_seqs) * (heads * (state_dim * value_dim + 3 * 64) + 4)   # as tgo_ssd_scan says
         ws = torch.empty(floats, dtype=torch.float32, device=xbc.device)
         _check(lib.tgo_ssd_scan(
             _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y),
@@ -1126,7 +1129,7 @@ def channel_scan(x: torch.Tensor, z: torch.Tensor, dt_raw: torch.Tensor, dt_bias
     assert q_start.dtype == state_slots.dtype == torch.int32
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
     assert conv_in is None or (conv_in.shape == (T, C) and conv_in.stride(1) == 1 and conv_in.dtype == x.dtype)
-    lib = load_library("state_space")
+    lib = entry_points("state_space")
     _check(lib.tgo_channel_scan(
         _ptr(x), c_ll(x.stride(0)), _ptr(z), c_ll(z.stride(0)), c_int(dtype_code(x.dtype)), _ptr(dt_raw),
         c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a2), _ptr(bm), _ptr(cm), c_ll(bm.stride(0)),
@@ -1172,7 +1175,7 @@ def delta_prepare(x: torch.Tensor, w: torch.Tensor, b_raw: torch.Tensor, a_raw: 
     qk = buf[:n_qk].view(T, groups, 2, wide)
     v = buf[n_qk:n_qk + T * heads * value_dim].view(T, heads * value_dim)
     records = buf[n_qk + n_v:].view(T, heads, 12)
-    lib = load_library("delta")
+    lib = entry_points("delta")
     _check(lib.tgo_delta_prepare(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w), _ptr(b_raw), _ptr(a_raw),
         c_ll(a_raw.stride(0)), _ptr(dt_bias), _ptr(decay), _ptr(qk), _ptr(v), _ptr(records),
@@ -1207,7 +1210,7 @@ def delta_scan(prepared: tuple, y: torch.Tensor, num_seqs: int, heads: int, grou
     _delta_args(prepared, conv_in, heads, groups, key_dim, value_dim, num_seqs, q_start, state_slots, state)
     qk, v, records = prepared
     assert y.dtype == torch.float32 and y.is_contiguous() and y.shape == v.shape and y.is_cuda
-    lib = load_library("delta")
+    lib = entry_points("delta")
     _check(lib.tgo_delta_scan(
         _ptr(qk), _ptr(v), _ptr(records), _ptr(y), c_int(num_seqs), c_int(heads), c_int(groups),
         c_int(key_dim), c_int(value_dim), _ptr(q_start), _ptr(state_slots), _ptr(state),
@@ -1219,7 +1222,7 @@ def delta_scan(prepared: tuple, y: torch.Tensor, num_seqs: int, heads: int, grou
 def delta_step_supports(heads: int, groups: int, key_dim: int, value_dim: int, state: torch.Tensor,
                         mem_offset: int) -> bool:
     """Whether the kernel for requests of one token each takes these sizes."""
-    return bool(load_library("delta").tgo_delta_step_supports(
+    return bool(entry_points("delta").tgo_delta_step_supports(
         c_int(heads), c_int(groups), c_int(key_dim), c_int(value_dim), c_ll(state.stride(0)), c_ll(mem_offset)))
 
 
@@ -1236,7 +1239,7 @@ def delta_step(prepared: tuple, z: torch.Tensor, gain: torch.Tensor, eps: float,
     assert z.shape == out.shape == v.shape and z.stride(1) == 1 and out.is_contiguous()
     assert z.dtype == out.dtype == conv_in.dtype and num_seqs == v.shape[0]
     assert gain.dtype == torch.float32 and gain.numel() == value_dim and gain.is_contiguous()
-    lib = load_library("delta")
+    lib = entry_points("delta")
     _check(lib.tgo_delta_step(
         _ptr(qk), _ptr(v), _ptr(records), _ptr(z), c_ll(z.stride(0)), _ptr(gain), c_float(eps),
         _ptr(out), c_int(num_seqs), c_int(heads), c_int(groups), c_int(key_dim), c_int(value_dim),
@@ -1251,7 +1254,7 @@ ROUTER_SCORES = {"chosen": 0, "all": 1, "sigmoid": 2}
 
 def moe_tile_rows() -> int:
     """Rows of one expert a tile of the routed products holds at most."""
-    return int(load_library("moe").tgo_moe_tile_rows())
+    return int(entry_points("moe").tgo_moe_tile_rows())
 
 
 # Rows an expert on average from which the routed products read copies of x's rows in place order:
@@ -1264,7 +1267,7 @@ MOE_GATHER_ROWS = 24
 def moe_error() -> int:
     """The code a wait of the routed products left when it ran out, or 0. Synchronises."""
     value = ctypes.c_int(0)
-    _check(load_library("moe").tgo_moe_error(ctypes.byref(value)), "moe_error")
+    _check(entry_points("moe").tgo_moe_error(ctypes.addressof(value)), "moe_error")
     return int(value.value)
 
 
@@ -1321,34 +1324,35 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     assert residual is None or residual.dtype == torch.float32
     dev, pairs = x.device, T * top
     max_tiles = min(pairs, pairs // moe_tile_rows() + E)
-    ints = torch.empty(3 * pairs + 3 * E + 2 + 3 * max_tiles, dtype=torch.int32, device=dev)
-    ids, perm, place = ints[:pairs], ints[pairs:2 * pairs], ints[2 * pairs:3 * pairs]
-    o = 3 * pairs
-    counts, fill, offsets = ints[o:o + E], ints[o + E:o + 2 * E], ints[o + 2 * E:o + 3 * E + 1]
-    tile_info = ints[o + 3 * E + 1:o + 3 * E + 2]
-    tiles = ints[o + 3 * E + 2:]
-    wts = torch.empty(pairs, dtype=torch.float32, device=dev)
-    logits = torch.empty((T, w_router.shape[0]), dtype=torch.float32, device=dev)
-    launches = c_int(0)
-    gate = torch.empty(T, dtype=torch.float32, device=dev) if extra_gated else None
-    hidden = torch.empty((pairs, ff), dtype=x.dtype, device=dev)
-    y = torch.empty((pairs, d), dtype=torch.float32, device=dev)
-    xg = torch.empty((pairs, d), dtype=x.dtype, device=dev) \
-        if x.dtype == torch.bfloat16 and pairs >= MOE_GATHER_ROWS * E else None
+    width = x.element_size()
+    copies = x.dtype == torch.bfloat16 and pairs >= MOE_GATHER_ROWS * E
+    # one workspace: (name, bytes) in their order, each at a multiple of 256
+    at, where = 0, {}
+    for name, size in (("ids", 4 * pairs), ("perm", 4 * pairs), ("place", 4 * pairs), ("counts", 4 * E), ("fill", 4 * E),
+                       ("offsets", 4 * (E + 1)), ("tile_info", 4), ("tiles", 12 * max_tiles), ("wts", 4 * pairs),
+                       ("logits", 4 * T * w_router.shape[0]), ("gate", 4 * T if extra_gated else 0),
+                       ("hidden", width * pairs * ff), ("y", 4 * pairs * d), ("xg", width * pairs * d if copies else 0)):
+        where[name] = at
+        at += (size + 255) // 256 * 256
+    ws = torch.empty(at, dtype=torch.uint8, device=dev)
+    base = ws.data_ptr()
+    w = {name: base + o for name, o in where.items()}
+    gate, xg = w["gate"] if extra_gated else 0, w["xg"] if copies else 0
+    launches = ctypes.c_int(0)
     out = residual if residual is not None else torch.empty((T, d), dtype=torch.float32, device=dev)
-    lib = load_library("moe")
+    lib = entry_points("moe")
     _check(lib.tgo_moe_route(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w_router), _ptr(b_router),
-        c_int(T), c_int(d), c_int(outputs), c_int(top), _ptr(logits), _ptr(ids), _ptr(wts), _ptr(counts), _ptr(fill),
-        _ptr(offsets), _ptr(perm), _ptr(place), _ptr(tile_info), _ptr(tiles), c_int(max_tiles),
-        c_int(ROUTER_SCORES[scores]), _ptr(correction), c_int(E), _ptr(gate), c_int(groups), c_int(keep),
-        c_int(1 if renormalize else 0), c_float(route_scale), c_int(group_best), ctypes.byref(launches),
+        c_int(T), c_int(d), c_int(outputs), c_int(top), w["logits"], w["ids"], w["wts"], w["counts"], w["fill"],
+        w["offsets"], w["perm"], w["place"], w["tile_info"], w["tiles"], c_int(max_tiles),
+        c_int(ROUTER_SCORES[scores]), _ptr(correction), c_int(E), gate, c_int(groups), c_int(keep),
+        c_int(1 if renormalize else 0), c_float(route_scale), c_int(group_best), ctypes.addressof(launches),
         _stream()), "moe_route", f"(E={E}+{identity}, top={top})")
     _check(lib.tgo_moe_experts(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w_gate), _ptr(w_up),
-        _ptr(w_down), _ptr(hidden), _ptr(y), _ptr(wts), _ptr(extra), _ptr(out), c_int(T), c_int(d),
-        c_int(ff), c_int(top), c_int(PLAIN_ACTIVATIONS[activation]), _ptr(perm), _ptr(offsets), _ptr(xg), _ptr(tile_info),
-        _ptr(tiles), c_int(max_tiles), _ptr(ids if identity else None), c_int(E), _ptr(gate),
+        _ptr(w_down), w["hidden"], w["y"], w["wts"], _ptr(extra), _ptr(out), c_int(T), c_int(d),
+        c_int(ff), c_int(top), c_int(PLAIN_ACTIVATIONS[activation]), w["perm"], w["offsets"], xg, w["tile_info"],
+        w["tiles"], c_int(max_tiles), w["ids"] if identity else 0, c_int(E), gate,
         _ptr(beside), c_int(dtype_code(beside.dtype) if beside is not None else 0),
         c_int(1 if residual is not None else 0), _stream()), "moe_experts", f"(d={d}, ff={ff})")
     LAUNCHES[0] += launches.value + 1            # beside the two that _check counted
@@ -1372,7 +1376,7 @@ def attention_mixed(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_h
     assert positions.dtype == torch.int32
     assert mix is None or (mix.dtype == torch.float32 and mix.is_contiguous() and
                            mix.shape == (num_heads, num_heads))
-    lib = load_library("attention_mixed")
+    lib = entry_points("attention_mixed")
     _check(lib.tgo_attention_mixed(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(dtype_code(q.dtype)),
         c_int(T), c_int(num_heads), c_int(num_kv_heads), c_int(key_dim), c_int(value_dim),
@@ -1385,7 +1389,7 @@ def attention_mixed(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_h
 def attention_mixed_tile_supports(num_heads: int, num_kv_heads: int, key_dim: int, value_dim: int,
                                   window: int) -> bool:
     """Whether the tensor-core tile kernel of the mixed-head attention takes these sizes."""
-    lib = load_library("attention_mixed")
+    lib = entry_points("attention_mixed")
     return bool(lib.tgo_attention_mixed_tile_supports(c_int(num_heads), c_int(num_kv_heads),
                                                       c_int(key_dim), c_int(value_dim), c_int(window)))
 
@@ -1405,7 +1409,7 @@ def attention_mixed_tile(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
     assert tile_tok0.dtype == torch.int32 and tile_ntok.dtype == torch.int32
     assert mix is None or (mix.dtype == torch.float32 and mix.is_contiguous() and
                            mix.shape == (num_heads, num_heads))
-    lib = load_library("attention_mixed")
+    lib = entry_points("attention_mixed")
     _check(lib.tgo_attention_mixed_tile(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(tile_tok0.numel()),
         c_int(num_heads), c_int(num_kv_heads), c_int(key_dim), c_int(value_dim), _ptr(k_cache),
@@ -1418,7 +1422,7 @@ def attention_mixed_tile(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
 def attention_mixed_decode_supports(num_heads: int, num_kv_heads: int, key_dim: int,
                                     value_dim: int, window: int) -> bool:
     """Whether the split-key decode kernels of the mixed-head attention take these sizes."""
-    lib = load_library("attention_mixed")
+    lib = entry_points("attention_mixed")
     return bool(lib.tgo_attention_mixed_decode_supports(
         c_int(num_heads), c_int(num_kv_heads), c_int(key_dim), c_int(value_dim), c_int(window)))
 
@@ -1445,7 +1449,7 @@ def attention_mixed_decode(q: torch.Tensor, out: torch.Tensor, num_heads: int, n
     scores = torch.empty((T, num_heads, stride), dtype=torch.float32, device=dev)
     stats = torch.empty((T, splits, num_heads, 2), dtype=torch.float32, device=dev)
     partial = torch.empty((T, splits, num_heads * value_dim), dtype=torch.float32, device=dev)
-    lib = load_library("attention_mixed")
+    lib = entry_points("attention_mixed")
     _check(lib.tgo_attention_mixed_decode(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(T), c_int(num_heads),
         c_int(num_kv_heads), c_int(key_dim), c_int(value_dim), _ptr(k_cache), _ptr(v_cache),
@@ -1477,7 +1481,7 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tens
     assert state_slots.dtype == torch.int32 and state_slots.numel() == num_seqs
     if rope is not None:
         assert rope.dtype == torch.float32 and rope.shape == (T, rotary_dim) and rope.is_contiguous()
-    lib = load_library("retention")
+    lib = entry_points("retention")
     _check(lib.tgo_retention(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0)), _ptr(v), c_ll(v.stride(0)),
         c_int(dtype_code(q.dtype)), _ptr(out), c_int(num_seqs), c_int(num_heads), c_int(key_dim),
@@ -1489,11 +1493,11 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tens
 
 def retention_chunk_tokens() -> int:
     """Tokens of one request a chunk of the chunked retention kernels holds at most."""
-    return int(load_library("retention").tgo_retention_chunk_tokens())
+    return int(entry_points("retention").tgo_retention_chunk_tokens())
 
 
 def retention_chunked_supports(num_heads: int, key_dim: int, value_dim: int) -> bool:
-    return bool(load_library("retention").tgo_retention_chunked_supports(
+    return bool(entry_points("retention").tgo_retention_chunked_supports(
         c_int(num_heads), c_int(key_dim), c_int(value_dim)))
 
 
@@ -1533,7 +1537,7 @@ def retention_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: to
         assert chunk_ntok.numel() == chunks and chunk_first.numel() == num_seqs
         scratch = torch.empty((chunks, num_heads, key_dim, value_dim), dtype=torch.float32,
                               device=q.device)
-    lib = load_library("retention")
+    lib = entry_points("retention")
     _check(lib.tgo_retention_chunked(
         _ptr(q), c_ll(q.stride(0)), _ptr(k), c_ll(k.stride(0)), _ptr(v), c_ll(v.stride(0)),
         c_int(dtype_code(q.dtype)), _ptr(out), c_int(num_seqs), c_int(num_heads), c_int(key_dim),
@@ -1554,7 +1558,7 @@ def sgemm_tn(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     assert w.shape[1] == K and out.shape == (M, N)
     assert x.dtype == w.dtype == out.dtype == torch.float32
     assert x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
-    lib = load_library("sgemm")
+    lib = entry_points("sgemm")
     _check(lib.tgo_sgemm_tn(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), _stream()),
            "sgemm_tn", f"(M={M}, N={N}, K={K})")
 
@@ -1581,7 +1585,7 @@ def gemm_skinny(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate:
     else:
         assert out.dtype in (torch.bfloat16, torch.float32) and out.shape == (M, N)
         omode = 0 if out.dtype == torch.bfloat16 else 1
-    lib = load_library("gemm_skinny")
+    lib = entry_points("gemm_skinny")
     _check(lib.tgo_gemm_skinny(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K),
                                c_int(omode), _stream()), "gemm_skinny", f"(M={M}, N={N}, K={K})")
 
@@ -1616,7 +1620,7 @@ def folds_norm(M: int, N: int, K: int) -> bool:
     """Whether the weight-streaming product of these sizes can take its rows as NormedRows."""
     key = (M, N, K)
     if key not in _folds:
-        _folds[key] = bool(load_library("gemm_skinny").tgo_gemm_skinny_folds_norm(
+        _folds[key] = bool(entry_points("gemm_skinny").tgo_gemm_skinny_folds_norm(
             c_int(M), c_int(N), c_int(K)))
     return _folds[key]
 
@@ -1635,7 +1639,7 @@ def gemm_skinny_normed(x: NormedRows, w: torch.Tensor, out: torch.Tensor, gated:
     else:
         assert out.dtype in (torch.bfloat16, torch.float32) and out.shape == (M, N)
         omode = 0 if out.dtype == torch.bfloat16 else 1
-    lib = load_library("gemm_skinny")
+    lib = entry_points("gemm_skinny")
     _check(lib.tgo_gemm_skinny_normed(_ptr(x.h), _ptr(x.gain), c_float(x.eps), _ptr(w), _ptr(out),
                                       c_int(M), c_int(N), c_int(K), c_int(omode), _stream()),
            "gemm_skinny_normed", f"(M={M}, N={N}, K={K})")
@@ -1781,7 +1785,7 @@ def num_sms(device) -> int:
 def flash_supports(head_dim: int, group: int) -> bool:
     """Whether the tensor-core attention kernel has an instance for this head size and
     group (others go to the generic kernel)."""
-    return bool(load_library("attention_flash").tgo_attention_flash_supports(
+    return bool(entry_points("attention_flash").tgo_attention_flash_supports(
         c_int(head_dim), c_int(group)))
 
 
@@ -1791,14 +1795,14 @@ USE_TMA_DECODE = True       # decode attention with head size 128: cache pages b
 def attention_decode_tma_supports(head_dim: int, group: int, page_size: int) -> bool:
     if head_dim != 128:                  # do not build the library for models that cannot use it
         return False
-    return bool(load_library("attention_decode_tma").tgo_attention_decode_tma_supports(
+    return bool(entry_points("attention_decode_tma").tgo_attention_decode_tma_supports(
         c_int(head_dim), c_int(group), c_int(page_size)))
 
 
 def attention_decode_tma_error() -> int:
     """1 if a wait of the TMA-fed decode attention kernel ever ran out, else 0. Synchronises."""
     value = ctypes.c_int(0)
-    _check(load_library("attention_decode_tma").tgo_attention_decode_tma_error(ctypes.byref(value)),
+    _check(entry_points("attention_decode_tma").tgo_attention_decode_tma_error(ctypes.addressof(value)),
            "attention_decode_tma_error")
     return int(value.value)
 
@@ -1842,7 +1846,7 @@ def attention_decode_fused(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ou
     if n_splits > 1:
         part_o = torch.empty((T, num_heads, n_splits, head_dim), dtype=torch.float32, device=q.device)
         part_ml = torch.empty((T, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
-    _check(load_library("attention_decode_tma").tgo_attention_decode_tma_fused(
+    _check(entry_points("attention_decode_tma").tgo_attention_decode_tma_fused(
         _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
         c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]),
         _ptr(positions), _ptr(seq_ids), c_int(T), c_int(num_heads), c_int(num_kv_heads),
@@ -1851,7 +1855,7 @@ def attention_decode_fused(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, ou
         c_float(eps), _ptr(rope), _ptr(slots), _stream()),
         "attention_decode_tma_fused", f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads})")
     if n_splits > 1:
-        _check(load_library("attention_flash").tgo_attention_flash_combine(
+        _check(entry_points("attention_flash").tgo_attention_flash_combine(
             _ptr(part_o), _ptr(part_ml), _ptr(out), c_ll(out.stride(0)), c_int(T), c_int(num_heads),
             c_int(head_dim), c_int(n_splits), _stream()), "attention_flash_combine")
 
@@ -1884,10 +1888,10 @@ def attention_flash(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_h
         part_o = torch.empty((T, num_heads, n_splits, head_dim), dtype=torch.float32,
                              device=q.device)
         part_ml = torch.empty((T, num_heads, n_splits, 2), dtype=torch.float32, device=q.device)
-    lib = load_library("attention_flash")
+    lib = entry_points("attention_flash")
     if tma:
         # decode with the pages brought in by TMA
-        _check(load_library("attention_decode_tma").tgo_attention_decode_tma(
+        _check(entry_points("attention_decode_tma").tgo_attention_decode_tma(
             _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
             c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables),
             c_int(block_tables.shape[1]), _ptr(positions), _ptr(seq_ids), c_int(T), c_int(num_heads),
@@ -1916,7 +1920,7 @@ def attention_flash(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv_h
 
 
 def attention_tc_supports(head_dim: int, group: int, page_size: int) -> bool:
-    return bool(load_library("attention_tc").tgo_attention_tc_supports(c_int(head_dim), c_int(group),
+    return bool(entry_points("attention_tc").tgo_attention_tc_supports(c_int(head_dim), c_int(group),
                                                                        c_int(page_size)))
 
 
@@ -1924,7 +1928,7 @@ def attention_tc_error() -> int:
     """The code a wait of the tcgen05 attention kernel left when it ran out (1 producer,
     2 issuer, 3 softmax), or 0. Synchronises with the device."""
     value = ctypes.c_int(0)
-    _check(load_library("attention_tc").tgo_attention_tc_error(ctypes.byref(value)), "attention_tc_error")
+    _check(entry_points("attention_tc").tgo_attention_tc_error(ctypes.addressof(value)), "attention_tc_error")
     return int(value.value)
 
 
@@ -1953,7 +1957,7 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
     assert q.stride(1) == 1 and out.stride(1) == 1 and k_cache.is_contiguous() and v_cache.is_contiguous()
     assert k_cache.shape == v_cache.shape and k_cache.shape[1:] == (num_kv_heads, page_size, head_dim)
     assert block_tables.dtype == torch.int32 and block_tables.is_contiguous()
-    lib = load_library("attention_tc")
+    lib = entry_points("attention_tc")
     _check(lib.tgo_attention_tc_prefill(
         _ptr(q), c_ll(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
         c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]),
@@ -1969,7 +1973,7 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
 
 def flash_tile_rows() -> int:
     """Query rows (token x head of the group) one prefill tile of the attention kernel holds."""
-    return int(load_library("attention_flash").tgo_attention_flash_tile_rows())
+    return int(entry_points("attention_flash").tgo_attention_flash_tile_rows())
 
 
 def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
@@ -1978,7 +1982,7 @@ def argmax(logits: torch.Tensor, out: torch.Tensor) -> None:
     n, V = logits.shape
     assert logits.dtype == torch.float32 and logits.stride(1) == 1
     assert out.dtype == torch.int32 and out.numel() == n
-    lib = load_library("sampling")
+    lib = entry_points("sampling")
     part_v = torch.empty((n, 32), dtype=torch.float32, device=logits.device)
     part_i = torch.empty((n, 32), dtype=torch.int32, device=logits.device)
     _check(lib.tgo_argmax(_ptr(logits), c_ll(logits.stride(0)), c_int(n), c_int(V), _ptr(out),
@@ -2014,7 +2018,7 @@ def sample(logits: torch.Tensor, temperature: torch.Tensor, top_k: torch.Tensor,
             assert top_ids.dtype == torch.int32 and top_logprobs.dtype == torch.float32
             assert top_ids.shape == top_logprobs.shape == (n, width)
             assert top_ids.is_contiguous() and top_logprobs.is_contiguous()
-    lib = load_library("sampling")
+    lib = entry_points("sampling")
     _check(lib.tgo_sample(_ptr(logits), c_ll(logits.stride(0)), c_int(n), c_int(V),
                           _ptr(temperature), _ptr(top_k), _ptr(top_p), _ptr(draws), _ptr(out),
                           _ptr(report), _ptr(logprob), _ptr(top_ids), _ptr(top_logprobs),
@@ -2031,7 +2035,7 @@ def logits_adjust(row: torch.Tensor, bias_ids: Optional[torch.Tensor],
     assert row.dtype == torch.float32 and row.dim() == 1 and row.is_contiguous()
     nb = 0 if bias_ids is None else bias_ids.numel()
     ni = 0 if ids is None else ids.numel()
-    lib = load_library("sampling")
+    lib = entry_points("sampling")
     _check(lib.tgo_logits_adjust(_ptr(row), _ptr(bias_ids), _ptr(bias), c_int(nb), _ptr(ids),
                                  _ptr(counts), c_int(ni), c_float(repetition), c_float(presence),
                                  c_float(frequency), c_int(row.numel()), _stream()),
@@ -2092,7 +2096,7 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, accumulate: boo
     else:
         omode = 0 if out.dtype == torch.bfloat16 else 1
         assert out.dtype in (torch.bfloat16, torch.float32)
-    lib = load_library("gemm_tc")
+    lib = entry_points("gemm_tc")
     tail_ws, tail_flags = _tc_tail_buffers(x.device)
     _check(lib.tgo_gemm_tc(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), c_int(omode),
                            _ptr(tail_ws), _ptr(tail_flags), _ptr(gemm_tc_error_flag(x.device)),
@@ -2103,7 +2107,7 @@ def gemm_tc_force_tile(rows: int = 0, width: int = 0, cut_last_round: bool = Tru
     """For tests and tuning: `gemm_tc` runs tiles of rows x width (rows 128
     or 256; width a multiple of 16 up to 256) instead of choosing; 0 gives the choice back.
     cut_last_round False: the tiles of the last round are not cut along K."""
-    lib = load_library("gemm_tc")
+    lib = entry_points("gemm_tc")
     _check(lib.tgo_gemm_tc_force_tile(c_int(rows), c_int(width), c_int(0 if cut_last_round else 1)),
            "gemm_tc_force_tile", f"(rows={rows}, width={width})")
 
@@ -2111,9 +2115,9 @@ def gemm_tc_force_tile(rows: int = 0, width: int = 0, cut_last_round: bool = Tru
 def gemm_tc_last_plan() -> tuple:
     """(rows, width, parts) of the last `gemm_tc`: its tile and into how many
     parts along K the tiles of its last round were cut (1: not cut)."""
-    lib = load_library("gemm_tc")
-    r, w, c = c_int(0), c_int(0), c_int(0)
-    lib.tgo_gemm_tc_last_plan(ctypes.byref(r), ctypes.byref(w), ctypes.byref(c))
+    lib = entry_points("gemm_tc")
+    r, w, c = ctypes.c_int(0), ctypes.c_int(0), ctypes.c_int(0)
+    lib.tgo_gemm_tc_last_plan(ctypes.addressof(r), ctypes.addressof(w), ctypes.addressof(c))
     return r.value, w.value, c.value
 
 
