@@ -241,9 +241,11 @@ __device__ __forceinline__ float at_capped(float qk, float cap_log2, float scale
     return fmaf(-2.f * cap_log2, r, cap_log2);
 }
 
-// DH: head size, 64 or 128. XF: the scores go through the cap or take the bias by distance before
-// the softmax (the plain form folds the scale into the exponential's argument).
-template <int DH, bool XF>
+// DH: head size, 64 or 128. MODE: 0 nothing of ApExtra but the counters (an instance of its own: the
+// others hold 16 bytes more in local memory), 1 all but the changed scores, 2 the scores go through the
+// cap or take the bias by distance before the softmax (the others fold the scale into the
+// exponential's argument).
+template <int DH, int MODE>
 __global__ void __launch_bounds__(AP_THREADS, 1)
 attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
                                const __grid_constant__ CUtensorMap map_q, bf16* __restrict__ out,
@@ -254,6 +256,8 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                                int n_tiles, int H, int Hkv, float scale_log2, int window, const ApExtra ex) {
     constexpr int NH = DH / 64;                                 // 64-column blocks of a row
     constexpr int OC = DH / 2;                                  // output columns of a softmax thread
+    constexpr bool XF = MODE == 2;
+    const int keep = MODE > 0 ? ex.keep_first : 0;
     unsigned int* const ticket = ex.ticket ? ex.ticket : ap_counters;
     extern __shared__ unsigned char at_raw[];
     unsigned char* base = (unsigned char*)(((uintptr_t)at_raw + 1023) & ~(uintptr_t)1023);
@@ -315,8 +319,8 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
     auto page_range = [&](int j, bool kept, int key_lo, int key_hi, int& first, int& last) {
         first = j * pages_per_tile;
         last = first + pages_per_tile;
-        if (j * AT_BN < ex.keep_first) key_lo = j * AT_BN;
-        if (kept && ex.keep_first < key_hi) key_hi = ex.keep_first;
+        if (MODE > 0 && j * AT_BN < keep) key_lo = j * AT_BN;
+        if (MODE > 0 && kept && keep < key_hi) key_hi = keep;
         while (first < last && (first + 1) * page_size <= key_lo) ++first;
         while (last > first && (last - 1) * page_size >= key_hi) --last;
     };
@@ -365,7 +369,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int key_lo = (window > 0 && p0 - window + 1 > 0) ? p0 - window + 1 : 0;
             const int key_hi = p_last + 1;
             const int t_lo = key_lo / AT_BN, t_hi = (key_hi + AT_BN - 1) / AT_BN;
-            int n_kept = ex.keep_first > 0 ? (ex.keep_first + AT_BN - 1) / AT_BN : 0;
+            int n_kept = keep > 0 ? (keep + AT_BN - 1) / AT_BN : 0;
             if (n_kept > t_lo) n_kept = t_lo;
             const int n_it = p0 < 0 ? 0 : n_kept + t_hi - t_lo;
             if (lane == 0) {
@@ -411,19 +415,19 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             const int* bt = block_tables + (size_t)rec.seq * max_blocks;
             const int pg_lo = rec.t_lo * pages_per_tile;
             if (rec.n_it > 0) {
-                int pg_hi = (rec.t_lo + rec.n_it - rec.n_kept) * pages_per_tile;
+                int pg_hi = (rec.t_lo + rec.n_it - (MODE > 0 ? rec.n_kept : 0)) * pages_per_tile;
                 if (pg_hi > max_blocks) pg_hi = max_blocks;
                 if (pg_hi - pg_lo > AT_PAGES_CAP) pg_hi = pg_lo + AT_PAGES_CAP;
                 for (int i = pg_lo + lane; i < pg_hi; i += 32) s_pages[i - pg_lo] = bt[i];
             }
             __syncwarp();
             auto page_of = [&](int pi) {
-                return pi >= pg_lo && pi - pg_lo < AT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi];
+                return (MODE == 0 || pi >= pg_lo) && pi - pg_lo < AT_PAGES_CAP ? s_pages[pi - pg_lo] : bt[pi];
             };
             for (int it = 0; it < rec.n_it; ++it, ++g) {
                 const uint32_t s = g & 1u, ph = (g >> 1) & 1u;
-                const bool kept = it < rec.n_kept;
-                const int j = kept ? it : rec.t_lo + it - rec.n_kept;
+                const bool kept = MODE > 0 && it < rec.n_kept;
+                const int j = kept ? it : rec.t_lo + it - (MODE > 0 ? rec.n_kept : 0);
                 int first, last;
                 page_range(j, kept, rec.key_lo, rec.key_hi, first, last);
                 ok = __all_sync(0xffffffffu, at_wait(&empty[s], ph ^ 1u, 1));
@@ -547,7 +551,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             for (int it = 0; it < n_it; ++it, ++g) {
                 const uint32_t s = g & 1u, ph = (g >> 1) & 1u;
                 const uint32_t tm_s = tmem + 128u * s;
-                const int tile_lo = (it < rec.n_kept ? it : rec.t_lo + it - rec.n_kept) * AT_BN;
+                const int tile_lo = (MODE == 0 ? rec.t_lo + it : it < rec.n_kept ? it : rec.t_lo + it - rec.n_kept) * AT_BN;
                 const int kbase = tile_lo + 64 * half;
                 if (ok) ok = at_wait(&s_full[s], ph, 3);
                 at_fence_after();
@@ -585,7 +589,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
 #pragma unroll
                     for (int i = 0; i < 64; ++i) {
                         const int key = kbase + i;
-                        sc[i] = (key <= pos && (key >= vis_lo || key < ex.keep_first)) ? sc[i] : -INFINITY;
+                        sc[i] = (key <= pos && (key >= vis_lo || (MODE > 0 && key < keep))) ? sc[i] : -INFINITY;
                         mx4[i & 3] = fmaxf(mx4[i & 3], sc[i]);
                     }
                 }
@@ -621,7 +625,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                 if (tile_lo + AT_BN > key_hi || tile_lo < key_lo) {     // rows of V that nobody may read
                     if (ok) ok = at_wait(&v_full[s], ph, 3);
                     const int key = tile_lo + row;
-                    if (key >= key_hi || (key < key_lo && key >= ex.keep_first)) {
+                    if (key >= key_hi || (key < key_lo && (MODE == 0 || key >= keep))) {
                         unsigned char* vrow = sV + s * AT_TILE_BYTES + row * 128 + (NH > 1 ? half * AT_BLOCK_BYTES : half * 64);
 #pragma unroll
                         for (int c = 0; c < 4 * NH; ++c) *(uint4*)(vrow + c * 16) = make_uint4(0u, 0u, 0u, 0u);
@@ -655,16 +659,16 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             if (at_bar_or(!ok)) break;
             l += s_xl[(half ^ 1) * 128 + row];
             {
-                const int head = rec.kvh * G + (row_ok ? row : 0) % G;
+                const int head = MODE > 0 ? rec.kvh * G + (row_ok ? row : 0) % G : 0;
                 float corr = 1.f;
-                if (ex.sinks) {                    // the sink joins the denominator last
+                if (MODE > 0 && ex.sinks) {                    // the sink joins the denominator last
                     const float sk = ex.sinks[head] * 1.4426950408889634f;
                     const float mn = fmaxf(m_used, sk);
                     corr = exp2f(m_used - mn);
                     l = l * corr + exp2f(sk - mn);
                 }
                 float inv = l > 0.f ? corr / l : 0.f;
-                if (ex.gate && row_ok)
+                if (MODE > 0 && ex.gate && row_ok)
                     inv *= 1.f / (1.f + __expf(-__bfloat162float(ex.gate[(size_t)(rec.tok0 + row / G) * ex.gate_stride + head])));
 #pragma unroll
                 for (int c = 0; c < NH; ++c) {
@@ -809,7 +813,7 @@ TGO_API int tgo_attention_tc_error(int* value) {
     return (int)cudaMemcpyFromSymbol(value, at_error_flag, sizeof(int));
 }
 
-template <int DH, bool XF>
+template <int DH, int MODE>
 static int at_go(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mq, void* out, long long out_stride,
                  int page_size, int shift, const int* block_tables, int max_blocks, const int* positions,
                  const int* seq_ids, const int* tile_tok0, const int* tile_ntok, int n_tiles, int H, int Hkv,
@@ -823,7 +827,7 @@ static int at_go(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap
     if (e != cudaSuccess) return (int)e;
     if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
     if (!sms_of[dev]) {
-        e = cudaFuncSetAttribute(attention_tc_persistent_kernel<DH, XF>,
+        e = cudaFuncSetAttribute(attention_tc_persistent_kernel<DH, MODE>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         if (e != cudaSuccess) return (int)e;
         int n = 0;
@@ -832,7 +836,7 @@ static int at_go(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap
     }
     const int sms = sms_of[dev];
     const int items = n_tiles * Hkv;
-    attention_tc_persistent_kernel<DH, XF><<<dim3(items < sms ? items : sms), AP_THREADS, smem, stream>>>(
+    attention_tc_persistent_kernel<DH, MODE><<<dim3(items < sms ? items : sms), AP_THREADS, smem, stream>>>(
         mk, mv, mq, (bf16*)out, out_stride, page_size, shift, block_tables, max_blocks,
         positions, seq_ids, tile_tok0, tile_ntok, n_tiles, H, Hkv, scale_log2, window, ex);
     return launch_status();
@@ -881,10 +885,13 @@ TGO_API int tgo_attention_tc_prefill(const void* q, long long q_stride, int n_to
         const cudaError_t e = cudaMemsetAsync(counters, 0, 2 * sizeof(int), stream);
         if (e != cudaSuccess) return (int)e;
     }
-#define AT_GO(DH, XF)                                                                                             \
-    return at_go<DH, XF>(*mk, *mv, *mq, out, out_stride, page_size, shift, block_tables, max_blocks, positions,    \
+#define AT_GO(DH, MODE)                                                                                           \
+    return at_go<DH, MODE>(*mk, *mv, *mq, out, out_stride, page_size, shift, block_tables, max_blocks, positions,    \
                          seq_ids, tile_tok0, tile_ntok, n_tiles, H, Hkv, scale * log2e, window, ex, stream)
-    if (dh == 128) { if (softcap > 0.f || dist_bias) AT_GO(128, true); else AT_GO(128, false); }
-    if (softcap > 0.f || dist_bias) AT_GO(64, true); else AT_GO(64, false);
+    const int mode = softcap > 0.f || dist_bias ? 2 : sinks || gate || ex.keep_first ? 1 : 0;
+    if (dh == 128) { if (mode == 2) AT_GO(128, 2); if (mode == 1) AT_GO(128, 1); AT_GO(128, 0); }
+    if (mode == 2) AT_GO(64, 2);
+    if (mode == 1) AT_GO(64, 1);
+    AT_GO(64, 0);
 #undef AT_GO
 }
