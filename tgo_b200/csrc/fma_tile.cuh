@@ -56,6 +56,41 @@ struct FmaTile {
             }
         }
     }
+    // The same over channels k0 .. k0 + n - 1 of a tile that was laid down across its rows: column c of
+    // channel k stands at c ^ 4 ((k >> SHIFT) & 7) (ft_swizzle), in A and, with BSWZ, in B. n and k0 are
+    // multiples of 1 << SHIFT.
+    template <int SHIFT, bool BSWZ>
+    __device__ __forceinline__ void add_swizzled(const float* __restrict__ A, int lda, const float* __restrict__ B, int ldb,
+                                                 int k0, int n) {
+#pragma unroll 1
+        for (int kb = 0; kb < n; kb += 1 << SHIFT) {
+            const int x = 4 * (((k0 + kb) >> SHIFT) & 7);
+            const float* b0 = B + (size_t)kb * ldb;
+            const float* a0 = A + (size_t)kb * lda;
+#pragma unroll
+            for (int k = 0; k < (1 << SHIFT); ++k, a0 += lda, b0 += ldb) {
+                unsigned long long b[2 * RN];
+#pragma unroll
+                for (int c = 0; c < RN; ++c) {
+                    const ulonglong2 v = *(const ulonglong2*)(b0 + (BSWZ ? (4 * (c * TX + tx)) ^ x : 4 * (c * TX + tx)));
+                    b[2 * c] = v.x;
+                    b[2 * c + 1] = v.y;
+                }
+#pragma unroll
+                for (int r = 0; r < RM; ++r) {
+                    const float4 v = *(const float4*)(a0 + ((4 * (r * TY + ty)) ^ x));
+                    const float a[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const unsigned long long aa = ft_pair(a[i], a[i]);
+#pragma unroll
+                        for (int j = 0; j < 2 * RN; ++j)
+                            asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(acc[4 * r + i][j]) : "l"(aa), "l"(b[j]));
+                    }
+                }
+            }
+        }
+    }
     __device__ __forceinline__ void scale_row(int i, float f) {
 #pragma unroll
         for (int j = 0; j < 2 * RN; ++j) {
@@ -68,6 +103,11 @@ struct FmaTile {
         return make_float4(a.x, a.y, b.x, b.y);
     }
 };
+
+// Where column c of channel k stands in a tile of channel rows that threads fill from row-major memory: a
+// warp then stores four rows x eight runs of 1 << shift channels without meeting a bank twice (rows of
+// 64 + 4 floats), and groups of four columns stay together.
+__device__ __forceinline__ int ft_swizzle(int c, int k, int shift) { return c ^ (4 * ((k >> shift) & 7)); }
 
 __device__ __forceinline__ void ft_copy16(float* dst, const float* src, bool ok) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"

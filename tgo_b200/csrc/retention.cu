@@ -488,7 +488,7 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 // Register tiles of 8 x 8 and 4 x 8 outputs (fma_tile.cuh) instead of 4 x 4; what a product sums
 // over is the slow axis of both of its operands in shared memory. Bound by the FMA pipes; a true
 // 32-bit product has no faster unit. MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16
-// rows; the kernels above in brackets): summaries 140 us (255), scan 40 (139), outputs 312 (879).
+// rows; the kernels above in brackets): summaries 138 us (255), scan 40 (139), outputs 208 (879).
 //   summaries   a block makes U for 128 columns of V: K (scaled rows) and V as they lie;
 //   scan        four neighbouring elements a thread, eight summaries asked for while the eight before
 //               them are used: bound by memory (every summary read once, every state written once);
@@ -542,11 +542,15 @@ __device__ __forceinline__ void rotated8(const T* __restrict__ x, const float* _
     const int p0 = low ? d0 : d0 - half;
     float g[8];
     taken8(x + (low ? d0 + half : p0), act, g);
+    float c[8], s[8];
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-        const float c = cs[p0 + i], s = cs[half + p0 + i];
-        f[i] = low ? f[i] * c - g[i] * s : f[i] * c + g[i] * s;
+    for (int i = 0; i < 2; ++i) {
+        const float4 a = ((const float4*)(cs + p0))[i], b = ((const float4*)(cs + half + p0))[i];
+        c[4 * i] = a.x; c[4 * i + 1] = a.y; c[4 * i + 2] = a.z; c[4 * i + 3] = a.w;
+        s[4 * i] = b.x; s[4 * i + 1] = b.y; s[4 * i + 2] = b.z; s[4 * i + 3] = b.w;
     }
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = low ? f[i] * c[i] - g[i] * s[i] : f[i] * c[i] + g[i] * s[i];
 }
 
 // The powers of the decay, 0 .. RC_CHUNK, by repeated multiplication.
@@ -674,17 +678,18 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
     const int tok0 = chunk_tok0[ci], n = chunk_ntok[ci];
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
     rf_powers(pw, decay[h]);
-    // a lane a row: the stores of a warp hit 32 neighbouring places, a row's line is read from L1
+    // a warp takes four rows x eight runs of eight channels: 128 bytes a row, and stores that meet no
+    // bank twice (ft_swizzle). (A lane a row, every load touched 32 lines: ncu showed the L1 87 % busy.)
     for (int i = threadIdx.x; i < 2 * RC_CHUNK * (DK / 8); i += RC_THREADS) {
         const int which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
-        const int r = j % RC_CHUNK, d = (j / RC_CHUNK) * 8;
+        const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
         float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (r < n) {
             const size_t t = (size_t)(tok0 + r);
             rotated8(which ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
                      rope ? rope + t * rot : nullptr, d, rot, act, f);
         }
-        float* dst = (which ? KV : Qt) + d * RF_LDN + r;
+        float* dst = (which ? KV : Qt) + d * RF_LDN + ft_swizzle(r, d, 3);
 #pragma unroll
         for (int x = 0; x < 8; ++x) dst[x * RF_LDN] = which ? f[x] * k_scale : f[x];
     }
@@ -694,7 +699,7 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
         a.ty = ty;
         a.tx = tx;
         a.clear();
-        if (4 * tx <= 4 * ty + 3) a.add(Qt, RF_LDN, KV, RF_LDN, DK);
+        if (4 * tx <= 4 * ty + 3) a.template add_swizzled<3, true>(Qt, RF_LDN, KV, RF_LDN, 0, DK);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
             const float4 r = a.get(i, 0);
@@ -733,7 +738,8 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
             ft_wait<RF_PSTAGES - 2>();
             __syncthreads();
             load_p(turn + RF_PSTAGES - 1);
-            o.add(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS, RF_PK);
+            o.template add_swizzled<3, false>(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS,
+                                     turn * RF_PK, RF_PK);
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) o.scale_row(i, pw[4 * ty + i + 1]);
@@ -813,7 +819,7 @@ static int retention_chunked(const T* q, long long q_stride, const T* k, long lo
     // rows that can be read eight channels at a time, rotated halves of whole eights
     auto whole = [&](const void* p, long long stride) { return (uintptr_t)p % 16 == 0 && stride * sizeof(T) % 16 == 0; };
     if ((dk == 64 || dk == 128) && dv % 8 == 0 && rot % 16 == 0 && whole(q, q_stride) && whole(k, k_stride) &&
-        whole(v, v_stride) && (uintptr_t)out % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)scratch % 16 == 0) {
+        whole(v, v_stride) && (uintptr_t)rope % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)scratch % 16 == 0) {
 #define RF_GO(DK)                                                                                                    \
     return retention_tiled<T, DK>(q, q_stride, k, k_stride, v, v_stride, out, B, H, dv, decay, k_scale, act, rope,    \
                                   rot, q_start, state_slots, state, chunks, chunk_tok0, chunk_ntok, chunk_first, scratch, stream)

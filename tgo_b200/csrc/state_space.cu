@@ -415,7 +415,7 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
 // sums lose nothing), summaries (the sum of S's line), a scan over the chunks, which leaves the
 // state before each chunk in its summary's place, and outputs. Float32 products in register tiles
 // (fma_tile.cuh), bound by the FMA pipes. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128): 711 us
-// by the walk above, 263 so (summaries 54, scan over the chunks 32, outputs 173); error against 64 bits
+// by the walk above, 242 so (summaries 54, scan over the chunks 32, outputs 152); error against 64 bits
 // 1.2e-7 (1.9e-7 by the walk).
 // The walk stays for the float32 engine, whose sums do not depend on how a prompt is cut, for
 // steps of few tokens a request, and for other sizes.
@@ -623,19 +623,20 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const flo
             ft_copy16(Ss + r * (P + 4) + c, Sc + (size_t)(n0 + r) * P + c, true);
         }
         ft_commit();
-        // a lane a row: the stores of a warp hit 32 neighbouring places
+        // a warp takes four rows x eight runs of four states: 128 bytes a row, no bank met twice (ft_swizzle)
         for (int i = threadIdx.x; i < 2 * SD_CHUNK * 16; i += THREADS) {
-            const int r = i % SD_CHUNK, c = ((i / SD_CHUNK) % 16) * 4, which = i / (SD_CHUNK * 16);
+            const int which = i / (SD_CHUNK * 16), j = i % (SD_CHUNK * 16);
+            const int r = 4 * ((j / 32) % (SD_CHUNK / 4)) + (j % 32) / 8, c = 4 * (j % 8 + 8 * (j / (8 * SD_CHUNK)));
             float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
             if (r < n) v = *(const float4*)((which ? brow : crow) + (size_t)r * C + n0 + c);
-            float* dst = (which ? Bt : Ct) + c * SD_LD + r;
+            float* dst = (which ? Bt : Ct) + c * SD_LD + ft_swizzle(r, c, 2);
             dst[0] = v.x; dst[SD_LD] = v.y; dst[2 * SD_LD] = v.z; dst[3 * SD_LD] = v.w;
         }
         ft_wait<0>();
         __syncthreads();
         if (busy) {
-            g.add(Ct, SD_LD, Bt, SD_LD, 64);
-            o.add(Ct, SD_LD, Ss, P + 4, 64);
+            g.template add_swizzled<2, true>(Ct, SD_LD, Bt, SD_LD, 0, 64);
+            o.template add_swizzled<2, false>(Ct, SD_LD, Ss, P + 4, 0, 64);
         }
     }
     __syncthreads();
