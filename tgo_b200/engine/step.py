@@ -222,15 +222,24 @@ class Engine:
     # ------------------------------------------------------------- decode graphs
     BUCKETS = (1, 2, 4, 8, 16, 24, 32, 48, 64, 96, 128, 192, 256)
     WIDTH_QUANTUM = 64          # block-table columns of the smallest graph variant; then 128, 256, ...
+    # Decode steps of short contexts run in a graph of this many columns. The width bounds the keys a
+    # graph's launches are planned for: in one of 64 columns (1024 keys) the attention of one to eight
+    # requests of 50 keys is cut eight ways and joined, in one of 16 it runs whole and a layer has one
+    # launch less. 24 steps of 4 layers of width 2048, 64 columns against 16: four requests of 33 + 24
+    # tokens 5.68 ms / 5.36, eight of 100 + 24 6.24 / 5.90. Graphs of 32 columns lost (eight of 400 7.03 /
+    # 7.12, two of 480 5.52 / 5.74): from there on cutting pays.
+    SHORT_WIDTH = 16
 
-    def _graph_width(self, entries: List[StepEntry]) -> int:
-        """Block-table columns of the graph a step runs through: the smallest of 64, 128,
-        256, ... that holds the longest table of the step (a few variants however long the
+    def _graph_width(self, entries: List[StepEntry], short: int = 0) -> int:
+        """Block-table columns of the graph a step runs through: `short`, or else the smallest of 64,
+        128, 256, ... that holds the longest table of the step (a few variants however long the
         contexts grow; the kernels read only the columns a request has)."""
         if self._begun is not None:
             raw = max(1, self._begun[1][2])
         else:
             raw = max(1, self.cache.step_widest_table([e.request_id for e in entries]))
+        if raw <= short:
+            return short
         q = self.WIDTH_QUANTUM
         while q < raw:
             q *= 2
@@ -243,7 +252,7 @@ class Engine:
         valid until the next step of the same bucket."""
         B = len(entries)
         bucket = next((b for b in self.BUCKETS if b >= B), B)
-        width = self._graph_width(entries)
+        width = self._graph_width(entries, self.SHORT_WIDTH)
         key = (bucket, width)
         entry = self._graphs.get(key)
         if entry is None:
