@@ -367,14 +367,28 @@ __device__ __forceinline__ void dl_keep_block(float* kept, const T* __restrict__
 }
 
 // ----------------------------------------------------------------------------------- scan
-// A block per (request, head, 16 or 32 columns of dv). L lanes of a warp share a column (the column in
-// the low bits of the lane): slice s keeps its rows 4 s + 4 L i + (0..3) in registers for the whole walk
-// over the request's tokens. Four tokens cost eight products of a vector with S, one transposing
-// exchange over the slices that leaves one of the eight sums in each, four broadcasts of the reads by
-// k, ten multiply-adds for the four u, and one update of S. DS_TOK tokens at a time come through shared
-// memory by asynchronous copies, two buffers. The order of every sum depends on the sizes alone.
+// A block per (request, head, 16 columns of dv). The L slices of a warp (the lane's high bits) each keep
+// rows 4 s + 4 L i + (0..3) of NC columns in registers for the whole walk over the request's tokens: with
+// sixteen slices two columns a thread, so that a row of k or q read from shared memory serves both. Four
+// tokens cost eight products of a vector with S a column, an exchange over the slices that leaves a read
+// by k and one by q in each, broadcasts of the reads by k, ten multiply-adds for the four u, and one
+// update of S; two rows of a column share a packed FMA. The second half of the slices hold a thread's two
+// columns the other way round, so that the exchange's widest step selects nothing, and the reads by q are
+// exchanged on their own: S waits only for those by k. DS_TOK tokens at a time come through shared memory
+// by asynchronous copies, two buffers. The order of every sum depends on the sizes alone.
+//
+// What bounds it is a chain: a multiprocessor has four to twelve warps (the heads' columns over 16), and
+// each four's update waits for its exchange. Counted before (a column a thread): 260 instructions a warp
+// and four for two columns, 2.3 warps a scheduler; the packed pairs, the second column, the exchange
+// without its widest selects and pointers that step instead of being made anew leave half a column.
+// Registers for three blocks a multiprocessor (at four the next rows are not asked for ahead: 64-wide keys
+// 84 us for 50; at two a third request waits: 202 for 191).
+// MEASURED (B200, 16 heads of 128 x 128, bfloat16 engine; before in brackets): 2048 tokens 193 us (276),
+// requests of 1111, 852 and 593 tokens 191 (329), eight of 300 .. 116 tokens 109 (187); 8 heads of 64 x 64,
+// 700 tokens 50 (78). With a request's blocks apart on the grid the second took 230: some multiprocessors
+// got three blocks of the longest.
 #define DS_TOK 16
-#define DS_THREADS 256
+#define DS_THREADS 128
 
 __device__ __forceinline__ void ds_copy4(float* dst, const float* src, bool valid) {
     const int n = valid ? 4 : 0;
@@ -393,23 +407,41 @@ __device__ __forceinline__ void ds_copy16(float* dst, const void* src, bool vali
 template <typename T> __device__ __forceinline__ bool dl_slow(float pm1) { return false; }
 template <> __device__ __forceinline__ bool dl_slow<float>(float pm1) { return pm1 > -0.3f; }
 
+__device__ __forceinline__ unsigned long long ds_pair(float lo, float hi) {
+    unsigned long long v;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(v) : "f"(lo), "f"(hi));
+    return v;
+}
+__device__ __forceinline__ float2 ds_split(unsigned long long v) {
+    float2 f;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+    return f;
+}
+__device__ __forceinline__ void ds_fma(unsigned long long& d, unsigned long long a, unsigned long long b) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(d) : "l"(a), "l"(b));
+}
+
 template <typename T, int L, int NQ>
-__global__ void __launch_bounds__(DS_THREADS)
+__global__ void __launch_bounds__(DS_THREADS, 3)
 delta_scan_kernel(const float* __restrict__ qk, const float* __restrict__ v, const float4* __restrict__ records,
                   float* __restrict__ y, int H, int G, int dk, int dv,
                   const int* __restrict__ q_start, const int* __restrict__ state_slots, float* __restrict__ state,
                   long long state_stride, long long mem_offset, const T* __restrict__ conv_in,
                   long long conv_in_stride, int taps, long long conv_offset) {
-    constexpr int NI = 4 * NQ, DKP = L * NI, CG = 32 / L, COLS = DS_THREADS / L;
+    constexpr int NC = L / 8;                            // columns a thread
+    constexpr int NI = 4 * NQ, DKP = L * NI, CG = 32 / L, COLS = NC * DS_THREADS / L;
     constexpr int BUF = DS_TOK * (2 * DKP + COLS + 12);
     extern __shared__ __align__(16) float smem[];        // 2 x { qk [TOK][2 DKP], records [TOK][12], v [TOK][COLS] }
     pdl_wait();
-    const int b = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * COLS;
+    // a request's blocks are neighbours, so that a multiprocessor's few are of different requests
+    const int each = H * ((dv + COLS - 1) / COLS);
+    const int b = blockIdx.x / each, h = blockIdx.x % H, c0 = blockIdx.x % each / H * COLS;
     const int t0 = q_start[b], n_tok = q_start[b + 1] - t0;
     if (n_tok <= 0) return;
     const int g = h / (H / G);
     const int lane = threadIdx.x & 31, cg = lane % CG, s = lane / CG;
-    const int col = (threadIdx.x >> 5) * CG + cg, c = c0 + col;
+    const int col = ((threadIdx.x >> 5) * CG + cg) * NC;
+    const int swap = s >> 3, mine = s & 3;               // place a of a thread is column a ^ swap of its NC
     float* row = state + (size_t)state_slots[b] * state_stride;
     float* Sg = row + mem_offset + (size_t)h * dk * dv;
     // the memory comes and goes through shared memory ([dk][COLS + 1] floats fit in the buffers)
@@ -418,17 +450,39 @@ delta_scan_kernel(const float* __restrict__ qk, const float* __restrict__ v, con
         smem[n * (COLS + 1) + cc] = c0 + cc < dv ? Sg[(size_t)n * dv + c0 + cc] : 0.f;
     }
     __syncthreads();
-    float S[NI];
+    unsigned long long S[NC][NI / 2];                    // two rows of a column
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        const int n = 4 * s + 4 * L * (i >> 2) + (i & 3);
-        S[i] = n < dk ? smem[n * (COLS + 1) + col] : 0.f;
-    }
+    for (int a = 0; a < NC; ++a)
+#pragma unroll
+        for (int i = 0; i < NI; i += 2) {
+            const int n = 4 * s + 4 * L * (i >> 2) + (i & 3);
+            S[a][i / 2] = ds_pair(n < dk ? smem[n * (COLS + 1) + col + (a ^ swap)] : 0.f,
+                                  n + 1 < dk ? smem[(n + 1) * (COLS + 1) + col + (a ^ swap)] : 0.f);
+        }
     __syncthreads();
     auto stage = [&](int base, int buf) {
         float* qks = smem + buf * BUF;
         float* rs = qks + DS_TOK * 2 * DKP;
         float* vs = rs + DS_TOK * 12;
+        if (n_tok - base >= DS_TOK) {                    // whole: pointers that step from row to row
+            constexpr int QR = DKP / 2, RQ = DS_THREADS / QR, RV = DS_THREADS / COLS;
+            static_assert(DS_THREADS % QR == 0 && DS_TOK % RQ == 0 && DS_TOK % RV == 0, "rows a pass");
+            const float* src = qk + ((size_t)(t0 + base + threadIdx.x / QR) * G + g) * 2 * DKP + 4 * (threadIdx.x % QR);
+#pragma unroll
+            for (int i = 0; i < DS_TOK / RQ; ++i, src += (size_t)RQ * G * 2 * DKP)
+                ds_copy16(qks + 4 * (threadIdx.x + i * DS_THREADS), src, true);
+            const int cc = threadIdx.x % COLS;
+            const bool ok = c0 + cc < dv;
+            const float* vrc = ok ? v + ((size_t)(t0 + base + threadIdx.x / COLS) * H + h) * dv + c0 + cc : v;
+#pragma unroll
+            for (int i = 0; i < DS_TOK / RV; ++i, vrc += ok ? (size_t)RV * H * dv : 0)
+                ds_copy4(vs + threadIdx.x + i * DS_THREADS, vrc, ok);
+            if (threadIdx.x < 3 * DS_TOK)
+                ds_copy16(rs + 4 * threadIdx.x, records + ((size_t)(t0 + base + threadIdx.x / 3) * H + h) * 3 +
+                                                    threadIdx.x % 3, true);
+            asm volatile("cp.async.commit_group;\n" ::);
+            return;
+        }
         const int nt = n_tok - base < DS_TOK ? n_tok - base : DS_TOK, ne = (nt + 3) & ~3;
         for (int i = threadIdx.x; i < ne * (2 * DKP / 4); i += DS_THREADS) {
             const int r = i / (2 * DKP / 4), q = i % (2 * DKP / 4);
@@ -447,9 +501,32 @@ delta_scan_kernel(const float* __restrict__ qk, const float* __restrict__ v, con
         }
         asm volatile("cp.async.commit_group;\n" ::);
     };
-    // the sum this slice ends with: the read by k of token `mine` of the four, or (by_q) by its q
-    const int vec = s / (L / 8), mine = vec & 3;
-    const bool stores = vec >= 4 && (s % (L / 8)) == 0 && c < dv;
+    // A slice ends with the reads of its place 0 by k and q of token `mine`
+    const int own = c0 + col + swap;
+    const bool stores = (s & 4) && own < dv;
+    auto joined = [&](const unsigned long long (&two)[NC][4]) {
+        float sum[NC][4];
+#pragma unroll
+        for (int a = 0; a < NC; ++a)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const float2 f = ds_split(two[a][j]);
+                sum[a][j] = f.x + f.y;
+            }
+        if (NC == 2)
+#pragma unroll
+            for (int j = 0; j < 4; ++j) sum[0][j] += __shfl_xor_sync(0xffffffffu, sum[NC - 1][j], CG * 8);
+#pragma unroll
+        for (int half = 2; half > 0; half >>= 1) {       // a slice keeps half of its sums
+            const bool up = s & half;
+#pragma unroll
+            for (int i = 0; i < half; ++i) {
+                const float give = up ? sum[0][i] : sum[0][i + half], have = up ? sum[0][i + half] : sum[0][i];
+                sum[0][i] = have + __shfl_xor_sync(0xffffffffu, give, CG * half);
+            }
+        }
+        return sum[0][0] + __shfl_xor_sync(0xffffffffu, sum[0][0], CG * 4);
+    };
     stage(0, 0);
     for (int base = 0, buf = 0; base < n_tok; base += DS_TOK, buf ^= 1) {
         const int nt = n_tok - base < DS_TOK ? n_tok - base : DS_TOK;
@@ -463,87 +540,91 @@ delta_scan_kernel(const float* __restrict__ qk, const float* __restrict__ v, con
         const float* qks = smem + buf * BUF;
         const float* rs = qks + DS_TOK * 2 * DKP;
         const float* vs = rs + DS_TOK * 12;
-        float* yt = y + ((size_t)(t0 + base + mine) * H + h) * dv + c;
+        float* yt = y + ((size_t)(t0 + base + mine) * H + h) * dv + own;
         auto four = [&](int r) {
             const float* q0 = qks + r * 2 * DKP + 4 * s;
-            float4 ka[NQ][4];
-            float sum[8];                                // four reads by k, four by q
+            ulonglong2 ka[NQ][4];
+            unsigned long long by_k[NC][4], by_q[NC][4];
 #pragma unroll
-            for (int j = 0; j < 8; ++j) sum[j] = 0.f;
+            for (int a = 0; a < NC; ++a)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) by_k[a][j] = by_q[a][j] = 0ull;
 #pragma unroll
             for (int i = 0; i < NQ; ++i)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    const float4 kk = *(const float4*)(q0 + j * 2 * DKP + DKP + 4 * L * i);
-                    const float4 qq = *(const float4*)(q0 + j * 2 * DKP + 4 * L * i);
-                    ka[i][j] = kk;
-                    sum[j] = fmaf(kk.x, S[4 * i], sum[j]);
-                    sum[4 + j] = fmaf(qq.x, S[4 * i], sum[4 + j]);
-                    sum[j] = fmaf(kk.y, S[4 * i + 1], sum[j]);
-                    sum[4 + j] = fmaf(qq.y, S[4 * i + 1], sum[4 + j]);
-                    sum[j] = fmaf(kk.z, S[4 * i + 2], sum[j]);
-                    sum[4 + j] = fmaf(qq.z, S[4 * i + 2], sum[4 + j]);
-                    sum[j] = fmaf(kk.w, S[4 * i + 3], sum[j]);
-                    sum[4 + j] = fmaf(qq.w, S[4 * i + 3], sum[4 + j]);
+                    ka[i][j] = *(const ulonglong2*)(q0 + j * 2 * DKP + DKP + 4 * L * i);
+#pragma unroll
+                    for (int a = 0; a < NC; ++a) {
+                        ds_fma(by_k[a][j], ka[i][j].x, S[a][2 * i]);
+                        ds_fma(by_k[a][j], ka[i][j].y, S[a][2 * i + 1]);
+                    }
                 }
+            const float read_k = joined(by_k);
+#pragma unroll
+            for (int i = 0; i < NQ; ++i)
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const ulonglong2 qq = *(const ulonglong2*)(q0 + j * 2 * DKP + 4 * L * i);
+#pragma unroll
+                    for (int a = 0; a < NC; ++a) {
+                        ds_fma(by_q[a][j], qq.x, S[a][2 * i]);
+                        ds_fma(by_q[a][j], qq.y, S[a][2 * i + 1]);
+                    }
+                }
+            const float read_q = joined(by_q);           // beside the reads by k: what S waits for are those
             float4 ra[4];                                // (b P_j, the three k_m.k_j terms); zeros past the end
             float2 rc[4];                                // P_j, E_j
-            float vj[4];
+            float vj[4][NC];
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 ra[j] = *(const float4*)(rs + 12 * (r + j));
                 rc[j] = *(const float2*)(rs + 12 * (r + j) + 8);
-                vj[j] = vs[(r + j) * COLS + col];
+#pragma unroll
+                for (int a = 0; a < NC; ++a) vj[j][a] = vs[(r + j) * COLS + col + (a ^ swap)];
             }
             const float2 total = *(const float2*)(rs + 12 * r + 10);         // P_last, P_last - 1
             const float4 rd = *(const float4*)(rs + 12 * (r + mine) + 4);
             const float p_mine = rs[12 * (r + mine) + 8];
+            float u[NC][4];
 #pragma unroll
-            for (int half = 4; half > 0; half >>= 1) {   // a slice keeps half of its sums
-                const int o = half * (L / 8);
-                const bool up = s & o;
-#pragma unroll
-                for (int i = 0; i < half; ++i) {
-                    const float give = up ? sum[i] : sum[i + half], have = up ? sum[i + half] : sum[i];
-                    sum[i] = have + __shfl_xor_sync(0xffffffffu, give, CG * o);
-                }
-            }
-#pragma unroll
-            for (int o = L / 16; o > 0; o >>= 1) sum[0] += __shfl_xor_sync(0xffffffffu, sum[0], CG * o);
-            float u[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const float x = __shfl_sync(0xffffffffu, sum[0], j * (L / 8) * CG + cg);
-                u[j] = fmaf(-ra[j].x, x, vj[j]);
-            }
-            u[1] = fmaf(-ra[1].y, u[0], u[1]);
-            u[2] = fmaf(-ra[2].y, u[0], u[2]);
-            u[3] = fmaf(-ra[3].y, u[0], u[3]);
-            u[2] = fmaf(-ra[2].z, u[1], u[2]);
-            u[3] = fmaf(-ra[3].z, u[1], u[3]);
-            u[3] = fmaf(-ra[3].w, u[2], u[3]);
-            const float o0 = fmaf(rd.y, u[1], fmaf(rd.x, u[0], p_mine * sum[0]));
-            const float o1 = fmaf(rd.w, u[3], rd.z * u[2]);
-            if (stores && r + mine < nt) *yt = o0 + o1;
-            yt += (size_t)4 * H * dv;
-#pragma unroll
-            for (int j = 0; j < 4; ++j) u[j] *= rc[j].y;                      // decayed by the later ones
-            const bool slow = dl_slow<T>(total.y);
-            const float f = slow ? total.y : total.x;
-#pragma unroll
-            for (int i = 0; i < NQ; ++i) {
-                float4 a = make_float4(f * S[4 * i], f * S[4 * i + 1], f * S[4 * i + 2], f * S[4 * i + 3]);
+            for (int a = 0; a < NC; ++a) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                    a.x = fmaf(ka[i][j].x, u[j], a.x);
-                    a.y = fmaf(ka[i][j].y, u[j], a.y);
-                    a.z = fmaf(ka[i][j].z, u[j], a.z);
-                    a.w = fmaf(ka[i][j].w, u[j], a.w);
+                    const float x = __shfl_sync(0xffffffffu, read_k, (((a ^ swap) << 3) + j) * CG + cg);
+                    u[a][j] = fmaf(-ra[j].x, x, vj[j][a]);
                 }
-                S[4 * i] = slow ? S[4 * i] + a.x : a.x;
-                S[4 * i + 1] = slow ? S[4 * i + 1] + a.y : a.y;
-                S[4 * i + 2] = slow ? S[4 * i + 2] + a.z : a.z;
-                S[4 * i + 3] = slow ? S[4 * i + 3] + a.w : a.w;
+                u[a][1] = fmaf(-ra[1].y, u[a][0], u[a][1]);
+                u[a][2] = fmaf(-ra[2].y, u[a][0], u[a][2]);
+                u[a][3] = fmaf(-ra[3].y, u[a][0], u[a][3]);
+                u[a][2] = fmaf(-ra[2].z, u[a][1], u[a][2]);
+                u[a][3] = fmaf(-ra[3].z, u[a][1], u[a][3]);
+                u[a][3] = fmaf(-ra[3].w, u[a][2], u[a][3]);
+            }
+            const float o0 = fmaf(rd.y, u[0][1], fmaf(rd.x, u[0][0], p_mine * read_q));
+            const float o1 = fmaf(rd.w, u[0][3], rd.z * u[0][2]);
+            if (stores && r + mine < nt) *yt = o0 + o1;
+            yt += (size_t)4 * H * dv;
+            const bool slow = dl_slow<T>(total.y);
+            const float f = slow ? total.y : total.x;
+            const unsigned long long ff = ds_pair(f, f);
+#pragma unroll
+            for (int a = 0; a < NC; ++a) {
+                unsigned long long uu[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const float e = u[a][j] * rc[j].y;                        // decayed by the later ones
+                    uu[j] = ds_pair(e, e);
+                }
+#pragma unroll
+                for (int i = 0; i < 2 * NQ; ++i) {
+                    unsigned long long x;
+                    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(x) : "l"(ff), "l"(S[a][i]));
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) ds_fma(x, i & 1 ? ka[i / 2][j].y : ka[i / 2][j].x, uu[j]);
+                    if (slow) asm("add.rn.f32x2 %0, %0, %1;" : "+l"(x) : "l"(S[a][i]));
+                    S[a][i] = x;
+                }
             }
         };
         if (nt == DS_TOK) {                              // unrolled: the next four's rows load while these are joined
@@ -555,10 +636,14 @@ delta_scan_kernel(const float* __restrict__ qk, const float* __restrict__ v, con
         __syncthreads();
     }
 #pragma unroll
-    for (int i = 0; i < NI; ++i) {
-        const int n = 4 * s + 4 * L * (i >> 2) + (i & 3);
-        if (n < dk) smem[n * (COLS + 1) + col] = S[i];
-    }
+    for (int a = 0; a < NC; ++a)
+#pragma unroll
+        for (int i = 0; i < NI; i += 2) {
+            const int n = 4 * s + 4 * L * (i >> 2) + (i & 3);
+            const float2 f = ds_split(S[a][i / 2]);
+            if (n < dk) smem[n * (COLS + 1) + col + (a ^ swap)] = f.x;
+            if (n + 1 < dk) smem[(n + 1) * (COLS + 1) + col + (a ^ swap)] = f.y;
+        }
     __syncthreads();
     for (int i = threadIdx.x; i < dk * COLS; i += DS_THREADS) {
         const int n = i / COLS, cc = i % COLS;
@@ -572,11 +657,13 @@ static int launch_delta_scan(const float* qk, const float* v, const float* recor
                              int B, int H, int G, int dk, int dv, const int* q_start, const int* state_slots,
                              float* state, long long state_stride, long long mem_offset, const T* conv_in,
                              long long conv_in_stride, int taps, long long conv_offset, cudaStream_t stream) {
-    constexpr int DKP = 4 * L * NQ, COLS = DS_THREADS / L;
+    constexpr int DKP = 4 * L * NQ, COLS = DS_THREADS / 8;
     const size_t smem = 2 * (size_t)DS_TOK * (2 * DKP + COLS + 12) * sizeof(float);
     auto kernel = delta_scan_kernel<T, L, NQ>;
     if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return tgo_launch_pdl(kernel, dim3(B, H, (dv + COLS - 1) / COLS), dim3(DS_THREADS), smem, stream, qk, v,
+    const long long blocks = (long long)B * H * ((dv + COLS - 1) / COLS);
+    if (blocks > 0x7fffffffLL) return TGO_E_BAD_ARG;
+    return tgo_launch_pdl(kernel, dim3((unsigned)blocks), dim3(DS_THREADS), smem, stream, qk, v,
                           (const float4*)records, y, H, G, dk, dv, q_start, state_slots, state,
                           state_stride, mem_offset, conv_in, conv_in_stride, taps, conv_offset);
 }
