@@ -1077,7 +1077,7 @@ def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
     assert torch.equal(state[untouched], before[untouched])
 
 
-@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 3, 64, 128), (2, 2, 128, 128)])
+@pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 1, 128, 64), (3, 3, 64, 128), (2, 2, 128, 128)])
 @pytest.mark.parametrize("lens", [[128], [1, 63, 64, 65, 200, 3], [700, 129]])
 def test_selective_scan_by_chunks(H, G, N, P, lens, monkeypatch):
     """Requests that end before, on and after a chunk, fast and slow decays, against the recurrence

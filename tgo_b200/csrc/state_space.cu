@@ -415,7 +415,7 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
 // sums lose nothing), summaries (the sum of S's line), a scan over the chunks, which leaves the
 // state before each chunk in its summary's place, and outputs. Float32 products in register tiles
 // (fma_tile.cuh), bound by the FMA pipes. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128): 711 us
-// by the walk above, 242 so (summaries 54, scan over the chunks 32, outputs 152); error against 64 bits
+// by the walk above, 224 so (summaries 54, scan over the chunks 32, outputs 134, 148 with a head a block); error against 64 bits
 // 1.2e-7 (1.9e-7 by the walk).
 // The walk stays for the float32 engine, whose sums do not depend on how a prompt is cut, for
 // steps of few tokens a request, and for other sizes.
@@ -581,46 +581,50 @@ ssd_scan_kernel(int H, int NP, const int* __restrict__ q_start, const int* __res
     *sp = s;
 }
 
-// A block: a chunk's rows of one head. B, C and the state come 64 of the N states at a time; C . B
-// and S^T C grow side by side in registers, then A times v is added.
-template <int N, int P>
-__global__ void __launch_bounds__(2 * P, 512 / (2 * P))
+// A block: a chunk's rows of HEADS neighbouring heads of one group, 2 P threads each. B, C and the states
+// come 64 of the N states at a time; C . B, which the heads share, and S^T C grow side by side in
+// registers, then A times v is added.
+template <int N, int P, int HEADS>
+__global__ void __launch_bounds__(HEADS * 2 * P, 512 / (HEADS * 2 * P))
 ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const float* __restrict__ D,
                    const int4* __restrict__ chunks, const float* __restrict__ dts, const double* __restrict__ cum,
                    const float* __restrict__ U, float* __restrict__ y) {
-    constexpr int THREADS = 2 * P, TX = P / 8;           // 16 x TX threads, 4 x 8 outputs each
-    constexpr int GN = SD_CHUNK / (4 * TX);              // columns of C . B a thread owns, in fours
+    constexpr int EACH = 2 * P, THREADS = HEADS * EACH, TX = P / 8;        // 16 x TX threads a head, 4 x 8 outputs each
+    constexpr int TG = HEADS * TX, GN = SD_CHUNK / (4 * TG);               // columns of C . B a thread owns, in fours
     extern __shared__ __align__(16) float smem[];
-    float* Ct = smem;                                    // [64][SD_LD] state-major; later A [SD_CHUNK][SD_LD] token-j-major
-    float* Bt = Ct + 64 * SD_LD;                         // [64][SD_LD]; later v [SD_CHUNK][P + 4]
-    float* Ss = Bt + (64 * SD_LD > SD_CHUNK * (P + 4) ? 64 * SD_LD : SD_CHUNK * (P + 4));      // [64][P + 4]
-    __shared__ double ls[SD_CHUNK];
-    __shared__ float ds[SD_CHUNK];
+    float* Ct = smem;                                    // [64][SD_LD] state-major; later a head's A, token-j-major
+    float* Bt = Ct + 64 * SD_LD;                         // [64][SD_LD]; later the second head's A
+    float* Ss = Bt + 64 * SD_LD;                         // [HEADS][64][P + 4]; later v [HEADS][SD_CHUNK][P + 4]
+    __shared__ double ls[HEADS][SD_CHUNK];
+    __shared__ float ds[HEADS][SD_CHUNK];
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
-    const int h = blockIdx.y, n = ch.y;
+    const int h0 = blockIdx.y * HEADS, hh = threadIdx.x / EACH, h = h0 + hh, t = threadIdx.x % EACH, n = ch.y;
     if (n == 0) return;
     const float* rows = xbc + (size_t)ch.x * C;
-    const float* brow = rows + H * P + (h / (H / G)) * N;
+    const float* brow = rows + H * P + (h0 / (H / G)) * N;
     const float* crow = brow + (size_t)G * N;
     const size_t at = ((size_t)blockIdx.x * H + h) * SD_CHUNK;
     const float* Sc = U + ((size_t)blockIdx.x * H + h) * N * P;
-    for (int i = threadIdx.x; i < SD_CHUNK; i += THREADS) {
-        ls[i] = cum[at + i];
-        ds[i] = dts[at + i];
+    float* Sh = Ss + hh * 64 * (P + 4);
+    for (int i = t; i < SD_CHUNK; i += EACH) {
+        ls[hh][i] = cum[at + i];
+        ds[hh][i] = dts[at + i];
     }
-    FmaTile<1, GN, 16, TX> g;
+    FmaTile<1, GN, 16, TG> g;
     FmaTile<1, 2, 16, TX> o;
-    g.ty = o.ty = threadIdx.x / TX;
-    g.tx = o.tx = threadIdx.x % TX;
+    g.ty = threadIdx.x / TG;
+    g.tx = threadIdx.x % TG;
+    o.ty = t / TX;
+    o.tx = t % TX;
     g.clear();
     o.clear();
-    const bool busy = 4 * (o.ty & ~(32 / TX - 1)) < n;   // the warp's first row exists
+    const bool busy = 4 * (o.ty & ~(32 / TX - 1)) < n, g_busy = 4 * (g.ty & ~(32 / TG - 1)) < n;   // a warp's first row exists
     for (int n0 = 0; n0 < N; n0 += 64) {
         if (n0) __syncthreads();
-        for (int i = threadIdx.x; i < 64 * (P / 4); i += THREADS) {
+        for (int i = t; i < 64 * (P / 4); i += EACH) {
             const int r = i / (P / 4), c = (i % (P / 4)) * 4;
-            ft_copy16(Ss + r * (P + 4) + c, Sc + (size_t)(n0 + r) * P + c, true);
+            ft_copy16(Sh + r * (P + 4) + c, Sc + (size_t)(n0 + r) * P + c, true);
         }
         ft_commit();
         // a warp takes four rows x eight runs of four states: 128 bytes a row, no bank met twice (ft_swizzle)
@@ -634,41 +638,46 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const flo
         }
         ft_wait<0>();
         __syncthreads();
-        if (busy) {
-            g.template add_swizzled<2, true>(Ct, SD_LD, Bt, SD_LD, 0, 64);
-            o.template add_swizzled<2, false>(Ct, SD_LD, Ss, P + 4, 0, 64);
-        }
+        if (g_busy) g.template add_swizzled<2, true>(Ct, SD_LD, Bt, SD_LD, 0, 64);
+        if (busy) o.template add_swizzled<2, false>(Ct, SD_LD, Sh, P + 4, 0, 64);
     }
     __syncthreads();
-    // A over C, v over B
-    if (busy)
+    // A over C and B, v over S
+    if (g_busy)
 #pragma unroll
         for (int c = 0; c < GN; ++c)
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
                 const int cj = g.col(c) + j;
-                float a[4];
+                float z[4];
 #pragma unroll
                 for (int i = 0; i < 4; ++i) {
-                    const int ri = 4 * g.ty + i;
                     const float4 x = g.get(i, c);
-                    const float z = j == 0 ? x.x : j == 1 ? x.y : j == 2 ? x.z : x.w;
-                    a[i] = cj <= ri ? z * expf((float)(ls[ri] - ls[cj])) : 0.f;
+                    z[i] = j == 0 ? x.x : j == 1 ? x.y : j == 2 ? x.z : x.w;
                 }
-                *(float4*)(Ct + cj * SD_LD + 4 * g.ty) = make_float4(a[0], a[1], a[2], a[3]);
+#pragma unroll
+                for (int e = 0; e < HEADS; ++e) {
+                    float a[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int ri = 4 * g.ty + i;
+                        a[i] = cj <= ri ? z[i] * expf((float)(ls[e][ri] - ls[e][cj])) : 0.f;
+                    }
+                    *(float4*)(Ct + (e * 64 + cj) * SD_LD + 4 * g.ty) = make_float4(a[0], a[1], a[2], a[3]);
+                }
             }
-    for (int i = threadIdx.x; i < SD_CHUNK * (P / 4); i += THREADS) {
+    for (int i = t; i < SD_CHUNK * (P / 4); i += EACH) {
         const int r = i / (P / 4), c = (i % (P / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < n) v = *(const float4*)(rows + (size_t)r * C + h * P + c);
-        const float w = ds[r];
-        *(float4*)(Bt + r * (P + 4) + c) = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+        const float w = ds[hh][r];
+        *(float4*)(Sh + r * (P + 4) + c) = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
     }
     __syncthreads();
     if (!busy) return;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o.scale_row(i, expf((float)ls[4 * o.ty + i]));
-    o.add(Ct, SD_LD, Bt, P + 4, min(n, 4 * (o.ty | (32 / TX - 1)) + 4));
+    for (int i = 0; i < 4; ++i) o.scale_row(i, expf((float)ls[hh][4 * o.ty + i]));
+    o.add(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, min(n, 4 * (o.ty | (32 / TX - 1)) + 4));
     const float Dh = D ? D[h] : 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -690,8 +699,9 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
                   const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
                   float* state, long long state_stride, long long offset, float* ws, cudaStream_t stream) {
     constexpr size_t s1 = (size_t)SD_CHUNK * (N + 4 + P + 4) * sizeof(float);
-    constexpr size_t vb = 64 * SD_LD > SD_CHUNK * (P + 4) ? 64 * SD_LD : SD_CHUNK * (P + 4);
-    constexpr size_t s3 = ((size_t)64 * SD_LD + vb + 64 * (P + 4)) * sizeof(float);
+    constexpr int PAIR = P == 64 ? 2 : 1;                // heads a block of the outputs where a group has an even number
+    constexpr size_t s3 = ((size_t)2 * 64 * SD_LD + 64 * (P + 4)) * sizeof(float);
+    constexpr size_t s3p = ((size_t)2 * 64 * SD_LD + PAIR * 64 * (P + 4)) * sizeof(float);
     static bool sized[64] = {};                          // per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -699,7 +709,8 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
     if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
     if (!sized[dev]) {
         if ((e = cudaFuncSetAttribute(ssd_summaries_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1)) != cudaSuccess) return (int)e;
-        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
+        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3p)) != cudaSuccess) return (int)e;
+        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
         sized[dev] = true;
     }
     const int n_chunks = T / SD_CHUNK + B;               // at least as many as there are
@@ -716,7 +727,13 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
     rc = tgo_launch_pdl(ssd_scan_kernel, dim3(B, H, (N * P / 4 + 255) / 256), dim3(256), 0, stream, H, N * P, q_start,
                         state_slots, (const double*)cum, U, state, state_stride, offset);
     if (rc) return rc;
-    return tgo_launch_pdl(ssd_outputs_kernel<N, P>, dim3(n_chunks, H), dim3(2 * P), s3, stream, xbc, C, H, G, D,
+    // Two heads a block from more (chunk, head) pairs than multiprocessors: 2048 tokens of 64 heads 134 us
+    // against 148, 700 of 24 25.1 against 27.1; 160 of 8 (24 pairs) 24.4 against 20.7, 512 of 16 (144) 24.9
+    // against 21.3.
+    if (PAIR == 2 && H / G % 2 == 0 && (long long)n_chunks * H > 148)
+        return tgo_launch_pdl(ssd_outputs_kernel<N, P, PAIR>, dim3(n_chunks, H / PAIR), dim3(PAIR * 2 * P), s3p, stream, xbc, C,
+                              H, G, D, (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+    return tgo_launch_pdl(ssd_outputs_kernel<N, P, 1>, dim3(n_chunks, H), dim3(2 * P), s3, stream, xbc, C, H, G, D,
                           (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
 }
 
