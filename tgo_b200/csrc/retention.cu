@@ -488,7 +488,8 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 // Register tiles of 8 x 8 and 4 x 8 outputs (fma_tile.cuh) instead of 4 x 4; what a product sums
 // over is the slow axis of both of its operands in shared memory. Bound by the FMA pipes; a true
 // 32-bit product has no faster unit. MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16
-// rows; the kernels above in brackets): summaries 138 us (255), scan 40 (139), outputs 208 (879).
+// rows; the kernels above in brackets): summaries 122 us (255), scan 40 (139), outputs 186 (879); 138 and
+// 206 where each run's loads were waited for before the next were asked for.
 //   summaries   a block makes U for 128 columns of V: K (scaled rows) and V as they lie;
 //   scan        four neighbouring elements a thread, eight summaries asked for while the eight before
 //               them are used: bound by memory (every summary read once, every state written once);
@@ -502,13 +503,18 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 #define RF_PK 16                      // channels of P a turn
 #define RF_PSTAGES 3
 
-// Eight channels' values of a row, after the activation.
-template <typename T>
-__device__ __forceinline__ void taken8(const T* __restrict__ x, int act, float (&f)[8]);
-template <>
-__device__ __forceinline__ void taken8<bf16>(const bf16* __restrict__ x, int act, float (&f)[8]) {
-    const uint4 u = *(const uint4*)x;
-    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+// Eight channels of a row as they lie, and their values after the activation. Asked for first and turned
+// later, so that several are under way at once.
+template <typename T> struct Raw8;
+template <> struct Raw8<bf16> { uint4 u; };
+template <> struct Raw8<float> { float4 a, b; };
+__device__ __forceinline__ void load8(Raw8<bf16>& w, const bf16* __restrict__ x) { w.u = *(const uint4*)x; }
+__device__ __forceinline__ void load8(Raw8<float>& w, const float* __restrict__ x) {
+    w.a = ((const float4*)x)[0];
+    w.b = ((const float4*)x)[1];
+}
+__device__ __forceinline__ void taken8(const Raw8<bf16>& raw, int act, float (&f)[8]) {
+    const uint32_t w[4] = {raw.u.x, raw.u.y, raw.u.z, raw.u.w};
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
         const float2 v = __bfloat1622float2(*(const __nv_bfloat162*)&w[i]);
@@ -519,39 +525,42 @@ __device__ __forceinline__ void taken8<bf16>(const bf16* __restrict__ x, int act
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.f + expf(-f[i]));
 }
-template <>
-__device__ __forceinline__ void taken8<float>(const float* __restrict__ x, int act, float (&f)[8]) {
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float4 v = ((const float4*)x)[i];
-        f[4 * i] = v.x; f[4 * i + 1] = v.y; f[4 * i + 2] = v.z; f[4 * i + 3] = v.w;
-    }
+__device__ __forceinline__ void taken8(const Raw8<float>& raw, int act, float (&f)[8]) {
+    f[0] = raw.a.x; f[1] = raw.a.y; f[2] = raw.a.z; f[3] = raw.a.w;
+    f[4] = raw.b.x; f[5] = raw.b.y; f[6] = raw.b.z; f[7] = raw.b.w;
     if (act == 1)
 #pragma unroll
         for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.f + expf(-f[i]));
 }
 
-// Eight neighbouring channels d0 .. d0 + 7 of a row, rotated: d0 and rot / 2 are multiples of 8.
-template <typename T>
-__device__ __forceinline__ void rotated8(const T* __restrict__ x, const float* __restrict__ cs, int d0, int rot, int act,
-                                         float (&f)[8]) {
-    taken8(x + d0, act, f);
-    if (!cs || d0 >= rot) return;
-    const int half = rot >> 1;
-    const bool low = d0 < half;
-    const int p0 = low ? d0 : d0 - half;
-    float g[8];
-    taken8(x + (low ? d0 + half : p0), act, g);
-    float c[8], s[8];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-        const float4 a = ((const float4*)(cs + p0))[i], b = ((const float4*)(cs + half + p0))[i];
-        c[4 * i] = a.x; c[4 * i + 1] = a.y; c[4 * i + 2] = a.z; c[4 * i + 3] = a.w;
-        s[4 * i] = b.x; s[4 * i + 1] = b.y; s[4 * i + 2] = b.z; s[4 * i + 3] = b.w;
+// Eight neighbouring channels d0 .. d0 + 7 of a row, rotated: d0 and rot / 2 are multiples of 8. Without a
+// rotation the partner is the run itself and nothing else is read.
+template <typename T> struct Rot8 {
+    Raw8<T> x, g;
+    float4 c0, c1, s0, s1;
+    __device__ __forceinline__ void load(const T* __restrict__ row, const float* __restrict__ cs, int d0, int rot) {
+        const int half = rot >> 1;
+        const bool turned = cs && d0 < rot;
+        load8(x, row + d0);
+        if (cs && rot > 0) {
+            const int p0 = !turned ? 0 : d0 < half ? d0 : d0 - half;
+            load8(g, row + (!turned ? d0 : d0 < half ? d0 + half : p0));
+            c0 = ((const float4*)(cs + p0))[0]; c1 = ((const float4*)(cs + p0))[1];
+            s0 = ((const float4*)(cs + half + p0))[0]; s1 = ((const float4*)(cs + half + p0))[1];
+        }
     }
+    __device__ __forceinline__ void values(bool rope, int d0, int rot, int act, float (&f)[8]) const {
+        taken8(x, act, f);
+        if (!rope || d0 >= rot) return;
+        const bool low = d0 < (rot >> 1);
+        float o[8];
+        taken8(g, act, o);
+        const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
+        const float n[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = low ? f[i] * c[i] - g[i] * s[i] : f[i] * c[i] + g[i] * s[i];
-}
+        for (int i = 0; i < 8; ++i) f[i] = low ? f[i] * c[i] - o[i] * n[i] : f[i] * c[i] + o[i] * n[i];
+    }
+};
 
 // The powers of the decay, 0 .. RC_CHUNK, by repeated multiplication.
 __device__ __forceinline__ void rf_powers(float* pw, float g) {
@@ -561,14 +570,25 @@ __device__ __forceinline__ void rf_powers(float* pw, float g) {
     }
 }
 
-// Columns c0 .. c0 + RF_SLICE - 1 of the chunk's values, rows past n and columns past dv zero.
+// Columns c0 .. c0 + RF_SLICE - 1 of the chunk's values, rows past n and columns past dv zero: asked for,
+// then put into shared memory.
+#define RF_V_RUNS (RC_CHUNK * (RF_SLICE / 8) / RC_THREADS)
 template <typename T>
-__device__ __forceinline__ void rf_load_v(float* Vs, const T* __restrict__ v, long long v_stride, int h, int dv, int c0,
-                                          int tok0, int n, int act) {
-    for (int i = threadIdx.x; i < RC_CHUNK * (RF_SLICE / 8); i += RC_THREADS) {
-        const int r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
+__device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[RF_V_RUNS], const T* __restrict__ v, long long v_stride, int h, int dv,
+                                         int c0, int tok0, int n) {
+#pragma unroll
+    for (int j = 0; j < RF_V_RUNS; ++j) {
+        const int i = threadIdx.x + j * RC_THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
+        load8(raw[j], v + (size_t)(tok0 + (r < n ? r : 0)) * v_stride + (size_t)h * dv + (c0 + c < dv ? c0 + c : 0));
+    }
+}
+template <typename T>
+__device__ __forceinline__ void rf_put_v(float* Vs, const Raw8<T> (&raw)[RF_V_RUNS], int dv, int c0, int n, int act) {
+#pragma unroll
+    for (int j = 0; j < RF_V_RUNS; ++j) {
+        const int i = threadIdx.x + j * RC_THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
         float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (r < n && c0 + c < dv) taken8(v + (size_t)(tok0 + r) * v_stride + (size_t)h * dv + c0 + c, act, f);
+        if (r < n && c0 + c < dv) taken8(raw[j], act, f);
         *(float4*)(Vs + r * RF_LDS + c) = make_float4(f[0], f[1], f[2], f[3]);
         *(float4*)(Vs + r * RF_LDS + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
     }
@@ -586,23 +606,36 @@ retention_summaries_tiled_kernel(const T* __restrict__ k, long long k_stride, co
     __shared__ float pw[RC_CHUNK + 1];
     pdl_wait();
     const int ci = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * RF_SLICE;
-    const int tok0 = chunk_tok0[ci], n = chunk_ntok[ci];
+    const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
+    Raw8<T> vr[RF_V_RUNS];
+    rf_ask_v(vr, v, v_stride, h, dv, c0, tok0, n);
     rf_powers(pw, decay[h]);
     __syncthreads();
-    for (int i = threadIdx.x; i < RC_CHUNK * (DK / 8); i += RC_THREADS) {
-        const int r = i / (DK / 8), d = (i % (DK / 8)) * 8;
-        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (r < n) {
-            const size_t t = (size_t)(tok0 + r);
-            rotated8(k + t * k_stride + (size_t)h * DK, rope ? rope + t * rot : nullptr, d, rot, act, f);
-            const float w = pw[n - 1 - r];
+    // two runs of K a thread at a time, beside the values: a thread a run after the other had its loads
+    // waited for one by one (ncu: 2.7 of 9 cycles an instruction)
+    constexpr int RUNS = RC_CHUNK * (DK / 8) / RC_THREADS;
 #pragma unroll
-            for (int x = 0; x < 8; ++x) f[x] = f[x] * k_scale * w;
+    for (int j0 = 0; j0 < RUNS; j0 += 2) {
+        Rot8<T> kr[2];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = threadIdx.x + (j0 + j) * RC_THREADS, r = i / (DK / 8), d = (i % (DK / 8)) * 8;
+            const size_t t = (size_t)(tok0 + (r < n ? r : 0));
+            kr[j].load(k + t * k_stride + (size_t)h * DK, rope ? rope + t * rot : nullptr, d, rot);
         }
-        *(float4*)(Ks + r * (DK + 4) + d) = make_float4(f[0], f[1], f[2], f[3]);
-        *(float4*)(Ks + r * (DK + 4) + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = threadIdx.x + (j0 + j) * RC_THREADS, r = i / (DK / 8), d = (i % (DK / 8)) * 8;
+            float f[8];
+            kr[j].values(rope != nullptr, d, rot, act, f);
+            const float w = r < n ? pw[n - 1 - r] : 0.f;
+#pragma unroll
+            for (int x = 0; x < 8; ++x) f[x] = r < n ? f[x] * k_scale * w : 0.f;
+            *(float4*)(Ks + r * (DK + 4) + d) = make_float4(f[0], f[1], f[2], f[3]);
+            *(float4*)(Ks + r * (DK + 4) + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        }
     }
-    rf_load_v(Vs, v, v_stride, h, dv, c0, tok0, n, act);
+    rf_put_v(Vs, vr, dv, c0, n, act);
     __syncthreads();
     FmaTile<DK / 64, 2, 16, 16> t;
     t.ty = threadIdx.x / 16;
@@ -675,23 +708,34 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
     __shared__ float pw[RC_CHUNK + 1];
     pdl_wait();
     const int ci = blockIdx.x, h = blockIdx.y;
-    const int tok0 = chunk_tok0[ci], n = chunk_ntok[ci];
+    const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
     const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
     rf_powers(pw, decay[h]);
     // a warp takes four rows x eight runs of eight channels: 128 bytes a row, and stores that meet no
     // bank twice (ft_swizzle). (A lane a row, every load touched 32 lines: ncu showed the L1 87 % busy.)
-    for (int i = threadIdx.x; i < 2 * RC_CHUNK * (DK / 8); i += RC_THREADS) {
-        const int which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
-        const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
-        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (r < n) {
-            const size_t t = (size_t)(tok0 + r);
-            rotated8(which ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
-                     rope ? rope + t * rot : nullptr, d, rot, act, f);
-        }
-        float* dst = (which ? KV : Qt) + d * RF_LDN + ft_swizzle(r, d, 3);
+    // Two runs are asked for at a time.
+    constexpr int RUNS = 2 * RC_CHUNK * (DK / 8) / RC_THREADS;
+#pragma unroll 1
+    for (int j0 = 0; j0 < RUNS; j0 += 2) {
+        Rot8<T> run[2];
 #pragma unroll
-        for (int x = 0; x < 8; ++x) dst[x * RF_LDN] = which ? f[x] * k_scale : f[x];
+        for (int e = 0; e < 2; ++e) {
+            const int i = threadIdx.x + (j0 + e) * RC_THREADS, which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
+            const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
+            const size_t t = (size_t)(tok0 + (r < n ? r : 0));
+            run[e].load(which ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
+                        rope ? rope + t * rot : nullptr, d, rot);
+        }
+#pragma unroll
+        for (int e = 0; e < 2; ++e) {
+            const int i = threadIdx.x + (j0 + e) * RC_THREADS, which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
+            const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
+            float f[8];
+            run[e].values(rope != nullptr, d, rot, act, f);
+            float* dst = (which ? KV : Qt) + d * RF_LDN + ft_swizzle(r, d, 3);
+#pragma unroll
+            for (int x = 0; x < 8; ++x) dst[x * RF_LDN] = r >= n ? 0.f : which ? f[x] * k_scale : f[x];
+        }
     }
     __syncthreads();
     {
@@ -729,7 +773,8 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
         __syncthreads();                                 // K (or the last slice's V) and P have been read
 #pragma unroll
         for (int s = 0; s < RF_PSTAGES - 1; ++s) load_p(s);
-        rf_load_v(KV, v, v_stride, h, dv, c0, tok0, n, act);
+        Raw8<T> vr[RF_V_RUNS];
+        rf_ask_v(vr, v, v_stride, h, dv, c0, tok0, n);
         FmaTile<1, 2, 16, 16> o;                         // 64 x 128
         o.ty = ty;
         o.tx = tx;
@@ -740,6 +785,7 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
             load_p(turn + RF_PSTAGES - 1);
             o.template add_swizzled<3, false>(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS,
                                      turn * RF_PK, RF_PK);
+            if (turn == 0) rf_put_v(KV, vr, dv, c0, n, act);    // seen past the next turn's barrier
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) o.scale_row(i, pw[4 * ty + i + 1]);
