@@ -327,6 +327,27 @@ def test_attention_generic_tiles(H, Hkv, dh, ps, dtype, monkeypatch):
         assert not outs[0][-1].any()
 
 
+@pytest.mark.parametrize("H,Hkv", [(4, 4), (4, 2), (6, 2), (5, 1), (12, 2)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_attention_generic_tiles_keep_requests_apart(H, Hkv, dtype, monkeypatch):
+    """Groups of heads that do not fill a warp's rows, requests that meet inside a warp, one of them with
+    values that are not finite: the others' rows are finite and every row is that of a warp a query."""
+    def crafted(b, K, V):
+        if b == 1:
+            V[0], V[1, :, ::2], V[5] = float("nan"), float("inf"), float("-inf")
+    case = paged_case([6, 3, 1, 9, 2], [40, 35, 70, 0, 33], H, Hkv, 36, 8, dtype, seed=H, crafted=crafted)
+    outs = []
+    for start in (4, 10 ** 9):
+        monkeypatch.setattr(ops(), "GENERIC_TILES_FROM", start)
+        outs.append(torch.full_like(case["q"], 7.0))
+        ops().attention_generic(case["q"], outs[-1], H, Hkv, 36, case["kc"], case["vc"], 8, case["bt"], case["seq"],
+                                case["pos"], 36 ** -0.5, 0)
+    others = case["seq"] != 1
+    assert bool(torch.isfinite(outs[1][others].float()).all()) and bool(torch.isnan(outs[1][~others].float()).any())
+    assert torch.equal(torch.isnan(outs[0]), torch.isnan(outs[1]))
+    assert torch.equal(outs[0].nan_to_num(nan=5.0), outs[1].nan_to_num(nan=5.0))
+
+
 @pytest.mark.parametrize("H,Hkv,dh,ps", SHAPES)
 @pytest.mark.parametrize("window", [0, 100])
 def test_attention_decode_split(H, Hkv, dh, ps, window):

@@ -241,7 +241,8 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
 #pragma unroll
                 for (int r = 0; r < AGT_R; ++r) {
                     const float wj = __shfl_sync(0xffffffffu, w[r], jj);
-                    if (k0 + jj > pos[r]) continue;      // past this row's keys: nothing is added, not even 0 x NaN
+                    // another request's keys, or past this row's: nothing is added, not even 0 x NaN
+                    if (tok[r] < ta || tok[r] >= tb || k0 + jj > pos[r]) continue;
 #pragma unroll
                     for (int i = 0; i < NV; ++i) {
                         acc[r][i].x = fmaf(wj, v4[i].x, acc[r][i].x);
