@@ -170,3 +170,25 @@ extern "C" int negative() { return -3; }
                 fast(bad)
         with pytest.raises(TypeError):
             fast(*([0] * 49))
+
+
+def test_kernels_are_called_by_ctypes_where_the_extension_fails(monkeypatch, tmp_path, capfd):
+    """The extension that calls the kernels does not compile, or what was built does not load: ctypes calls
+    them, and building everything goes on. A library of kernels that fails still raises."""
+    from tgo_b200.kernels import build as kb
+    broken = tmp_path / "broken.so"
+    broken.write_bytes(b"no library")
+
+    def fails(name, **kw):
+        raise kb.KernelBuildError(f"the compiler failed on {name}")
+    for compiles in (fails, lambda name, **kw: str(broken)):
+        monkeypatch.setattr(kb, "compile_library", compiles)
+        assert kb._find_binder() is kb._bind_ctypes
+        assert "ctypes" in capfd.readouterr().err
+    monkeypatch.setattr(kb, "compile_library", lambda name, verbose=True: fails(name))
+    monkeypatch.setattr(kb, "library_path", lambda name: str(tmp_path / name))
+    monkeypatch.setattr(kb, "LIBRARIES", {"fastcall": kb.LIBRARIES["fastcall"]})
+    kb.build_all(verbose=False)
+    monkeypatch.setattr(kb, "LIBRARIES", {"fastcall": ([], []), "other": ([], []), "third": ([], [])})
+    with pytest.raises(kb.KernelBuildError, match="other|third"):
+        kb.build_all(verbose=False)

@@ -53,6 +53,7 @@ LIBRARIES = {
     # calls of the other libraries' entry points (a Python extension; see `entry_points`)
     "fastcall": (["fastcall.cpp"], []),
 }
+OPTIONAL = ("fastcall",)         # the package runs without, a little slower
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 PYTHON_INCLUDE = sysconfig.get_paths()["include"]
 
@@ -235,16 +236,22 @@ _entries = {}
 
 
 def _find_binder():
+    """What turns an address into a callable: the extension, or ctypes where the calling convention or the
+    Python headers are missing and where the extension does not compile or load."""
     import platform
     if platform.machine() != "x86_64" or not sys.platform.startswith("linux") or \
             not os.path.exists(os.path.join(PYTHON_INCLUDE, "Python.h")):
         return _bind_ctypes
     import importlib.machinery
     import importlib.util
-    path = compile_library("fastcall")
-    loader = importlib.machinery.ExtensionFileLoader("tgo_fastcall", path)
-    module = importlib.util.module_from_spec(importlib.util.spec_from_loader("tgo_fastcall", loader))
-    loader.exec_module(module)
+    try:
+        path = compile_library("fastcall")
+        loader = importlib.machinery.ExtensionFileLoader("tgo_fastcall", path)
+        module = importlib.util.module_from_spec(importlib.util.spec_from_loader("tgo_fastcall", loader))
+        loader.exec_module(module)
+    except (KernelBuildError, ImportError, OSError) as e:
+        _say(f"[tgo_b200] the kernels are called by ctypes: {str(e)[:500]}")
+        return _bind_ctypes
     return lambda fn: module.bind(ctypes.cast(fn, ctypes.c_void_p).value)
 
 
@@ -262,6 +269,15 @@ def entry_points(name: str):
     return got
 
 
+def _compile_or_do_without(name: str, verbose: bool) -> None:
+    try:
+        compile_library(name, verbose=verbose)
+    except KernelBuildError as e:
+        if name not in OPTIONAL:
+            raise
+        _say(f"[tgo_b200] {name} is done without: {str(e)[:500]}")
+
+
 def compile_together(names, verbose: bool = True) -> None:
     """Build several libraries at once, a compiler process each (a model's first step would
     otherwise build the ones it needs one after the other as it reaches them)."""
@@ -269,14 +285,14 @@ def compile_together(names, verbose: bool = True) -> None:
     todo = [n for n in dict.fromkeys(names) if n not in _loaded and not os.path.exists(library_path(n))]
     if len(todo) <= 1:
         for n in todo:
-            compile_library(n, verbose=verbose)
+            _compile_or_do_without(n, verbose)
         return
     with ThreadPoolExecutor(max_workers=min(len(todo), os.cpu_count() or 2, 8)) as pool:
-        for f in [pool.submit(compile_library, n, verbose) for n in todo]:
+        for f in [pool.submit(_compile_or_do_without, n, verbose) for n in todo]:
             f.result()
 
 
 def build_all(verbose: bool = True) -> None:
     compile_together(sorted(LIBRARIES), verbose=verbose)
     for name in sorted(LIBRARIES):           # whatever was there already is checked to exist
-        compile_library(name, verbose=verbose)
+        _compile_or_do_without(name, verbose)
