@@ -192,3 +192,23 @@ def test_kernels_are_called_by_ctypes_where_the_extension_fails(monkeypatch, tmp
     monkeypatch.setattr(kb, "LIBRARIES", {"fastcall": ([], []), "other": ([], []), "third": ([], [])})
     with pytest.raises(kb.KernelBuildError, match="other|third"):
         kb.build_all(verbose=False)
+
+
+def test_python_extension_is_built_for_each_interpreter(monkeypatch, tmp_path):
+    """A build folder shared by interpreters of unlike binary interfaces holds an extension for each, and
+    building one leaves the other's."""
+    from tgo_b200.kernels import build as kb
+    if kb.find_host_compiler() is None or kb._find_binder() is kb._bind_ctypes:
+        pytest.skip("no extension here")
+    monkeypatch.setattr(kb, "_build_dir_found", str(tmp_path))
+    mine, books = kb.library_path("fastcall"), kb.library_path("host_runtime")
+    with monkeypatch.context() as m:
+        m.setattr(kb.sysconfig, "get_config_var", lambda name: "cpython-399td-x86_64-linux-gnu")
+        other = kb.library_path("fastcall")
+        assert kb.library_path("host_runtime") == books
+    assert other != mine
+    with open(other, "w") as f:
+        f.write("another interpreter's")
+    assert kb.compile_library("fastcall", verbose=False) == mine
+    import os
+    assert os.path.exists(other) and os.path.exists(mine)

@@ -54,6 +54,7 @@ LIBRARIES = {
     "fastcall": (["fastcall.cpp"], []),
 }
 OPTIONAL = ("fastcall",)         # the package runs without, a little slower
+PYTHON_LIBRARIES = ("fastcall",)  # compiled against the Python headers: good for one binary interface
 HOST_FLAGS = ["-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden"]
 PYTHON_INCLUDE = sysconfig.get_paths()["include"]
 
@@ -135,9 +136,17 @@ def _digest(sources, link_flags) -> str:
     return h.hexdigest()[:16]
 
 
+def _file_stem(name: str) -> str:
+    """What the names of a library's builds begin with. The folder may be shared by several interpreters:
+    what is compiled against Python's headers names the interface it was compiled for."""
+    if name in PYTHON_LIBRARIES:
+        return f"libtgo_{name}.{sysconfig.get_config_var('SOABI') or sys.implementation.cache_tag}_"
+    return f"libtgo_{name}_"
+
+
 def library_path(name: str) -> str:
     sources, link_flags = LIBRARIES[name]
-    return os.path.join(_build_dir(), f"libtgo_{name}_{_digest(sources, link_flags)}.so")
+    return os.path.join(_build_dir(), f"{_file_stem(name)}{_digest(sources, link_flags)}.so")
 
 
 def compile_library(name: str, verbose: bool = True, ptxas_info: bool = False) -> str:
@@ -179,7 +188,7 @@ def compile_library(name: str, verbose: bool = True, ptxas_info: bool = False) -
         raise KernelBuildError(f"the compiler failed on {name}:\n{' '.join(cmd)}\n{text}")
     os.replace(tmp, out)
     # older builds of the same library (other source hashes) are of no use any more
-    prefix = f"libtgo_{name}_"
+    prefix = _file_stem(name)
     for other in os.listdir(os.path.dirname(out)):
         if other.startswith(prefix) and other.endswith(".so") and \
                 os.path.join(os.path.dirname(out), other) != out:
