@@ -212,3 +212,20 @@ def test_python_extension_is_built_for_each_interpreter(monkeypatch, tmp_path):
     assert kb.compile_library("fastcall", verbose=False) == mine
     import os
     assert os.path.exists(other) and os.path.exists(mine)
+
+
+def test_engine_compiles_all_it_calls_at_once(monkeypatch):
+    """Everything an engine on a GPU will load is compiled when it is made, side by side: the libraries its
+    model names, the books, and what calls the kernels."""
+    import types
+
+    import torch
+    from tgo_b200.engine import step
+    asked = []
+    monkeypatch.setattr(step, "compile_together", lambda names, **kw: asked.extend(names))
+    monkeypatch.setattr(step, "NativeCacheManager", lambda *a: None)
+    monkeypatch.setattr(step, "CacheStorage", lambda *a: None)
+    model = types.SimpleNamespace(device=torch.device("cuda"), groups=[], dtype=torch.bfloat16, state_shapes=[],
+                                  libraries=lambda page_size: ["moe", "gemm_tc"])
+    step.Engine(model, max_tokens=64)
+    assert {"host_runtime", "fastcall", "moe", "gemm_tc"} <= set(asked)

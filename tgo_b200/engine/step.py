@@ -56,7 +56,7 @@ class Engine:
         if self.device.type == "cuda":
             # the libraries the model's parts say they call, compiled side by side (each
             # would otherwise be built when the first step reaches it, one after the other)
-            compile_together(["host_runtime"] + model.libraries(page_size))
+            compile_together(["host_runtime", "fastcall"] + model.libraries(page_size))
         pages = [num_pages for _ in model.groups]
         # the books and the packing of a step are kept by the native host library
         self.cache = NativeCacheManager(model.groups, page_size, pages, num_slots)
