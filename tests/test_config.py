@@ -229,3 +229,40 @@ def test_engine_compiles_all_it_calls_at_once(monkeypatch):
                                   libraries=lambda page_size: ["moe", "gemm_tc"])
     step.Engine(model, max_tokens=64)
     assert {"host_runtime", "fastcall", "moe", "gemm_tc"} <= set(asked)
+
+
+@pytest.mark.parametrize("which", ["grouped", "latent"])
+def test_counters_live_until_the_launch(which, monkeypatch):
+    """The counters a launch draws its items from are still held when the launch is made: memory that went
+    back to the allocator before it may be another thread's by then."""
+    import gc
+    import types
+    import weakref
+
+    import torch
+    from tgo_b200.kernels import ops
+    made, launched = [], []
+    empty = torch.empty
+
+    def recorded(*a, **kw):
+        t = empty(*a, **kw)
+        made.append(weakref.ref(t))
+        return t
+
+    def launch(*args):
+        gc.collect()
+        launched.append([r() is not None and r().data_ptr() in args for r in made])
+        return 0
+    fake = types.SimpleNamespace(tgo_attention_tc_prefill=launch, tgo_attention_latent_tc=launch)
+    for name, value in (("_need_cuda", lambda *a: None), ("_stream", lambda: 0), ("entry_points", lambda name: fake)):
+        monkeypatch.setattr(ops, name, value)
+    i32 = torch.zeros(4, dtype=torch.int32)
+    q, out = torch.zeros(4, 256, dtype=torch.bfloat16), torch.zeros(4, 256, dtype=torch.bfloat16)
+    cache = torch.zeros(3, 1, 16, 128, dtype=torch.bfloat16)
+    monkeypatch.setattr(torch, "empty", recorded)
+    if which == "grouped":
+        ops.attention_tc_prefill(q, out, 2, 1, 128, cache, cache, 16, i32.view(2, 2), i32, i32, i32, i32, 0.1, 0,
+                                 own_counters=True)
+    else:
+        ops.attention_latent_tc(q, out, 2, 128, 64, cache, 16, i32.view(2, 2), i32, i32, 0.1, 0, None, i32, i32)
+    assert launched == [[True]]

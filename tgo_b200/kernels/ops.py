@@ -627,12 +627,12 @@ def attention_latent_tc(q: torch.Tensor, out: torch.Tensor, num_heads: int, key_
     assert block_tables.is_contiguous() and block_tables.dtype == torch.int32 and block_tables.dim() == 2
     assert sinks is None or (sinks.dtype == torch.float32 and sinks.numel() == num_heads)
     assert tile_tok0.dtype == tile_ntok.dtype == torch.int32
+    counter = torch.empty(1, dtype=torch.int32, device=q.device)
     _check(entry_points("attention_latent_tc").tgo_attention_latent_tc(
         _ptr(q), c_ll(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_ll(out.stride(0)), _ptr(cache),
         c_int(cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(positions),
         _ptr(seq_ids), _ptr(tile_tok0), _ptr(tile_ntok), c_int(tile_tok0.numel()), c_int(num_heads), c_int(key_dim),
-        c_int(value_dim), c_float(scale), c_int(window), _ptr(sinks),
-        _ptr(torch.empty(1, dtype=torch.int32, device=q.device)), _stream()), "attention_latent_tc",
+        c_int(value_dim), c_float(scale), c_int(window), _ptr(sinks), _ptr(counter), _stream()), "attention_latent_tc",
         f"(heads={num_heads}, dk={key_dim}, dv={value_dim})")
 
 
@@ -1958,6 +1958,7 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
     assert k_cache.shape == v_cache.shape and k_cache.shape[1:] == (num_kv_heads, page_size, head_dim)
     assert block_tables.dtype == torch.int32 and block_tables.is_contiguous()
     lib = entry_points("attention_tc")
+    counters = torch.empty(2, dtype=torch.int32, device=q.device) if own_counters else None
     _check(lib.tgo_attention_tc_prefill(
         _ptr(q), c_ll(q.stride(0)), c_int(q.shape[0]), _ptr(out), c_ll(out.stride(0)), _ptr(k_cache), _ptr(v_cache),
         c_int(k_cache.shape[0]), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]),
@@ -1966,8 +1967,7 @@ def attention_tc_prefill(q: torch.Tensor, out: torch.Tensor, num_heads: int, num
         _ptr(sinks), c_float(softcap or 0.0), c_int(keep_first), _ptr(dist_bias),
         c_int(dist_bias.shape[0] if dist_bias is not None else 0), _ptr(gate),
         c_ll(gate.stride(0) if gate is not None else 0),
-        _ptr(torch.empty(2, dtype=torch.int32, device=q.device) if own_counters else None),
-        _stream()), "attention_tc_prefill",
+        _ptr(counters), _stream()), "attention_tc_prefill",
         f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads}, page_size={page_size})")
 
 
