@@ -114,15 +114,20 @@ __global__ void attention_generic_kernel(
 // ------------------------------------------------------------- prompt portions, every earlier key
 // The same sums in the same order, for steps that bring several tokens a request and see every
 // earlier key (window 0: the keys are then cut into the same 32 for every query). A block takes
-// AGT_Q query rows (the heads of one kv head x consecutive tokens) and brings each 32 keys and
-// values into shared memory once for all of them; a warp owns AGT_R rows, a lane one key for the
-// scores and 4 NV channels for the sums. Bound by reads of shared memory (a 16-byte read of a key
-// row feeds 4 AGT_R FMA). Rows of another request in the block are walked after the first's.
+// AGT_Q query rows (the heads of one kv head x consecutive tokens of one request) and brings each 32
+// keys and values into shared memory once for all of them; a warp owns AGT_R rows, a lane one key for
+// the scores and 4 NV channels for the sums. Bound by reads of shared memory (a 16-byte read of a key
+// row feeds 4 AGT_R FMA). The first `n_blocks` blocks of a kv head take the first run of tokens of one
+// request among their AGT_Q / G tokens; where requests meet inside those, the runs that begin there go
+// to the blocks behind them, so that no request waits for another's keys.
 // The caller picks this kernel from four tokens a request on (bits do not depend on it): MEASURED
-// (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this about 140.
+// (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this about 140; 64 tokens beside
+// fifteen single ones of 1000 keys, 16/4 heads of 128: 946 and 302 us (1258 when a block walked the requests
+// that meet in it in turn), 8/8 heads of 64: 556 and 178 (2691).
 #define AGT_WARPS 4
 #define AGT_R 4
 #define AGT_Q (AGT_WARPS * AGT_R)
+#define AGT_MAX_SMEM ((int)((32 * (AG_MAX_DH + 4) + 32 * AG_MAX_DH + AGT_Q * AG_MAX_DH) * sizeof(float)))
 
 __device__ __forceinline__ float4 ag_load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 ag_load4(const bf16* p) {
@@ -131,10 +136,38 @@ __device__ __forceinline__ float4 ag_load4(const bf16* p) {
     return make_float4(a.x, a.y, b.x, b.y);
 }
 
+// The request of a token, -1 for one that brings nothing.
+__device__ __forceinline__ int agt_request(const int* __restrict__ positions, const int* __restrict__ seq_ids, int t) {
+    return positions[t] >= 0 ? seq_ids[t] : -1;
+}
+
+// The token where the k-th run begins that does not begin with a block's tokens, or -1. The whole block calls.
+__device__ __forceinline__ int agt_run(int k, int nt, int Tn, const int* __restrict__ positions, const int* __restrict__ seq_ids) {
+    __shared__ int s_before[AGT_WARPS], s_at;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    for (int base = 0, seen = 0; base < Tn; base += 32 * AGT_WARPS) {
+        const int t = base + threadIdx.x;
+        const bool begins = t < Tn && t % nt && agt_request(positions, seq_ids, t) != agt_request(positions, seq_ids, t - 1);
+        const unsigned ballot = __ballot_sync(0xffffffffu, begins);
+        if (lane == 0) s_before[warp] = __popc(ballot);
+        const int n = __syncthreads_count(begins);
+        if (k < seen + n) {
+            int rank = seen + __popc(ballot & ((1u << lane) - 1u));
+            for (int w = 0; w < warp; ++w) rank += s_before[w];
+            if (begins && rank == k) s_at = t;
+            __syncthreads();
+            return s_at;
+        }
+        seen += n;
+        __syncthreads();                                 // s_before is written again
+    }
+    return -1;
+}
+
 template <typename T, int NV>
-__global__ void __launch_bounds__(32 * AGT_WARPS)
+__global__ void __launch_bounds__(32 * AGT_WARPS, NV == 1 ? 4 : 2)
 attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* __restrict__ out, long long out_stride,
-                               int Tn, int H, int Hkv, int dh, int dv, const T* __restrict__ k_cache,
+                               int Tn, int n_blocks, int H, int Hkv, int dh, int dv, const T* __restrict__ k_cache,
                                const T* __restrict__ v_cache, int page_size, const int* __restrict__ block_tables,
                                int max_blocks, const int* __restrict__ seq_ids, const int* __restrict__ positions,
                                float scale, const float* __restrict__ sinks, float softcap, int v_row,
@@ -147,32 +180,30 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
     float* qs = vs + 32 * dv;                            // [AGT_Q][dh]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int G = H / Hkv, kvh = blockIdx.y;
-    const int nt = AGT_Q / G, nq = nt * G;               // tokens and rows of a block (G <= AGT_Q)
-    const int t0 = blockIdx.x * nt, t_end = t0 + nt < Tn ? t0 + nt : Tn;
-    for (int i = threadIdx.x; i < nq * dh; i += blockDim.x) {
-        const int r = i / dh, t = t0 + r / G;
-        qs[i] = t < t_end ? to_f32(q[(size_t)t * q_stride + (size_t)(kvh * G + r % G) * dh + i % dh]) : 0.f;
-    }
-    float m[AGT_R], l[AGT_R];
-    float4 acc[AGT_R][NV];
-    int tok[AGT_R], pos[AGT_R];
+    const int nt = AGT_Q / G;                            // tokens of a block (G <= AGT_Q)
+    for (int run = blockIdx.x;; run += gridDim.x - n_blocks) {       // a first run, or the others a block has to take
+        const int t0 = run < n_blocks ? run * nt : agt_run(run - n_blocks, nt, Tn, positions, seq_ids);
+        if (t0 < 0) return;
+        const int b = agt_request(positions, seq_ids, t0);
+        int t_end = t0 + 1, p_last = positions[t0];
+        for (; t_end % nt && t_end < Tn && agt_request(positions, seq_ids, t_end) == b; ++t_end) p_last = max(p_last, positions[t_end]);
+        const int nq = (t_end - t0) * G;
+        for (int i = threadIdx.x; i < AGT_Q * dh; i += blockDim.x) {
+            const int r = i / dh;
+            qs[i] = r < nq ? to_f32(q[(size_t)(t0 + r / G) * q_stride + (size_t)(kvh * G + r % G) * dh + i % dh]) : 0.f;
+        }
+        float m[AGT_R], l[AGT_R];
+        float4 acc[AGT_R][NV];
+        int tok[AGT_R], pos[AGT_R];
 #pragma unroll
-    for (int r = 0; r < AGT_R; ++r) {
-        const int row = warp * AGT_R + r;
-        m[r] = -INFINITY;
-        l[r] = 0.f;
-        tok[r] = row < nq ? t0 + row / G : t_end;
-        pos[r] = tok[r] < t_end ? positions[tok[r]] : -1;
+        for (int r = 0; r < AGT_R; ++r) {
+            const int row = warp * AGT_R + r;
+            m[r] = -INFINITY;
+            l[r] = 0.f;
+            tok[r] = row < nq ? t0 + row / G : t_end;
+            pos[r] = tok[r] < t_end ? positions[tok[r]] : -1;
 #pragma unroll
-        for (int i = 0; i < NV; ++i) acc[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    }
-    for (int ta = t0; ta < t_end;) {                     // a run of tokens of one request
-        int tb = ta + 1, p_last = positions[ta];
-        const int b = p_last >= 0 ? seq_ids[ta] : -1;
-        for (; tb < t_end; ++tb) {
-            const int p = positions[tb];
-            if ((p >= 0 ? seq_ids[tb] : -1) != b) break;
-            p_last = p > p_last ? p : p_last;
+            for (int i = 0; i < NV; ++i) acc[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         const int* bt = block_tables + (size_t)(b < 0 ? 0 : b) * max_blocks;
         for (int k0 = 0; k0 <= p_last; k0 += 32) {
@@ -192,6 +223,7 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
                 *(float4*)(vs + r * dv + c) = v;
             }
             __syncthreads();
+            if (warp * AGT_R >= nq) continue;            // none of the run's rows are this warp's
             float a[AGT_R], w[AGT_R];
 #pragma unroll
             for (int r = 0; r < AGT_R; ++r) a[r] = 0.f;
@@ -210,10 +242,9 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
             int most = 0;
 #pragma unroll
             for (int r = 0; r < AGT_R; ++r) {
-                const bool mine = tok[r] >= ta && tok[r] < tb && k0 <= pos[r];
                 const int p = pos[r], j = k0 + lane;
                 w[r] = 0.f;
-                if (!mine) continue;                     // the same for the whole warp
+                if (k0 > p) continue;                    // the same for the whole warp
                 float s = -INFINITY;
                 if (j <= p) {
                     s = a[r] * scale;
@@ -241,8 +272,7 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
 #pragma unroll
                 for (int r = 0; r < AGT_R; ++r) {
                     const float wj = __shfl_sync(0xffffffffu, w[r], jj);
-                    // another request's keys, or past this row's: nothing is added, not even 0 x NaN
-                    if (tok[r] < ta || tok[r] >= tb || k0 + jj > pos[r]) continue;
+                    if (k0 + jj > pos[r]) continue;      // past this row's keys: nothing is added, not even 0 x NaN
 #pragma unroll
                     for (int i = 0; i < NV; ++i) {
                         acc[r][i].x = fmaf(wj, v4[i].x, acc[r][i].x);
@@ -253,34 +283,35 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
                 }
             }
         }
-        ta = tb;
-    }
 #pragma unroll
-    for (int r = 0; r < AGT_R; ++r) {
-        if (tok[r] >= t_end) continue;
-        const int h = kvh * G + (warp * AGT_R + r) % G;
-        if (sinks && pos[r] >= 0) {                      // the sink joins the denominator last
-            const float sk = sinks[h];
-            const float m_new = fmaxf(m[r], sk);
-            const float corr = expf(m[r] - m_new);
-            l[r] = l[r] * corr + expf(sk - m_new);
+        for (int r = 0; r < AGT_R; ++r) {
+            if (tok[r] >= t_end) continue;
+            const int h = kvh * G + (warp * AGT_R + r) % G;
+            if (sinks && pos[r] >= 0) {                  // the sink joins the denominator last
+                const float sk = sinks[h];
+                const float m_new = fmaxf(m[r], sk);
+                const float corr = expf(m[r] - m_new);
+                l[r] = l[r] * corr + expf(sk - m_new);
+#pragma unroll
+                for (int i = 0; i < NV; ++i) {
+                    acc[r][i].x *= corr; acc[r][i].y *= corr; acc[r][i].z *= corr; acc[r][i].w *= corr;
+                }
+            }
+            float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
+            if (gate) inv *= 1.f / (1.f + expf(-to_f32(gate[(size_t)tok[r] * gate_stride + h])));
+            T* o = out + (size_t)tok[r] * out_stride + (size_t)h * dv;
 #pragma unroll
             for (int i = 0; i < NV; ++i) {
-                acc[r][i].x *= corr; acc[r][i].y *= corr; acc[r][i].z *= corr; acc[r][i].w *= corr;
+                const int d = (lane + 32 * i) * 4;
+                if (d >= dv) continue;
+                o[d] = from_f32<T>(acc[r][i].x * inv);
+                o[d + 1] = from_f32<T>(acc[r][i].y * inv);
+                o[d + 2] = from_f32<T>(acc[r][i].z * inv);
+                o[d + 3] = from_f32<T>(acc[r][i].w * inv);
             }
         }
-        float inv = l[r] > 0.f ? 1.f / l[r] : 0.f;
-        if (gate) inv *= 1.f / (1.f + expf(-to_f32(gate[(size_t)tok[r] * gate_stride + h])));
-        T* o = out + (size_t)tok[r] * out_stride + (size_t)h * dv;
-#pragma unroll
-        for (int i = 0; i < NV; ++i) {
-            const int d = (lane + 32 * i) * 4;
-            if (d >= dv) continue;
-            o[d] = from_f32<T>(acc[r][i].x * inv);
-            o[d + 1] = from_f32<T>(acc[r][i].y * inv);
-            o[d + 2] = from_f32<T>(acc[r][i].z * inv);
-            o[d + 3] = from_f32<T>(acc[r][i].w * inv);
-        }
+        if (run < n_blocks) return;
+        __syncthreads();                                 // the run's queries, keys and values have been read
     }
 }
 
@@ -293,26 +324,35 @@ TGO_API int tgo_attention_generic_tiles_takes(int H, int Hkv, int dh, int dv, in
 
 TGO_API int tgo_attention_generic_tiles(const void* q, long long q_stride, void* out, long long out_stride, int dtype,
                                         int T, int H, int Hkv, int dh, int dv, const void* k_cache,
-                                        const void* v_cache, int page_size, const int* block_tables, int max_blocks,
-                                        const int* seq_ids, const int* positions, float scale, const float* sinks,
-                                        float softcap, int v_row, const float* dist_bias, int n_dist,
+                                        const void* v_cache, int page_size, const int* block_tables, int n_seqs,
+                                        int max_blocks, const int* seq_ids, const int* positions, float scale,
+                                        const float* sinks, float softcap, int v_row, const float* dist_bias, int n_dist,
                                         const void* gate, long long gate_stride, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (v_row <= 0) v_row = dv;
-    if (!tgo_attention_generic_tiles_takes(H, Hkv, dh, dv, v_row) || Hkv > 65535 || page_size <= 0 || max_blocks <= 0 ||
-        !(softcap >= 0.f) || (dist_bias && n_dist <= 0) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15) ||
+    if (!tgo_attention_generic_tiles_takes(H, Hkv, dh, dv, v_row) || Hkv > 65535 || page_size <= 0 || n_seqs <= 0 ||
+        max_blocks <= 0 || !(softcap >= 0.f) || (dist_bias && n_dist <= 0) || ((uintptr_t)k_cache & 15) || ((uintptr_t)v_cache & 15) ||
         (dtype != TGO_BF16 && dtype != TGO_F32))
         return TGO_E_BAD_ARG;
-    const int nt = AGT_Q / (H / Hkv);
-    const dim3 grid((T + nt - 1) / nt, Hkv);
+    // a block for the first run of every nt tokens, and as many as there are requests for the others
+    const int nt = AGT_Q / (H / Hkv), n_blocks = (T + nt - 1) / nt;
+    const dim3 grid(n_blocks + (n_seqs < T ? n_seqs : T), Hkv);
     const size_t smem = (size_t)(32 * (dh + 4) + 32 * dv + AGT_Q * dh) * sizeof(float);
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return (int)e;
+    if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
 #define AGT_GO(TT, NV)                                                                                         \
     do {                                                                                                        \
-        const cudaError_t e = cudaFuncSetAttribute(attention_generic_tiles_kernel<TT, NV>,                      \
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);     \
-        if (e != cudaSuccess) return (int)e;                                                                    \
+        static int sized[64] = {};                       /* per device: the shared memory asked for there */    \
+        if (sized[dev] < (int)smem) {                                                                           \
+            e = cudaFuncSetAttribute(attention_generic_tiles_kernel<TT, NV>,                                    \
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, AGT_MAX_SMEM);                \
+            if (e != cudaSuccess) return (int)e;                                                                \
+            sized[dev] = AGT_MAX_SMEM;                                                                          \
+        }                                                                                                       \
         attention_generic_tiles_kernel<TT, NV><<<grid, 32 * AGT_WARPS, smem, stream>>>(                         \
-            (const TT*)q, q_stride, (TT*)out, out_stride, T, H, Hkv, dh, dv, (const TT*)k_cache,                \
+            (const TT*)q, q_stride, (TT*)out, out_stride, T, n_blocks, H, Hkv, dh, dv, (const TT*)k_cache,      \
             (const TT*)v_cache, page_size, block_tables, max_blocks, seq_ids, positions, scale, sinks, softcap, \
             v_row, dist_bias, n_dist, (const TT*)gate, gate_stride);                                            \
     } while (0)

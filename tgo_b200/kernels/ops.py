@@ -244,8 +244,8 @@ def attention_generic(q: torch.Tensor, out: torch.Tensor, num_heads: int, num_kv
         _check(lib.tgo_attention_generic_tiles(
             _ptr(q), c_ll(q.stride(0)), _ptr(out), c_ll(out.stride(0)), c_int(dtype_code(q.dtype)), c_int(T),
             c_int(num_heads), c_int(num_kv_heads), c_int(head_dim), c_int(value_dim or head_dim), _ptr(k_cache),
-            _ptr(v_cache), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[1]), _ptr(seq_ids),
-            _ptr(positions), c_float(scale), _ptr(sinks), c_float(softcap or 0.0), c_int(value_row),
+            _ptr(v_cache), c_int(page_size), _ptr(block_tables), c_int(block_tables.shape[0]), c_int(block_tables.shape[1]),
+            _ptr(seq_ids), _ptr(positions), c_float(scale), _ptr(sinks), c_float(softcap or 0.0), c_int(value_row),
             _ptr(dist_bias), c_int(dist_bias.shape[0] if dist_bias is not None else 0), _ptr(gate),
             c_ll(gate.stride(0) if gate is not None else 0), _stream()), "attention_generic_tiles",
             f"(head_dim={head_dim}, heads={num_heads}/{num_kv_heads})")
