@@ -1135,6 +1135,40 @@ def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
     assert torch.equal(state[untouched], before[untouched])
 
 
+def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
+    """One request through the selective scan by chunks or in order: outputs and state."""
+    T = xbc.shape[0]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    y, state = torch.empty(T, H * P, device=DEV), torch.zeros(1, H * N * P, device=DEV)
+    monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1 if chunks else 1 << 30)
+    launches = o.LAUNCHES[0]
+    o.selective_scan(xbc, dt_raw, None, a_log, None, y, 1, H, G, N, P, i32([0, T]), i32([0]), state, 0)
+    assert o.LAUNCHES[0] == launches + (4 if chunks else 1)
+    return y, state
+
+
+@pytest.mark.parametrize("H,G,N,P", [(64, 8, 128, 64), (3, 1, 64, 64), (2, 1, 128, 128)])
+def test_selective_scan_by_chunks_looks_forward_only(H, G, N, P, monkeypatch):
+    """A number that is not finite at a token leaves every output before it as it is without it; one in x
+    leaves the other channels' too. Two heads a block and one."""
+    o, T = ops(), 200
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log = torch.linspace(-3.0, 1.0, H, device=DEV)
+    clean, _ = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P)
+    assert bool(torch.isfinite(clean).all())
+    for t in (0, 1, 14, 15, 40, 63, 64, 100, 199):
+        for bad in (float("nan"), float("inf"), float("-inf")):
+            for col in (9, H * P + 5, H * P + G * N + 7):                # of x, of B and of C
+                y = xbc.clone()
+                y[t, col] = bad
+                got, _ = chunked_scan(o, monkeypatch, y, dt_raw, a_log, H, G, N, P)
+                assert torch.equal(got[:t], clean[:t]), (t, bad, col)
+                assert not bool(torch.isfinite(got[t, :P]).all())
+                if col == 9:
+                    others = [c for c in range(H * P) if c != 9]
+                    assert torch.equal(got[:, others], clean[:, others]), (t, bad)
+
+
 @pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 1, 128, 64), (3, 3, 64, 128), (2, 2, 128, 128)])
 @pytest.mark.parametrize("lens", [[128], [1, 63, 64, 65, 200, 3], [700, 129]])
 def test_selective_scan_by_chunks(H, G, N, P, lens, monkeypatch):

@@ -666,18 +666,24 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const flo
                     *(float4*)(Ct + (e * 64 + cj) * SD_LD + 4 * g.ty) = make_float4(a[0], a[1], a[2], a[3]);
                 }
             }
+    bool odd = false;                                    // a value that is not finite among the chunk's
     for (int i = t; i < SD_CHUNK * (P / 4); i += EACH) {
         const int r = i / (P / 4), c = (i % (P / 4)) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < n) v = *(const float4*)(rows + (size_t)r * C + h * P + c);
         const float w = ds[hh][r];
-        *(float4*)(Sh + r * (P + 4) + c) = make_float4(v.x * w, v.y * w, v.z * w, v.w * w);
+        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
+        *(float4*)(Sh + r * (P + 4) + c) = v;
+        odd = odd || ft_not_finite(v);
     }
-    __syncthreads();
+    const bool triangle = __syncthreads_or(odd);
     if (!busy) return;
 #pragma unroll
     for (int i = 0; i < 4; ++i) o.scale_row(i, expf((float)ls[hh][4 * o.ty + i]));
-    o.add(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, min(n, 4 * (o.ty | (32 / TX - 1)) + 4));
+    // tokens past a row have factors of 0: added where all values are finite, left out where they are not
+    const int first_row = 4 * (o.ty & ~(32 / TX - 1)), end = min(n, 4 * (o.ty | (32 / TX - 1)) + 4);
+    o.add(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, triangle ? first_row : end);
+    if (triangle) o.add_triangle(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, first_row, end);
     const float Dh = D ? D[h] : 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
