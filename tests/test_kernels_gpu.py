@@ -1135,6 +1135,38 @@ def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
     assert torch.equal(state[untouched], before[untouched])
 
 
+@pytest.mark.parametrize("dk,dv", [(64, 136), (128, 256)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_retention_by_tiled_chunks_looks_forward_only(dk, dv, dtype):
+    """A value, key or query that is not finite at a token leaves every output before it, and the other
+    channels of the value, as they are without it."""
+    o, H, n = ops(), 2, 150
+    z = (rnd(n, H * (2 * dk + dv), seed=dk + dv) * 0.5).to(dtype)
+    C = o.retention_chunk_tokens()
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    nt = [min(C, n - a) for a in range(0, n, C)]
+
+    def run(z):
+        out, state = torch.empty(n, H * dv, device=DEV), torch.zeros(1, H, dk, dv, device=DEV)
+        o.retention_chunked(z[:, :H * dk], z[:, H * dk:2 * H * dk], z[:, 2 * H * dk:], out, 1, H, dk, dv,
+                            torch.tensor([0.9, 0.99], device=DEV), dk ** -0.5, None, 0, i32([0, n]), i32([0]), state,
+                            i32(list(range(0, n, C))), i32(nt), i32([0]))
+        return out
+    clean = run(z)
+    assert bool(torch.isfinite(clean).all())
+    for t in (0, 1, 6, 7, 37, 63, 64, 75, 149):
+        for bad in (float("nan"), float("inf"), float("-inf")):
+            for col in (3, H * dk + 5, 2 * H * dk + 9):                  # a query, a key and a value of head 0
+                y = z.clone()
+                y[t, col] = bad
+                got = run(y)
+                assert torch.equal(got[:t], clean[:t]), (t, bad, col)
+                assert not bool(torch.isfinite(got[t, :dv]).all()) and torch.equal(got[:, dv:], clean[:, dv:])
+                if col >= 2 * H * dk:
+                    others = [c for c in range(dv) if c != 9]
+                    assert torch.equal(got[:, others], clean[:, others]), (t, bad)
+
+
 def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
     """One request through the selective scan by chunks or in order: outputs and state."""
     T = xbc.shape[0]

@@ -571,7 +571,7 @@ __device__ __forceinline__ void rf_powers(float* pw, float g) {
 }
 
 // Columns c0 .. c0 + RF_SLICE - 1 of the chunk's values, rows past n and columns past dv zero: asked for,
-// then put into shared memory.
+// then put into shared memory; true if a thread's are not all finite.
 #define RF_V_RUNS (RC_CHUNK * (RF_SLICE / 8) / RC_THREADS)
 template <typename T>
 __device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[RF_V_RUNS], const T* __restrict__ v, long long v_stride, int h, int dv,
@@ -583,15 +583,19 @@ __device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[RF_V_RUNS], const T* __r
     }
 }
 template <typename T>
-__device__ __forceinline__ void rf_put_v(float* Vs, const Raw8<T> (&raw)[RF_V_RUNS], int dv, int c0, int n, int act) {
+__device__ __forceinline__ bool rf_put_v(float* Vs, const Raw8<T> (&raw)[RF_V_RUNS], int dv, int c0, int n, int act) {
+    bool odd = false;
 #pragma unroll
     for (int j = 0; j < RF_V_RUNS; ++j) {
         const int i = threadIdx.x + j * RC_THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
         float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
         if (r < n && c0 + c < dv) taken8(raw[j], act, f);
-        *(float4*)(Vs + r * RF_LDS + c) = make_float4(f[0], f[1], f[2], f[3]);
-        *(float4*)(Vs + r * RF_LDS + c + 4) = make_float4(f[4], f[5], f[6], f[7]);
+        const float4 lo = make_float4(f[0], f[1], f[2], f[3]), hi = make_float4(f[4], f[5], f[6], f[7]);
+        *(float4*)(Vs + r * RF_LDS + c) = lo;
+        *(float4*)(Vs + r * RF_LDS + c + 4) = hi;
+        odd = odd || ft_not_finite(lo) || ft_not_finite(hi);
     }
+    return odd;
 }
 
 template <typename T, int DK>
@@ -706,6 +710,7 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
     float* Ps = At + RC_CHUNK * RF_LDN;                  // [RF_PSTAGES][RF_PK][RF_LDS]
     float* KV = Ps + RF_PSTAGES * RF_PK * RF_LDS;        // K [DK][RF_LDN], later V [RC_CHUNK][RF_LDS]
     __shared__ float pw[RC_CHUNK + 1];
+    __shared__ int s_odd;                                // a value that is not finite among the slice's
     pdl_wait();
     const int ci = blockIdx.x, h = blockIdx.y;
     const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
@@ -756,8 +761,9 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
         }
     }
     const float* Pc = P + ((size_t)ci * H + h) * DK * dv;
-    // the warp's rows end at 4 ty + 3 of its upper half: later tokens of the chunk are zeros of A
-    const int j_end = min(n, 4 * (ty | 1) + 4);
+    // the warp's rows end at 4 ty + 3 of its upper half: later tokens of the chunk are zeros of A. So are those
+    // between a row and that end: added where all values are finite, left out where they are not.
+    const int first_row = 4 * (ty & ~1), j_end = min(n, 4 * (ty | 1) + 4);
     for (int c0 = blockIdx.z * RF_SLICE; c0 < dv; c0 += gridDim.z * RF_SLICE) {
         auto load_p = [&](int turn) {
             if (turn < DK / RF_PK) {
@@ -771,6 +777,7 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
             ft_commit();
         };
         __syncthreads();                                 // K (or the last slice's V) and P have been read
+        if (threadIdx.x == 0) s_odd = 0;
 #pragma unroll
         for (int s = 0; s < RF_PSTAGES - 1; ++s) load_p(s);
         Raw8<T> vr[RF_V_RUNS];
@@ -785,11 +792,12 @@ retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, cons
             load_p(turn + RF_PSTAGES - 1);
             o.template add_swizzled<3, false>(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS,
                                      turn * RF_PK, RF_PK);
-            if (turn == 0) rf_put_v(KV, vr, dv, c0, n, act);    // seen past the next turn's barrier
+            if (turn == 0 && rf_put_v(KV, vr, dv, c0, n, act)) s_odd = 1;     // seen past the next turn's barrier
         }
 #pragma unroll
         for (int i = 0; i < 4; ++i) o.scale_row(i, pw[4 * ty + i + 1]);
-        o.add(At, RF_LDN, KV, RF_LDS, j_end);
+        o.add(At, RF_LDN, KV, RF_LDS, s_odd ? first_row : j_end);
+        if (s_odd) o.add_triangle(At, RF_LDN, KV, RF_LDS, first_row, j_end);
 #pragma unroll
         for (int i = 0; i < 4; ++i)
             if (4 * ty + i < n)
