@@ -1199,6 +1199,26 @@ def test_selective_scan_by_chunks_looks_forward_only(H, G, N, P, monkeypatch):
                 if col == 9:
                     others = [c for c in range(H * P) if c != 9]
                     assert torch.equal(got[:, others], clean[:, others]), (t, bad)
+        y = dt_raw.clone()
+        y[t, 0] = float("nan")
+        got, _ = chunked_scan(o, monkeypatch, xbc, y, a_log, H, G, N, P)
+        assert torch.equal(got[:t], clean[:t]) and torch.equal(got[:, P:], clean[:, P:])
+        assert bool(torch.isnan(got[t:, :P]).all())
+
+
+@pytest.mark.parametrize("H,G,N,P", [(6, 3, 128, 64), (3, 1, 64, 128)])
+def test_selective_scan_by_chunks_with_decays_of_zero(H, G, N, P, monkeypatch):
+    """Heads whose state is gone after a token (exp(A_log) up to infinity in 32 bits): what the walk in order
+    gives, within the rounding of sums of at most N + 64 float32 terms."""
+    o, T = ops(), 300
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log = torch.linspace(60.0, 100.0, H, device=DEV)
+    a_log[0] = 0.0
+    got, state = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P)
+    want, state2 = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=False)
+    assert bool(torch.isfinite(want).all())
+    assert (got - want).norm() <= 6e-6 * want.norm() and (state - state2).norm() <= 6e-6 * state2.norm()
+    assert ((got - want).abs() <= 1e-4 * want.abs().clamp(min=1.0)).all()
 
 
 @pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 1, 128, 64), (3, 3, 64, 128), (2, 2, 128, 128)])

@@ -477,7 +477,10 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
             const float z = to_f32(dt_raw[(size_t)(tok0 + t) * dt_stride + h]) + bias;
             dt[i] = z > 20.f ? z : log1pf(expf(z));
         }
-        l[i] = -(double)A * (double)dt[i];
+        // A decay below 2^-369 is 0 in 32 bits, beside whatever it is multiplied by: held at exp(-256), so that
+        // differences of sums stay numbers where A is infinite. (NaN stays NaN.)
+        l[i] = t < n ? -(double)A * (double)dt[i] : 0.0;
+        if (l[i] < -256.0) l[i] = -256.0;
     }
     double incl = l[0] + l[1];
 #pragma unroll
@@ -485,9 +488,10 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
         const double a = __shfl_up_sync(0xffffffffu, incl, o);
         if (lane >= o) incl += a;
     }
+    const double before = __shfl_up_sync(0xffffffffu, incl, 1);
     const size_t at = ((size_t)ci * H + h) * SD_CHUNK + 2 * lane;
     *(float2*)(dts + at) = make_float2(dt[0], dt[1]);
-    *(double2*)(cum + at) = make_double2(incl - l[1], incl);
+    *(double2*)(cum + at) = make_double2((lane ? before : 0.0) + l[0], incl);
 }
 
 template <int N, int P>
