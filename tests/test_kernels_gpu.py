@@ -1086,6 +1086,31 @@ def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
 
 
+def test_routed_experts_activation_in_32_bits():
+    """SiLU of products far below zero. The products are sums of two exact numbers, so that the hidden rows
+    show the activation alone: within 2^-21 (the exponential's 2 units in the last place, a sum, a
+    product and a division of half a unit each: 2^-21.2) and one rounding to bfloat16 of the value in 64 bits."""
+    o, d = ops(), 256
+    a = torch.cat([torch.arange(-88, -64, 0.5), torch.arange(-64, -32, 0.25), torch.arange(-32, -16, 0.125),
+                   torch.arange(-16, 16, 0.25)])
+    x = torch.zeros(a.numel(), d)
+    x[:, 0], x[:, 1] = a, 1.0
+    wg, wu = torch.zeros(1, d, d), torch.zeros(1, d, d)
+    wg[0, :, 0], wg[0, :, 1], wu[0, :, 1] = 1.0, torch.arange(d) / 8192.0, 1.0
+    x, wg, wu, wd = (t.to(torch.bfloat16).to(DEV) for t in (x, wg, wu, torch.eye(d)[None]))
+    got = o.moe_feed_forward(x, torch.zeros(1, d, device=DEV), None, wg, wu, wd, 1, "silu").double()
+    z = x.double() @ wg[0].double().t()
+    want = z / (1.0 + torch.exp(-z))
+    half = torch.exp2(torch.floor(torch.log2(want.abs())) - 8)           # half of what bfloat16 is spaced by
+    assert o.moe_error() == 0 and torch.equal(got, got.to(torch.bfloat16).double())
+    assert ((got - want).abs() <= half + 2.0 ** -21 * want.abs()).all()
+    # a product that overflows to infinity keeps it, one to the other side is no number (0 x infinity)
+    x, wg = torch.zeros(2, d, dtype=x.dtype, device=DEV), torch.zeros_like(wg)
+    x[:, 1], x[0, 0], x[1, 0], wg[0, 0, 0] = 1.0, 3e38, -3e38, 2.0
+    got = o.moe_feed_forward(x, torch.zeros(1, d, device=DEV), None, wg, wu, wd, 1, "silu")
+    assert got[0, 0] == float("inf") and bool(torch.isnan(got[1, 0]))
+
+
 @pytest.mark.parametrize("dk,dv,rot,act", [(64, 8, 0, 0), (64, 128, 32, 1), (128, 136, 128, 0), (128, 256, 64, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):

@@ -517,10 +517,17 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
 
 __device__ int moe_error_flag = 0;
 
-// act of the products' results: the hardware's exponential and reciprocal for the sigmoid (relative
-// error about 2^-21; the result is rounded to bfloat16)
-__device__ __forceinline__ float moe_act_fast(float z, int act) {
-    return act == 0 ? __fdividef(z, 1.f + __expf(-z)) : moe_act(z, act);
+// act of the products' results. SiLU as z / (1 + e^-z) for z >= 0 and z e^z / (1 + e^z) below, so that the
+// divisor lies in [1, 2] and the quotient needs no scaling: the hardware's reciprocal and one correction by the
+// remainder, within 0.51 units in the last place. (With a plain division, whose rare cases are a branch an
+// element, 64 tokens took 64 us instead of 49.)
+__device__ __forceinline__ float moe_act_tile(float z, int act) {
+    if (act != 0) return moe_act(z, act);
+    const float e = expf(-fabsf(z)), d = 1.f + e, n = z >= 0.f ? z : z * e;
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(d));
+    const float q = n * r;
+    return z < __int_as_float(0x7f800000) ? fmaf(fmaf(-q, d, n), r, q) : z;
 }
 
 template <int MODE>
@@ -628,7 +635,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                     float v[32];
 #pragma unroll
                     for (int i = 0; i < 32; ++i)
-                        v[i] = moe_act_fast(__uint_as_float(a[i]), act) * (GATED ? __uint_as_float(u[GATED ? i : 0]) : 1.f);
+                        v[i] = moe_act_tile(__uint_as_float(a[i]), act) * (GATED ? __uint_as_float(u[GATED ? i : 0]) : 1.f);
                     // 64 bytes a row, pieces of 16 shifted by row so that neither side meets a bank twice
 #pragma unroll
                     for (int q = 0; q < 4; ++q)
