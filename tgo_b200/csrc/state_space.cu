@@ -755,16 +755,17 @@ TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, lon
            offset % 4 == 0;
 }
 
-// As tgo_selective_scan with dt_raw in bfloat16; ws: (T / tgo_ssd_chunk_tokens() + B) times (H (N P + 3
-// tgo_ssd_chunk_tokens()) + 4) floats, 16-byte aligned: a summary, the steps' sizes and logarithms, and
-// what each chunk is.
+// As tgo_selective_scan with dt_raw in bfloat16; ws: ws_floats floats, 16-byte aligned, at least (T /
+// tgo_ssd_chunk_tokens() + B) times (H (N P + 3 tgo_ssd_chunk_tokens()) + 4): a summary, the steps' sizes and
+// logarithms, and what each chunk is.
 TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long dt_stride, const float* dt_bias,
                          const float* A_log, const float* D, float* y, int T, int B, int H, int G, int N, int P,
                          const int* q_start, const int* state_slots, float* state, long long state_stride,
-                         long long ssm_offset, float* ws, cudaStream_t stream) {
+                         long long ssm_offset, float* ws, long long ws_floats, cudaStream_t stream) {
     if (B <= 0 || T <= 0) return 0;
     if (!tgo_ssd_takes(xbc, y, state, state_stride, ssm_offset, H, G, N, P) || C != H * P + 2 * G * N ||
-        state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16)
+        state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16 ||
+        ws_floats < (long long)(T / SD_CHUNK + B) * ((long long)H * (N * P + 3 * SD_CHUNK) + 4))
         return TGO_E_BAD_ARG;
 #define SD_GO(N, P)                                                                                                    \
     return ssd_go<N, P>(xbc, C, (const bf16*)dt_raw, dt_stride, dt_bias, A_log, D, y, T, B, H, G, q_start, state_slots, state, \

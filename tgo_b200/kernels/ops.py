@@ -1086,12 +1086,14 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
     if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and \
             lib.tgo_ssd_takes(_ptr(xbc), _ptr(y), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(heads),
                               c_int(groups), c_int(state_dim), c_int(value_dim)):
-        floats = (T // 64 + num_seqs) * (heads * (state_dim * value_dim + 3 * 64) + 4)   # as tgo_ssd_scan says
+        chunk = lib.tgo_ssd_chunk_tokens()
+        floats = (T // chunk + num_seqs) * (heads * (state_dim * value_dim + 3 * chunk) + 4)     # as tgo_ssd_scan says
         ws = torch.empty(floats, dtype=torch.float32, device=xbc.device)
         _check(lib.tgo_ssd_scan(
             _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y),
             c_int(T), c_int(num_seqs), c_int(heads), c_int(groups), c_int(state_dim), c_int(value_dim), _ptr(q_start),
-            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), _ptr(ws), _stream()), "ssd_scan",
+            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), _ptr(ws), c_ll(floats),
+            _stream()), "ssd_scan",
             f"(heads={heads}, groups={groups}, state={state_dim}, vdim={value_dim})")
         LAUNCHES[0] += 3
         return
