@@ -269,14 +269,14 @@ def test_counters_live_until_the_launch(which, monkeypatch):
 
 
 def test_chunked_scan_refuses_a_short_workspace():
-    """The library says how long a chunk is, and a workspace of one float less than its chunks need is
-    refused before anything is launched (the addresses below are never read)."""
+    """The library says how long a chunk is, and a workspace of one float less than its chunks need for one
+    head is refused before anything is launched (the addresses below are never read)."""
     from tgo_b200.kernels import ops
     from tgo_b200.kernels.build import entry_points
     lib = entry_points("state_space")
     T, B, H, G, N, P = 300, 3, 4, 2, 128, 64
     chunk = lib.tgo_ssd_chunk_tokens()
-    floats = (T // chunk + B) * (H * (N * P + 3 * chunk) + 4)
+    floats = (T // chunk + B) * (N * P + 3 * chunk + 4)
     at = 1 << 20
     for short in (floats - 1, 0, -1):
         assert lib.tgo_ssd_scan(at, H * P + 2 * G * N, at, H, 0, at, 0, at, T, B, H, G, N, P, at, at, at, H * N * P, 0, at,

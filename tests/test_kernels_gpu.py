@@ -1193,14 +1193,15 @@ def test_retention_by_tiled_chunks_looks_forward_only(dk, dv, dtype):
 
 
 def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
-    """One request through the selective scan by chunks or in order: outputs and state."""
+    """One request through the selective scan by chunks or in order (None: as the rule has it beyond the
+    shortest steps): outputs and state."""
     T = xbc.shape[0]
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
     y, state = torch.empty(T, H * P, device=DEV), torch.zeros(1, H * N * P, device=DEV)
-    monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1 if chunks else 1 << 30)
+    monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1 << 30 if chunks is False else 1)
     launches = o.LAUNCHES[0]
     o.selective_scan(xbc, dt_raw, None, a_log, None, y, 1, H, G, N, P, i32([0, T]), i32([0]), state, 0)
-    assert o.LAUNCHES[0] == launches + (4 if chunks else 1)
+    assert chunks is None or o.LAUNCHES[0] == launches + (4 if chunks else 1)
     return y, state
 
 
@@ -1244,6 +1245,42 @@ def test_selective_scan_by_chunks_with_decays_of_zero(H, G, N, P, monkeypatch):
     assert bool(torch.isfinite(want).all())
     assert (got - want).norm() <= 6e-6 * want.norm() and (state - state2).norm() <= 6e-6 * state2.norm()
     assert ((got - want).abs() <= 1e-4 * want.abs().clamp(min=1.0)).all()
+
+
+def test_selective_scan_by_chunks_takes_a_bounded_workspace():
+    """16000 tokens of 64 heads of 64 x 128 (a state's size a chunk and head: 525 MB) run in groups of heads
+    over at most 256 MB beside the result."""
+    o, T, H, G, N, P = ops(), 16000, 64, 8, 128, 64
+    xbc, dt_raw = torch.zeros(T, H * P + 2 * G * N, device=DEV), torch.zeros(T, H, dtype=torch.bfloat16, device=DEV)
+    y, state, i32 = torch.empty(T, H * P, device=DEV), torch.zeros(1, H * N * P, device=DEV), torch.int32
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    before = torch.cuda.memory_allocated()
+    o.selective_scan(xbc, dt_raw, None, torch.zeros(H, device=DEV), None, y, 1, H, G, N, P,
+                     torch.tensor([0, T], dtype=i32, device=DEV), torch.tensor([0], dtype=i32, device=DEV), state, 0)
+    torch.cuda.synchronize()
+    assert torch.cuda.max_memory_allocated() - before <= (256 << 20) + (1 << 20)
+    assert not y.any() and not state.any()
+
+
+@pytest.mark.parametrize("H,G,N,P", [(24, 4, 128, 64), (3, 1, 128, 64), (5, 1, 64, 128)])
+def test_selective_scan_by_chunks_in_groups_of_heads(H, G, N, P, monkeypatch):
+    """Heads in groups of every size, down to one, give the bits of all at once; none at all walks."""
+    o, T = ops(), 700
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log = torch.linspace(-3.0, 1.0, H, device=DEV)
+    y, state = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P)
+    a_head = 4 * (T // 64 + 1) * (N * P + 3 * 64 + 4)
+    for heads in sorted({1, 2, 3, H // 2 + 1} - {H}):
+        monkeypatch.setattr(o, "SSD_WORKSPACE_BYTES", heads * a_head)
+        launches = o.LAUNCHES[0]
+        y2, state2 = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=None)
+        assert (o.LAUNCHES[0] - launches) % 4 == 0 and o.LAUNCHES[0] - launches > 4
+        assert torch.equal(y, y2) and torch.equal(state, state2)
+    monkeypatch.setattr(o, "SSD_WORKSPACE_BYTES", 1000)
+    launches = o.LAUNCHES[0]
+    chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=None)
+    assert o.LAUNCHES[0] == launches + 1
 
 
 @pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 1, 128, 64), (3, 3, 64, 128), (2, 2, 128, 128)])

@@ -417,6 +417,8 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
 // (fma_tile.cuh), bound by the FMA pipes. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128): 711 us
 // by the walk above, 224 so (summaries 54, scan over the chunks 32, outputs 134, 148 with a head a block); error against 64 bits
 // 1.2e-7 (1.9e-7 by the walk).
+// The workspace is a state's size a chunk and head; a call whose workspace does not hold all heads takes
+// them in groups, one after the other over the same memory (heads do not meet; the sums are the same).
 // The walk stays for the float32 engine, whose sums do not depend on how a prompt is cut, for
 // steps of few tokens a request, and for other sizes.
 #define SD_CHUNK 64
@@ -496,7 +498,7 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
 
 template <int N, int P>
 __global__ void __launch_bounds__(N * P / 64, 512 / (N * P / 64))
-ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, const int4* __restrict__ chunks,
+ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int h0, const int4* __restrict__ chunks,
                      const float* __restrict__ dts, const double* __restrict__ cum, float* __restrict__ U) {
     constexpr int THREADS = N * P / 64;
     extern __shared__ __align__(16) float smem[];
@@ -505,10 +507,10 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, const i
     __shared__ float ws[SD_CHUNK];
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
-    const int h = blockIdx.y, n = ch.y;
+    const int h = h0 + blockIdx.y, n = ch.y;             // the workspace holds the group's gridDim.y heads
     if (n == 0) return;
     const float* rows = xbc + (size_t)ch.x * C;
-    const size_t at = ((size_t)blockIdx.x * H + h) * SD_CHUNK;
+    const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * SD_CHUNK;
     for (int i = threadIdx.x; i < n * (N / 4); i += THREADS) {
         const int r = i / (N / 4), c = (i % (N / 4)) * 4;
         ft_copy16(Bs + r * (N + 4) + c, rows + (size_t)r * C + H * P + (h / (H / G)) * N + c, true);
@@ -530,7 +532,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, const i
     t.tx = threadIdx.x % (P / 8);
     t.clear();
     t.add(Bs, N + 4, Vs, P + 4, n);
-    float* Uo = U + ((size_t)blockIdx.x * H + h) * N * P;
+    float* Uo = U + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * N * P;
 #pragma unroll
     for (int i = 0; i < 8; ++i)
 #pragma unroll
@@ -590,7 +592,7 @@ ssd_scan_kernel(int H, int NP, const int* __restrict__ q_start, const int* __res
 // registers, then A times v is added.
 template <int N, int P, int HEADS>
 __global__ void __launch_bounds__(HEADS * 2 * P, 512 / (HEADS * 2 * P))
-ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const float* __restrict__ D,
+ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first, const float* __restrict__ D,
                    const int4* __restrict__ chunks, const float* __restrict__ dts, const double* __restrict__ cum,
                    const float* __restrict__ U, float* __restrict__ y) {
     constexpr int EACH = 2 * P, THREADS = HEADS * EACH, TX = P / 8;        // 16 x TX threads a head, 4 x 8 outputs each
@@ -603,13 +605,13 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, const flo
     __shared__ float ds[HEADS][SD_CHUNK];
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
-    const int h0 = blockIdx.y * HEADS, hh = threadIdx.x / EACH, h = h0 + hh, t = threadIdx.x % EACH, n = ch.y;
+    const int h0 = first + blockIdx.y * HEADS, hh = threadIdx.x / EACH, h = h0 + hh, t = threadIdx.x % EACH, n = ch.y;
     if (n == 0) return;
     const float* rows = xbc + (size_t)ch.x * C;
     const float* brow = rows + H * P + (h0 / (H / G)) * N;
     const float* crow = brow + (size_t)G * N;
-    const size_t at = ((size_t)blockIdx.x * H + h) * SD_CHUNK;
-    const float* Sc = U + ((size_t)blockIdx.x * H + h) * N * P;
+    const size_t place = (size_t)(blockIdx.x * gridDim.y + blockIdx.y) * HEADS + hh, at = place * SD_CHUNK;
+    const float* Sc = U + place * N * P;
     float* Sh = Ss + hh * 64 * (P + 4);
     for (int i = t; i < SD_CHUNK; i += EACH) {
         ls[hh][i] = cum[at + i];
@@ -707,7 +709,7 @@ TGO_API int tgo_ssd_chunk_tokens() { return SD_CHUNK; }
 template <int N, int P>
 static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stride, const float* dt_bias, const float* A_log,
                   const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
-                  float* state, long long state_stride, long long offset, float* ws, cudaStream_t stream) {
+                  float* state, long long state_stride, long long offset, float* ws, long long ws_floats, cudaStream_t stream) {
     constexpr size_t s1 = (size_t)SD_CHUNK * (N + 4 + P + 4) * sizeof(float);
     constexpr int PAIR = P == 64 ? 2 : 1;                // heads a block of the outputs where a group has an even number
     constexpr size_t s3 = ((size_t)2 * 64 * SD_LD + 64 * (P + 4)) * sizeof(float);
@@ -724,27 +726,38 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
         sized[dev] = true;
     }
     const int n_chunks = T / SD_CHUNK + B;               // at least as many as there are
-    float* U = ws;
-    double* cum = (double*)(U + (size_t)n_chunks * H * N * P);
-    float* dts = (float*)(cum + (size_t)n_chunks * H * SD_CHUNK);
-    int4* chunks = (int4*)(dts + (size_t)n_chunks * H * SD_CHUNK);
-    int rc = tgo_launch_pdl(ssd_steps_kernel<bf16>, dim3(n_chunks, (H + 7) / 8), dim3(256), 0, stream, dt_raw, dt_stride, dt_bias,
-                            A_log, H, q_start, B, chunks, dts, cum);
-    if (rc) return rc;
-    rc = tgo_launch_pdl(ssd_summaries_kernel<N, P>, dim3(n_chunks, H), dim3(N * P / 64), s1, stream, xbc, C, H, G,
-                        (const int4*)chunks, (const float*)dts, (const double*)cum, U);
-    if (rc) return rc;
-    rc = tgo_launch_pdl(ssd_scan_kernel, dim3(B, H, (N * P / 4 + 255) / 256), dim3(256), 0, stream, H, N * P, q_start,
-                        state_slots, (const double*)cum, U, state, state_stride, offset);
-    if (rc) return rc;
-    // Two heads a block from more (chunk, head) pairs than multiprocessors: 2048 tokens of 64 heads 134 us
-    // against 148, 700 of 24 25.1 against 27.1; 160 of 8 (24 pairs) 24.4 against 20.7, 512 of 16 (144) 24.9
-    // against 21.3.
-    if (PAIR == 2 && H / G % 2 == 0 && (long long)n_chunks * H > 148)
-        return tgo_launch_pdl(ssd_outputs_kernel<N, P, PAIR>, dim3(n_chunks, H / PAIR), dim3(PAIR * 2 * P), s3p, stream, xbc, C,
-                              H, G, D, (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
-    return tgo_launch_pdl(ssd_outputs_kernel<N, P, 1>, dim3(n_chunks, H), dim3(2 * P), s3, stream, xbc, C, H, G, D,
-                          (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+    const bool pairs = PAIR == 2 && H / G % 2 == 0;
+    // heads a group: what the workspace holds, an even number where two share a block
+    long long each = (ws_floats / n_chunks - 4) / (N * P + 3 * SD_CHUNK);
+    if (each > H) each = H;
+    if (pairs && each > 1) each &= ~1ll;
+    for (int h0 = 0; h0 < H; h0 += (int)each) {
+        const int nh = H - h0 < each ? H - h0 : (int)each;
+        float* U = ws;
+        double* cum = (double*)(U + (size_t)n_chunks * nh * N * P);
+        float* dts = (float*)(cum + (size_t)n_chunks * nh * SD_CHUNK);
+        int4* chunks = (int4*)(dts + (size_t)n_chunks * nh * SD_CHUNK);
+        int rc = tgo_launch_pdl(ssd_steps_kernel<bf16>, dim3(n_chunks, (nh + 7) / 8), dim3(256), 0, stream, dt_raw + h0, dt_stride,
+                                dt_bias ? dt_bias + h0 : dt_bias, A_log + h0, nh, q_start, B, chunks, dts, cum);
+        if (rc) return rc;
+        rc = tgo_launch_pdl(ssd_summaries_kernel<N, P>, dim3(n_chunks, nh), dim3(N * P / 64), s1, stream, xbc, C, H, G, h0,
+                            (const int4*)chunks, (const float*)dts, (const double*)cum, U);
+        if (rc) return rc;
+        rc = tgo_launch_pdl(ssd_scan_kernel, dim3(B, nh, (N * P / 4 + 255) / 256), dim3(256), 0, stream, nh, N * P, q_start,
+                            state_slots, (const double*)cum, U, state, state_stride, offset + (long long)h0 * N * P);
+        if (rc) return rc;
+        // Two heads a block from more (chunk, head) pairs than multiprocessors: 2048 tokens of 64 heads 134 us
+        // against 148, 700 of 24 25.1 against 27.1; 160 of 8 (24 pairs) 24.4 against 20.7, 512 of 16 (144) 24.9
+        // against 21.3.
+        if (pairs && nh % 2 == 0 && (long long)n_chunks * nh > 148)
+            rc = tgo_launch_pdl(ssd_outputs_kernel<N, P, PAIR>, dim3(n_chunks, nh / PAIR), dim3(PAIR * 2 * P), s3p, stream, xbc, C,
+                                H, G, h0, D, (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+        else
+            rc = tgo_launch_pdl(ssd_outputs_kernel<N, P, 1>, dim3(n_chunks, nh), dim3(2 * P), s3, stream, xbc, C, H, G, h0, D,
+                                (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+        if (rc) return rc;
+    }
+    return 0;
 }
 
 // 1 if the chunked scan takes these sizes and places (places as addresses); bfloat16 engine only.
@@ -756,8 +769,8 @@ TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, lon
 }
 
 // As tgo_selective_scan with dt_raw in bfloat16; ws: ws_floats floats, 16-byte aligned, at least (T /
-// tgo_ssd_chunk_tokens() + B) times (H (N P + 3 tgo_ssd_chunk_tokens()) + 4): a summary, the steps' sizes and
-// logarithms, and what each chunk is.
+// tgo_ssd_chunk_tokens() + B) times (h (N P + 3 tgo_ssd_chunk_tokens()) + 4) for the h of the H heads that are
+// taken at a time (at least one): a summary, the steps' sizes and logarithms, and what each chunk is.
 TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long dt_stride, const float* dt_bias,
                          const float* A_log, const float* D, float* y, int T, int B, int H, int G, int N, int P,
                          const int* q_start, const int* state_slots, float* state, long long state_stride,
@@ -765,11 +778,11 @@ TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long 
     if (B <= 0 || T <= 0) return 0;
     if (!tgo_ssd_takes(xbc, y, state, state_stride, ssm_offset, H, G, N, P) || C != H * P + 2 * G * N ||
         state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16 ||
-        ws_floats < (long long)(T / SD_CHUNK + B) * ((long long)H * (N * P + 3 * SD_CHUNK) + 4))
+        ws_floats < (long long)(T / SD_CHUNK + B) * (N * P + 3 * SD_CHUNK + 4))
         return TGO_E_BAD_ARG;
 #define SD_GO(N, P)                                                                                                    \
     return ssd_go<N, P>(xbc, C, (const bf16*)dt_raw, dt_stride, dt_bias, A_log, D, y, T, B, H, G, q_start, state_slots, state, \
-                        state_stride, ssm_offset, ws, stream)
+                        state_stride, ssm_offset, ws, ws_floats, stream)
     if (N == 128) { if (P == 64) SD_GO(128, 64); SD_GO(128, 128); }
     if (P == 64) SD_GO(64, 64);
     SD_GO(64, 128);
