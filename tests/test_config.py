@@ -281,3 +281,12 @@ def test_chunked_scan_refuses_a_short_workspace():
     for short in (floats - 1, 0, -1):
         assert lib.tgo_ssd_scan(at, H * P + 2 * G * N, at, H, 0, at, 0, at, T, B, H, G, N, P, at, at, at, H * N * P, 0, at,
                                 short, 0) == ops.E_BAD_ARG
+
+
+@pytest.mark.parametrize("N,K,E,top,tokens", [(1536, 4096, 16, 2, (8, 16, 33, 64)), (768, 4096, 128, 8, (4,))])
+def test_routed_products_stay_off_the_narrowest_tiles(N, K, E, top, tokens):
+    """Decode batches for which tiles of 32 gated columns were slower than all wider ones (and than the
+    kernels before them): 108 us against 68 to 81 at the first, 173 against 85 to 98 at the fourth."""
+    from tgo_b200.kernels.build import entry_points
+    for T in tokens:
+        assert entry_points("moe").tgo_moe_tile_width(N, K, E, T * top, 1, 148) >= 64
