@@ -1086,6 +1086,38 @@ def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
 
 
+@pytest.mark.parametrize("T,E,identity,top", [(9, 4, 0, 2), (9, 4, 4, 3), (200, 4, 0, 2), (200, 4, 4, 3)])
+@pytest.mark.parametrize("strided", [False, True])
+def test_routed_experts_of_strided_rows_and_identities(T, E, identity, top, strided):
+    """Rows of x with a stride of their own and router outputs that stand for the row itself, with few rows
+    an expert (gathered) and many (copied in place order; identities have no place there)."""
+    o, d, ff = ops(), 136, 104
+    assert (T * top >= o.MOE_GATHER_ROWS * E) == (T == 200)
+    x = rnd(T, d + 24, seed=1).to(torch.bfloat16)[:, 8:d + 8] if strided else rnd(T, d, seed=1).to(torch.bfloat16)
+    wr = rnd(E + identity, d, seed=2) * d ** -0.5
+    wg, wu = ((rnd(E, ff, d, seed=s) * d ** -0.5).to(torch.bfloat16) for s in (3, 4))
+    wd = (rnd(E, d, ff, seed=5) * ff ** -0.5).to(torch.bfloat16)
+    got = o.moe_feed_forward(x, wr, None, wg, wu, wd, top, "silu", scores="all", identity=identity)
+    assert o.moe_error() == 0
+    p = torch.softmax(x.double() @ wr.double().t(), -1)
+    ids = torch.topk(p, top, -1).indices
+    wt = torch.gather(p, 1, ids)
+    wt = wt / wt.sum(-1, keepdim=True)
+    want, size = torch.zeros(T, d, dtype=torch.float64, device=DEV), torch.zeros(T, d, dtype=torch.float64, device=DEV)
+    for e in range(E + identity):
+        row, place = torch.nonzero(ids == e, as_tuple=True)
+        xe, we = x[row].double(), wt[row, place][:, None]
+        if e >= E:
+            want.index_add_(0, row, xe * we)
+            continue
+        h = torch.nn.functional.silu(xe @ wg[e].double().t()) * (xe @ wu[e].double().t())
+        want.index_add_(0, row, (h @ wd[e].double().t()) * we)
+        size.index_add_(0, row, (h.abs() @ wd[e].double().abs().t()) * we)
+    assert not identity or (ids >= E).any()
+    # hidden rows are rounded to bfloat16 (2^-9 each); the rest is float32
+    assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
+
+
 def test_routed_experts_activation_in_32_bits():
     """SiLU of products far below zero. The products are sums of two exact numbers, so that the hidden rows
     show the activation alone: within 2^-21 (the exponential's 2 units in the last place, a sum, a
@@ -1158,6 +1190,32 @@ def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
         assert (got - want).norm() <= 3e-6 * want.norm() and (state[slots[b]].double() - S).norm() <= 3e-6 * S.norm()
     untouched = [i for i in range(B + 2) if i not in slots]
     assert torch.equal(state[untouched], before[untouched])
+
+
+@pytest.mark.parametrize("lens", [[0, 70, 0, 0, 64, 0], [130, 0, 1]])
+def test_retention_by_tiled_chunks_beside_empty_requests(lens):
+    """Requests without tokens between others: the others' outputs and states, the same bits; theirs stay."""
+    o, H, dk, dv = ops(), 2, 64, 128
+    C, z = o.retention_chunk_tokens(), rnd(sum(lens), H * (2 * dk + dv), seed=5) * 0.5
+    state = rnd(len(lens), H, dk, dv, seed=1)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+
+    def run(lens, slots):
+        starts, t0, nt, first = [0], [], [], []
+        for n in lens:
+            first.append(len(t0))
+            t0 += range(starts[-1], starts[-1] + n, C)
+            nt += [min(C, n - a) for a in range(0, n, C)]
+            starts.append(starts[-1] + n)
+        out, s = torch.full((sum(lens), H * dv), float("nan"), device=DEV), state.clone()
+        o.retention_chunked(z[:, :H * dk], z[:, H * dk:2 * H * dk], z[:, 2 * H * dk:], out, len(lens), H, dk, dv,
+                            torch.tensor([0.9, 0.99], device=DEV), dk ** -0.5, None, 0, i32(starts), i32(slots), s,
+                            i32(t0), i32(nt), i32(first))
+        return out, s
+    full = [i for i, n in enumerate(lens) if n]
+    got, want = run(lens, list(range(len(lens)))), run([lens[i] for i in full], full)
+    assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
+    assert torch.equal(got[1][[i for i, n in enumerate(lens) if not n]], state[[i for i, n in enumerate(lens) if not n]])
 
 
 @pytest.mark.parametrize("dk,dv", [(64, 136), (128, 256)])
@@ -1245,6 +1303,31 @@ def test_selective_scan_by_chunks_with_decays_of_zero(H, G, N, P, monkeypatch):
     assert bool(torch.isfinite(want).all())
     assert (got - want).norm() <= 6e-6 * want.norm() and (state - state2).norm() <= 6e-6 * state2.norm()
     assert ((got - want).abs() <= 1e-4 * want.abs().clamp(min=1.0)).all()
+
+
+@pytest.mark.parametrize("lens", [[0, 70, 0, 0, 64, 0], [130, 0, 1]])
+def test_selective_scan_by_chunks_beside_empty_requests(lens, monkeypatch):
+    """Requests without tokens between others: the others' outputs and states, the same bits; theirs stay."""
+    o, H, G, N, P, T = ops(), 4, 2, 64, 64, sum(lens)
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=1), rnd(T, H, seed=3).to(torch.bfloat16)
+    state = rnd(len(lens), H * N * P, seed=6)
+    monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1)
+    monkeypatch.setattr(o, "SSD_TOKENS_A_REQUEST", 1)
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+
+    def run(lens, slots):
+        starts = [0]
+        for n in lens:
+            starts.append(starts[-1] + n)
+        y, s = torch.full((T, H * P), float("nan"), device=DEV), state.clone()
+        launches = o.LAUNCHES[0]
+        o.selective_scan(xbc, dt_raw, None, torch.linspace(-3.0, 1.0, H, device=DEV), None, y, len(lens), H, G, N, P,
+                         i32(starts), i32(slots), s, 0)
+        assert o.LAUNCHES[0] == launches + 4
+        return y, s
+    full = [i for i, n in enumerate(lens) if n]
+    got, want = run(lens, list(range(len(lens)))), run([lens[i] for i in full], full)
+    assert bool(torch.isfinite(got[0]).all()) and torch.equal(got[0], want[0]) and torch.equal(got[1], want[1])
 
 
 def test_selective_scan_by_chunks_takes_a_bounded_workspace():
@@ -1371,6 +1454,61 @@ def test_attention_latent_tc(H, dk, dv, ps, window, sink):
     assert o.attention_latent_tc_error() == 0
     assert bool(torch.isfinite(want).all())
     assert torch.allclose(out.float(), want, **tol(torch.bfloat16))
+
+
+def with_empty_requests(H, Hkv, dh, ps):
+    """Prompt portions and single tokens in turn, every other single token one that brings nothing, more than
+    a GPU's worth of items: blocks draw empty items between full ones, in both places of their rings."""
+    extents = [40, 1, 1, 150, 1, 1, 1, 5] * 40
+    firsts = [0, 30, 200, 60, 3, 500, 77, 9] * 40
+    case = paged_case(extents, firsts, H, Hkv, dh, ps, torch.bfloat16, seed=dh)
+    empty = torch.zeros(case["q"].shape[0], dtype=torch.bool, device=DEV)
+    t = 0
+    for i, n in enumerate(extents):
+        if n == 1 and i % 2:
+            empty[t] = True
+        t += n
+    case["pos"][empty] = -1
+    return case, empty
+
+
+@pytest.mark.parametrize("H,Hkv,dh,ps", [(4, 1, 64, 16), (8, 2, 128, 32)])
+@pytest.mark.parametrize("extra", ["none", "sink", "all"])
+def test_attention_tc_requests_that_bring_nothing(H, Hkv, dh, ps, extra):
+    """Zeros for the tokens that bring nothing; the others as the generic kernel has them."""
+    case, empty = with_empty_requests(H, Hkv, dh, ps)
+    o, T, scale = ops(), case["q"].shape[0], dh ** -0.5
+    kw = dict(softcap=2.0 if extra == "all" else 0.0, dist_bias=rnd(70, H, seed=1) if extra == "all" else None,
+              sinks=rnd(H, seed=2) if extra != "none" else None,
+              gate=rnd(T, H, seed=3).to(torch.bfloat16) if extra == "all" else None)
+    t0, nt = attention_part().step_tiles(Ctx(case, False), 128 // (H // Hkv))
+    out = torch.full_like(case["q"], 9.0)
+    o.attention_tc_prefill(case["q"], out, H, Hkv, dh, case["kc"], case["vc"], ps, case["bt"], case["pos"],
+                           case["seq"], t0, nt, scale, 100, own_counters=True, **kw)
+    want = torch.empty_like(case["q"].float())
+    kw["gate"] = kw["gate"].float() if kw["gate"] is not None else None
+    o.attention_generic(case["q"].float(), want, H, Hkv, dh, case["kc"].float(), case["vc"].float(), ps, case["bt"],
+                        case["seq"], case["pos"], scale, 100, **kw)
+    assert o.attention_tc_error() == 0 and bool(torch.isfinite(want).all())
+    assert not out[empty].any() and torch.allclose(out.float(), want, **tol(torch.bfloat16))
+
+
+@pytest.mark.parametrize("H,dk,dv,ps", [(16, 576, 512, 16), (40, 200, 64, 32)])
+@pytest.mark.parametrize("sink", [False, True])
+def test_attention_latent_tc_requests_that_bring_nothing(H, dk, dv, ps, sink):
+    """Zeros for the tokens that bring nothing; the others as the generic kernel has them."""
+    case, empty = with_empty_requests(H, 1, dk, ps)
+    o, T, scale = ops(), case["q"].shape[0], dk ** -0.5
+    sinks = rnd(H, seed=2) if sink else None
+    t0, nt = attention_part().step_tiles(Ctx(case, False), 128 // H)
+    out = torch.full((T, H * dv), 9.0, dtype=torch.bfloat16, device=DEV)
+    o.attention_latent_tc(case["q"], out, H, dk, dv, case["kc"], ps, case["bt"], case["seq"], case["pos"], scale, 0,
+                          sinks, t0, nt)
+    want, kc = torch.empty(T, H * dv, device=DEV), case["kc"].float()
+    o.attention_generic(case["q"].float(), want, H, 1, dk, kc, kc, ps, case["bt"], case["seq"], case["pos"], scale, 0,
+                        value_dim=dv, sinks=sinks, value_row=dk)
+    assert o.attention_latent_tc_error() == 0 and bool(torch.isfinite(want).all())
+    assert not out[empty].any() and torch.allclose(out.float(), want, **tol(torch.bfloat16))
 
 
 @pytest.mark.parametrize("H,Hkv,ps", [(16, 4, 16), (5, 1, 8), (12, 1, 32), (16, 2, 64)])
