@@ -21,8 +21,9 @@
 // MEASURED (B200, 2048 tokens of 16 heads, rows of 576, values of 512; mma.sync tiles of eight warps in
 // brackets): 130 us (511), 560 TFLOP/s of the products an ideal kernel would make.
 //
-// Every wait has a time limit (about two seconds), after which the CTA stops issuing, frees its
-// tensor memory and returns. No cluster, no multicast.
+// Every wait has a time limit (about two seconds), after which the CTA stops issuing, waits, with the same
+// limit, for its copies and products under way, frees its tensor memory and returns. No cluster, no
+// multicast.
 #include "tcgen.cuh"
 
 #define LT_THREADS 416
@@ -83,8 +84,9 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     uint64_t* p_free = bars + 18;        // [2]
     uint64_t* o_free = bars + 20;        // [1]
     uint64_t* o_done = bars + 21;        // [1]
-    uint32_t* tmem_slot = (uint32_t*)(bars + 22);
-    LtItem* ring = (LtItem*)(bars + 24);                 // [2]
+    uint64_t* settled = bars + 22;       // [2]: after a wait ran out, one an issuer
+    uint32_t* tmem_slot = (uint32_t*)(bars + 24);
+    LtItem* ring = (LtItem*)(bars + 26);                 // [2]
     float* s_xm = (float*)(ring + 2);                    // [2][2 halves][128 rows]
 
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -101,7 +103,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
         for (int i = 0; i < LT_K_SLOTS; ++i) { tg_init(&k_full[i], 1); tg_init(&k_empty[i], 1); }
         for (int i = 0; i < 2; ++i) {
             tg_init(&v_full[i], 1); tg_init(&v_empty[i], 1); tg_init(&v_ok[i], 1);
-            tg_init(&s_full[i], 1); tg_init(&p_full[i], 8); tg_init(&p_free[i], 1);
+            tg_init(&s_full[i], 1); tg_init(&p_full[i], 8); tg_init(&p_free[i], 1); tg_init(&settled[i], 1);
         }
         tg_init(o_free, 8);
         tg_init(o_done, 1);
@@ -121,7 +123,10 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             LtItem* rec = &ring[n & 1u];
             // the products with the last item's Q have run, and everybody has read its record
             ok = __all_sync(0xffffffffu, tg_wait(q_empty, (n & 1u) ^ 1u, err, 1));
-            if (!ok) break;
+            if (!ok) {
+                tg_settle_copies(q_full, 1, n, err, 1);
+                break;
+            }
             int item = 0;
             if (lane == 0) item = (int)atomicAdd(ticket, 1u);
             item = __shfl_sync(0xffffffffu, item, 0);
@@ -180,6 +185,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         }
+        if (!ok) tg_settle_copies(k_full, LT_K_SLOTS, g, err, 3);
     } else if (warp == 10) {
         // ---------------------------------------------------------- V
         bool ok = true;
@@ -199,9 +205,9 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     const int k0 = (rec.t_lo + it) * 128 + 32 * q;
                     if (k0 >= rec.key_hi || k0 + 32 <= rec.key_lo) continue;         // P is zero there
                     const uint32_t s = g % LT_V_SLOTS, ph = (g / LT_V_SLOTS) & 1u;
-                    ++g;
                     ok = __all_sync(0xffffffffu, tg_wait(&v_empty[s], ph ^ 1u, err, 5));
                     if (!ok) break;
+                    ++g;
                     unsigned char* slot = sV + s * LT_BLOCK;
                     // boxes whose rows somebody may read: [b_lo, b_hi)
                     int b_lo = 0, b_hi = vboxes;
@@ -232,6 +238,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         }
+        if (!ok) tg_settle_copies(v_full, LT_V_SLOTS, g, err, 5);
     } else if (warp == 1) {
         // ---------------------------------------------------------- issuer of S = Q K^T
         if (lane == 0) {
@@ -239,7 +246,8 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             uint32_t g = 0, t = 0;                       // K slots and key tiles so far
             bool ok = true;
             for (uint32_t n = 0; ok; ++n) {
-                if (!tg_wait(q_full, n & 1u, err, 7)) break;
+                ok = tg_wait(q_full, n & 1u, err, 7);
+                if (!ok) break;
                 const LtItem* rec = &ring[n & 1u];
                 if (!rec->valid) break;
                 const int n_it = rec->n_it;
@@ -260,6 +268,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
                 tg_commit(q_empty);                      // the item's products with Q have run
             }
+            if (!ok) tg_settle_products(&settled[0], err, 8);
         }
     } else if (warp == 11) {
         // ---------------------------------------------------------- issuer of O += P V
@@ -267,7 +276,8 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             uint32_t g = 0, t = 0, okph = 0;
             bool ok = true;
             for (uint32_t n = 0; ok; ++n) {
-                if (!tg_wait(q_full, n & 1u, err, 10)) break;
+                ok = tg_wait(q_full, n & 1u, err, 10);
+                if (!ok) break;
                 const LtItem rec = ring[n & 1u];
                 if (!rec.valid) break;
                 tg_arrive(q_empty);
@@ -302,6 +312,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     tg_commit(o_done);
                 }
             }
+            if (!ok) tg_settle_products(&settled[1], err, 12);
         }
     } else {
         // ---------------------------------------------------------- softmax

@@ -40,8 +40,9 @@
 // keys' tiles are walked before the window's. MEASURED, 2348 + 1611 tokens' worth of keys for 2048 +
 // 1536 queries of 16/4 heads of 128, window 1024, sink: 60 us; 390 us for the mma.sync tiles.
 //
-// Every wait has a time limit (about two seconds): it records a code, the CTA stops issuing,
-// frees its tensor memory and returns. No cluster, no multicast.
+// Every wait has a time limit (about two seconds): it records a code, the CTA stops issuing, waits, with
+// the same limit, for its copies and products under way, frees its tensor memory and returns. No cluster,
+// no multicast.
 #include <cuda.h>
 
 #include <mutex>
@@ -206,6 +207,16 @@ __device__ __forceinline__ uint32_t at_pack(float lo, float hi) {
 // warps have each read the record; so no waiter ever falls two phases behind a barrier.
 #define AP_THREADS 416
 
+// Before a CTA gives up: the last copies into a ring of two that `sent` copies have gone through are waited
+// for, and the products that a thread has issued (`bar` is used by nobody else), each with the time limit.
+__device__ __forceinline__ void at_settle_copies(uint64_t* full, uint32_t sent, int code) {
+    for (uint32_t j = sent > 2u ? sent - 2u : 0u; j < sent; ++j) at_wait(&full[j & 1u], (j >> 1) & 1u, code);
+}
+__device__ __forceinline__ void at_settle_products(uint64_t* bar, int code) {
+    at_commit(bar);
+    at_wait(bar, 0, code);
+}
+
 struct ApItem {          // what warp 0 tells the others about an item
     int valid;           // 0: no more items
     int tok0, n_rows, p0, n_it, t_lo, key_lo, key_hi, seq, kvh;
@@ -276,8 +287,9 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
     uint64_t* o_free = bars + 16;       // [2]
     uint64_t* o_done = bars + 18;       // [1]
     uint64_t* p_free = bars + 19;       // [2]
-    uint32_t* tmem_slot = (uint32_t*)(bars + 21);
-    ApItem* ring = (ApItem*)(bars + 22);                        // [4]
+    uint64_t* settled = bars + 21;      // [2]: after a wait ran out, one an issuer
+    uint32_t* tmem_slot = (uint32_t*)(bars + 23);
+    ApItem* ring = (ApItem*)(bars + 24);                        // [4]
     float* s_xm = (float*)(ring + 4);   // [2][2 halves][128 rows]
     float* s_xl = s_xm + 512;           // [2 halves][128 rows]
     int* s_pages_k = (int*)(s_xl + 256);          // [AT_PAGES_CAP]
@@ -300,6 +312,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             at_mbar_init(&v_full[i], 1); at_mbar_init(&v_empty[i], 1);
             at_mbar_init(&s_full[i], 1); at_mbar_init(&p_full[i], 8);
             at_mbar_init(&o_free[i], 8); at_mbar_init(&p_free[i], 1);
+            at_mbar_init(&settled[i], 1);
         }
         at_mbar_init(o_done, 1);
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -346,7 +359,10 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             // the Q buffer (and with it the turn to publish) is free once the products of the
             // item two back have run and everybody has read its record
             ok = __all_sync(0xffffffffu, at_wait(&q_empty[qb], qph ^ 1u, 1));
-            if (!ok) break;
+            if (!ok) {
+                at_settle_copies(q_full, n, 1);
+                break;
+            }
             // An item is drawn only now, when the CTA has room for it: the CTA then holds the
             // item it computes and the one it loads, and no third. (Drawn one turn earlier, as
             // this kernel did at first, two items lay reserved behind the running one; with
@@ -443,6 +459,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             }
             __syncwarp();
         }
+        if (!ok) at_settle_copies(full, g, 1);
     } else if (warp == 1) {
         // ---------------------------------------------------------- issuer of S = Q K^T
         // (a thread can start a product about every 80 cycles, so the two kinds of product
@@ -454,7 +471,8 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             bool ok = true;
             for (uint32_t n = 0; ok; ++n) {
                 const uint32_t qb = n & 1u;
-                if (!at_wait(&q_full[qb], (n >> 1) & 1u, 2)) break;
+                ok = at_wait(&q_full[qb], (n >> 1) & 1u, 2);
+                if (!ok) break;
                 const ApItem* rec = &ring[n & 3];
                 if (!rec->valid) break;
                 const int n_it = rec->n_it;
@@ -477,6 +495,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                 }
                 at_commit(&q_empty[qb]);               // the item's products with Q have run
             }
+            if (!ok) at_settle_products(&settled[0], 2);
         }
     } else if (warp == 11) {
         // ---------------------------------------------------------- issuer of O += P V
@@ -486,7 +505,8 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
             uint32_t g = 0;
             bool ok = true;
             for (uint32_t n = 0; ok; ++n) {
-                if (!at_wait(&q_full[n & 1u], (n >> 1) & 1u, 2)) break;
+                ok = at_wait(&q_full[n & 1u], (n >> 1) & 1u, 2);
+                if (!ok) break;
                 const ApItem* rec = &ring[n & 3];
                 if (!rec->valid) break;
                 const int n_it = rec->n_it;
@@ -509,6 +529,7 @@ attention_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_k, const 
                     at_commit(o_done);
                 }
             }
+            if (!ok) at_settle_products(&settled[1], 2);
         }
     } else {
         // ---------------------------------------------------------- softmax
@@ -818,7 +839,7 @@ static int at_go(const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap
                  int page_size, int shift, const int* block_tables, int max_blocks, const int* positions,
                  const int* seq_ids, const int* tile_tok0, const int* tile_ntok, int n_tiles, int H, int Hkv,
                  float scale_log2, int window, const ApExtra& ex, cudaStream_t stream) {
-    constexpr size_t smem = 1024 + 6 * (size_t)AT_TILE_BYTES + 22 * 8 + 4 * sizeof(ApItem) +
+    constexpr size_t smem = 1024 + 6 * (size_t)AT_TILE_BYTES + 24 * 8 + 4 * sizeof(ApItem) +
                             768 * sizeof(float) + 2 * AT_PAGES_CAP * sizeof(int);
     // per device: its SM count, and whether this kernel's attribute is set there
     static int sms_of[64] = {};

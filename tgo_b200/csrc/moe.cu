@@ -547,11 +547,13 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     uint64_t* empty = full + 8;
     uint64_t* acc_full = empty + 8;                            // [2]
     uint64_t* acc_empty = acc_full + 2;                        // [2]
-    uint32_t* tmem_slot = (uint32_t*)(acc_empty + 2);
+    uint64_t* settled = acc_empty + 2;                         // after a wait ran out
+    uint32_t* tmem_slot = (uint32_t*)(settled + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 8; ++i) { tg_init(&full[i], 1); tg_init(&empty[i], 1); }
         for (int i = 0; i < 2; ++i) { tg_init(&acc_full[i], 1); tg_init(&acc_empty[i], 4); }
+        tg_init(settled, 1);
         tg_init_done();
     }
     if (warp == 1) tg_alloc512(tmem_slot);
@@ -586,6 +588,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                 if (lane < groups && gather) tg_gather4(st + lane * 512, &map_a, kb * MT_BK, src[0], src[1], src[2], src[3], &full[s]);
             }
         }
+        if (!ok) tg_settle_copies(full, stages, it, &moe_error_flag, 1);
     } else if (warp == 1) {
         if (lane == 0) {
             const uint32_t idesc = tg_idesc(nm);
@@ -609,6 +612,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
                 }
                 tg_commit(&acc_full[buf]);
             }
+            if (!ok) tg_settle_products(settled, &moe_error_flag, 3);
         }
     } else {
         const int quarter = warp & 3;                          // tensor-memory lanes this warp may read

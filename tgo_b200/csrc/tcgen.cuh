@@ -52,6 +52,11 @@ __device__ __forceinline__ void tg_gather4(void* dst, const CUtensorMap* map, in
                  "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];"
                  ::"r"(tg_smem(dst)), "l"(map), "r"(tg_smem(bar)), "r"(x), "r"(r0), "r"(r1), "r"(r2), "r"(r3) : "memory");
 }
+// Before a CTA gives up: the last copies into a ring of `slots` that `sent` copies have gone through are
+// waited for, each with the time limit.
+__device__ __forceinline__ void tg_settle_copies(uint64_t* full, uint32_t slots, uint32_t sent, int* err, int code) {
+    for (uint32_t j = sent > slots ? sent - slots : 0u; j < sent; ++j) tg_wait(&full[j % slots], (j / slots) & 1u, err, code);
+}
 // D (tensor memory) (+)= A B^T, both operands in shared memory
 __device__ __forceinline__ void tg_mma(uint32_t d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
     asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
@@ -66,6 +71,12 @@ __device__ __forceinline__ void tg_mma_ts(uint32_t d, uint32_t a, uint64_t b, ui
 }
 __device__ __forceinline__ void tg_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(tg_smem(bar)) : "memory");
+}
+// Before a CTA gives up: the products a thread has issued are waited for. `bar` (one arrival) is used by
+// nobody else.
+__device__ __forceinline__ void tg_settle_products(uint64_t* bar, int* err, int code) {
+    tg_commit(bar);
+    tg_wait(bar, 0, err, code);
 }
 __device__ __forceinline__ void tg_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void tg_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
