@@ -16,6 +16,15 @@
 
 typedef __nv_bfloat16 bf16;
 
+// Multiprocessors of the current device (148 where it cannot be asked), kept per device.
+static inline int tgo_multiprocessors() {
+    static int kept[64] = {};
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
+    if (!kept[dev] && cudaDeviceGetAttribute(&kept[dev], cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) kept[dev] = 0;
+    return kept[dev] > 0 ? kept[dev] : 148;
+}
+
 __device__ __forceinline__ float to_f32(float x) { return x; }
 __device__ __forceinline__ float to_f32(bf16 x) { return __bfloat162float(x); }
 

@@ -700,14 +700,6 @@ moe_gather_kernel(const bf16* __restrict__ x, long long x_stride, bf16* __restri
     for (int c = threadIdx.x; c < d / 8; c += 128) dst[c] = src[c];
 }
 
-static int moe_sms() {
-    static int cached[64] = {};
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 148;
-    if (!cached[dev]) cudaDeviceGetAttribute(&cached[dev], cudaDevAttrMultiProcessorCount, dev);
-    return cached[dev] > 0 ? cached[dev] : 148;
-}
-
 // The column tile: a round of items costs its k-blocks at the slower of their products (2 cycles a
 // column) and of their bytes (70 a cycle) and 200 cycles each, and about 1500 cycles; the number of planned
 // tiles is the device's to know, `m_est` what evenly spread tokens would make. MEASURED (B200, 104 sizes: 8
@@ -750,12 +742,12 @@ static int moe_tc_launch(const void* a, long long a_rows, long long a_stride, co
         if (err != cudaSuccess) return (int)err;
         sized[dev] = true;
     }
-    const int bn = moe_tc_width(N, K, E, pairs, MODE == 1, moe_sms());
+    const int bn = moe_tc_width(N, K, E, pairs, MODE == 1, tgo_multiprocessors());
     CUtensorMap ma, m0, m1;
     if (!tg_map(&ma, a, a_rows, K, a_stride, gather ? 1 : 32) || !tg_map(&m0, b0, (long long)E * N, K, K, bn) ||
         !tg_map(&m1, b1 ? b1 : b0, (long long)E * N, K, K, bn))
         return TGO_E_BAD_ARG;
-    return tgo_launch_pdl(moe_tc_kernel<MODE>, dim3(moe_sms()), dim3(MT_THREADS), MT_SMEM, stream, ma, m0, m1, (bf16*)hidden, y,
+    return tgo_launch_pdl(moe_tc_kernel<MODE>, dim3(tgo_multiprocessors()), dim3(MT_THREADS), MT_SMEM, stream, ma, m0, m1, (bf16*)hidden, y,
                           N, K, bn, top, act, gather ? 1 : 0, perm, tile_info, tiles);
 }
 

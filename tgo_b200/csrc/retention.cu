@@ -837,7 +837,7 @@ static int retention_tiled(const T* q, long long q_stride, const T* k, long long
                         decay, q_start, state_slots, chunk_first, scratch, state);
     if (rc) return rc;
     // two blocks an SM: with fewer (chunk, head) pairs than twice that a block takes one slice
-    const int z = (long long)chunks * H < 592 ? slices : 1;
+    const int z = (long long)chunks * H < 4 * tgo_multiprocessors() ? slices : 1;
     return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RC_THREADS), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
                           H, dv, decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, (const float*)scratch);
 }

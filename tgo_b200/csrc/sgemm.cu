@@ -165,12 +165,7 @@ TGO_API int tgo_sgemm_tn(const float* x, const float* w, float* y, int M, int N,
                          cudaStream_t stream) {
     if (M <= 0 || N <= 0) return 0;
     if (K <= 0) return TGO_E_BAD_ARG;
-    static int sms = 0;
-    if (!sms) {
-        int dev = 0;
-        if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
-            sms = 148;
-    }
+    const int sms = tgo_multiprocessors();
     // The tile: a round (as many tiles as SMs) costs `fixed` once and `round` each, in us at K = 2048,
     // fitted to the times of 15 products of 1 to 1200 rows (64 x 128: 123 us for one round, 597 for
     // six; 64 x 64: 88, 133 for two, 688 for twelve; 16 x 64: 54, 132 for four, 1450 for forty-six).

@@ -749,7 +749,7 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
         // Two heads a block from more (chunk, head) pairs than multiprocessors: 2048 tokens of 64 heads 134 us
         // against 148, 700 of 24 25.1 against 27.1; 160 of 8 (24 pairs) 24.4 against 20.7, 512 of 16 (144) 24.9
         // against 21.3.
-        if (pairs && nh % 2 == 0 && (long long)n_chunks * nh > 148)
+        if (pairs && nh % 2 == 0 && (long long)n_chunks * nh > tgo_multiprocessors())
             rc = tgo_launch_pdl(ssd_outputs_kernel<N, P, PAIR>, dim3(n_chunks, nh / PAIR), dim3(PAIR * 2 * P), s3p, stream, xbc, C,
                                 H, G, h0, D, (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
         else
