@@ -290,3 +290,19 @@ def test_routed_products_stay_off_the_narrowest_tiles(N, K, E, top, tokens):
     from tgo_b200.kernels.build import entry_points
     for T in tokens:
         assert entry_points("moe").tgo_moe_tile_width(N, K, E, T * top, 1, 148) >= 64
+
+
+def test_selective_scan_of_no_requests_at_all(monkeypatch):
+    """A step without requests launches what does nothing; the rule for chunks does not divide by their count."""
+    import types
+
+    import torch
+    from tgo_b200.kernels import ops
+    seen = []
+    lib = types.SimpleNamespace(tgo_ssd_chunk_tokens=lambda: 64, tgo_selective_scan=lambda *a: seen.append(a) or 0)
+    for name, value in (("_need_cuda", lambda *a: None), ("_stream", lambda: 0), ("entry_points", lambda name: lib)):
+        monkeypatch.setattr(ops, name, value)
+    z = torch.zeros
+    ops.selective_scan(z(0, 2 * 64 + 2 * 64), z(0, 2, dtype=torch.bfloat16), None, z(2), None, z(0, 128), 0, 2, 1, 64, 64,
+                       z(1, dtype=torch.int32), z(0, dtype=torch.int32), z(1, 2 * 64 * 64), 0)
+    assert len(seen) == 1

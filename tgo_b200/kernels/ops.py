@@ -1087,7 +1087,7 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
     lib = entry_points("state_space")
     chunk = lib.tgo_ssd_chunk_tokens()
-    n_chunks, a_head = T // chunk + num_seqs, state_dim * value_dim + 3 * chunk      # as tgo_ssd_scan says
+    n_chunks, a_head = max(1, T // chunk + num_seqs), state_dim * value_dim + 3 * chunk      # as tgo_ssd_scan says
     most = min(heads, (SSD_WORKSPACE_BYTES // (4 * n_chunks) - 4) // a_head)         # heads at a time
     if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and most > 0 and \
             lib.tgo_ssd_takes(_ptr(xbc), _ptr(y), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(heads),
