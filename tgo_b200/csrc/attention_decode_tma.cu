@@ -537,7 +537,7 @@ flash_decode_tma_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_
     __syncthreads();                           // all tiles read: the ring is free for the join
     // Only a join kernel is let in early. A product that came in beside the last blocks of a small grid
     // was placed two blocks an SM, and so was the one after it: 27 us for a gate/up product of 8 rows
-    // that takes 17.
+    // that takes 17. (Measured with up to eight requests; decoding 64 is as fast either way.)
     if (n_splits > 1) pdl_launch_late();
     float* so = (float*)ring;                  // [4][16][DH]
     if constexpr (KEYS_ON_M) {

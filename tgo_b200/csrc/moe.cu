@@ -519,8 +519,8 @@ __device__ int moe_error_flag = 0;
 
 // act of the products' results. SiLU as z / (1 + e^-z) for z >= 0 and z e^z / (1 + e^z) below, so that the
 // divisor lies in [1, 2] and the quotient needs no scaling: the hardware's reciprocal and one correction by the
-// remainder, within 0.51 units in the last place. (With a plain division, whose rare cases are a branch an
-// element, 64 tokens took 64 us instead of 49.)
+// remainder. (With a plain division, whose rare cases are a branch an element, the up product of 64 tokens
+// took 64 us instead of 51, that of 2048 103 instead of 90.)
 __device__ __forceinline__ float moe_act_tile(float z, int act) {
     if (act != 0) return moe_act(z, act);
     const float e = expf(-fabsf(z)), d = 1.f + e, n = z >= 0.f ? z : z * e;

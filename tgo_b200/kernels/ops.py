@@ -1057,7 +1057,8 @@ def causal_conv_act(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
 # Steps of at least so many tokens, and so many a request on average, run the selective scan by
 # chunks in the bfloat16 engine (64 heads of 64 x 128, a call's wall time, walk against chunks: 64
 # tokens 28 against 36 us, 128 47 / 47, 256 90 / 60; 16 requests of 128 359 / 288; 256 tokens beside 31
-# single ones 198 / 226, 32 requests of 16 114 / 208: a chunk costs its two state-sized rows)
+# single ones 198 / 226, 32 requests of 16 114 / 208: a chunk costs its two state-sized rows). The mean is
+# all the host knows without the lengths: one long portion beside many single tokens (1500 beside 31) walks.
 SSD_MIN_TOKENS = 160
 SSD_TOKENS_A_REQUEST = 64
 # What the workspace of a call may take: up to here all heads run at once (7700 tokens of the size above),

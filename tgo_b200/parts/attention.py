@@ -105,6 +105,8 @@ def decode_splits(ctx, num_kv_heads: int, window: int, device, **kernel) -> int:
 
 
 def tc_kernel_takes(q_dtype, head_dim: int, group: int, page_size: int) -> bool:
+    """Whether prompt portions run on the tcgen05 kernel. (It has an instance for heads of 64, which the
+    attention with sinks takes; on this path it has not been measured against the mma.sync tiles.)"""
     return USE_TC_ATTENTION and q_dtype == torch.bfloat16 and head_dim == 128 and \
         ops.attention_tc_supports(head_dim, group, page_size)
 
