@@ -506,8 +506,8 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
 // 32 KB of them, four in flight an SM) and by the operands' way into the SM (about 70 bytes a
 // cycle) for full tiles. MEASURED (B200, 32 experts, top 4, ff 768 of width 2048, gated; mma.sync
 // tiles of 64 x 64 fed by cp.async before): 2048 tokens, up 91 us (250) and down 41 (135), 570 and
-// 620 TFLOP/s with the copy of x's rows before them 8 us; 64 tokens, 40 us (66) and 21 (25), 5.0
-// and 4.8 TB/s of weights.
+// 620 TFLOP/s with the copy of x's rows before them 8 us; 64 tokens, from a flushed L2, 51 us (71) and 23
+// (25), 4.0 and 4.4 TB/s of weights.
 #define MT_BK 64
 #define MT_A_BYTES (MOE_TILE * MT_BK * 2)
 #define MT_RING (192 * 1024)
