@@ -1,6 +1,7 @@
 """Each CUDA kernel alone against a plain float32 (or float64) torch restatement of the
 same operation, at sizes other than the tiny models': widths that are no power of two,
 head sizes in steps of 16, odd head counts and groups, scattered pages, windows."""
+import ctypes
 import math
 
 import numpy as np
@@ -205,6 +206,47 @@ def test_sgemm_tiles(M, N, K):
     bound = K * 2.0 ** -24 * (x.double().abs() @ w.double().abs().t())
     assert ((outs[0].double() - want).abs() <= bound + 1e-30).all()
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 1, 256), (31, 127, 260), (33, 129, 576), (64, 128, 640), (97, 257, 1020), (161, 130, 2048),
+                                   (330, 40, 6144)])
+def test_sgemm_by_parts(M, N, K):
+    """Three bfloat16 parts a number: the same bits from every tile and beside any rows, an error below that of a
+    chain of FMA, and the plain kernel's result where one is not finite."""
+    from tgo_b200.kernels.build import load_library
+    lib = load_library("sgemm")
+    x, w = rnd(M, K, seed=5), rnd(N, K, seed=6)
+    assert lib.tgo_sgemm_part_bytes(ctypes.c_void_p(w.data_ptr()), K, N) > 0
+    outs = []
+    try:
+        for columns in (160, 128, 96, 64, 32, 0):
+            lib.tgo_sgemm_force_columns(columns)
+            outs.append(torch.full((M, N), float("nan"), device=DEV))
+            ops().sgemm_tn(x, w, outs[-1])
+    finally:
+        lib.tgo_sgemm_force_columns(0)
+    assert all(torch.equal(o, outs[0]) for o in outs)
+    last = torch.empty(1, N, device=DEV)
+    ops().sgemm_tn(x[M - 1:].contiguous(), w, last)
+    assert torch.equal(last[0], outs[0][M - 1])
+    # a k-block of 64: four cuts of less than 2^-23 of its sum's size, the products left out (2^-26 a term)
+    # and a rounded addition: K / 64 times 2^-21 of the sum of sizes is above all of them
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    assert ((outs[0].double() - want).abs() <= (K + 63) // 64 * 2.0 ** -21 * size).all()
+    plain, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    x[M // 2, 3], x[M - 1, K - 1], w[N // 2, 7] = float("inf"), float("nan"), -3.4e38
+    x[0, 7] = 1e-3
+    ops().sgemm_tn(x, w, got)
+    try:
+        lib.tgo_sgemm_force_tile(1)
+        ops().sgemm_tn(x, w, plain)
+    finally:
+        lib.tgo_sgemm_force_tile(0)
+    odd = ~torch.isfinite(plain)
+    assert torch.equal(torch.isfinite(got), ~odd)
+    assert torch.equal(got[odd].nan_to_num(7.0), plain[odd].nan_to_num(7.0))
+    assert torch.allclose(got[~odd], plain[~odd], rtol=1e-4, atol=1e-3)
+    assert ops().sgemm_error() == 0
 
 
 # ----------------------------------------------------------------------- attention

@@ -1564,7 +1564,8 @@ def retention_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: to
 
 
 def sgemm_tn(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
-    """out[M,N] = x[M,K] . w[N,K]^T, all float32, plain FMA."""
+    """out[M,N] = x[M,K] . w[N,K]^T in true float32: on the tensor cores by parts where the sizes
+    allow it (whatever M is), else by plain FMA."""
     _need_cuda(x, w, out)
     M, K = x.shape
     N = w.shape[0]
@@ -1572,8 +1573,22 @@ def sgemm_tn(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     assert x.dtype == w.dtype == out.dtype == torch.float32
     assert x.is_contiguous() and w.is_contiguous() and out.is_contiguous()
     lib = entry_points("sgemm")
+    row = lib.tgo_sgemm_part_bytes(_ptr(w), c_int(K), c_int(N)) if M > 0 else 0
+    if row:
+        parts = torch.empty(M * row, dtype=torch.uint8, device=x.device)
+        _check(lib.tgo_sgemm_split(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), _ptr(parts), _stream()),
+               "sgemm_tn", f"(M={M}, N={N}, K={K})")
+        LAUNCHES[0] += 1
+        return
     _check(lib.tgo_sgemm_tn(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), _stream()),
            "sgemm_tn", f"(M={M}, N={N}, K={K})")
+
+
+def sgemm_error() -> int:
+    """The code a wait of the float32 products left when it ran out, or 0. Synchronises."""
+    value = ctypes.c_int(0)
+    _check(entry_points("sgemm").tgo_sgemm_error(ctypes.addressof(value)), "sgemm_error")
+    return int(value.value)
 
 
 SKINNY_MAX_ROWS = 8
@@ -1715,7 +1730,7 @@ def linear(x: torch.Tensor, w: torch.Tensor, out_dtype: Optional[torch.dtype] = 
     belongs to: either it is added there and None is returned, or the product is returned
     for the caller to add (the block hands it to the next norm).
 
-    float32: this package's plain-FMA kernel. bfloat16 with few rows (a decode step): this
+    float32: this package's true float32 product (`sgemm_tn`). bfloat16 with few rows (a decode step): this
     package's weight-streaming kernel, which does the residual add in its epilogue.
     bfloat16 with many rows (TC_MIN_ROWS): this package's tcgen05 kernel (TMA-fed,
     accumulators in tensor memory); between them the library product. out_dtype float32
@@ -2156,6 +2171,10 @@ def kernel_wait_errors() -> dict:
         code = moe_error()
         if code:
             out["moe"] = code
+    if "sgemm" in _loaded:
+        code = sgemm_error()
+        if code:
+            out["sgemm"] = code
     for key, flag in _tc_err.items():
         code = int(flag.item())
         if code:
