@@ -2155,6 +2155,8 @@ def kernel_wait_errors() -> dict:
     trusted. Looks only at libraries that are loaded; synchronises with the device."""
     from .build import _loaded
     out = {}
+    if not torch.cuda.is_initialized():      # no kernel has run, though a library may be loaded for its host rules
+        return out
     if "attention_tc" in _loaded:
         code = attention_tc_error()
         if code:
