@@ -15,7 +15,7 @@
 // The columns of S are independent, so a block owns a slice of dv columns of one
 // (request, head): grid (requests, heads, slices). The powers of the decay come from a table
 // made by repeated multiplication.
-#include "fma_tile.cuh"
+#include "split3.cuh"
 
 #define RT_CHUNK 32
 #define RT_THREADS 256
@@ -485,23 +485,26 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 }
 
 // ------------------------------------------------ the same, for heads of 64 or 128 key channels
-// Register tiles of 8 x 8 and 4 x 8 outputs (fma_tile.cuh) instead of 4 x 4; what a product sums
-// over is the slow axis of both of its operands in shared memory. Bound by the FMA pipes; a true
-// 32-bit product has no faster unit. MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16
-// rows; the kernels above in brackets): summaries 122 us (255), scan 40 (139), outputs 186 (879); 138 and
-// 206 where each run's loads were waited for before the next were asked for.
-//   summaries   a block makes U for 128 columns of V: K (scaled rows) and V as they lie;
+// The products in true float32 on the tensor cores: each number as three bfloat16 parts (split3.cuh), values that
+// are bfloat16 numbers already as one. A block makes 128 columns of V: channels of V are the accumulators' lanes,
+// tokens (or key channels) their columns, so that every operand is laid down as it lies in memory and a warp's results
+// leave as whole lines.
+//   summaries   U^T = V^T K: K's scaled and rotated rows and V, one product of 64 tokens;
 //   scan        four neighbouring elements a thread, eight summaries asked for while the eight before
 //               them are used: bound by memory (every summary read once, every state written once);
-//   outputs     a block takes a chunk's 64 rows and, 128 columns at a time, decay^(i+1) Q P + A V:
-//               Q and K are laid down channel-major once, A token-major; P comes 16 channels at a
-//               time, two turns ahead. The columns are shared out over blocks when there are few
-//               chunks.
+//   outputs     by halves of 64 key channels, one after the other through the same shared memory (two blocks an SM
+//               hide each other's loads): Q K^T and P^T Q^T; then A = decay^(i-j) Q K^T goes back to
+//               shared memory as parts, V^T A^T is made, and out = decay^(i+1) (Q P) + A V.
+// Zeros of A times a value that is not finite are not zero: such a number is laid down as 0, which leaves what does
+// not depend on it as it is, bit for bit, and a block that met one makes plain sums too and writes those that are not finite.
+// MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
+// summaries @S@ us (122), scan 40, outputs @O@ us (190). Bound by the bytes of U, P and the outputs, and by the
+// conversions' instructions.
 #define RF_SLICE 128
-#define RF_LDN (RC_CHUNK + 4)         // rows of a channel-major tile
-#define RF_LDS (RF_SLICE + 4)
-#define RF_PK 16                      // channels of P a turn
-#define RF_PSTAGES 3
+#define RF_TILE 8192                  // 64 rows of 64 bfloat16 numbers
+#define RF_LOOP_LD 129                // rows of the plain sums' tiles
+
+__device__ int retention_error_flag = 0;
 
 // Eight channels of a row as they lie, and their values after the activation. Asked for first and turned
 // later, so that several are under way at once.
@@ -533,32 +536,36 @@ __device__ __forceinline__ void taken8(const Raw8<float>& raw, int act, float (&
         for (int i = 0; i < 8; ++i) f[i] = f[i] / (1.f + expf(-f[i]));
 }
 
-// Eight neighbouring channels d0 .. d0 + 7 of a row, rotated: d0 and rot / 2 are multiples of 8. Without a
-// rotation the partner is the run itself and nothing else is read.
-template <typename T> struct Rot8 {
-    Raw8<T> x, g;
+// Two runs of eight channels of a row that a rotation turns into each other, or two runs that it leaves as they are:
+// pair p of DK / 16; rot is a multiple of 16.
+template <typename T> struct Pair8 {
+    Raw8<T> x, y;
     float4 c0, c1, s0, s1;
-    __device__ __forceinline__ void load(const T* __restrict__ row, const float* __restrict__ cs, int d0, int rot) {
-        const int half = rot >> 1;
-        const bool turned = cs && d0 < rot;
-        load8(x, row + d0);
-        if (cs && rot > 0) {
-            const int p0 = !turned ? 0 : d0 < half ? d0 : d0 - half;
-            load8(g, row + (!turned ? d0 : d0 < half ? d0 + half : p0));
-            c0 = ((const float4*)(cs + p0))[0]; c1 = ((const float4*)(cs + p0))[1];
-            s0 = ((const float4*)(cs + half + p0))[0]; s1 = ((const float4*)(cs + half + p0))[1];
+    int lo, hi;
+    bool turned;
+    __device__ __forceinline__ void load(const T* __restrict__ row, const float* __restrict__ cs, int p, int rot) {
+        turned = cs && 16 * p < rot;
+        lo = turned ? 8 * p : 16 * p;
+        hi = turned ? lo + (rot >> 1) : lo + 8;
+        load8(x, row + lo);
+        load8(y, row + hi);
+        if (turned) {
+            c0 = *(const float4*)(cs + lo); c1 = *(const float4*)(cs + lo + 4);
+            s0 = *(const float4*)(cs + hi); s1 = *(const float4*)(cs + hi + 4);
         }
     }
-    __device__ __forceinline__ void values(bool rope, int d0, int rot, int act, float (&f)[8]) const {
+    __device__ __forceinline__ void values(int act, float (&f)[8], float (&g)[8]) const {
         taken8(x, act, f);
-        if (!rope || d0 >= rot) return;
-        const bool low = d0 < (rot >> 1);
-        float o[8];
-        taken8(g, act, o);
+        taken8(y, act, g);
+        if (!turned) return;
         const float c[8] = {c0.x, c0.y, c0.z, c0.w, c1.x, c1.y, c1.z, c1.w};
         const float n[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
 #pragma unroll
-        for (int i = 0; i < 8; ++i) f[i] = low ? f[i] * c[i] - o[i] * n[i] : f[i] * c[i] + o[i] * n[i];
+        for (int i = 0; i < 8; ++i) {
+            const float a = f[i], b = g[i];
+            f[i] = a * c[i] - b * n[i];
+            g[i] = b * c[i] + a * n[i];
+        }
     }
 };
 
@@ -570,88 +577,167 @@ __device__ __forceinline__ void rf_powers(float* pw, float g) {
     }
 }
 
-// Columns c0 .. c0 + RF_SLICE - 1 of the chunk's values, rows past n and columns past dv zero: asked for,
-// then put into shared memory; true if a thread's are not all finite.
-#define RF_V_RUNS (RC_CHUNK * (RF_SLICE / 8) / RC_THREADS)
-template <typename T>
-__device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[RF_V_RUNS], const T* __restrict__ v, long long v_stride, int h, int dv,
-                                         int c0, int tok0, int n) {
+// Columns c0 .. c0 + 127 of the chunk's values, asked for and then laid down (rows of tokens, two tiles of 64 columns a
+// part); rows past n and columns past dv are zeros. True: a thread's are not all finite.
+template <int THREADS> __device__ constexpr int rf_v_runs() { return RC_CHUNK * (RF_SLICE / 8) / THREADS; }
+template <typename T, int THREADS>
+__device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[rf_v_runs<THREADS>()], const T* __restrict__ v, long long v_stride, int h,
+                                         int dv, int c0, int tok0, int n) {
 #pragma unroll
-    for (int j = 0; j < RF_V_RUNS; ++j) {
-        const int i = threadIdx.x + j * RC_THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
+    for (int j = 0; j < rf_v_runs<THREADS>(); ++j) {
+        const int i = threadIdx.x + j * THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
         load8(raw[j], v + (size_t)(tok0 + (r < n ? r : 0)) * v_stride + (size_t)h * dv + (c0 + c < dv ? c0 + c : 0));
     }
 }
-template <typename T>
-__device__ __forceinline__ bool rf_put_v(float* Vs, const Raw8<T> (&raw)[RF_V_RUNS], int dv, int c0, int n, int act) {
+template <typename T, int VP, int THREADS>
+__device__ __forceinline__ bool rf_put_v(uint32_t tile, const Raw8<T> (&raw)[rf_v_runs<THREADS>()], int dv, int c0, int n, int act) {
     bool odd = false;
 #pragma unroll
-    for (int j = 0; j < RF_V_RUNS; ++j) {
-        const int i = threadIdx.x + j * RC_THREADS, r = i / (RF_SLICE / 8), c = (i % (RF_SLICE / 8)) * 8;
-        float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-        if (r < n && c0 + c < dv) taken8(raw[j], act, f);
-        const float4 lo = make_float4(f[0], f[1], f[2], f[3]), hi = make_float4(f[4], f[5], f[6], f[7]);
-        *(float4*)(Vs + r * RF_LDS + c) = lo;
-        *(float4*)(Vs + r * RF_LDS + c + 4) = hi;
-        odd = odd || ft_not_finite(lo) || ft_not_finite(hi);
+    for (int j = 0; j < rf_v_runs<THREADS>(); ++j) {
+        const int i = threadIdx.x + j * THREADS, r = i / (RF_SLICE / 8), piece = i % (RF_SLICE / 8);
+        const bool ok = r < n && c0 + 8 * piece < dv;
+        const uint32_t dst = tile + (piece >> 3) * RF_TILE + s3_place(r, piece & 7);
+        if constexpr (VP == 1) {
+            uint4 w = ok ? raw[j].u : make_uint4(0u, 0u, 0u, 0u);
+            odd = s3_finite8(w) || odd;
+            s3_store16(dst, w);
+        } else {
+            float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+            if (ok) taken8(raw[j], act, f);
+            uint4 part[3];
+            odd = s3_split8_finite(f, part) || odd;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) s3_store16(dst + q * 2 * RF_TILE, part[q]);
+        }
     }
     return odd;
 }
+// The parts of eight numbers to their place in three tiles `step` bytes apart.
+__device__ __forceinline__ bool rf_put8(uint32_t tile, uint32_t step, int row, int piece, const float (&f)[8]) {
+    uint4 part[3];
+    const bool odd = s3_split8_finite(f, part);
+    const uint32_t dst = tile + s3_place(row, piece);
+#pragma unroll
+    for (int q = 0; q < 3; ++q) s3_store16(dst + q * step, part[q]);
+    return odd;
+}
+// The value of column c of a token, as the plain sums take it.
+template <typename T>
+__device__ __forceinline__ float rf_value(const T* __restrict__ v, long long v_stride, size_t t, int h, int dv, int c, int act) {
+    return taken(v[t * v_stride + (size_t)h * dv + c], act);
+}
+__device__ __forceinline__ bool rf_not_finite(float x) { return !(fabsf(x) < __int_as_float(0x7f800000)); }
+// A block's products are there (`phase` of their barrier), for all threads or for none.
+__device__ __forceinline__ bool rf_made(uint64_t* bar, uint32_t phase, int code) {
+    const bool ok = __syncthreads_and(tg_wait(bar, phase, &retention_error_flag, code));
+    tg_after();
+    return ok;
+}
 
-template <typename T, int DK>
-__global__ void __launch_bounds__(RC_THREADS, 2)
-retention_summaries_tiled_kernel(const T* __restrict__ k, long long k_stride, const T* __restrict__ v, long long v_stride,
-                                 int H, int dv, const float* __restrict__ decay, float k_scale, int act,
-                                 const float* __restrict__ rope, int rot, const int* __restrict__ chunk_tok0,
-                                 const int* __restrict__ chunk_ntok, float* __restrict__ U) {
-    extern __shared__ __align__(16) float smem[];
-    float* Ks = smem;                                    // [RC_CHUNK][DK + 4]
-    float* Vs = Ks + RC_CHUNK * (DK + 4);                // [RC_CHUNK][RF_LDS]
+// VP: parts a value has (1: bfloat16 rows without an activation). A block makes the columns of up to two slices.
+template <typename T, int DK, int VP>
+__global__ void __launch_bounds__(RC_THREADS, VP == 1 ? 2 : 1)
+retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const T* __restrict__ v, long long v_stride,
+                              int H, int dv, const float* __restrict__ decay, float k_scale, int act,
+                              const float* __restrict__ rope, int rot, const int* __restrict__ chunk_tok0,
+                              const int* __restrict__ chunk_ntok, int slices, float* __restrict__ U) {
+    constexpr int KB = DK / 64;                          // tiles of a part of K
+    extern __shared__ unsigned char rf_raw[];
+    unsigned char* base = (unsigned char*)(((uintptr_t)rf_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sV = base + 3 * KB * RF_TILE;         // K's parts, then either slice's of V
     __shared__ float pw[RC_CHUNK + 1];
+    __shared__ __align__(8) uint64_t bars[2];            // one a slice
+    __shared__ uint32_t tmem_slot;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) tg_alloc<2 * DK>(&tmem_slot);
+    if (threadIdx.x == 0) { tg_init(&bars[0], 1); tg_init(&bars[1], 1); tg_init_done(); }
     pdl_wait();
-    const int ci = blockIdx.x, h = blockIdx.y, c0 = blockIdx.z * RF_SLICE;
+    const int ci = blockIdx.x, h = blockIdx.y, first = blockIdx.z * slices * RF_SLICE;
     const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
-    Raw8<T> vr[RF_V_RUNS];
-    rf_ask_v(vr, v, v_stride, h, dv, c0, tok0, n);
+    const int ns = min(slices, (dv - first + RF_SLICE - 1) / RF_SLICE);
+    Raw8<T> vr[rf_v_runs<RC_THREADS>()];
+    rf_ask_v<T, RC_THREADS>(vr, v, v_stride, h, dv, first, tok0, n);
     rf_powers(pw, decay[h]);
+    tg_before();
     __syncthreads();
-    // two runs of K a thread at a time, beside the values: a thread a run after the other had its loads
-    // waited for one by one (ncu: 2.7 of 9 cycles an instruction)
-    constexpr int RUNS = RC_CHUNK * (DK / 8) / RC_THREADS;
+    tg_after();
+    const uint32_t tmem = tmem_slot;
+    bool odd = false;
+    constexpr int PAIRS = RC_CHUNK * (DK / 16) / RC_THREADS;
+    Pair8<T> kr[PAIRS];
 #pragma unroll
-    for (int j0 = 0; j0 < RUNS; j0 += 2) {
-        Rot8<T> kr[2];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = threadIdx.x + (j0 + j) * RC_THREADS, r = i / (DK / 8), d = (i % (DK / 8)) * 8;
-            const size_t t = (size_t)(tok0 + (r < n ? r : 0));
-            kr[j].load(k + t * k_stride + (size_t)h * DK, rope ? rope + t * rot : nullptr, d, rot);
-        }
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = threadIdx.x + (j0 + j) * RC_THREADS, r = i / (DK / 8), d = (i % (DK / 8)) * 8;
-            float f[8];
-            kr[j].values(rope != nullptr, d, rot, act, f);
-            const float w = r < n ? pw[n - 1 - r] : 0.f;
-#pragma unroll
-            for (int x = 0; x < 8; ++x) f[x] = r < n ? f[x] * k_scale * w : 0.f;
-            *(float4*)(Ks + r * (DK + 4) + d) = make_float4(f[0], f[1], f[2], f[3]);
-            *(float4*)(Ks + r * (DK + 4) + d + 4) = make_float4(f[4], f[5], f[6], f[7]);
-        }
+    for (int j = 0; j < PAIRS; ++j) {
+        const int i = threadIdx.x + j * RC_THREADS, r = i / (DK / 16);
+        const size_t t = (size_t)(tok0 + (r < n ? r : 0));
+        kr[j].load(k + t * k_stride + (size_t)h * DK, rope ? rope + t * rot : nullptr, i % (DK / 16), rot);
     }
-    rf_put_v(Vs, vr, dv, c0, n, act);
-    __syncthreads();
-    FmaTile<DK / 64, 2, 16, 16> t;
-    t.ty = threadIdx.x / 16;
-    t.tx = threadIdx.x % 16;
-    t.clear();
-    t.add(Ks, DK + 4, Vs, RF_LDS, n);
+#pragma unroll
+    for (int j = 0; j < PAIRS; ++j) {
+        const int r = (threadIdx.x + j * RC_THREADS) / (DK / 16);
+        float f[8], g[8];
+        kr[j].values(act, f, g);
+        const float w = r < n ? pw[n - 1 - r] : 0.f;
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            f[x] = r < n ? f[x] * k_scale * w : 0.f;
+            g[x] = r < n ? g[x] * k_scale * w : 0.f;
+        }
+        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].lo / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].lo / 8) & 7, f) || odd;
+        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].hi / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].hi / 8) & 7, g) || odd;
+    }
+    for (int s = 0; s < ns; ++s) {
+        unsigned char* sv = sV + s * 2 * VP * RF_TILE;
+        odd = rf_put_v<T, VP, RC_THREADS>(tg_smem(sv), vr, dv, first + s * RF_SLICE, n, act) || odd;
+        if (s + 1 < ns) rf_ask_v<T, RC_THREADS>(vr, v, v_stride, h, dv, first + (s + 1) * RF_SLICE, tok0, n);
+        s3_fence();
+        odd = __syncthreads_or(odd);
+        if (warp == 0 && tg_elect()) {
+            s3_products<VP, 3, RC_CHUNK / 16>(tmem + (uint32_t)(DK * s), tg_desc_mn(sv, RF_TILE), 2 * RF_TILE >> 4, 128,
+                                              tg_desc_mn(base, RF_TILE), KB * RF_TILE >> 4, 128, tg_idesc(DK, true, true), false);
+            tg_commit(&bars[s]);
+        }
+        __syncwarp();
+    }
+    bool ok = true;
+    for (int s = 0; s < ns && ok; ++s) ok = rf_made(&bars[s], 0, 1);
     float* Uo = U + ((size_t)ci * H + h) * DK * dv;
+    if (ok) {
+        const int d0 = (warp >> 2) * (DK / 2);
+        for (int s = 0; s < ns; ++s) {
+            const int c = first + s * RF_SLICE + (warp & 3) * 32 + lane;
 #pragma unroll
-    for (int i = 0; i < DK / 16; ++i)
+            for (int x = 0; x < DK / 2; x += 32) {
+                uint32_t r[32];
+                tg_ld32(tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(DK * s + d0 + x), r);
+                tg_wait_ld();
+                float* dst = Uo + (size_t)(d0 + x) * dv + c;
+                if (c < dv)
 #pragma unroll
-        for (int c = 0; c < 2; ++c)
-            if (c0 + t.col(c) < dv) *(float4*)(Uo + (size_t)t.row(i) * dv + c0 + t.col(c)) = t.get(i, c);
+                    for (int i = 0; i < 32; ++i, dst += dv) *dst = __uint_as_float(r[i]);
+            }
+        }
+        if (odd) {
+            float* Kf = (float*)base;
+            load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
+            __syncthreads();
+            for (int i = threadIdx.x; i < DK * RF_SLICE * ns; i += RC_THREADS) {
+                const int d = i / (RF_SLICE * ns), c = first + i % (RF_SLICE * ns);
+                if (c >= dv) continue;
+                float s = 0.f;
+                for (int j = 0; j < n; ++j)
+                    s = fmaf(Kf[j * RF_LOOP_LD + d] * pw[n - 1 - j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
+                if (rf_not_finite(s)) Uo[(size_t)d * dv + c] = s;
+            }
+        }
+    } else {
+        for (int s = 0; s < ns; ++s) tg_wait(&bars[s], 0, &retention_error_flag, 1);      // products that may still be under way
+    }
+    tg_before();
+    __syncthreads();
+    if (warp == 0) {
+        tg_after();
+        tg_free<2 * DK>(tmem);
+    }
 }
 
 // grid (requests, heads, ceil(dk dv / 1024)): a thread four neighbouring elements of the state
@@ -697,128 +783,232 @@ retention_scan4_kernel(int H, int dkdv, const float* __restrict__ decay, const i
     *sp = s;
 }
 
-template <typename T, int DK>
-__global__ void __launch_bounds__(RC_THREADS, 2)
-retention_outputs_tiled_kernel(const T* __restrict__ q, long long q_stride, const T* __restrict__ k, long long k_stride,
-                               const T* __restrict__ v, long long v_stride, float* __restrict__ out, int H, int dv,
-                               const float* __restrict__ decay, float k_scale, int act, const float* __restrict__ rope,
-                               int rot, const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_ntok,
-                               const float* __restrict__ P) {
-    extern __shared__ __align__(16) float smem[];
-    float* Qt = smem;                                    // [DK][RF_LDN]
-    float* At = Qt + DK * RF_LDN;                        // [RC_CHUNK][RF_LDN], token j major
-    float* Ps = At + RC_CHUNK * RF_LDN;                  // [RF_PSTAGES][RF_PK][RF_LDS]
-    float* KV = Ps + RF_PSTAGES * RF_PK * RF_LDS;        // K [DK][RF_LDN], later V [RC_CHUNK][RF_LDS]
+// Shared memory: Q's parts (a part DK / 64 tiles), two buffers of P's (64 channels x 128 columns, two tiles a part),
+// K's parts, over which A's and one slice's values come to lie (24 KB more than K at DK = 128).
+#define RF_OUT_THREADS 512
+template <int DK> __host__ __device__ constexpr int rf_out_k() { return 3 * (DK / 64) * RF_TILE + 2 * 6 * RF_TILE; }
+template <int DK> __host__ __device__ constexpr int rf_out_bytes() { return rf_out_k<DK>() + 9 * RF_TILE; }
+
+template <typename T, int DK, int VP>
+__global__ void __launch_bounds__(RF_OUT_THREADS, 1)
+retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T* __restrict__ k, long long k_stride,
+                            const T* __restrict__ v, long long v_stride, float* __restrict__ out, int H, int dv,
+                            const float* __restrict__ decay, float k_scale, int act, const float* __restrict__ rope,
+                            int rot, const int* __restrict__ chunk_tok0, const int* __restrict__ chunk_ntok, int slices,
+                            const float* __restrict__ P) {
+    constexpr int HALVES = DK / 64, THREADS = RF_OUT_THREADS;
+    extern __shared__ unsigned char rf_raw[];
+    unsigned char* sQ = (unsigned char*)(((uintptr_t)rf_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sP = sQ + 3 * HALVES * RF_TILE;       // [2]
+    unsigned char* sK = sQ + rf_out_k<DK>();
+    unsigned char* sA = sK;
+    unsigned char* sV = sK + 3 * RF_TILE;
     __shared__ float pw[RC_CHUNK + 1];
-    __shared__ int s_odd;                                // a value that is not finite among the slice's
+    __shared__ __align__(8) uint64_t bars[4];
+    __shared__ uint32_t tmem_slot;
+    uint64_t *s_done = bars, *p_done = bars + 1 /* [2] */, *v_done = bars + 3;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (warp == 0) tg_alloc512(&tmem_slot);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 4; ++i) tg_init(&bars[i], 1);
+        tg_init_done();
+    }
     pdl_wait();
-    const int ci = blockIdx.x, h = blockIdx.y;
+    const int ci = blockIdx.x, h = blockIdx.y, first = blockIdx.z * slices * RF_SLICE;
     const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
-    const int ty = threadIdx.x / 16, tx = threadIdx.x % 16;
-    rf_powers(pw, decay[h]);
-    // a warp takes four rows x eight runs of eight channels: 128 bytes a row, and stores that meet no
-    // bank twice (ft_swizzle). (A lane a row, every load touched 32 lines: ncu showed the L1 87 % busy.)
-    // Two runs are asked for at a time.
-    constexpr int RUNS = 2 * RC_CHUNK * (DK / 8) / RC_THREADS;
-#pragma unroll 1
-    for (int j0 = 0; j0 < RUNS; j0 += 2) {
-        Rot8<T> run[2];
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int i = threadIdx.x + (j0 + e) * RC_THREADS, which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
-            const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
-            const size_t t = (size_t)(tok0 + (r < n ? r : 0));
-            run[e].load(which ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
-                        rope ? rope + t * rot : nullptr, d, rot);
-        }
-#pragma unroll
-        for (int e = 0; e < 2; ++e) {
-            const int i = threadIdx.x + (j0 + e) * RC_THREADS, which = i / (RC_CHUNK * (DK / 8)), j = i % (RC_CHUNK * (DK / 8));
-            const int r = 4 * ((j / 32) % (RC_CHUNK / 4)) + (j % 32) / 8, d = 8 * (j % 8 + 8 * (j / (8 * RC_CHUNK)));
-            float f[8];
-            run[e].values(rope != nullptr, d, rot, act, f);
-            float* dst = (which ? KV : Qt) + d * RF_LDN + ft_swizzle(r, d, 3);
-#pragma unroll
-            for (int x = 0; x < 8; ++x) dst[x * RF_LDN] = r >= n ? 0.f : which ? f[x] * k_scale : f[x];
-        }
-    }
-    __syncthreads();
-    {
-        FmaTile<1, 1, 16, 16> a;                         // A[i][j], 64 x 64
-        a.ty = ty;
-        a.tx = tx;
-        a.clear();
-        if (4 * tx <= 4 * ty + 3) a.template add_swizzled<3, true>(Qt, RF_LDN, KV, RF_LDN, 0, DK);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const float4 r = a.get(i, 0);
-            const float x[4] = {r.x, r.y, r.z, r.w};
-#pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int gap = 4 * ty + i - (4 * tx + j);
-                At[(4 * tx + j) * RF_LDN + 4 * ty + i] = gap >= 0 ? x[j] * pw[gap >= 0 ? gap : 0] : 0.f;
-            }
-        }
-    }
+    const int ns = min(slices, (dv - first + RF_SLICE - 1) / RF_SLICE), stages = ns * HALVES;
     const float* Pc = P + ((size_t)ci * H + h) * DK * dv;
-    // the warp's rows end at 4 ty + 3 of its upper half: later tokens of the chunk are zeros of A. So are those
-    // between a row and that end: added where all values are finite, left out where they are not.
-    const int first_row = 4 * (ty & ~1), j_end = min(n, 4 * (ty | 1) + 4);
-    for (int c0 = blockIdx.z * RF_SLICE; c0 < dv; c0 += gridDim.z * RF_SLICE) {
-        auto load_p = [&](int turn) {
-            if (turn < DK / RF_PK) {
-                float* dst = Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS;
-                for (int i = threadIdx.x; i < RF_PK * (RF_SLICE / 4); i += RC_THREADS) {
-                    const int d = i / (RF_SLICE / 4), c = (i % (RF_SLICE / 4)) * 4;
-                    const bool ok = c0 + c < dv;
-                    ft_copy16(dst + d * RF_LDS + c, ok ? Pc + (size_t)(turn * RF_PK + d) * dv + c0 + c : Pc, ok);
-                }
-            }
-            ft_commit();
-        };
-        __syncthreads();                                 // K (or the last slice's V) and P have been read
-        if (threadIdx.x == 0) s_odd = 0;
+    // Q and K
+    constexpr int PAIRS = 2 * RC_CHUNK * (DK / 16) / THREADS;
+    Pair8<T> run[PAIRS];
 #pragma unroll
-        for (int s = 0; s < RF_PSTAGES - 1; ++s) load_p(s);
-        Raw8<T> vr[RF_V_RUNS];
-        rf_ask_v(vr, v, v_stride, h, dv, c0, tok0, n);
-        FmaTile<1, 2, 16, 16> o;                         // 64 x 128
-        o.ty = ty;
-        o.tx = tx;
-        o.clear();
-        for (int turn = 0; turn < DK / RF_PK; ++turn) {
-            ft_wait<RF_PSTAGES - 2>();
-            __syncthreads();
-            load_p(turn + RF_PSTAGES - 1);
-            o.template add_swizzled<3, false>(Qt + turn * RF_PK * RF_LDN, RF_LDN, Ps + (turn % RF_PSTAGES) * RF_PK * RF_LDS, RF_LDS,
-                                     turn * RF_PK, RF_PK);
-            if (turn == 0 && rf_put_v(KV, vr, dv, c0, n, act)) s_odd = 1;     // seen past the next turn's barrier
+    for (int j = 0; j < PAIRS; ++j) {
+        const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
+        const size_t t = (size_t)(tok0 + (r < n ? r : 0));
+        run[j].load(i / (RC_CHUNK * (DK / 16)) ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
+                    rope ? rope + t * rot : nullptr, i % (DK / 16), rot);
+    }
+    // P: a stage is 64 channels x 128 columns (the halves of a slice one after the other), eight columns a thread and run
+    float4 p[2][2];
+    auto ask_p = [&](int stage) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = threadIdx.x + j * THREADS, d = 64 * (stage % HALVES) + i / 16, c = first + stage / HALVES * RF_SLICE + (i % 16) * 8;
+            const float4* src = (const float4*)(Pc + (size_t)d * dv + (c < dv ? c : 0));
+            p[j][0] = src[0];
+            p[j][1] = src[1];
         }
+    };
+    ask_p(0);
+    rf_powers(pw, decay[h]);
+    tg_before();
+    __syncthreads();
+    tg_after();
+    // columns: Q K^T by halves (0, 64); P Q of slice s and half x at 128 + 64 (2 s + x); A V of slice s at 384 + 64 s
+    const uint32_t tmem = tmem_slot, lanes = (uint32_t)((warp & 3) * 32) << 16;
+    bool odd = false, ok = true;
+    const bool issuer = warp == 0 && tg_elect();
 #pragma unroll
-        for (int i = 0; i < 4; ++i) o.scale_row(i, pw[4 * ty + i + 1]);
-        o.add(At, RF_LDN, KV, RF_LDS, s_odd ? first_row : j_end);
-        if (s_odd) o.add_triangle(At, RF_LDN, KV, RF_LDS, first_row, j_end);
+    for (int j = 0; j < PAIRS; ++j) {
+        const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
+        const bool key = i / (RC_CHUNK * (DK / 16));
+        float f[8], g[8];
+        run[j].values(act, f, g);
+        const float w = r >= n ? 0.f : key ? k_scale : 1.f;
+        if (r >= n || key)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-            if (4 * ty + i < n)
+            for (int x = 0; x < 8; ++x) { f[x] = r >= n ? 0.f : f[x] * w; g[x] = r >= n ? 0.f : g[x] * w; }
+        const uint32_t tile = tg_smem(key ? sK : sQ);
+        odd = rf_put8(tile + (uint32_t)(run[j].lo / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].lo / 8) & 7, f) || odd;
+        odd = rf_put8(tile + (uint32_t)(run[j].hi / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].hi / 8) & 7, g) || odd;
+    }
+    s3_fence();
+    __syncthreads();
+    if (issuer) {                                        // rows 64.. of the accumulators are nobody's
 #pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    if (c0 + o.col(c) < dv)
-                        *(float4*)(out + ((size_t)(tok0 + 4 * ty + i) * H + h) * dv + c0 + o.col(c)) = o.get(i, c);
+        for (int x = 0; x < HALVES; ++x)
+            s3_products<3, 3, 4>(tmem + 64u * x, tg_desc(sQ + x * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_desc(sK + x * RF_TILE),
+                                 HALVES * RF_TILE >> 4, 2, tg_idesc(64), false);
+        tg_commit(s_done);
+    }
+    __syncwarp();
+    Raw8<T> vr[rf_v_runs<THREADS>()];
+    for (int stage = 0; stage < stages; ++stage) {
+        const int b = stage & 1;
+        unsigned char* buf = sP + b * 6 * RF_TILE;
+        if (stage > 1) ok = ok && tg_wait(&p_done[b], ((stage >> 1) & 1) ^ 1, &retention_error_flag, 1);
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const int i = threadIdx.x + j * THREADS, d = i / 16, piece = i % 16;
+            float f[8] = {p[j][0].x, p[j][0].y, p[j][0].z, p[j][0].w, p[j][1].x, p[j][1].y, p[j][1].z, p[j][1].w};
+            if (first + stage / HALVES * RF_SLICE + piece * 8 >= dv)
+#pragma unroll
+                for (int x = 0; x < 8; ++x) f[x] = 0.f;
+            odd = rf_put8(tg_smem(buf) + (uint32_t)((piece >> 3) * RF_TILE), 2 * RF_TILE, d, piece & 7, f) || odd;
+        }
+        if (stage + 1 < stages) ask_p(stage + 1);
+        if (stage == HALVES - 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first, tok0, n);
+        s3_fence();
+        ok = __syncthreads_and(ok);
+        if (!ok) break;
+        if (issuer) {
+            tg_after();
+            s3_products<3, 3, 4>(tmem + 128u + 64u * (2 * (stage / HALVES) + stage % HALVES), tg_desc_mn(buf, RF_TILE), 2 * RF_TILE >> 4, 128,
+                                 tg_desc(sQ + stage % HALVES * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_idesc(64, false, true), false);
+            tg_commit(&p_done[b]);
+        }
+        __syncwarp();
+        if (stage != HALVES - 1) continue;
+        // beside the first slice: A's parts (a lane a token, 16 earlier tokens a warp) and the slice's values
+        ok = rf_made(s_done, 0, 2);
+        if (!ok) break;
+        if ((warp & 3) < 2) {
+            const int i = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16;
+            uint32_t s0[16], s1[16];
+            tg_ld16(tmem + lanes + (uint32_t)j0, s0);
+            if (HALVES > 1) tg_ld16(tmem + lanes + 64u + (uint32_t)j0, s1);
+            tg_wait_ld();
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                float f[8];
+#pragma unroll
+                for (int x = 0; x < 8; ++x) {
+                    const int gap = i - (j0 + 8 * y + x);
+                    const float s = __uint_as_float(s0[8 * y + x]) + (HALVES > 1 ? __uint_as_float(s1[8 * y + x]) : 0.f);
+                    f[x] = gap >= 0 ? s * pw[gap >= 0 ? gap : 0] : 0.f;
+                }
+                odd = rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f) || odd;
+            }
+        }
+        odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act) || odd;
+        if (ns > 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first + RF_SLICE, tok0, n);
+        s3_fence();
+        __syncthreads();
+        if (issuer) {
+            s3_products<VP, 3, 4>(tmem + 384u, tg_desc_mn(sV, RF_TILE), 2 * RF_TILE >> 4, 128, tg_desc(sA), RF_TILE >> 4, 2,
+                                  tg_idesc(64, false, true), false);
+            tg_commit(v_done);
+        }
+        __syncwarp();
+    }
+    if (ok) ok = rf_made(v_done, 0, 3);                  // and with it all that was issued before
+    if (ok && ns > 1) {
+        odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first + RF_SLICE, n, act) || odd;
+        s3_fence();
+        __syncthreads();
+        if (issuer) {
+            s3_products<VP, 3, 4>(tmem + 448u, tg_desc_mn(sV, RF_TILE), 2 * RF_TILE >> 4, 128, tg_desc(sA), RF_TILE >> 4, 2,
+                                  tg_idesc(64, false, true), false);
+            tg_commit(v_done);
+        }
+        __syncwarp();
+    }
+    if (ok) {
+        const int i0 = (warp >> 2) * 16;
+        for (int s = 0; s < ns && ok; ++s) {
+            if (s > 0) ok = rf_made(v_done, 1, 4);
+            const int c = first + s * RF_SLICE + (warp & 3) * 32 + lane;
+            uint32_t a[16], p0[16], p1[16];
+            tg_ld16(tmem + lanes + 384u + 64u * s + (uint32_t)i0, a);
+            tg_ld16(tmem + lanes + 128u + 128u * s + (uint32_t)i0, p0);
+            if (HALVES > 1) tg_ld16(tmem + lanes + 192u + 128u * s + (uint32_t)i0, p1);
+            tg_wait_ld();
+            float* dst = out + ((size_t)(tok0 + i0) * H + h) * dv + c;
+            if (c < dv && ok)
+#pragma unroll
+                for (int i = 0; i < 16; ++i, dst += (size_t)H * dv)
+                    if (i0 + i < n) {
+                        const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
+                        *dst = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
+                    }
+        }
+    }
+    if (!ok) {                                           // products that may still be under way
+        for (int x = 0; x < 8; ++x) tg_wait(&bars[x >> 1], x & 1, &retention_error_flag, 5);
+    } else if (__syncthreads_or(odd)) {                  // plain sums: a term past a row is not added at all
+        float* Qf = (float*)sQ;                          // [64][RF_LOOP_LD], then K's
+        float* Kf = Qf + RC_CHUNK * RF_LOOP_LD;
+        float* Af = Kf + RC_CHUNK * RF_LOOP_LD;          // [64][65]
+        load_rotated(Qf, RF_LOOP_LD, q, q_stride, h, DK, rope, rot, tok0, n, 1.f, act);
+        load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
+        __syncthreads();
+        for (int x = threadIdx.x; x < n * RC_CHUNK; x += THREADS) {
+            const int i = x / RC_CHUNK, j = x % RC_CHUNK;
+            float s = 0.f;
+            for (int d = 0; j <= i && d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Kf[j * RF_LOOP_LD + d], s);
+            Af[i * (RC_CHUNK + 1) + j] = j <= i ? s * pw[i - j] : 0.f;
+        }
+        __syncthreads();
+        for (int x = threadIdx.x; x < n * RF_SLICE * ns; x += THREADS) {
+            const int i = x / (RF_SLICE * ns), c = first + x % (RF_SLICE * ns);
+            if (c >= dv) continue;
+            float s = 0.f;
+            for (int d = 0; d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Pc[(size_t)d * dv + c], s);
+            s *= pw[i + 1];
+            for (int j = 0; j <= i; ++j)
+                s = fmaf(Af[i * (RC_CHUNK + 1) + j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
+            if (rf_not_finite(s)) out[((size_t)(tok0 + i) * H + h) * dv + c] = s;
+        }
+    }
+    tg_before();
+    __syncthreads();
+    if (warp == 0) {
+        tg_after();
+        tg_free512(tmem);
     }
 }
 
-template <typename T, int DK>
-static int retention_tiled(const T* q, long long q_stride, const T* k, long long k_stride, const T* v, long long v_stride,
+template <typename T, int DK, int VP>
+static int retention_tc(const T* q, long long q_stride, const T* k, long long k_stride, const T* v, long long v_stride,
                            float* out, int B, int H, int dv, const float* decay, float k_scale, int act,
                            const float* rope, int rot, const int* q_start, const int* state_slots, float* state,
                            int chunks, const int* chunk_tok0, const int* chunk_ntok, const int* chunk_first,
                            float* scratch, cudaStream_t stream) {
-    constexpr size_t s1 = (size_t)RC_CHUNK * (DK + 4 + RF_LDS) * sizeof(float);
-    constexpr size_t kv = (size_t)(DK * RF_LDN > RC_CHUNK * RF_LDS ? DK * RF_LDN : RC_CHUNK * RF_LDS);
-    constexpr size_t s3 = ((size_t)(DK + RC_CHUNK) * RF_LDN + RF_PSTAGES * RF_PK * RF_LDS + kv) * sizeof(float);
-    auto k1 = retention_summaries_tiled_kernel<T, DK>;
-    auto k3 = retention_outputs_tiled_kernel<T, DK>;
+    constexpr size_t s1 = 1024 + (size_t)(3 * (DK / 64) + 4 * VP) * RF_TILE, s3 = 1024 + rf_out_bytes<DK>();
+    static_assert(s1 >= 1024 + RC_CHUNK * RF_LOOP_LD * sizeof(float), "the plain sums' tiles");
+    static_assert(s3 >= 1024 + RC_CHUNK * (2 * RF_LOOP_LD + RC_CHUNK + 1) * sizeof(float), "the plain sums' tiles");
+    auto k1 = retention_summaries_tc_kernel<T, DK, VP>;
+    auto k3 = retention_outputs_tc_kernel<T, DK, VP>;
     static bool sized[64] = {};                          // per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -829,18 +1019,21 @@ static int retention_tiled(const T* q, long long q_stride, const T* k, long long
         if ((e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
         sized[dev] = true;
     }
-    const int slices = (dv + RF_SLICE - 1) / RF_SLICE;
-    int rc = tgo_launch_pdl(k1, dim3(chunks, H, slices), dim3(RC_THREADS), s1, stream, k, k_stride, v, v_stride, H, dv,
-                            decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, scratch);
+    // two slices a block, which share Q's and K's parts, unless blocks of one are fewer than the multiprocessors
+    const int slices = (dv + RF_SLICE - 1) / RF_SLICE, per = (long long)chunks * H * slices > tgo_multiprocessors() ? 2 : 1;
+    const int z = (slices + per - 1) / per;
+    int rc = tgo_launch_pdl(k1, dim3(chunks, H, z), dim3(RC_THREADS), s1, stream, k, k_stride, v, v_stride, H, dv,
+                            decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, per, scratch);
     if (rc) return rc;
     rc = tgo_launch_pdl(retention_scan4_kernel, dim3(B, H, (DK * dv / 4 + 255) / 256), dim3(256), 0, stream, H, DK * dv,
                         decay, q_start, state_slots, chunk_first, scratch, state);
     if (rc) return rc;
-    // two blocks an SM: with fewer (chunk, head) pairs than twice that a block takes one slice
-    const int z = (long long)chunks * H < 4 * tgo_multiprocessors() ? slices : 1;
-    return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RC_THREADS), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
-                          H, dv, decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, (const float*)scratch);
+    return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RF_OUT_THREADS), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
+                          H, dv, decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, per, (const float*)scratch);
 }
+
+// The code a wait of the chunks' products left when it ran out (0: none did). Synchronises.
+TGO_API int tgo_retention_error(int* value) { return (int)cudaMemcpyFromSymbol(value, retention_error_flag, sizeof(int)); }
 
 static inline size_t summaries_smem(int dk) {
     return ((size_t)RC_CHUNK * (dk + 1) + (size_t)RC_CHUNK * RC_VS + RC_CHUNK + 1) * sizeof(float);
@@ -874,11 +1067,16 @@ static int retention_chunked(const T* q, long long q_stride, const T* k, long lo
     auto whole = [&](const void* p, long long stride) { return (uintptr_t)p % 16 == 0 && stride * sizeof(T) % 16 == 0; };
     if ((dk == 64 || dk == 128) && dv % 8 == 0 && rot % 16 == 0 && whole(q, q_stride) && whole(k, k_stride) &&
         whole(v, v_stride) && (uintptr_t)rope % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)state % 16 == 0 && (uintptr_t)scratch % 16 == 0) {
-#define RF_GO(DK)                                                                                                    \
-    return retention_tiled<T, DK>(q, q_stride, k, k_stride, v, v_stride, out, B, H, dv, decay, k_scale, act, rope,    \
-                                  rot, q_start, state_slots, state, chunks, chunk_tok0, chunk_ntok, chunk_first, scratch, stream)
-        if (dk == 128) RF_GO(128);
-        RF_GO(64);
+#define RF_GO(DK, VP)                                                                                                \
+    return retention_tc<T, DK, VP>(q, q_stride, k, k_stride, v, v_stride, out, B, H, dv, decay, k_scale, act, rope,  \
+                                   rot, q_start, state_slots, state, chunks, chunk_tok0, chunk_ntok, chunk_first, scratch, stream)
+        if constexpr (sizeof(T) == 2)
+            if (act == 0) {
+                if (dk == 128) RF_GO(128, 1);
+                RF_GO(64, 1);
+            }
+        if (dk == 128) RF_GO(128, 3);
+        RF_GO(64, 3);
 #undef RF_GO
     }
     const size_t s1 = summaries_smem(dk), s3 = outputs_smem(dk);

@@ -21,8 +21,86 @@ __device__ __forceinline__ void s3_split8(const float (&v)[8], uint4& hi, uint4&
     s3_split2(v[4], v[5], hi.z, mid.z, lo.z);
     s3_split2(v[6], v[7], hi.w, mid.w, lo.w);
 }
+// Whether one of two packed bfloat16 numbers is infinite or NaN.
+__device__ __forceinline__ bool s3_odd2(uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; }
+__device__ __forceinline__ bool s3_odd8(uint4 w) { return s3_odd2(w.x) || s3_odd2(w.y) || s3_odd2(w.z) || s3_odd2(w.w); }
+// The same with every part finite, for products whose masked terms must stay zero: a number that rounds past the
+// largest bfloat16 has its hi cut instead, one that is not finite is taken for 0. True: there was one of those.
+__device__ __noinline__ bool s3_mend8(const float* v, uint32_t* hi, uint32_t* mid, uint32_t* lo) {
+    bool odd = false;
+    for (int i = 0; i < 8; ++i) {
+        float x = v[i];
+        const bool ok = fabsf(x) < __int_as_float(0x7f800000);
+        odd = odd || !ok;
+        x = ok ? x : 0.f;
+        uint32_t h = __float_as_uint(__bfloat162float(__float2bfloat16_rn(x)));
+        if ((h & 0x7f800000u) == 0x7f800000u) h = __float_as_uint(x) & 0xffff0000u;
+        const float r = x - __uint_as_float(h);
+        const uint32_t m = __float_as_uint(__bfloat162float(__float2bfloat16_rn(r)));
+        const uint32_t l = __float_as_uint(__bfloat162float(__float2bfloat16_rn(r - __uint_as_float(m))));
+        const int at = 16 * (i & 1);
+        hi[i >> 1] = at ? hi[i >> 1] | h : h >> 16;
+        mid[i >> 1] = at ? mid[i >> 1] | m : m >> 16;
+        lo[i >> 1] = at ? lo[i >> 1] | l : l >> 16;
+    }
+    return odd;
+}
+__device__ __forceinline__ bool s3_split8_finite(const float (&v)[8], uint4 (&part)[3]) {
+    s3_split8(v, part[0], part[1], part[2]);
+    // the rest of what is not finite, or rounds to infinity, is not finite: 0 times it is not 0
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+    __nv_bfloat162 seen = zero;
+    seen = __hfma2(*(const __nv_bfloat162*)&part[1].x, zero, seen);
+    seen = __hfma2(*(const __nv_bfloat162*)&part[1].y, zero, seen);
+    seen = __hfma2(*(const __nv_bfloat162*)&part[1].z, zero, seen);
+    seen = __hfma2(*(const __nv_bfloat162*)&part[1].w, zero, seen);
+    if (!(*(const uint32_t*)&seen & 0x7fff7fffu)) return false;
+    float f[8];
+    uint32_t w[3][4];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[i] = v[i];
+    const bool odd = s3_mend8(f, w[0], w[1], w[2]);
+#pragma unroll
+    for (int p = 0; p < 3; ++p) part[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
+    return odd;
+}
+// ... of numbers that are bfloat16 numbers already.
+__device__ __forceinline__ bool s3_finite8(uint4& v) {
+    if (!s3_odd8(v)) return false;
+    uint32_t w[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        if ((w[i] & 0x7f80u) == 0x7f80u) w[i] &= 0xffff0000u;
+        if ((w[i] & 0x7f800000u) == 0x7f800000u) w[i] &= 0xffffu;
+    }
+    v = make_uint4(w[0], w[1], w[2], w[3]);
+    return true;
+}
 __device__ __forceinline__ void s3_store16(uint32_t addr, uint4 v) {
     asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
 }
 // Generic stores to shared memory, made visible to the products that read them.
 __device__ __forceinline__ void s3_fence() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+
+// A 16-byte piece's place in a tile of 128-byte rows with the 128-byte swizzle.
+__device__ __forceinline__ uint32_t s3_place(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
+// D += A B^T over 16 KSTEPS of k and every kept pair of parts, the smallest first. Part p of A starts a_part * p
+// after da and a k-step a_k after the one before (descriptor units of 16 bytes); AP, BP: parts there are (1: the
+// numbers are bfloat16 numbers themselves). One thread issues.
+template <int AP, int BP, int KSTEPS>
+__device__ __forceinline__ void s3_products(uint32_t d, uint64_t da, uint32_t a_part, uint32_t a_k, uint64_t db, uint32_t b_part,
+                                            uint32_t b_k, uint32_t idesc, bool more) {
+    uint32_t acc = more ? 1u : 0u;
+#pragma unroll
+    for (int sum = 2; sum >= 0; --sum)
+#pragma unroll
+        for (int p = 0; p < AP; ++p) {
+            const int q = sum - p;
+            if (q < 0 || q >= BP) continue;
+#pragma unroll
+            for (int k = 0; k < KSTEPS; ++k) {
+                tg_mma(d, da + (uint64_t)(a_part * p + a_k * k), db + (uint64_t)(b_part * q + b_k * k), idesc, acc);
+                acc = 1u;
+            }
+        }
+}

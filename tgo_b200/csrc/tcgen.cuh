@@ -95,6 +95,14 @@ __device__ __forceinline__ void tg_alloc512(uint32_t* slot) {
 __device__ __forceinline__ void tg_free512(uint32_t tmem) {
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
 }
+// ... some of them, so that several CTAs of an SM can each have their share (a power of two from 32 on)
+template <int COLS> __device__ __forceinline__ void tg_alloc(uint32_t* slot) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tg_smem(slot)), "r"((uint32_t)COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+template <int COLS> __device__ __forceinline__ void tg_free(uint32_t tmem) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"((uint32_t)COLS) : "memory");
+}
 // Descriptor of an operand tile: rows of 128 bytes with the 128-byte swizzle, groups of eight rows
 // 1024 bytes apart. K-major: the rows are the M or N index, 16 values of k are 2 units further.
 __device__ __forceinline__ uint64_t tg_desc(const void* tile) {
@@ -115,9 +123,9 @@ __device__ __forceinline__ uint64_t tg_desc_mn(const void* tile, uint32_t block)
     d |= (uint64_t)2 << 61;
     return d;
 }
-// float32 sums of bfloat16 products, M = 128, both operands K-major (b_mn: B is MN-major)
-__device__ __forceinline__ uint32_t tg_idesc(int n, bool b_mn = false) {
-    return (1u << 4) | (1u << 7) | (1u << 10) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+// float32 sums of bfloat16 products, M = 128, both operands K-major (a_mn, b_mn: A, B is MN-major)
+__device__ __forceinline__ uint32_t tg_idesc(int n, bool b_mn = false, bool a_mn = false) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | (a_mn ? 1u << 15 : 0u) | (b_mn ? 1u << 16 : 0u) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
 }
 __device__ __forceinline__ void tg_ld32(uint32_t taddr, uint32_t (&r)[32]) {
     asm volatile(

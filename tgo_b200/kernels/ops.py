@@ -1504,6 +1504,13 @@ def retention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: torch.Tens
         f"(heads={num_heads}, dk={key_dim}, dv={value_dim})")
 
 
+def retention_error() -> int:
+    """The code a wait of the chunked retention kernels left when it ran out, or 0. Synchronises."""
+    value = ctypes.c_int(0)
+    _check(entry_points("retention").tgo_retention_error(ctypes.addressof(value)), "retention_error")
+    return int(value.value)
+
+
 def retention_chunk_tokens() -> int:
     """Tokens of one request a chunk of the chunked retention kernels holds at most."""
     return int(entry_points("retention").tgo_retention_chunk_tokens())
@@ -2177,6 +2184,10 @@ def kernel_wait_errors() -> dict:
         code = sgemm_error()
         if code:
             out["sgemm"] = code
+    if "retention" in _loaded:
+        code = retention_error()
+        if code:
+            out["retention"] = code
     for key, flag in _tc_err.items():
         code = int(flag.item())
         if code:
