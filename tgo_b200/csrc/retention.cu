@@ -492,14 +492,16 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 //   summaries   U^T = V^T K: K's scaled and rotated rows and V, one product of 64 tokens;
 //   scan        four neighbouring elements a thread, eight summaries asked for while the eight before
 //               them are used: bound by memory (every summary read once, every state written once);
-//   outputs     by halves of 64 key channels, one after the other through the same shared memory (two blocks an SM
-//               hide each other's loads): Q K^T and P^T Q^T; then A = decay^(i-j) Q K^T goes back to
-//               shared memory as parts, V^T A^T is made, and out = decay^(i+1) (Q P) + A V.
+//   outputs     Q and K once for up to two slices: Q K^T by halves of 64 channels; P comes 64 channels x 128 columns
+//               at a time through two buffers, P^T Q^T; A = decay^(i-j) Q K^T goes back to shared memory as
+//               parts (over K's), V^T A^T; out = decay^(i+1) (Q P) + A V. A warp of its own issues the products while
+//               sixteen lay the next operands down. (One slice a block, halves of Q, K and P one after the
+//               other, two blocks an SM: 167 us.)
 // Zeros of A times a value that is not finite are not zero: such a number is laid down as 0, which leaves what does
 // not depend on it as it is, bit for bit, and a block that met one makes plain sums too and writes those that are not finite.
 // MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
-// summaries @S@ us (122), scan 40, outputs @O@ us (190). Bound by the bytes of U, P and the outputs, and by the
-// conversions' instructions.
+// summaries 50 us (122), scan 40, outputs 119 us (190). The summaries are bound by the bytes of U; a block of the outputs
+// by its chain: loads 5000 cycles, parts of Q and K 3000, 168 products of 75 cycles, results 2300.
 #define RF_SLICE 128
 #define RF_TILE 8192                  // 64 rows of 64 bfloat16 numbers
 #define RF_LOOP_LD 129                // rows of the plain sums' tiles
@@ -785,12 +787,12 @@ retention_scan4_kernel(int H, int dkdv, const float* __restrict__ decay, const i
 
 // Shared memory: Q's parts (a part DK / 64 tiles), two buffers of P's (64 channels x 128 columns, two tiles a part),
 // K's parts, over which A's and one slice's values come to lie (24 KB more than K at DK = 128).
-#define RF_OUT_THREADS 512
+#define RF_OUT_THREADS 512           // and a warp that issues the products
 template <int DK> __host__ __device__ constexpr int rf_out_k() { return 3 * (DK / 64) * RF_TILE + 2 * 6 * RF_TILE; }
 template <int DK> __host__ __device__ constexpr int rf_out_bytes() { return rf_out_k<DK>() + 9 * RF_TILE; }
 
 template <typename T, int DK, int VP>
-__global__ void __launch_bounds__(RF_OUT_THREADS, 1)
+__global__ void __launch_bounds__(RF_OUT_THREADS + 32, 1)
 retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T* __restrict__ k, long long k_stride,
                             const T* __restrict__ v, long long v_stride, float* __restrict__ out, int H, int dv,
                             const float* __restrict__ decay, float k_scale, int act, const float* __restrict__ rope,
@@ -804,13 +806,14 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     unsigned char* sA = sK;
     unsigned char* sV = sK + 3 * RF_TILE;
     __shared__ float pw[RC_CHUNK + 1];
-    __shared__ __align__(8) uint64_t bars[4];
+    __shared__ __align__(8) uint64_t bars[9];
     __shared__ uint32_t tmem_slot;
     uint64_t *s_done = bars, *p_done = bars + 1 /* [2] */, *v_done = bars + 3;
+    uint64_t *qk_full = bars + 4, *p_full = bars + 5 /* [2] */, *a_full = bars + 7, *v_full = bars + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) tg_alloc512(&tmem_slot);
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 4; ++i) tg_init(&bars[i], 1);
+        for (int i = 0; i < 9; ++i) tg_init(&bars[i], i < 4 ? 1 : THREADS / 32);
         tg_init_done();
     }
     pdl_wait();
@@ -818,168 +821,189 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
     const int ns = min(slices, (dv - first + RF_SLICE - 1) / RF_SLICE), stages = ns * HALVES;
     const float* Pc = P + ((size_t)ci * H + h) * DK * dv;
-    // Q and K
-    constexpr int PAIRS = 2 * RC_CHUNK * (DK / 16) / THREADS;
-    Pair8<T> run[PAIRS];
-#pragma unroll
-    for (int j = 0; j < PAIRS; ++j) {
-        const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
-        const size_t t = (size_t)(tok0 + (r < n ? r : 0));
-        run[j].load(i / (RC_CHUNK * (DK / 16)) ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
-                    rope ? rope + t * rot : nullptr, i % (DK / 16), rot);
-    }
-    // P: a stage is 64 channels x 128 columns (the halves of a slice one after the other), eight columns a thread and run
-    float4 p[2][2];
-    auto ask_p = [&](int stage) {
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = threadIdx.x + j * THREADS, d = 64 * (stage % HALVES) + i / 16, c = first + stage / HALVES * RF_SLICE + (i % 16) * 8;
-            const float4* src = (const float4*)(Pc + (size_t)d * dv + (c < dv ? c : 0));
-            p[j][0] = src[0];
-            p[j][1] = src[1];
-        }
-    };
-    ask_p(0);
-    rf_powers(pw, decay[h]);
-    tg_before();
-    __syncthreads();
-    tg_after();
     // columns: Q K^T by halves (0, 64); P Q of slice s and half x at 128 + 64 (2 s + x); A V of slice s at 384 + 64 s
-    const uint32_t tmem = tmem_slot, lanes = (uint32_t)((warp & 3) * 32) << 16;
     bool odd = false, ok = true;
-    const bool issuer = warp == 0 && tg_elect();
-#pragma unroll
-    for (int j = 0; j < PAIRS; ++j) {
-        const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
-        const bool key = i / (RC_CHUNK * (DK / 16));
-        float f[8], g[8];
-        run[j].values(act, f, g);
-        const float w = r >= n ? 0.f : key ? k_scale : 1.f;
-        if (r >= n || key)
-#pragma unroll
-            for (int x = 0; x < 8; ++x) { f[x] = r >= n ? 0.f : f[x] * w; g[x] = r >= n ? 0.f : g[x] * w; }
-        const uint32_t tile = tg_smem(key ? sK : sQ);
-        odd = rf_put8(tile + (uint32_t)(run[j].lo / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].lo / 8) & 7, f) || odd;
-        odd = rf_put8(tile + (uint32_t)(run[j].hi / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].hi / 8) & 7, g) || odd;
-    }
-    s3_fence();
-    __syncthreads();
-    if (issuer) {                                        // rows 64.. of the accumulators are nobody's
-#pragma unroll
-        for (int x = 0; x < HALVES; ++x)
-            s3_products<3, 3, 4>(tmem + 64u * x, tg_desc(sQ + x * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_desc(sK + x * RF_TILE),
-                                 HALVES * RF_TILE >> 4, 2, tg_idesc(64), false);
-        tg_commit(s_done);
-    }
-    __syncwarp();
-    Raw8<T> vr[rf_v_runs<THREADS>()];
-    for (int stage = 0; stage < stages; ++stage) {
-        const int b = stage & 1;
-        unsigned char* buf = sP + b * 6 * RF_TILE;
-        if (stage > 1) ok = ok && tg_wait(&p_done[b], ((stage >> 1) & 1) ^ 1, &retention_error_flag, 1);
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const int i = threadIdx.x + j * THREADS, d = i / 16, piece = i % 16;
-            float f[8] = {p[j][0].x, p[j][0].y, p[j][0].z, p[j][0].w, p[j][1].x, p[j][1].y, p[j][1].z, p[j][1].w};
-            if (first + stage / HALVES * RF_SLICE + piece * 8 >= dv)
-#pragma unroll
-                for (int x = 0; x < 8; ++x) f[x] = 0.f;
-            odd = rf_put8(tg_smem(buf) + (uint32_t)((piece >> 3) * RF_TILE), 2 * RF_TILE, d, piece & 7, f) || odd;
-        }
-        if (stage + 1 < stages) ask_p(stage + 1);
-        if (stage == HALVES - 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first, tok0, n);
-        s3_fence();
-        ok = __syncthreads_and(ok);
-        if (!ok) break;
-        if (issuer) {
+    if (warp == THREADS / 32) {
+        // ---------------------------------------------------------- issuer
+        tg_before();
+        __syncthreads();
+        tg_after();
+        const uint32_t tmem = tmem_slot;
+        const bool leader = tg_elect();
+        auto wait = [&](uint64_t* bar, uint32_t phase) {
+            ok = __all_sync(0xffffffffu, ok && tg_wait(bar, phase, &retention_error_flag, 6));
             tg_after();
-            s3_products<3, 3, 4>(tmem + 128u + 64u * (2 * (stage / HALVES) + stage % HALVES), tg_desc_mn(buf, RF_TILE), 2 * RF_TILE >> 4, 128,
-                                 tg_desc(sQ + stage % HALVES * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_idesc(64, false, true), false);
-            tg_commit(&p_done[b]);
+            return ok;
+        };
+        if (wait(qk_full, 0) && leader) {                // rows 64.. of the accumulators are nobody's
+#pragma unroll
+            for (int x = 0; x < HALVES; ++x)
+                s3_products<3, 3, 4>(tmem + 64u * x, tg_desc(sQ + x * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_desc(sK + x * RF_TILE),
+                                     HALVES * RF_TILE >> 4, 2, tg_idesc(64), false);
+            tg_commit(s_done);
         }
         __syncwarp();
-        if (stage != HALVES - 1) continue;
-        // beside the first slice: A's parts (a lane a token, 16 earlier tokens a warp) and the slice's values
-        ok = rf_made(s_done, 0, 2);
-        if (!ok) break;
-        if ((warp & 3) < 2) {
-            const int i = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16;
-            uint32_t s0[16], s1[16];
-            tg_ld16(tmem + lanes + (uint32_t)j0, s0);
-            if (HALVES > 1) tg_ld16(tmem + lanes + 64u + (uint32_t)j0, s1);
-            tg_wait_ld();
+        auto values = [&](int s) {
+            if (leader) {
+                s3_products<VP, 3, 4>(tmem + 384u + 64u * s, tg_desc_mn(sV, RF_TILE), 2 * RF_TILE >> 4, 128, tg_desc(sA), RF_TILE >> 4, 2,
+                                      tg_idesc(64, false, true), false);
+                tg_commit(v_done);
+            }
+            __syncwarp();
+        };
+        for (int stage = 0; stage < stages && ok; ++stage) {
+            const int b = stage & 1, x = stage % HALVES;
+            if (wait(&p_full[b], (stage >> 1) & 1) && leader) {
+                s3_products<3, 3, 4>(tmem + 128u + 64u * (2 * (stage / HALVES) + x), tg_desc_mn(sP + b * 6 * RF_TILE, RF_TILE),
+                                     2 * RF_TILE >> 4, 128, tg_desc(sQ + x * RF_TILE), HALVES * RF_TILE >> 4, 2, tg_idesc(64, false, true), false);
+                tg_commit(&p_done[b]);
+            }
+            __syncwarp();
+            if (stage == HALVES - 1 && ok && wait(a_full, 0)) values(0);
+        }
+        if (ns > 1 && ok && wait(v_full, 0)) values(1);
+    } else {
+        // ---------------------------------------------------------- parts and results
+        // Q and K
+        constexpr int PAIRS = 2 * RC_CHUNK * (DK / 16) / THREADS;
+        Pair8<T> run[PAIRS];
 #pragma unroll
-            for (int y = 0; y < 2; ++y) {
-                float f[8];
+        for (int j = 0; j < PAIRS; ++j) {
+            const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
+            const size_t t = (size_t)(tok0 + (r < n ? r : 0));
+            run[j].load(i / (RC_CHUNK * (DK / 16)) ? k + t * k_stride + (size_t)h * DK : q + t * q_stride + (size_t)h * DK,
+                        rope ? rope + t * rot : nullptr, i % (DK / 16), rot);
+        }
+        // P: a stage is 64 channels x 128 columns (the halves of a slice one after the other), eight columns a thread and run
+        float4 p[2][2];
+        auto ask_p = [&](int stage) {
 #pragma unroll
-                for (int x = 0; x < 8; ++x) {
-                    const int gap = i - (j0 + 8 * y + x);
-                    const float s = __uint_as_float(s0[8 * y + x]) + (HALVES > 1 ? __uint_as_float(s1[8 * y + x]) : 0.f);
-                    f[x] = gap >= 0 ? s * pw[gap >= 0 ? gap : 0] : 0.f;
+            for (int j = 0; j < 2; ++j) {
+                const int i = threadIdx.x + j * THREADS, d = 64 * (stage % HALVES) + i / 16, c = first + stage / HALVES * RF_SLICE + (i % 16) * 8;
+                const float4* src = (const float4*)(Pc + (size_t)d * dv + (c < dv ? c : 0));
+                p[j][0] = src[0];
+                p[j][1] = src[1];
+            }
+        };
+        ask_p(0);
+        rf_powers(pw, decay[h]);
+        tg_before();
+        __syncthreads();
+        tg_after();
+        const uint32_t tmem = tmem_slot, lanes = (uint32_t)((warp & 3) * 32) << 16;
+        auto full = [&](uint64_t* bar) {                     // a warp's share of an operand is laid down
+            s3_fence();
+            tg_before();
+            __syncwarp();
+            if (lane == 0) tg_arrive(bar);
+        };
+#pragma unroll
+        for (int j = 0; j < PAIRS; ++j) {
+            const int i = threadIdx.x + j * THREADS, r = (i / (DK / 16)) % RC_CHUNK;
+            const bool key = i / (RC_CHUNK * (DK / 16));
+            float f[8], g[8];
+            run[j].values(act, f, g);
+            const float w = r >= n ? 0.f : key ? k_scale : 1.f;
+            if (r >= n || key)
+#pragma unroll
+                for (int x = 0; x < 8; ++x) { f[x] = r >= n ? 0.f : f[x] * w; g[x] = r >= n ? 0.f : g[x] * w; }
+            const uint32_t tile = tg_smem(key ? sK : sQ);
+            odd = rf_put8(tile + (uint32_t)(run[j].lo / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].lo / 8) & 7, f) || odd;
+            odd = rf_put8(tile + (uint32_t)(run[j].hi / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].hi / 8) & 7, g) || odd;
+        }
+        full(qk_full);
+        Raw8<T> vr[rf_v_runs<THREADS>()];
+        for (int stage = 0; stage < stages; ++stage) {
+            const int b = stage & 1;
+            unsigned char* buf = sP + b * 6 * RF_TILE;
+            if (stage > 1) ok = __all_sync(0xffffffffu, tg_wait(&p_done[b], ((stage >> 1) & 1) ^ 1, &retention_error_flag, 1));
+            if (!ok) break;
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int i = threadIdx.x + j * THREADS, d = i / 16, piece = i % 16;
+                float f[8] = {p[j][0].x, p[j][0].y, p[j][0].z, p[j][0].w, p[j][1].x, p[j][1].y, p[j][1].z, p[j][1].w};
+                if (first + stage / HALVES * RF_SLICE + piece * 8 >= dv)
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) f[x] = 0.f;
+                odd = rf_put8(tg_smem(buf) + (uint32_t)((piece >> 3) * RF_TILE), 2 * RF_TILE, d, piece & 7, f) || odd;
+            }
+            if (stage + 1 < stages) ask_p(stage + 1);
+            if (stage == HALVES - 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first, tok0, n);
+            full(&p_full[b]);
+            if (stage != HALVES - 1) continue;
+            // beside the first slice: A's parts (a lane a token, 16 earlier tokens a warp) and the slice's values
+            ok = __all_sync(0xffffffffu, tg_wait(s_done, 0, &retention_error_flag, 2));
+            if (!ok) break;
+            tg_after();
+            if ((warp & 3) < 2) {
+                const int i = (warp & 3) * 32 + lane, j0 = (warp >> 2) * 16;
+                uint32_t s0[16], s1[16];
+                tg_ld16(tmem + lanes + (uint32_t)j0, s0);
+                if (HALVES > 1) tg_ld16(tmem + lanes + 64u + (uint32_t)j0, s1);
+                tg_wait_ld();
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    float f[8];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        const int gap = i - (j0 + 8 * y + x);
+                        const float s = __uint_as_float(s0[8 * y + x]) + (HALVES > 1 ? __uint_as_float(s1[8 * y + x]) : 0.f);
+                        f[x] = gap >= 0 ? s * pw[gap >= 0 ? gap : 0] : 0.f;
+                    }
+                    odd = rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f) || odd;
                 }
-                odd = rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f) || odd;
+            }
+            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act) || odd;
+            if (ns > 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first + RF_SLICE, tok0, n);
+            full(a_full);
+        }
+        if (ok) ok = __all_sync(0xffffffffu, tg_wait(v_done, 0, &retention_error_flag, 3));      // and with it all that was issued before
+        tg_after();
+        if (ok && ns > 1) {
+            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first + RF_SLICE, n, act) || odd;
+            full(v_full);
+        }
+        if (ok) {
+            const int i0 = (warp >> 2) * 16;
+            for (int s = 0; s < ns && ok; ++s) {
+                if (s > 0) ok = __all_sync(0xffffffffu, tg_wait(v_done, 1, &retention_error_flag, 4));
+                tg_after();
+                const int c = first + s * RF_SLICE + (warp & 3) * 32 + lane;
+                uint32_t a[16], p0[16], p1[16];
+                tg_ld16(tmem + lanes + 384u + 64u * s + (uint32_t)i0, a);
+                tg_ld16(tmem + lanes + 128u + 128u * s + (uint32_t)i0, p0);
+                if (HALVES > 1) tg_ld16(tmem + lanes + 192u + 128u * s + (uint32_t)i0, p1);
+                tg_wait_ld();
+                float* dst = out + ((size_t)(tok0 + i0) * H + h) * dv + c;
+                if (c < dv && ok)
+#pragma unroll
+                    for (int i = 0; i < 16; ++i, dst += (size_t)H * dv)
+                        if (i0 + i < n) {
+                            const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
+                            *dst = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
+                        }
             }
         }
-        odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act) || odd;
-        if (ns > 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first + RF_SLICE, tok0, n);
-        s3_fence();
-        __syncthreads();
-        if (issuer) {
-            s3_products<VP, 3, 4>(tmem + 384u, tg_desc_mn(sV, RF_TILE), 2 * RF_TILE >> 4, 128, tg_desc(sA), RF_TILE >> 4, 2,
-                                  tg_idesc(64, false, true), false);
-            tg_commit(v_done);
-        }
-        __syncwarp();
     }
-    if (ok) ok = rf_made(v_done, 0, 3);                  // and with it all that was issued before
-    if (ok && ns > 1) {
-        odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first + RF_SLICE, n, act) || odd;
-        s3_fence();
-        __syncthreads();
-        if (issuer) {
-            s3_products<VP, 3, 4>(tmem + 448u, tg_desc_mn(sV, RF_TILE), 2 * RF_TILE >> 4, 128, tg_desc(sA), RF_TILE >> 4, 2,
-                                  tg_idesc(64, false, true), false);
-            tg_commit(v_done);
-        }
-        __syncwarp();
-    }
-    if (ok) {
-        const int i0 = (warp >> 2) * 16;
-        for (int s = 0; s < ns && ok; ++s) {
-            if (s > 0) ok = rf_made(v_done, 1, 4);
-            const int c = first + s * RF_SLICE + (warp & 3) * 32 + lane;
-            uint32_t a[16], p0[16], p1[16];
-            tg_ld16(tmem + lanes + 384u + 64u * s + (uint32_t)i0, a);
-            tg_ld16(tmem + lanes + 128u + 128u * s + (uint32_t)i0, p0);
-            if (HALVES > 1) tg_ld16(tmem + lanes + 192u + 128u * s + (uint32_t)i0, p1);
-            tg_wait_ld();
-            float* dst = out + ((size_t)(tok0 + i0) * H + h) * dv + c;
-            if (c < dv && ok)
-#pragma unroll
-                for (int i = 0; i < 16; ++i, dst += (size_t)H * dv)
-                    if (i0 + i < n) {
-                        const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
-                        *dst = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
-                    }
-        }
-    }
+    ok = __syncthreads_and(ok);
+    odd = __syncthreads_or(odd);
     if (!ok) {                                           // products that may still be under way
         for (int x = 0; x < 8; ++x) tg_wait(&bars[x >> 1], x & 1, &retention_error_flag, 5);
-    } else if (__syncthreads_or(odd)) {                  // plain sums: a term past a row is not added at all
+    } else if (odd) {                                    // plain sums: a term past a row is not added at all
         float* Qf = (float*)sQ;                          // [64][RF_LOOP_LD], then K's
         float* Kf = Qf + RC_CHUNK * RF_LOOP_LD;
         float* Af = Kf + RC_CHUNK * RF_LOOP_LD;          // [64][65]
         load_rotated(Qf, RF_LOOP_LD, q, q_stride, h, DK, rope, rot, tok0, n, 1.f, act);
         load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
         __syncthreads();
-        for (int x = threadIdx.x; x < n * RC_CHUNK; x += THREADS) {
+        for (int x = threadIdx.x; x < n * RC_CHUNK; x += THREADS + 32) {
             const int i = x / RC_CHUNK, j = x % RC_CHUNK;
             float s = 0.f;
             for (int d = 0; j <= i && d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Kf[j * RF_LOOP_LD + d], s);
             Af[i * (RC_CHUNK + 1) + j] = j <= i ? s * pw[i - j] : 0.f;
         }
         __syncthreads();
-        for (int x = threadIdx.x; x < n * RF_SLICE * ns; x += THREADS) {
+        for (int x = threadIdx.x; x < n * RF_SLICE * ns; x += THREADS + 32) {
             const int i = x / (RF_SLICE * ns), c = first + x % (RF_SLICE * ns);
             if (c >= dv) continue;
             float s = 0.f;
@@ -994,7 +1018,7 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     __syncthreads();
     if (warp == 0) {
         tg_after();
-        tg_free512(tmem);
+        tg_free512(tmem_slot);
     }
 }
 
@@ -1028,7 +1052,7 @@ static int retention_tc(const T* q, long long q_stride, const T* k, long long k_
     rc = tgo_launch_pdl(retention_scan4_kernel, dim3(B, H, (DK * dv / 4 + 255) / 256), dim3(256), 0, stream, H, DK * dv,
                         decay, q_start, state_slots, chunk_first, scratch, state);
     if (rc) return rc;
-    return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RF_OUT_THREADS), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
+    return tgo_launch_pdl(k3, dim3(chunks, H, z), dim3(RF_OUT_THREADS + 32), s3, stream, q, q_stride, k, k_stride, v, v_stride, out,
                           H, dv, decay, k_scale, act, rope, rot, chunk_tok0, chunk_ntok, per, (const float*)scratch);
 }
 
