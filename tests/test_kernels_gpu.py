@@ -249,6 +249,42 @@ def test_sgemm_by_parts(M, N, K):
     assert ops().sgemm_error() == 0
 
 
+@pytest.mark.parametrize("T,H,G,dk,dv,rot", [(1, 1, 1, 16, 16, 16), (11, 3, 1, 48, 32, 16), (130, 2, 2, 64, 128, 0),
+                                             (1203, 16, 4, 128, 128, 64)])
+def test_projection_rows_eight_channels_at_a_time(T, H, G, dk, dv, rot):
+    """The form of whole runs of channels against 64 bits (a bfloat16 rounding of float32 arithmetic), tokens that
+    are not stored among them, single tokens and fours."""
+    o, ps = ops(), 16
+    w = H * dk + G * (dk + dv)
+    x = rnd(T, w, seed=dk).to(torch.bfloat16)
+    bias = rnd(w, seed=3)
+    rope = rnd(T, rot, seed=4) if rot else None
+    slots = torch.randperm(T + 40, generator=torch.Generator().manual_seed(1))[:T].to(torch.int32).to(DEV)
+    slots[T // 2] = -1
+    pages = (T + 40 + ps - 1) // ps
+    kc, vc = (torch.zeros((pages, G, ps, n), dtype=torch.bfloat16, device=DEV) for n in (dk, dv))
+    y, at = (x.double() + bias.double()), [H * dk, H * dk + G * dk]
+
+    def turned(z):
+        if rot:
+            c, s = rope[:, None, :rot // 2].double(), rope[:, None, rot // 2:].double()
+            lo, hi = z[..., :rot // 2], z[..., rot // 2:rot]
+            z = torch.cat([lo * c - hi * s, hi * c + lo * s, z[..., rot:]], -1)
+        return z
+    wq, wk, wv = turned(y[:, :at[0]].reshape(T, H, dk)), turned(y[:, at[0]:at[1]].reshape(T, G, dk)), y[:, at[1]:].reshape(T, G, dv)
+    o.qkv_bias_rope_cache(x[:, :at[0]], x[:, at[0]:at[1]], x[:, at[1]:], H, G, dk, dv, bias[:at[0]].contiguous(),
+                          bias[at[0]:at[1]].contiguous(), bias[at[1]:].contiguous(), rope, rot, False, slots, kc, vc, ps)
+    close = lambda a, b: bool(((a.double() - b).abs() <= 2.0 ** -8 * b.abs() + 1e-5).all())    # noqa: E731
+    assert close(x[:, :at[0]].reshape(T, H, dk), wq)
+    stored = slots >= 0
+    s = slots[stored].long()
+    assert close(kc[s // ps, :, s % ps], wk[stored]) and close(vc[s // ps, :, s % ps], wv[stored])
+    rest = torch.ones(pages * ps, dtype=torch.bool, device=DEV)
+    rest[s] = False
+    r = rest.nonzero().flatten()
+    assert not kc[r // ps, :, r % ps].any() and not vc[r // ps, :, r % ps].any()
+
+
 # ----------------------------------------------------------------------- attention
 
 
