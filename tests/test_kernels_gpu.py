@@ -1505,6 +1505,14 @@ def test_gated_group_norm_in_fours(n, groups, act, first, dtype):
     assert torch.allclose(out.double(), want, rtol=2.0 ** -8 if dtype == torch.bfloat16 else 1e-5, atol=1e-6)
 
 
+@pytest.mark.parametrize("n,groups", [(516, 2), (1024, 1), (1028, 3), (1536, 1), (2048, 2)])
+@pytest.mark.parametrize("act,first", [(None, False), ("silu", True)])
+def test_gated_group_norm_a_block_a_group(n, groups, act, first):
+    """Wider groups: four warps share one; cut turns of 512."""
+    for dtype in (torch.float32, torch.bfloat16):
+        test_gated_group_norm_in_fours(n, groups, act, first, dtype)
+
+
 @pytest.mark.parametrize("H,dk,dv,ps", [(16, 576, 512, 16), (5, 576, 512, 8), (128, 264, 256, 64), (24, 200, 64, 32), (3, 448, 320, 128)])
 @pytest.mark.parametrize("window,sink", [(0, False), (130, True), (300, False)])
 def test_attention_latent_tc(H, dk, dv, ps, window, sink):

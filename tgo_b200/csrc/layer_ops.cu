@@ -459,18 +459,20 @@ __device__ __forceinline__ float gate_value(float z, int act) {
 
 // Groups of up to 512 channels that can be read four at a time (16 bytes of o and of the gain, 8 or
 // 16 of the gate): a warp a (token, group), V fours a lane in registers between the sum of squares
-// and the scaling. Gate, gain and result as `gated_group_norm_kernel` below has them. Bound by
+// and the scaling; groups of up to 2048: the four warps of a block (WARPS) a group. Gate, gain and result as `gated_group_norm_kernel` below has them. Bound by
 // memory: every row read and written once. MEASURED (B200): 2048 tokens of 8 x 512 channels, silu,
-// 17 us (51 a channel a lane, four bytes at a time); 4096 tokens of 16 x 256 29 us (39).
-template <typename T, int V>
+// 17 us (51 a channel a lane, four bytes at a time); 4096 tokens of 16 x 256 29 us (39); 2048 of
+// 1536, no gate, 6.3 us (10.5).
+template <typename T, int V, int WARPS>
 __global__ void __launch_bounds__(128)
 gated_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride,
                             const float* __restrict__ gain, T* __restrict__ out, int n, int groups, float eps,
                             int gate_act, int gate_first, long long pairs) {
+    __shared__ float scratch[33];
     pdl_wait();
-    const long long w = (long long)blockIdx.x * 4 + (threadIdx.x >> 5);
+    const long long w = WARPS == 1 ? (long long)blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
     if (w >= pairs) return;
-    const int lane = threadIdx.x & 31;
+    const int lane = threadIdx.x % (32 * WARPS);
     const long long t = w / groups;
     const int g = (int)(w % groups);
     const float* x = o + (size_t)w * n;
@@ -478,7 +480,7 @@ gated_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ g
     float v[V][4], z[V][4];
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int i = 4 * lane + 128 * u;
+        const int i = 4 * lane + 128 * WARPS * u;
         const float4 a = i < n ? *(const float4*)(x + i) : make_float4(0.f, 0.f, 0.f, 0.f);
         v[u][0] = a.x; v[u][1] = a.y; v[u][2] = a.z; v[u][3] = a.w;
         z[u][0] = z[u][1] = z[u][2] = z[u][3] = 0.f;
@@ -502,12 +504,12 @@ gated_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ g
             if (gate_first) v[u][k] *= z[u][k];
             ss += v[u][k] * v[u][k];
         }
-    ss = warp_sum(ss);
+    ss = WARPS == 1 ? warp_sum(ss) : block_sum(ss, scratch);
     const float r = rsqrtf(ss / (float)n + eps);
     T* y = out + (size_t)w * n;
 #pragma unroll
     for (int u = 0; u < V; ++u) {
-        const int i = 4 * lane + 128 * u;
+        const int i = 4 * lane + 128 * WARPS * u;
         if (i >= n) break;
         const float4 gn = gain ? *(const float4*)(gain + g * n + i) : make_float4(1.f, 1.f, 1.f, 1.f);
         const float gk[4] = {gn.x, gn.y, gn.z, gn.w};
@@ -533,14 +535,15 @@ static int gated_group_norm_vec(const float* o, const T* gate, long long gate_st
                                 int n, int groups, float eps, int gate_act, int gate_first, cudaStream_t stream) {
     const long long pairs = (long long)T_ * groups;
     const size_t four = 4 * sizeof(T);
-    if (n > 512 || n % 4 || (uintptr_t)o % 16 || (uintptr_t)gain % 16 || (uintptr_t)out % four || (uintptr_t)gate % four ||
+    if (n > 2048 || n % 4 || (uintptr_t)o % 16 || (uintptr_t)gain % 16 || (uintptr_t)out % four || (uintptr_t)gate % four ||
         (gate && gate_stride % 4) || (pairs + 3) / 4 > 0x7fffffffLL)
         return -1;
-    const dim3 grid((unsigned)((pairs + 3) / 4)), block(128);
-#define GGV_GO(V)                                                                                                      \
-    tgo_launch_pdl(gated_group_norm_vec_kernel<T, V>, grid, block, 0, stream, o, gate, gate_stride, gain, out, n, groups, \
-                   eps, gate_act, gate_first, pairs)
-    return n <= 128 ? GGV_GO(1) : n <= 256 ? GGV_GO(2) : GGV_GO(4);
+    const dim3 block(128);
+#define GGV_GO(V, W)                                                                                                   \
+    tgo_launch_pdl(gated_group_norm_vec_kernel<T, V, W>, dim3((unsigned)(W == 1 ? (pairs + 3) / 4 : pairs)), block, 0, stream, o, \
+                   gate, gate_stride, gain, out, n, groups, eps, gate_act, gate_first, pairs)
+    if (n > 512) return pairs > 0x7fffffffLL ? -1 : n <= 1024 ? GGV_GO(2, 4) : GGV_GO(4, 4);
+    return n <= 128 ? GGV_GO(1, 1) : n <= 256 ? GGV_GO(2, 1) : GGV_GO(4, 1);
 #undef GGV_GO
 }
 
