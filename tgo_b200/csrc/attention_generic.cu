@@ -115,25 +115,36 @@ __global__ void attention_generic_kernel(
 // The same sums in the same order, for steps that bring several tokens a request and see every
 // earlier key (window 0: the keys are then cut into the same 32 for every query). A block takes
 // AGT_Q query rows (the heads of one kv head x consecutive tokens of one request) and brings each 32
-// keys and values into shared memory once for all of them; a warp owns AGT_R rows, a lane one key for
-// the scores and 4 NV channels for the sums. Bound by reads of shared memory (a 16-byte read of a key
-// row feeds 4 AGT_R FMA). The first `n_blocks` blocks of a kv head take the first run of tokens of one
+// keys and values into shared memory once for all of them, float32 ones by asynchronous copies one tile ahead; a
+// warp owns AGT_R rows, a lane one key for the scores and 4 NV channels for the sums. Tiles whose every key all
+// of a warp's rows see go side by side through the softmax and without a test a key. Bound by reads of shared memory
+// (a 16-byte read of a key row feeds 4 AGT_R FMA). The first `n_blocks` blocks of a kv head take the first run of tokens of one
 // request among their AGT_Q / G tokens; where requests meet inside those, the runs that begin there go
 // to the blocks behind them, so that no request waits for another's keys.
 // The caller picks this kernel from four tokens a request on (bits do not depend on it): MEASURED
-// (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this about 140; 64 tokens beside
-// fifteen single ones of 1000 keys, 16/4 heads of 128: 946 and 302 us (1258 when a block walked the requests
-// that meet in it in turn), 8/8 heads of 64: 556 and 178 (2691).
-#define AGT_WARPS 4
+// (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this 75 (139 with each tile waited
+// for, each row's sums by themselves and the weights by shuffles); 64 tokens beside
+// fifteen single ones of 1000 keys, 16/4 heads of 128: 946 and 93 us (302; 1258 when a block walked the requests
+// that meet in it in turn), 8/8 heads of 64: 556 and 101 (178; 2691).
+#define AGT_WARPS 8
 #define AGT_R 4
 #define AGT_Q (AGT_WARPS * AGT_R)
-#define AGT_MAX_SMEM ((int)((32 * (AG_MAX_DH + 4) + 32 * AG_MAX_DH + AGT_Q * AG_MAX_DH) * sizeof(float)))
+#define AGT_MAX_SMEM ((int)((2 * (32 * (AG_MAX_DH + 4) + 32 * AG_MAX_DH) + AGT_Q * (AG_MAX_DH + 32)) * sizeof(float)))
 
 __device__ __forceinline__ float4 ag_load4(const float* p) { return *(const float4*)p; }
 __device__ __forceinline__ float4 ag_load4(const bf16* p) {
     const uint2 v = *(const uint2*)p;
     const float2 a = __bfloat1622float2(*(const __nv_bfloat162*)&v.x), b = __bfloat1622float2(*(const __nv_bfloat162*)&v.y);
     return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// Four numbers of a row of the cache to shared memory as float32; zeros where !ok. float32 rows on their way when it returns.
+__device__ __forceinline__ void agt_copy4(float* dst, const float* src, bool ok) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;"
+                 ::"r"((uint32_t)__cvta_generic_to_shared(dst)), "l"(src), "r"(ok ? 16 : 0) : "memory");
+}
+__device__ __forceinline__ void agt_copy4(float* dst, const bf16* src, bool ok) {
+    *(float4*)dst = ok ? ag_load4(src) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // The request of a token, -1 for one that brings nothing.
@@ -165,7 +176,7 @@ __device__ __forceinline__ int agt_run(int k, int nt, int Tn, const int* __restr
 }
 
 template <typename T, int NV>
-__global__ void __launch_bounds__(32 * AGT_WARPS, NV == 1 ? 4 : 2)
+__global__ void __launch_bounds__(32 * AGT_WARPS, NV == 1 ? 2 : 1)
 attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* __restrict__ out, long long out_stride,
                                int Tn, int n_blocks, int H, int Hkv, int dh, int dv, const T* __restrict__ k_cache,
                                const T* __restrict__ v_cache, int page_size, const int* __restrict__ block_tables,
@@ -175,10 +186,10 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
                                long long gate_stride) {
     extern __shared__ __align__(16) float agt_smem[];
     const int ldk = dh + 4;                              // 16-byte reads of 8 rows hit 8 different places
-    float* ks = agt_smem;                                // [32][ldk]
-    float* vs = ks + 32 * ldk;                           // [32][dv]
-    float* qs = vs + 32 * dv;                            // [AGT_Q][dh]
+    const int buf_floats = 32 * (ldk + dv);              // keys [32][ldk], then values [32][dv]; two of them
+    float* qs = agt_smem + 2 * buf_floats;               // [AGT_Q][dh]
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    float* ws = qs + AGT_Q * dh + warp * AGT_R * 32;     // the warp's weights [AGT_R][32]
     const int G = H / Hkv, kvh = blockIdx.y;
     const int nt = AGT_Q / G;                            // tokens of a block (G <= AGT_Q)
     for (int run = blockIdx.x;; run += gridDim.x - n_blocks) {       // a first run, or the others a block has to take
@@ -206,23 +217,30 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
             for (int i = 0; i < NV; ++i) acc[r][i] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
         const int* bt = block_tables + (size_t)(b < 0 ? 0 : b) * max_blocks;
-        for (int k0 = 0; k0 <= p_last; k0 += 32) {
-            __syncthreads();                             // the last keys have been read
-            for (int i = threadIdx.x; i < 32 * (dh / 4); i += blockDim.x) {
-                const int r = i / (dh / 4), c = (i % (dh / 4)) * 4, j = k0 + r;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (j <= p_last)
-                    v = ag_load4(k_cache + (((size_t)bt[j / page_size] * Hkv + kvh) * page_size + (j % page_size)) * dh + c);
-                *(float4*)(ks + r * ldk + c) = v;
+        int pos_min = pos[0];
+#pragma unroll
+        for (int r = 1; r < AGT_R; ++r) pos_min = min(pos_min, pos[r]);
+        // AGT_WARPS threads a key: its place is looked up once
+        auto load = [&](int k0, int buf) {
+            if (k0 <= p_last) {
+                const int r = threadIdx.x / AGT_WARPS, j = k0 + r, c0 = (threadIdx.x % AGT_WARPS) * 4;
+                const bool ok = j <= p_last;
+                const size_t row = ok ? ((size_t)bt[j / page_size] * Hkv + kvh) * page_size + j % page_size : 0;
+                const T *kr = k_cache + row * dh, *vr = v_cache + row * v_row;
+                float *kd = agt_smem + buf * buf_floats + r * ldk, *vd = agt_smem + buf * buf_floats + 32 * ldk + r * dv;
+                for (int c = c0; c < dh; c += 4 * AGT_WARPS) agt_copy4(kd + c, kr + c, ok);
+                for (int c = c0; c < dv; c += 4 * AGT_WARPS) agt_copy4(vd + c, vr + c, ok);
             }
-            for (int i = threadIdx.x; i < 32 * (dv / 4); i += blockDim.x) {
-                const int r = i / (dv / 4), c = (i % (dv / 4)) * 4, j = k0 + r;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (j <= p_last)
-                    v = ag_load4(v_cache + (((size_t)bt[j / page_size] * Hkv + kvh) * page_size + (j % page_size)) * v_row + c);
-                *(float4*)(vs + r * dv + c) = v;
-            }
-            __syncthreads();
+            asm volatile("cp.async.commit_group;" ::: "memory");
+        };
+        __syncthreads();                                 // the last run's keys have been read
+        load(0, 0);
+        for (int k0 = 0, buf = 0; k0 <= p_last; k0 += 32, buf ^= 1) {
+            asm volatile("cp.async.wait_group 0;" ::: "memory");
+            __syncthreads();                             // this tile is there, the last one has been read
+            load(k0 + 32, buf ^ 1);
+            const float* ks = agt_smem + buf * buf_floats;
+            const float* vs = ks + 32 * ldk;
             if (warp * AGT_R >= nq) continue;            // none of the run's rows are this warp's
             float a[AGT_R], w[AGT_R];
 #pragma unroll
@@ -238,6 +256,65 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
                     a[r] = fmaf(q4.z, k4.z, a[r]);
                     a[r] = fmaf(q4.w, k4.w, a[r]);
                 }
+            }
+            if (k0 + 31 <= pos_min) {                    // every row sees every key
+                float m_new[AGT_R], sum[AGT_R];
+#pragma unroll
+                for (int r = 0; r < AGT_R; ++r) {
+                    const int p = pos[r], j = k0 + lane;
+                    float s = a[r] * scale;
+                    if (softcap > 0.f) s = softcap * tanhf(s / softcap);
+                    if (dist_bias) s += dist_bias[(size_t)((p - j) < n_dist ? (p - j) : n_dist - 1) * H + kvh * G + (warp * AGT_R + r) % G];
+                    a[r] = m_new[r] = s;
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < AGT_R; ++r) m_new[r] = fmaxf(m_new[r], __shfl_xor_sync(0xffffffffu, m_new[r], o));
+#pragma unroll
+                for (int r = 0; r < AGT_R; ++r) {
+                    m_new[r] = fmaxf(m[r], m_new[r]);
+                    sum[r] = w[r] = expf(a[r] - m_new[r]);
+                    ws[r * 32 + lane] = w[r];
+                }
+#pragma unroll
+                for (int o = 16; o > 0; o >>= 1)
+#pragma unroll
+                    for (int r = 0; r < AGT_R; ++r) sum[r] += __shfl_xor_sync(0xffffffffu, sum[r], o);
+#pragma unroll
+                for (int r = 0; r < AGT_R; ++r) {
+                    const float corr = expf(m[r] - m_new[r]);
+                    l[r] = l[r] * corr + sum[r];
+#pragma unroll
+                    for (int i = 0; i < NV; ++i) {
+                        acc[r][i].x *= corr; acc[r][i].y *= corr; acc[r][i].z *= corr; acc[r][i].w *= corr;
+                    }
+                    m[r] = m_new[r];
+                }
+                __syncwarp();
+#pragma unroll 2
+                for (int j0 = 0; j0 < 32; j0 += 4) {
+                    float4 w4[AGT_R];
+#pragma unroll
+                    for (int r = 0; r < AGT_R; ++r) w4[r] = *(const float4*)(ws + r * 32 + j0);
+#pragma unroll
+                    for (int jj = 0; jj < 4; ++jj)
+#pragma unroll
+                        for (int i = 0; i < NV; ++i) {
+                            const float4 v4 = (lane + 32 * i) * 4 < dv ? *(const float4*)(vs + (j0 + jj) * dv + (lane + 32 * i) * 4)
+                                                                       : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                            for (int r = 0; r < AGT_R; ++r) {
+                                const float wj = jj == 0 ? w4[r].x : jj == 1 ? w4[r].y : jj == 2 ? w4[r].z : w4[r].w;
+                                acc[r][i].x = fmaf(wj, v4.x, acc[r][i].x);
+                                acc[r][i].y = fmaf(wj, v4.y, acc[r][i].y);
+                                acc[r][i].z = fmaf(wj, v4.z, acc[r][i].z);
+                                acc[r][i].w = fmaf(wj, v4.w, acc[r][i].w);
+                            }
+                        }
+                }
+                __syncwarp();                            // the weights have been read
+                continue;
             }
             int most = 0;
 #pragma unroll
@@ -311,6 +388,7 @@ attention_generic_tiles_kernel(const T* __restrict__ q, long long q_stride, T* _
             }
         }
         if (run < n_blocks) return;
+        asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();                                 // the run's queries, keys and values have been read
     }
 }
@@ -337,7 +415,7 @@ TGO_API int tgo_attention_generic_tiles(const void* q, long long q_stride, void*
     // a block for the first run of every nt tokens, and as many as there are requests for the others
     const int nt = AGT_Q / (H / Hkv), n_blocks = (T + nt - 1) / nt;
     const dim3 grid(n_blocks + (n_seqs < T ? n_seqs : T), Hkv);
-    const size_t smem = (size_t)(32 * (dh + 4) + 32 * dv + AGT_Q * dh) * sizeof(float);
+    const size_t smem = (size_t)(2 * 32 * (dh + 4 + dv) + AGT_Q * (dh + 32)) * sizeof(float);
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess) return (int)e;
