@@ -1341,6 +1341,28 @@ def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
     return y, state
 
 
+@pytest.mark.parametrize("H,G,N,P,T", [(6, 2, 64, 64, 200), (40, 2, 128, 64, 65), (40, 2, 128, 64, 1500), (5, 1, 128, 128, 190),
+                                       (12, 1, 64, 64, 64), (17, 1, 64, 128, 257)])
+def test_selective_scan_by_chunks_heads_a_block(H, G, N, P, T, monkeypatch):
+    """Groups whose heads fill blocks and pairs of 128 channels or do not, whole and cut chunks, against the
+    recurrence in 64 bits: sums of N + 64 float32 terms behind at most T / 64 chunks."""
+    o = ops()
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + T), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log = torch.linspace(-2.0, 1.0, H, device=DEV)
+    y, state = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P)
+    x, B, C = (z.double() for z in xbc.split([H * P, G * N, G * N], 1))
+    B, C = (z.view(T, G, N).repeat_interleave(H // G, 1) for z in (B, C))
+    dt, S = torch.nn.functional.softplus(dt_raw.double()), torch.zeros(H, N, P, dtype=torch.float64, device=DEV)
+    want = torch.empty(T, H, P, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S = torch.exp(-torch.exp(a_log.double()) * dt[t])[:, None, None] * S + \
+            (dt[t][:, None] * B[t])[:, :, None] * x[t].view(H, 1, P)
+        want[t] = torch.einsum("hn,hnp->hp", C[t], S)
+    assert (y.view(T, H, P).double() - want).norm() <= 1e-6 * want.norm()
+    assert (state.view(H, N, P).double() - S).norm() <= 1e-6 * S.norm()
+    assert o.ssd_error() == 0
+
+
 @pytest.mark.parametrize("H,G,N,P", [(64, 8, 128, 64), (3, 1, 64, 64), (2, 1, 128, 128)])
 def test_selective_scan_by_chunks_looks_forward_only(H, G, N, P, monkeypatch):
     """A number that is not finite at a token leaves every output before it as it is without it; one in x

@@ -606,22 +606,14 @@ __device__ __forceinline__ bool rf_put_v(uint32_t tile, const Raw8<T> (&raw)[rf_
         } else {
             float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (ok) taken8(raw[j], act, f);
-            uint4 part[3];
-            odd = s3_split8_finite(f, part) || odd;
-#pragma unroll
-            for (int q = 0; q < 3; ++q) s3_store16(dst + q * 2 * RF_TILE, part[q]);
+            odd = s3_put8(f, dst, 2 * RF_TILE) || odd;
         }
     }
     return odd;
 }
 // The parts of eight numbers to their place in three tiles `step` bytes apart.
 __device__ __forceinline__ bool rf_put8(uint32_t tile, uint32_t step, int row, int piece, const float (&f)[8]) {
-    uint4 part[3];
-    const bool odd = s3_split8_finite(f, part);
-    const uint32_t dst = tile + s3_place(row, piece);
-#pragma unroll
-    for (int q = 0; q < 3; ++q) s3_store16(dst + q * step, part[q]);
-    return odd;
+    return s3_put8(f, tile + s3_place(row, piece), step);
 }
 // The value of column c of a token, as the plain sums take it.
 template <typename T>

@@ -45,25 +45,6 @@ __device__ __noinline__ bool s3_mend8(const float* v, uint32_t* hi, uint32_t* mi
     }
     return odd;
 }
-__device__ __forceinline__ bool s3_split8_finite(const float (&v)[8], uint4 (&part)[3]) {
-    s3_split8(v, part[0], part[1], part[2]);
-    // the rest of what is not finite, or rounds to infinity, is not finite: 0 times it is not 0
-    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
-    __nv_bfloat162 seen = zero;
-    seen = __hfma2(*(const __nv_bfloat162*)&part[1].x, zero, seen);
-    seen = __hfma2(*(const __nv_bfloat162*)&part[1].y, zero, seen);
-    seen = __hfma2(*(const __nv_bfloat162*)&part[1].z, zero, seen);
-    seen = __hfma2(*(const __nv_bfloat162*)&part[1].w, zero, seen);
-    if (!(*(const uint32_t*)&seen & 0x7fff7fffu)) return false;
-    float f[8];
-    uint32_t w[3][4];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) f[i] = v[i];
-    const bool odd = s3_mend8(f, w[0], w[1], w[2]);
-#pragma unroll
-    for (int p = 0; p < 3; ++p) part[p] = make_uint4(w[p][0], w[p][1], w[p][2], w[p][3]);
-    return odd;
-}
 // ... of numbers that are bfloat16 numbers already.
 __device__ __forceinline__ bool s3_finite8(uint4& v) {
     if (!s3_odd8(v)) return false;
@@ -84,6 +65,55 @@ __device__ __forceinline__ void s3_fence() { asm volatile("fence.proxy.async.sha
 
 // A 16-byte piece's place in a tile of 128-byte rows with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t s3_place(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
+// R eights to their places dst[r], dst[r] + step, dst[r] + 2 step with every part finite; true: a number was not. One test
+// for all of them, so that their chains of conversions run side by side.
+template <int R> __device__ __forceinline__ bool s3_put(const float (&v)[R][8], const uint32_t (&dst)[R], uint32_t step) {
+    uint4 part[R][3];
+    // the rest of what is not finite, or rounds to infinity, is not finite: 0 times it is not 0
+    const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
+    uint32_t any = 0;
+#pragma unroll
+    for (int r = 0; r < R; ++r) {
+        s3_split8(v[r], part[r][0], part[r][1], part[r][2]);
+        __nv_bfloat162 a = __hmul2(*(const __nv_bfloat162*)&part[r][1].x, zero), b = __hmul2(*(const __nv_bfloat162*)&part[r][1].y, zero);
+        a = __hfma2(*(const __nv_bfloat162*)&part[r][1].z, zero, a);
+        b = __hfma2(*(const __nv_bfloat162*)&part[r][1].w, zero, b);
+        any |= (*(const uint32_t*)&a | *(const uint32_t*)&b) & 0x7fff7fffu;
+    }
+    bool odd = false;
+    if (any) {
+#pragma unroll 1
+        for (int r = 0; r < R; ++r) {
+            float f[8];
+            uint32_t w[3][4];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+                f[i] = v[0][i];
+#pragma unroll
+                for (int q = 1; q < R; ++q) f[i] = r == q ? v[q][i] : f[i];
+            }
+            uint32_t to = dst[0];
+#pragma unroll
+            for (int q = 1; q < R; ++q) to = r == q ? dst[q] : to;
+            odd = s3_mend8(f, w[0], w[1], w[2]) || odd;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) s3_store16(to + q * step, make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]));
+        }
+        return odd;
+    }
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+#pragma unroll
+        for (int q = 0; q < 3; ++q) s3_store16(dst[r] + q * step, part[r][q]);
+    return false;
+}
+__device__ __forceinline__ bool s3_put8(const float (&v)[8], uint32_t dst, uint32_t step) {
+    float f[1][8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) f[0][i] = v[i];
+    const uint32_t to[1] = {dst};
+    return s3_put<1>(f, to, step);
+}
 // D += A B^T over 16 KSTEPS of k and every kept pair of parts, the smallest first. Part p of A starts a_part * p
 // after da and a k-step a_k after the one before (descriptor units of 16 bytes); AP, BP: parts there are (1: the
 // numbers are bfloat16 numbers themselves). One thread issues.

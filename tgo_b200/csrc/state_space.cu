@@ -19,7 +19,7 @@
 // A request's state row (float32, `state_stride` floats apart) holds the scan's state
 // [H][N][P] (or [channels][N]) at `ssm_offset` and the convolution's last taps - 1 inputs [taps - 1][C] (oldest
 // first) at `conv_offset`.
-#include "fma_tile.cuh"
+#include "split3.cuh"
 
 // ------------------------------------------------------------------------- convolution
 // y[t][c] = silu(bias[c] + sum_j w[c][j] x[t - (taps - 1 - j)][c]); inputs before the step's
@@ -413,16 +413,15 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
 //
 // Four launches: steps (dt and L of every token; L in 64 bits, so that the differences of large
 // sums lose nothing), summaries (the sum of S's line), a scan over the chunks, which leaves the
-// state before each chunk in its summary's place, and outputs. Float32 products in register tiles
-// (fma_tile.cuh), bound by the FMA pipes. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128): 711 us
-// by the walk above, 224 so (summaries 54, scan over the chunks 32, outputs 134, 148 with a head a block); error against 64 bits
-// 1.2e-7 (1.9e-7 by the walk).
+// state before each chunk in its summary's place, and outputs. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128):
+// 711 us by the walk above, 224 with float32 products in register tiles of packed FMA (summaries 52, scan over the
+// chunks 32, outputs 132), 148 with their parts on the tensor cores (30, 31, 82); errors against 64 bits, means of 15
+// draws: outputs 0.9e-7 (1.1e-7 by FMA), state 8.4e-8 (8.7e-8).
 // The workspace is a state's size a chunk and head; a call whose workspace does not hold all heads takes
 // them in groups, one after the other over the same memory (heads do not meet; the sums are the same).
 // The walk stays for the float32 engine, whose sums do not depend on how a prompt is cut, for
 // steps of few tokens a request, and for other sizes.
 #define SD_CHUNK 64
-#define SD_LD (SD_CHUNK + 4)
 
 // The request and tokens of chunk `ci` (chunks are numbered request after request): false past the
 // last. One warp.
@@ -496,47 +495,214 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
     *(double2*)(cum + at) = make_double2((lane ? before : 0.0) + l[0], incl);
 }
 
+// ---- the products, in true float32 on the tensor cores (split3.cuh): three bfloat16 parts a number
+// A block takes a chunk's rows of several heads of one group, whose B and C are the same, 128 of their channels ("a
+// pair": two heads of 64, or one of 128) at a time: channels are the accumulators' lanes, tokens or states their
+// columns, so that every operand is laid down as it lies in memory and a warp's results leave as whole lines.
+// Sixteen warps lay parts down and write results, one issues. In the outputs A = exp(L_i - L_j) dt_j (C . B) has D on
+// its diagonal, so that x goes in as it is and nothing is read for the results. Bound by the chains of conversions (about 2500
+// cycles a stage of 64 x 128 numbers for eight warps) and not by the products, 50 cycles each. Zeros of A times a value that is not finite are not
+// zero: such a number is laid down as 0, which leaves what does not depend on it as it is, bit for bit, and a
+// block that met one makes plain sums too and writes those that are not finite.
+#define SD_THREADS 512
+#define SD_HALF 256                   // of the outputs: one half lays the states and values down, the other A
+#define SD_HEADS 16                   // heads a block takes at most
+#define SD_TILE 8192                  // 64 rows of 64 bfloat16 numbers
+
+__device__ int ssd_error_flag = 0;
+
+__device__ __forceinline__ bool sd_not_finite(float x) { return !(fabsf(x) < __int_as_float(0x7f800000)); }
+__device__ __forceinline__ void sd_eight(float (&f)[8], float4 a, float4 b, float w, bool ok) {
+    f[0] = ok ? a.x * w : 0.f; f[1] = ok ? a.y * w : 0.f; f[2] = ok ? a.z * w : 0.f; f[3] = ok ? a.w * w : 0.f;
+    f[4] = ok ? b.x * w : 0.f; f[5] = ok ? b.y * w : 0.f; f[6] = ok ? b.z * w : 0.f; f[7] = ok ? b.w * w : 0.f;
+}
+// A warp's share of an operand is laid down.
+__device__ __forceinline__ void sd_full(uint64_t* bar) {
+    s3_fence();
+    tg_before();
+    __syncwarp();
+    if ((threadIdx.x & 31) == 0) tg_arrive(bar);
+}
+// For a whole warp: the phase of a barrier is over.
+__device__ __forceinline__ bool sd_wait(uint64_t* bar, uint32_t phase, int code) {
+    const bool ok = __all_sync(0xffffffffu, tg_wait(bar, phase, &ssd_error_flag, code));
+    tg_after();
+    return ok;
+}
+// Barrier of THREADS threads that leave together: whether no wait of theirs has run out.
+template <int THREADS> __device__ __forceinline__ bool sd_sync(bool ok) {
+    uint32_t r;
+    asm volatile("{\n\t.reg .pred p, q;\n\tsetp.ne.u32 p, %1, 0;\n\t"
+                 "bar.red.and.pred q, 1, %2, p;\n\tselp.u32 %0, 1, 0, q;\n\t}"
+                 : "=r"(r) : "r"((uint32_t)ok), "n"(THREADS) : "memory");
+    return r != 0;
+}
+// A chunk's B or C, 64 rows of N states: asked for, then laid down (rows of tokens, N / 64 tiles a part).
+template <int N> struct SdRows {
+    static constexpr int RUNS = SD_CHUNK * (N / 8) / SD_THREADS;
+    float4 v[RUNS][2];
+    __device__ __forceinline__ void load(const float* __restrict__ rows, int C, int n) {
+#pragma unroll
+        for (int j = 0; j < RUNS; ++j) {
+            const int i = threadIdx.x + j * SD_THREADS, r = i / (N / 8);
+            const float4* src = (const float4*)(rows + (size_t)(r < n ? r : 0) * C + (i % (N / 8)) * 8);
+            v[j][0] = src[0];
+            v[j][1] = src[1];
+        }
+    }
+    __device__ __forceinline__ bool put(uint32_t tile, int n) const {
+        float f[RUNS][8];
+        uint32_t dst[RUNS];
+#pragma unroll
+        for (int j = 0; j < RUNS; ++j) {
+            const int i = threadIdx.x + j * SD_THREADS, r = i / (N / 8), piece = i % (N / 8);
+            sd_eight(f[j], v[j][0], v[j][1], 1.f, r < n);
+            dst[j] = tile + (piece >> 3) * SD_TILE + s3_place(r, piece & 7);
+        }
+        return s3_put<RUNS>(f, dst, N / 64 * SD_TILE);
+    }
+};
+// x of a pair: 64 rows of 128 channels of neighbouring heads (channels past `width` are zeros), a row and head times
+// its weight; two tiles of 64 channels a part.
+template <int THREADS> struct SdPair {
+    static constexpr int RUNS = SD_CHUNK * 16 / THREADS;
+    float4 v[RUNS][2];
+    __device__ __forceinline__ void load(const float* __restrict__ rows, int C, int n, int width) {
+#pragma unroll
+        for (int j = 0; j < RUNS; ++j) {
+            const int i = threadIdx.x + j * THREADS, r = i / 16, c = (i % 16) * 8;
+            const float4* src = (const float4*)(rows + (size_t)(r < n ? r : 0) * C + (c < width ? c : 0));
+            v[j][0] = src[0];
+            v[j][1] = src[1];
+        }
+    }
+    // weights [128 / P][SD_CHUNK]; null: none
+    template <int P> __device__ __forceinline__ bool put(uint32_t tile, int n, int width, const float (*weights)[SD_CHUNK]) const {
+        bool odd = false;
+#pragma unroll
+        for (int j0 = 0; j0 < RUNS; j0 += 2) {
+            float f[2][8];
+            uint32_t dst[2];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                const int i = threadIdx.x + (j0 + j) * THREADS, r = i / 16, piece = i % 16;
+                const bool in = r < n && piece * 8 < width;
+                sd_eight(f[j], v[j0 + j][0], v[j0 + j][1], in && weights ? weights[piece * 8 / P][r] : 1.f, in);
+                dst[j] = tile + (piece >> 3) * SD_TILE + s3_place(r, piece & 7);
+            }
+            odd = s3_put<2>(f, dst, 2 * SD_TILE) || odd;
+        }
+        return odd;
+    }
+};
+
+// Shared memory: B's parts (N / 64 tiles a part), two buffers of a pair's weighted values (two tiles a part).
 template <int N, int P>
-__global__ void __launch_bounds__(N * P / 64, 512 / (N * P / 64))
-ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int h0, const int4* __restrict__ chunks,
+__global__ void __launch_bounds__(SD_THREADS + 32, 1)
+ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int first, int hb, const int4* __restrict__ chunks,
                      const float* __restrict__ dts, const double* __restrict__ cum, float* __restrict__ U) {
-    constexpr int THREADS = N * P / 64;
-    extern __shared__ __align__(16) float smem[];
-    float* Bs = smem;                                    // [SD_CHUNK][N + 4]
-    float* Vs = Bs + SD_CHUNK * (N + 4);                 // [SD_CHUNK][P + 4], rows times dt exp(L_n - L_j)
-    __shared__ float ws[SD_CHUNK];
+    constexpr int HP = 128 / P, NB = N / 64, STAGE = 6 * SD_TILE;
+    extern __shared__ unsigned char sd_raw[];
+    unsigned char* sB = (unsigned char*)(((uintptr_t)sd_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sV = sB + 3 * NB * SD_TILE;
+    __shared__ float ws[2][HP][SD_CHUNK];
+    __shared__ __align__(8) uint64_t bars[5];
+    __shared__ uint32_t tmem_slot;
+    uint64_t *v_full = bars, *v_done = bars + 2, *settled = bars + 4;
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
-    const int h = h0 + blockIdx.y, n = ch.y;             // the workspace holds the group's gridDim.y heads
+    const int n = ch.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (n == 0) return;
+    const int nh = gridDim.y * hb, l0 = blockIdx.y * hb, h0 = first + l0, pairs = (hb + HP - 1) / HP;
     const float* rows = xbc + (size_t)ch.x * C;
-    const size_t at = ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * SD_CHUNK;
-    for (int i = threadIdx.x; i < n * (N / 4); i += THREADS) {
-        const int r = i / (N / 4), c = (i % (N / 4)) * 4;
-        ft_copy16(Bs + r * (N + 4) + c, rows + (size_t)r * C + H * P + (h / (H / G)) * N + c, true);
+    const size_t at = (size_t)blockIdx.x * nh + l0;      // the workspace holds the nh heads from `first` on
+    if (warp == 0) tg_alloc<4 * N>(&tmem_slot);
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < 2; ++i) { tg_init(&v_full[i], SD_THREADS / 32); tg_init(&v_done[i], 1); }
+        tg_init(settled, 1);
+        tg_init_done();
     }
-    ft_commit();
-    for (int i = threadIdx.x; i < n; i += THREADS) ws[i] = dts[at + i] * expf((float)(cum[at + n - 1] - cum[at + i]));
+    tg_before();
     __syncthreads();
-    for (int i = threadIdx.x; i < n * (P / 4); i += THREADS) {
-        const int r = i / (P / 4), c = (i % (P / 4)) * 4;
-        float4 v = *(const float4*)(rows + (size_t)r * C + h * P + c);
-        const float w = ws[r];
-        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-        *(float4*)(Vs + r * (P + 4) + c) = v;
+    tg_after();
+    const uint32_t tmem = tmem_slot;
+    bool odd = false, ok = true;
+    if (warp == SD_THREADS / 32) {
+        const bool leader = tg_elect();
+        for (int q = 0; q < pairs; ++q) {
+            ok = sd_wait(&v_full[q & 1], (q >> 1) & 1, 1);
+            if (!ok) break;
+            if (leader) {
+#pragma unroll
+                for (int x = 0; x < 2; ++x)              // either half of the tokens for itself: the sums err less
+                    s3_products<3, 3, SD_CHUNK / 32>(tmem + (uint32_t)(N * (2 * (q & 1) + x)), tg_desc_mn(sV + (q & 1) * STAGE, SD_TILE) + 256u * x,
+                                                     2 * SD_TILE >> 4, 128, tg_desc_mn(sB, SD_TILE) + 256u * x, NB * SD_TILE >> 4, 128,
+                                                     tg_idesc(N, true, true), false);
+                tg_commit(&v_done[q & 1]);
+            }
+            __syncwarp();
+        }
+        if (!ok && leader) tg_settle_products(settled, &ssd_error_flag, 1);
+    } else {
+        SdRows<N> b;
+        b.load(rows + H * P + (h0 / (H / G)) * N, C, n);
+        SdPair<SD_THREADS> x;
+        x.load(rows + h0 * P, C, n, min(hb, HP) * P);
+        odd = b.put(tg_smem(sB), n);
+        for (int q = 0; q <= pairs; ++q) {
+            if (q < pairs) {
+                const int heads = min(HP, hb - q * HP);
+                // the buffers' products of the pair before the last have been waited for below
+                if (threadIdx.x < heads * SD_CHUNK) {
+                    const int e = threadIdx.x / SD_CHUNK, j = threadIdx.x % SD_CHUNK;
+                    const size_t o = (at + q * HP + e) * SD_CHUNK;
+                    ws[q & 1][e][j] = j < n ? dts[o + j] * expf((float)(cum[o + n - 1] - cum[o + j])) : 0.f;
+                }
+                ok = sd_sync<SD_THREADS>(ok);
+                if (!ok) break;
+                odd = x.put<P>(tg_smem(sV) + (q & 1) * STAGE, n, heads * P, ws[q & 1]) || odd;
+                sd_full(&v_full[q & 1]);
+                if (q + 1 < pairs) x.load(rows + (h0 + (q + 1) * HP) * P, C, n, min(HP, hb - (q + 1) * HP) * P);
+            }
+            if (q > 0) {                                 // the pair before this one
+                const int d = q - 1, row = (warp & 3) * 32 + lane, l = d * HP + row / P;
+                ok = sd_wait(&v_done[d & 1], (d >> 1) & 1, 2);
+                constexpr int COLS = N / 4;              // states a warp
+                const int n0 = (warp >> 2) * COLS;
+                const uint32_t t = tmem + ((uint32_t)((warp & 3) * 32) << 16) + (uint32_t)(2 * N * (d & 1) + n0);
+                float* dst = U + ((at + l) * N + n0) * P + row % P;
+#pragma unroll
+                for (int c = 0; c < COLS; c += 16, dst += 16 * P) {
+                    uint32_t r0[16], r1[16];
+                    tg_ld16(t + c, r0);
+                    tg_ld16(t + (uint32_t)(N + c), r1);
+                    tg_wait_ld();
+                    if (ok && l < hb)
+#pragma unroll
+                        for (int i = 0; i < 16; ++i) dst[i * P] = __uint_as_float(r0[i]) + __uint_as_float(r1[i]);
+                }
+                tg_before();                             // before the next products into this buffer
+            }
+        }
     }
-    ft_wait<0>();
+    ok = __syncthreads_and(ok);
+    if (__syncthreads_or(odd) && ok) {                   // plain sums
+        const float* br = rows + H * P + (h0 / (H / G)) * N;
+        for (int i = threadIdx.x; i < hb * N * P; i += SD_THREADS + 32) {
+            const int l = i / (N * P), m = i / P % N, c = i % P;
+            const size_t o = (at + l) * SD_CHUNK;
+            float sum = 0.f;
+            for (int j = 0; j < n; ++j)
+                sum = fmaf(br[(size_t)j * C + m], rows[(size_t)j * C + (h0 + l) * P + c] * (dts[o + j] * expf((float)(cum[o + n - 1] - cum[o + j]))), sum);
+            if (sd_not_finite(sum)) U[((at + l) * N + m) * P + c] = sum;
+        }
+    }
+    tg_before();
     __syncthreads();
-    FmaTile<2, 2, N / 8, P / 8> t;
-    t.ty = threadIdx.x / (P / 8);
-    t.tx = threadIdx.x % (P / 8);
-    t.clear();
-    t.add(Bs, N + 4, Vs, P + 4, n);
-    float* Uo = U + ((size_t)blockIdx.x * gridDim.y + blockIdx.y) * N * P;
-#pragma unroll
-    for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) *(float4*)(Uo + (size_t)t.row(i) * P + t.col(c)) = t.get(i, c);
+    if (warp == 0) {
+        tg_after();
+        tg_free<4 * N>(tmem_slot);
+    }
 }
 
 // grid (requests, heads, ceil(N P / 1024)): a thread four neighbouring elements of the state
@@ -587,133 +753,271 @@ ssd_scan_kernel(int H, int NP, const int* __restrict__ q_start, const int* __res
     *sp = s;
 }
 
-// A block: a chunk's rows of HEADS neighbouring heads of one group, 2 P threads each. B, C and the states
-// come 64 of the N states at a time; C . B, which the heads share, and S^T C grow side by side in
-// registers, then A times v is added.
-template <int N, int P, int HEADS>
-__global__ void __launch_bounds__(HEADS * 2 * P, 512 / (HEADS * 2 * P))
-ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first, const float* __restrict__ D,
+// Shared memory: C's parts; B's, over which a pair's A come to lie (24 KB a head); two buffers that the states (64 of
+// them x 128 channels a stage) and the values of a pair go through in turn.
+template <int N, int P> __host__ __device__ constexpr int sd_a_bytes() {
+    return 3 * (N / 64 > 128 / P ? N / 64 : 128 / P) * SD_TILE;
+}
+template <int N, int P> __host__ __device__ constexpr int sd_out_bytes() { return 3 * (N / 64) * SD_TILE + sd_a_bytes<N, P>() + 2 * 6 * SD_TILE; }
+
+template <int N, int P>
+__global__ void __launch_bounds__(SD_THREADS + 32, 1)
+ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first, int hb, const float* __restrict__ D,
                    const int4* __restrict__ chunks, const float* __restrict__ dts, const double* __restrict__ cum,
                    const float* __restrict__ U, float* __restrict__ y) {
-    constexpr int EACH = 2 * P, THREADS = HEADS * EACH, TX = P / 8;        // 16 x TX threads a head, 4 x 8 outputs each
-    constexpr int TG = HEADS * TX, GN = SD_CHUNK / (4 * TG);               // columns of C . B a thread owns, in fours
-    extern __shared__ __align__(16) float smem[];
-    float* Ct = smem;                                    // [64][SD_LD] state-major; later a head's A, token-j-major
-    float* Bt = Ct + 64 * SD_LD;                         // [64][SD_LD]; later the second head's A
-    float* Ss = Bt + 64 * SD_LD;                         // [HEADS][64][P + 4]; later v [HEADS][SD_CHUNK][P + 4]
-    __shared__ double ls[HEADS][SD_CHUNK];
-    __shared__ float ds[HEADS][SD_CHUNK];
+    constexpr int HP = 128 / P, HALVES = N / 64, STAGES = HALVES + 1, STAGE = 6 * SD_TILE;
+    extern __shared__ unsigned char sd_raw[];
+    unsigned char* sC = (unsigned char*)(((uintptr_t)sd_raw + 1023) & ~(uintptr_t)1023);
+    unsigned char* sB = sC + 3 * HALVES * SD_TILE;
+    unsigned char* sA = sB;
+    unsigned char* sR = sB + sd_a_bytes<N, P>();         // [2]
+    __shared__ double ls[SD_HEADS][SD_CHUNK];
+    __shared__ float ds[SD_HEADS][SD_CHUNK], el[SD_HEADS][SD_CHUNK];
+    __shared__ __align__(8) uint64_t bars[12];
+    __shared__ uint32_t tmem_slot;
+    uint64_t *cb_full = bars, *s_done = bars + 1, *r_full = bars + 2 /* [2] */, *r_done = bars + 4 /* [2] */, *y_done = bars + 6;
+    uint64_t *a_full = bars + 7, *y_free = bars + 8 /* [2] */, *settled = bars + 10, *a_done = bars + 11;
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
-    const int h0 = first + blockIdx.y * HEADS, hh = threadIdx.x / EACH, h = h0 + hh, t = threadIdx.x % EACH, n = ch.y;
+    const int n = ch.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (n == 0) return;
+    const int nh = gridDim.y * hb, l0 = blockIdx.y * hb, h0 = first + l0, pairs = (hb + HP - 1) / HP;
     const float* rows = xbc + (size_t)ch.x * C;
     const float* brow = rows + H * P + (h0 / (H / G)) * N;
     const float* crow = brow + (size_t)G * N;
-    const size_t place = (size_t)(blockIdx.x * gridDim.y + blockIdx.y) * HEADS + hh, at = place * SD_CHUNK;
-    const float* Sc = U + place * N * P;
-    float* Sh = Ss + hh * 64 * (P + 4);
-    for (int i = t; i < SD_CHUNK; i += EACH) {
-        ls[hh][i] = cum[at + i];
-        ds[hh][i] = dts[at + i];
+    const size_t at = (size_t)blockIdx.x * nh + l0;
+    if (warp == 0) tg_alloc512(&tmem_slot);
+    if (threadIdx.x == 0) {
+        tg_init(cb_full, SD_THREADS / 32);
+        tg_init(s_done, 1);
+        for (int i = 0; i < 2; ++i) { tg_init(&r_full[i], SD_HALF / 32); tg_init(&r_done[i], 1); tg_init(&y_free[i], SD_HALF / 32); }
+        tg_init(a_full, SD_HALF / 32);
+        tg_init(y_done, 1);
+        tg_init(a_done, 1);
+        tg_init(settled, 1);
+        tg_init_done();
     }
-    FmaTile<1, GN, 16, TG> g;
-    FmaTile<1, 2, 16, TX> o;
-    g.ty = threadIdx.x / TG;
-    g.tx = threadIdx.x % TG;
-    o.ty = t / TX;
-    o.tx = t % TX;
-    g.clear();
-    o.clear();
-    const bool busy = 4 * (o.ty & ~(32 / TX - 1)) < n, g_busy = 4 * (g.ty & ~(32 / TG - 1)) < n;   // a warp's first row exists
-    for (int n0 = 0; n0 < N; n0 += 64) {
-        if (n0) __syncthreads();
-        for (int i = t; i < 64 * (P / 4); i += EACH) {
-            const int r = i / (P / 4), c = (i % (P / 4)) * 4;
-            ft_copy16(Sh + r * (P + 4) + c, Sc + (size_t)(n0 + r) * P + c, true);
-        }
-        ft_commit();
-        // a warp takes four rows x eight runs of four states: 128 bytes a row, no bank met twice (ft_swizzle)
-        for (int i = threadIdx.x; i < 2 * SD_CHUNK * 16; i += THREADS) {
-            const int which = i / (SD_CHUNK * 16), j = i % (SD_CHUNK * 16);
-            const int r = 4 * ((j / 32) % (SD_CHUNK / 4)) + (j % 32) / 8, c = 4 * (j % 8 + 8 * (j / (8 * SD_CHUNK)));
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (r < n) v = *(const float4*)((which ? brow : crow) + (size_t)r * C + n0 + c);
-            float* dst = (which ? Bt : Ct) + c * SD_LD + ft_swizzle(r, c, 2);
-            dst[0] = v.x; dst[SD_LD] = v.y; dst[2 * SD_LD] = v.z; dst[3 * SD_LD] = v.w;
-        }
-        ft_wait<0>();
-        __syncthreads();
-        if (g_busy) g.template add_swizzled<2, true>(Ct, SD_LD, Bt, SD_LD, 0, 64);
-        if (busy) o.template add_swizzled<2, false>(Ct, SD_LD, Sh, P + 4, 0, 64);
+    for (int i = threadIdx.x; i < hb * SD_CHUNK; i += SD_THREADS + 32) {
+        const double l = cum[at * SD_CHUNK + i];
+        (&ls[0][0])[i] = l;
+        (&ds[0][0])[i] = dts[at * SD_CHUNK + i];
+        (&el[0][0])[i] = expf((float)l);
     }
+    tg_before();
     __syncthreads();
-    // A over C and B, v over S
-    if (g_busy)
+    tg_after();
+    // columns: a pair's 256 begin at 256 (q & 1): C S by halves of the states (0, 64), A v of either head (128, 192).
+    // C . B by halves lies in the second pair's first 128 until the first pair's A are made.
+    const uint32_t tmem = tmem_slot, lanes = (uint32_t)((warp & 3) * 32) << 16;
+    bool odd = false, ok = true;
+    if (warp == SD_THREADS / 32) {
+        // ---------------------------------------------------------- issuer
+        const bool leader = tg_elect();
+        ok = sd_wait(cb_full, 0, 3);
+        if (ok && leader) {                              // rows 64.. of the accumulators are nobody's
 #pragma unroll
-        for (int c = 0; c < GN; ++c)
+            for (int x = 0; x < HALVES; ++x)
+                s3_products<3, 3, 4>(tmem + 256u + 64u * x, tg_desc(sC + x * SD_TILE), HALVES * SD_TILE >> 4, 2, tg_desc(sB + x * SD_TILE),
+                                     HALVES * SD_TILE >> 4, 2, tg_idesc(64), false);
+            tg_commit(s_done);
+        }
+        __syncwarp();
+        for (int q = 0, stage = 0; q < pairs && ok; ++q) {
+            const uint32_t to = tmem + 256u * (q & 1);
+            if (q > 1) ok = sd_wait(&y_free[q & 1], ((q >> 1) & 1) ^ 1, 3);      // the results of the pair before the last are out
+            for (int x = 0; x < STAGES && ok; ++x, ++stage) {
+                unsigned char* buf = sR + (stage & 1) * STAGE;
+                ok = sd_wait(&r_full[stage & 1], (stage >> 1) & 1, 3);
+                if (ok && x == 1) ok = sd_wait(a_full, q & 1, 3);
+                if (!ok) break;
+                if (leader) {
+                    if (x != 1)
+                        s3_products<3, 3, 4>(to + 64u * (x >> 1), tg_desc_mn(buf, SD_TILE), 2 * SD_TILE >> 4, 128,
+                                             tg_desc(sC + (x >> 1) * SD_TILE), HALVES * SD_TILE >> 4, 2, tg_idesc(64, false, true), false);
+                    else
 #pragma unroll
-            for (int j = 0; j < 4; ++j) {
-                const int cj = g.col(c) + j;
-                float z[4];
-#pragma unroll
-                for (int i = 0; i < 4; ++i) {
-                    const float4 x = g.get(i, c);
-                    z[i] = j == 0 ? x.x : j == 1 ? x.y : j == 2 ? x.z : x.w;
+                        for (int e = 0; e < HP; ++e)     // both heads' lanes, of which e's are read
+                            s3_products<3, 3, 4>(to + 128u + 64u * e, tg_desc_mn(buf, SD_TILE), 2 * SD_TILE >> 4, 128,
+                                                 tg_desc(sA + 3 * e * SD_TILE), SD_TILE >> 4, 2, tg_idesc(64, false, true), false);
+                    tg_commit(&r_done[stage & 1]);
+                    if (x == 1) tg_commit(a_done);
+                    if (x == STAGES - 1) tg_commit(y_done);
                 }
+                __syncwarp();
+            }
+        }
+        if (!ok && leader) tg_settle_products(settled, &ssd_error_flag, 3);
+    } else {
+        {
+            SdRows<N> c, b;
+            c.load(crow, C, n);
+            b.load(brow, C, n);
+            odd = c.put(tg_smem(sC), n);
+            odd = b.put(tg_smem(sB), n) || odd;
+        }
+        sd_full(cb_full);
+        if (warp < SD_HALF / 32) {
+            // ------------------------------------------------------ the states and values of the pairs
+            // the states of a pair's heads [N][P] each: a stage is 64 states x 128 channels. The values come second, so
+            // that A v is made while the other states are laid down.
+            constexpr int RUNS = 64 * 16 / SD_HALF;
+            float4 p[RUNS][2];
+            auto ask = [&](int q, int x) {
 #pragma unroll
-                for (int e = 0; e < HEADS; ++e) {
-                    float a[4];
+                for (int j = 0; j < RUNS; ++j) {
+                    const int i = threadIdx.x + j * SD_HALF, m = 64 * x + i / 16, c = (i % 16) * 8;
+                    const int l = min(q * HP + c / P, hb - 1);
+                    const float4* src = (const float4*)(U + ((at + l) * N + m) * P + c % P);
+                    p[j][0] = src[0];
+                    p[j][1] = src[1];
+                }
+            };
+            ask(0, 0);
+            SdPair<SD_HALF> v;
+            for (int q = 0, stage = 0; q < pairs && ok; ++q) {
+                const int heads = min(HP, hb - q * HP), width = heads * P;
+                for (int x = 0; x < STAGES && ok; ++x, ++stage) {
+                    if (stage > 1) ok = sd_wait(&r_done[stage & 1], ((stage >> 1) & 1) ^ 1, 4);
+                    if (!ok) break;
+                    const uint32_t buf = tg_smem(sR) + (stage & 1) * STAGE;
+                    if (x != 1) {
 #pragma unroll
-                    for (int i = 0; i < 4; ++i) {
-                        const int ri = 4 * g.ty + i;
-                        a[i] = cj <= ri ? z[i] * expf((float)(ls[e][ri] - ls[e][cj])) : 0.f;
+                        for (int j0 = 0; j0 < RUNS; j0 += 2) {
+                            float f[2][8];
+                            uint32_t dst[2];
+#pragma unroll
+                            for (int j = 0; j < 2; ++j) {
+                                const int i = threadIdx.x + (j0 + j) * SD_HALF, piece = i % 16;
+                                sd_eight(f[j], p[j0 + j][0], p[j0 + j][1], 1.f, piece * 8 < width);
+                                dst[j] = buf + (piece >> 3) * SD_TILE + s3_place(i / 16, piece & 7);
+                            }
+                            odd = s3_put<2>(f, dst, 2 * SD_TILE) || odd;
+                        }
+                    } else {
+                        odd = v.template put<P>(buf, n, width, nullptr) || odd;
                     }
-                    *(float4*)(Ct + (e * 64 + cj) * SD_LD + 4 * g.ty) = make_float4(a[0], a[1], a[2], a[3]);
+                    sd_full(&r_full[stage & 1]);
+                    if (x == 0) v.load(rows + (h0 + q * HP) * P, C, n, width);
+                    else if (x + 1 < STAGES) ask(q, 1);
+                    else if (q + 1 < pairs) ask(q + 1, 0);
                 }
             }
-    bool odd = false;                                    // a value that is not finite among the chunk's
-    for (int i = t; i < SD_CHUNK * (P / 4); i += EACH) {
-        const int r = i / (P / 4), c = (i % (P / 4)) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (r < n) v = *(const float4*)(rows + (size_t)r * C + h * P + c);
-        const float w = ds[hh][r];
-        v.x *= w; v.y *= w; v.z *= w; v.w *= w;
-        *(float4*)(Sh + r * (P + 4) + c) = v;
-        odd = odd || ft_not_finite(v);
-    }
-    const bool triangle = __syncthreads_or(odd);
-    if (!busy) return;
+        } else {
+            // ------------------------------------------------------ A of the pairs, and their results
+            const int tid = threadIdx.x - SD_HALF, ai = tid / 4, aj = tid % 4 * 8;       // two eights of every A: aj, aj + 32
+            ok = sd_sync<SD_HALF>(sd_wait(s_done, 0, 6));
+            float s[16];
+            {                                            // C . B out of tensor memory, a row to four threads
+                float* st = (float*)sB;                  // B's parts have been read
+                if ((warp & 3) < 2) {
+                    const int i = (warp & 3) * 32 + lane, j0 = (warp >> 2 & 1) * 32;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) o.scale_row(i, expf((float)ls[hh][4 * o.ty + i]));
-    // tokens past a row have factors of 0: added where all values are finite, left out where they are not
-    const int first_row = 4 * (o.ty & ~(32 / TX - 1)), end = min(n, 4 * (o.ty | (32 / TX - 1)) + 4);
-    o.add(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, triangle ? first_row : end);
-    if (triangle) o.add_triangle(Ct + hh * 64 * SD_LD, SD_LD, Sh, P + 4, first_row, end);
-    const float Dh = D ? D[h] : 0.f;
+                    for (int c = 0; c < 32; c += 16) {
+                        uint32_t s0[16], s1[16];
+                        tg_ld16(tmem + lanes + 256u + (uint32_t)(j0 + c), s0);
+                        if (HALVES > 1) tg_ld16(tmem + lanes + 320u + (uint32_t)(j0 + c), s1);
+                        tg_wait_ld();
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const int r = 4 * o.ty + i;
-        if (r >= n) break;
+                        for (int x = 0; x < 16; ++x)
+                            st[i * (SD_CHUNK + 1) + j0 + c + x] = __uint_as_float(s0[x]) + (HALVES > 1 ? __uint_as_float(s1[x]) : 0.f);
+                    }
+                }
+                sd_sync<SD_HALF>(ok);
 #pragma unroll
-        for (int c = 0; c < 2; ++c) {
-            const float4 x = *(const float4*)(rows + (size_t)r * C + h * P + o.col(c));
-            float4 v = o.get(i, c);
-            v.x = fmaf(Dh, x.x, v.x); v.y = fmaf(Dh, x.y, v.y); v.z = fmaf(Dh, x.z, v.z); v.w = fmaf(Dh, x.w, v.w);
-            *(float4*)(y + (size_t)(ch.x + r) * H * P + h * P + o.col(c)) = v;
+                for (int x = 0; x < 16; ++x) s[x] = st[ai * (SD_CHUNK + 1) + aj + (x & 7) + (x >> 3) * 32];
+                sd_sync<SD_HALF>(ok);
+            }
+            for (int q = 0; q <= pairs && ok; ++q) {
+                if (q > 0) ok = sd_wait(a_done, (q - 1) & 1, 5);     // A's place is free
+                if (!ok) break;
+                if (q < pairs) {
+                    for (int e = 0; e < min(HP, hb - q * HP); ++e) {
+                        const double* l = ls[q * HP + e];
+                        const float* dt = ds[q * HP + e];
+                        const double li = l[ai];
+                        const float Dh = D ? D[h0 + q * HP + e] : 0.f;
+                        float f[2][8];
+#pragma unroll
+                        for (int x = 0; x < 16; ++x) {
+                            const int j = aj + (x & 7) + (x >> 3) * 32;
+                            const float a = s[x] * (expf((float)(li - l[j])) * dt[j]);       // 0 to infinity past the diagonal
+                            f[x >> 3][x & 7] = j > ai || ai >= n ? 0.f : j == ai ? a + Dh : a;
+                        }
+                        const uint32_t tile = tg_smem(sA) + (uint32_t)(3 * e * SD_TILE);
+                        const uint32_t dst[2] = {tile + s3_place(ai, aj / 8), tile + s3_place(ai, aj / 8 + 4)};
+                        odd = s3_put<2>(f, dst, SD_TILE) || odd;
+                    }
+                    sd_full(a_full);
+                }
+                if (q > 0) {
+                    const int d = q - 1, row = (warp & 3) * 32 + lane, l = d * HP + row / P, i0 = (warp >> 2 & 1) * 32;
+                    ok = sd_wait(y_done, d & 1, 5);
+                    if (!ok) break;
+                    const uint32_t t = tmem + lanes + 256u * (d & 1) + (uint32_t)i0;
+                    float* dst = y + (size_t)(ch.x + i0) * H * P + (h0 + l) * P + row % P;
+#pragma unroll
+                    for (int c = 0; c < 32; c += 16) {
+                        uint32_t a[16], p0[16], p1[16];
+                        tg_ld16(t + 128u + 64u * (row / P) + c, a);
+                        tg_ld16(t + c, p0);
+                        if (HALVES > 1) tg_ld16(t + 64u + c, p1);
+                        tg_wait_ld();
+                        if (l < hb)
+#pragma unroll
+                            for (int i = 0; i < 16; ++i)
+                                if (i0 + c + i < n) {
+                                    const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
+                                    dst[(size_t)(c + i) * H * P] = fmaf(far, el[l][i0 + c + i], __uint_as_float(a[i]));
+                                }
+                    }
+                    sd_full(&y_free[d & 1]);
+                }
+            }
         }
     }
+    ok = __syncthreads_and(ok);
+    if (__syncthreads_or(odd) && ok) {                   // plain sums: a token past a row is not added at all
+        float* Sf = (float*)sC;
+        for (int x = threadIdx.x; x < n * SD_CHUNK; x += SD_THREADS + 32) {
+            const int i = x / SD_CHUNK, j = x % SD_CHUNK;
+            float sum = 0.f;
+            for (int m = 0; j <= i && m < N; ++m) sum = fmaf(crow[(size_t)i * C + m], brow[(size_t)j * C + m], sum);
+            Sf[i * (SD_CHUNK + 1) + j] = sum;
+        }
+        __syncthreads();
+        for (int x = threadIdx.x; x < hb * n * P; x += SD_THREADS + 32) {
+            const int l = x / (n * P), i = x / P % n, c = x % P;
+            const size_t o = (at + l) * SD_CHUNK;
+            const float* Uc = U + (at + l) * N * P + c;
+            float sum = 0.f;
+            for (int m = 0; m < N; ++m) sum = fmaf(crow[(size_t)i * C + m], Uc[(size_t)m * P], sum);
+            sum *= expf((float)cum[o + i]);
+            for (int j = 0; j <= i; ++j)
+                sum = fmaf(Sf[i * (SD_CHUNK + 1) + j] * expf((float)(cum[o + i] - cum[o + j])),
+                           dts[o + j] * rows[(size_t)j * C + (h0 + l) * P + c], sum);
+            sum = fmaf(D ? D[h0 + l] : 0.f, rows[(size_t)i * C + (h0 + l) * P + c], sum);
+            if (sd_not_finite(sum)) y[(size_t)(ch.x + i) * H * P + (h0 + l) * P + c] = sum;
+        }
+    }
+    tg_before();
+    __syncthreads();
+    if (warp == 0) {
+        tg_after();
+        tg_free512(tmem_slot);
+    }
 }
+
+// The code a wait of the chunks' products left when it ran out (0: none did). Synchronises.
+TGO_API int tgo_ssd_error(int* value) { return (int)cudaMemcpyFromSymbol(value, ssd_error_flag, sizeof(int)); }
 
 TGO_API int tgo_ssd_chunk_tokens() { return SD_CHUNK; }
 template <int N, int P>
 static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stride, const float* dt_bias, const float* A_log,
                   const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
                   float* state, long long state_stride, long long offset, float* ws, long long ws_floats, cudaStream_t stream) {
-    constexpr size_t s1 = (size_t)SD_CHUNK * (N + 4 + P + 4) * sizeof(float);
-    constexpr int PAIR = P == 64 ? 2 : 1;                // heads a block of the outputs where a group has an even number
-    constexpr size_t s3 = ((size_t)2 * 64 * SD_LD + 64 * (P + 4)) * sizeof(float);
-    constexpr size_t s3p = ((size_t)2 * 64 * SD_LD + PAIR * 64 * (P + 4)) * sizeof(float);
+    constexpr int HP = 128 / P;
+    constexpr size_t s1 = 1024 + (3 * (N / 64) + 2 * 6) * SD_TILE, s3 = 1024 + sd_out_bytes<N, P>();
+    static_assert(s3 >= 1024 + SD_CHUNK * (SD_CHUNK + 1) * sizeof(float), "the plain sums' tile");
     static bool sized[64] = {};                          // per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
@@ -721,16 +1025,19 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
     if (dev < 0 || dev >= 64) return TGO_E_BAD_ARG;
     if (!sized[dev]) {
         if ((e = cudaFuncSetAttribute(ssd_summaries_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s1)) != cudaSuccess) return (int)e;
-        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P, PAIR>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3p)) != cudaSuccess) return (int)e;
-        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
+        if ((e = cudaFuncSetAttribute(ssd_outputs_kernel<N, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
         sized[dev] = true;
     }
     const int n_chunks = T / SD_CHUNK + B;               // at least as many as there are
-    const bool pairs = PAIR == 2 && H / G % 2 == 0;
-    // heads a group: what the workspace holds, an even number where two share a block
+    // Heads at a time: what the workspace holds, whole groups where it holds one. Heads a block: as many of a group as
+    // leave a block a multiprocessor, so that B and C are laid down once for them.
     long long each = (ws_floats / n_chunks - 4) / (N * P + 3 * SD_CHUNK);
     if (each > H) each = H;
-    if (pairs && each > 1) each &= ~1ll;
+    const int group = H / G;
+    int hb = 1;
+    for (int d = 1; d <= group && d <= each && d <= SD_HEADS; ++d)
+        if (group % d == 0 && (d <= HP || (long long)n_chunks * (each / d) >= tgo_multiprocessors())) hb = d;
+    each -= each % hb;
     for (int h0 = 0; h0 < H; h0 += (int)each) {
         const int nh = H - h0 < each ? H - h0 : (int)each;
         float* U = ws;
@@ -740,21 +1047,14 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
         int rc = tgo_launch_pdl(ssd_steps_kernel<bf16>, dim3(n_chunks, (nh + 7) / 8), dim3(256), 0, stream, dt_raw + h0, dt_stride,
                                 dt_bias ? dt_bias + h0 : dt_bias, A_log + h0, nh, q_start, B, chunks, dts, cum);
         if (rc) return rc;
-        rc = tgo_launch_pdl(ssd_summaries_kernel<N, P>, dim3(n_chunks, nh), dim3(N * P / 64), s1, stream, xbc, C, H, G, h0,
-                            (const int4*)chunks, (const float*)dts, (const double*)cum, U);
+        rc = tgo_launch_pdl(ssd_summaries_kernel<N, P>, dim3(n_chunks, nh / hb), dim3(SD_THREADS + 32), s1, stream, xbc, C, H, G, h0,
+                            hb, (const int4*)chunks, (const float*)dts, (const double*)cum, U);
         if (rc) return rc;
         rc = tgo_launch_pdl(ssd_scan_kernel, dim3(B, nh, (N * P / 4 + 255) / 256), dim3(256), 0, stream, nh, N * P, q_start,
                             state_slots, (const double*)cum, U, state, state_stride, offset + (long long)h0 * N * P);
         if (rc) return rc;
-        // Two heads a block from more (chunk, head) pairs than multiprocessors: 2048 tokens of 64 heads 134 us
-        // against 148, 700 of 24 25.1 against 27.1; 160 of 8 (24 pairs) 24.4 against 20.7, 512 of 16 (144) 24.9
-        // against 21.3.
-        if (pairs && nh % 2 == 0 && (long long)n_chunks * nh > tgo_multiprocessors())
-            rc = tgo_launch_pdl(ssd_outputs_kernel<N, P, PAIR>, dim3(n_chunks, nh / PAIR), dim3(PAIR * 2 * P), s3p, stream, xbc, C,
-                                H, G, h0, D, (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
-        else
-            rc = tgo_launch_pdl(ssd_outputs_kernel<N, P, 1>, dim3(n_chunks, nh), dim3(2 * P), s3, stream, xbc, C, H, G, h0, D,
-                                (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
+        rc = tgo_launch_pdl(ssd_outputs_kernel<N, P>, dim3(n_chunks, nh / hb), dim3(SD_THREADS + 32), s3, stream, xbc, C, H, G, h0, hb, D,
+                            (const int4*)chunks, (const float*)dts, (const double*)cum, (const float*)U, y);
         if (rc) return rc;
     }
     return 0;

@@ -1054,6 +1054,13 @@ def causal_conv_act(x: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
         LAUNCHES[0] += 1
 
 
+def ssd_error() -> int:
+    """The code a wait of the selective scan by chunks left when it ran out, or 0. Synchronises."""
+    value = ctypes.c_int(0)
+    _check(entry_points("state_space").tgo_ssd_error(ctypes.addressof(value)), "ssd_error")
+    return int(value.value)
+
+
 # Steps of at least so many tokens, and so many a request on average, run the selective scan by
 # chunks in the bfloat16 engine (64 heads of 64 x 128, a call's wall time, walk against chunks: 64
 # tokens 28 against 36 us, 128 47 / 47, 256 90 / 60; 16 requests of 128 359 / 288; 256 tokens beside 31
@@ -2184,6 +2191,10 @@ def kernel_wait_errors() -> dict:
         code = sgemm_error()
         if code:
             out["sgemm"] = code
+    if "state_space" in _loaded:
+        code = ssd_error()
+        if code:
+            out["selective_scan"] = code
     if "retention" in _loaded:
         code = retention_error()
         if code:
