@@ -12,7 +12,8 @@
 // 64 KB more). Per key tile of 128 the products take 3328 cycles (36 of 64, 8 of 128) and 208 KB come
 // into the SM: both near what it can do.
 //   warp 0      draws items (longest first) from a counter, asks TMA for Q, publishes a record;
-//   warps 12, 10  ask for K and for V, a page and block a lane;
+//   warps 12..14, 10 and 15  ask for K and for V, a warp a slot of its ring, a page and block a lane (a warp starts a
+//               copy about every 80 cycles, and a key tile in pages of 16 takes 72 of K and 32 of V: one warp each, 138 us);
 //   warps 1, 11   issue S = Q K^T and O += P V, a thread each;
 //   warps 2..9  softmax, two threads a row, as in attention_tc.cu (lazily moved maximum).
 // Rows of V that nobody may read are zeroed by warp 10 once they have landed (P is zero there, but the
@@ -26,7 +27,7 @@
 // multicast.
 #include "tcgen.cuh"
 
-#define LT_THREADS 416
+#define LT_THREADS 512
 #define LT_BLOCK 16384                   // 128 rows x 64 channels, or 32 rows x 256
 #define LT_MAX_BLOCKS 9                  // blocks of Q: rows up to 576 wide
 #define LT_K_SLOTS 3
@@ -57,6 +58,13 @@ __device__ __forceinline__ float lt_ex2(float x) {
 __device__ __forceinline__ void lt_load_3d(void* dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
     asm volatile("cp.async.bulk.tensor.3d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5}], [%2];"
                  ::"r"(tg_smem(dst)), "l"(map), "r"(tg_smem(bar)), "r"(x), "r"(y), "r"(z) : "memory");
+}
+
+// A warp that gives up waits for the last copies into its own slot; `count` uses of the ring have gone by.
+__device__ __forceinline__ void lt_settle_slot(uint64_t* full, uint32_t slots, uint32_t slot, uint32_t count, int* err, int code) {
+    if (count <= slot) return;
+    const uint32_t last = count - 1 - (count - 1 - slot) % slots;
+    tg_wait(&full[slot], (last / slots) & 1u, err, code);
 }
 
 __global__ void __launch_bounds__(LT_THREADS, 1)
@@ -99,7 +107,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
     }
     if (tid == 0) {
         tg_init(q_full, 1);
-        tg_init(q_empty, 12);
+        tg_init(q_empty, 15);
         for (int i = 0; i < LT_K_SLOTS; ++i) { tg_init(&k_full[i], 1); tg_init(&k_empty[i], 1); }
         for (int i = 0; i < 2; ++i) {
             tg_init(&v_full[i], 1); tg_init(&v_empty[i], 1); tg_init(&v_ok[i], 1);
@@ -155,7 +163,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
             }
             __syncwarp();
         }
-    } else if (warp == 12) {
+    } else if (warp >= 12 && warp < 12 + LT_K_SLOTS) {
         // ---------------------------------------------------------- K
         bool ok = true;
         uint32_t g = 0;
@@ -177,6 +185,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 const int at = (first + lane - j * ppt) * page_size * 128;
                 for (int c = 0; c < blocks; ++c, ++g) {
                     const uint32_t s = g % LT_K_SLOTS, ph = (g / LT_K_SLOTS) & 1u;
+                    if (s != (uint32_t)(warp - 12)) continue;
                     ok = __all_sync(0xffffffffu, tg_wait(&k_empty[s], ph ^ 1u, err, 3));
                     if (!ok) break;
                     if (lane == 0) tg_expect(&k_full[s], (uint32_t)(last - first) * (uint32_t)page_size * 128u);
@@ -185,8 +194,8 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         }
-        if (!ok) tg_settle_copies(k_full, LT_K_SLOTS, g, err, 3);
-    } else if (warp == 10) {
+        if (!ok) lt_settle_slot(k_full, LT_K_SLOTS, warp - 12, g, err, 3);
+    } else if (warp == 10 || warp == 15) {
         // ---------------------------------------------------------- V
         bool ok = true;
         uint32_t g = 0;
@@ -205,6 +214,10 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                     const int k0 = (rec.t_lo + it) * 128 + 32 * q;
                     if (k0 >= rec.key_hi || k0 + 32 <= rec.key_lo) continue;         // P is zero there
                     const uint32_t s = g % LT_V_SLOTS, ph = (g / LT_V_SLOTS) & 1u;
+                    if (s != (warp == 15 ? 1u : 0u)) {   // the other warp's
+                        ++g;
+                        continue;
+                    }
                     ok = __all_sync(0xffffffffu, tg_wait(&v_empty[s], ph ^ 1u, err, 5));
                     if (!ok) break;
                     ++g;
@@ -238,7 +251,7 @@ attention_latent_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __gr
                 }
             }
         }
-        if (!ok) tg_settle_copies(v_full, LT_V_SLOTS, g, err, 5);
+        if (!ok) lt_settle_slot(v_full, LT_V_SLOTS, warp == 15 ? 1 : 0, g, err, 5);
     } else if (warp == 1) {
         // ---------------------------------------------------------- issuer of S = Q K^T
         if (lane == 0) {
