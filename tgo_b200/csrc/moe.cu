@@ -513,7 +513,7 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
 #define MT_RING (192 * 1024)
 #define MT_STAGE_OUT 4096                  // per epilogue warp: 32 rows x 128 bytes on their way out
 #define MT_SMEM (MT_RING + 4 * MT_STAGE_OUT + 1024 + 256)
-#define MT_THREADS 192
+#define MT_THREADS 224
 
 __device__ int moe_error_flag = 0;
 
@@ -532,7 +532,7 @@ __device__ __forceinline__ float moe_act_tile(float z, int act) {
 
 template <int MODE>
 __global__ void __launch_bounds__(MT_THREADS, 1)
-moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b0,
+moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_tile, const __grid_constant__ CUtensorMap map_b0,
               const __grid_constant__ CUtensorMap map_b1, bf16* __restrict__ hidden, float* __restrict__ y, int N,
               int K, int bn, int top, int act, int gather, const int* __restrict__ perm,
               const int* __restrict__ tile_info, const int* __restrict__ tiles) {
@@ -551,7 +551,7 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     uint32_t* tmem_slot = (uint32_t*)(settled + 1);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (threadIdx.x == 0) {
-        for (int i = 0; i < 8; ++i) { tg_init(&full[i], 1); tg_init(&empty[i], 1); }
+        for (int i = 0; i < 8; ++i) { tg_init(&full[i], 2); tg_init(&empty[i], 1); }
         for (int i = 0; i < 2; ++i) { tg_init(&acc_full[i], 1); tg_init(&acc_empty[i], 4); }
         tg_init(settled, 1);
         tg_init_done();
@@ -564,28 +564,44 @@ moe_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__
     pdl_wait();
     const int n_nt = (N + bn - 1) / bn, total = tile_info[0] * n_nt, kbs = (K + MT_BK - 1) / MT_BK;
 
-    if (warp == 0) {
+    if (warp == 0 || warp == 6) {
+        // ---- rows (warp 0) and matrices (warp 6): a warp starts a copy about every 80 cycles
         uint32_t it = 0;
         bool ok = true;
         for (int w = blockIdx.x; w < total && ok; w += gridDim.x) {
             const int tile = w / n_nt, n0 = (w % n_nt) * bn;
             const int e = tiles[3 * tile], r0 = tiles[3 * tile + 1], rows = tiles[3 * tile + 2];
+            // more than three boxes of 32 rows come as one of 128: the rows after an expert's are the next one's, whose
+            // sums nobody stores
+            const bool whole = !gather && rows > 96;
             int src[4] = {0, 0, 0, 0};
-            if (gather)
+            if (gather && warp == 0)
 #pragma unroll
                 for (int j = 0; j < 4; ++j) src[j] = perm[r0 + min(4 * lane + j, rows - 1)] / top;
-            const int groups = gather ? (rows + 3) / 4 : (rows + 31) / 32, group_bytes = gather ? 512 : 4096;
+            const int groups = gather ? (rows + 3) / 4 : whole ? 1 : (rows + 31) / 32, group_bytes = gather ? 512 : whole ? MT_A_BYTES : 4096;
             for (int kb = 0; kb < kbs; ++kb, ++it) {
                 const int s = it % stages;
                 ok = __all_sync(0xffffffffu, tg_wait(&empty[s], ((it / stages) & 1) ^ 1, &moe_error_flag, 1));
                 if (!ok) break;
                 unsigned char* st = base + (size_t)s * stage_bytes;
-                if (lane == 0) tg_expect(&full[s], (uint32_t)(groups * group_bytes + nm * MT_BK * 2));
+                if (warp == 6) {
+                    if (lane == 0) {
+                        tg_expect(&full[s], (uint32_t)(nm * MT_BK * 2));
+                        tg_load_2d(st + MT_A_BYTES, &map_b0, kb * MT_BK, e * N + n0, &full[s]);
+                        if (GATED) tg_load_2d(st + MT_A_BYTES + bn * MT_BK * 2, &map_b1, kb * MT_BK, e * N + n0, &full[s]);
+                    }
+                    __syncwarp();
+                    continue;
+                }
+                if (lane == 0) tg_expect(&full[s], (uint32_t)(groups * group_bytes));
                 __syncwarp();
-                if (lane == 0) tg_load_2d(st + MT_A_BYTES, &map_b0, kb * MT_BK, e * N + n0, &full[s]);
-                if (GATED && lane == 1) tg_load_2d(st + MT_A_BYTES + bn * MT_BK * 2, &map_b1, kb * MT_BK, e * N + n0, &full[s]);
-                if (lane < groups && !gather) tg_load_2d(st + lane * 4096, &map_a, kb * MT_BK, r0 + 32 * lane, &full[s]);
-                if (lane < groups && gather) tg_gather4(st + lane * 512, &map_a, kb * MT_BK, src[0], src[1], src[2], src[3], &full[s]);
+                if (whole) {
+                    if (lane == 0) tg_load_2d(st, &map_tile, kb * MT_BK, r0, &full[s]);
+                } else if (!gather) {
+                    if (lane < groups) tg_load_2d(st + lane * 4096, &map_a, kb * MT_BK, r0 + 32 * lane, &full[s]);
+                } else if (lane < groups) {
+                    tg_gather4(st + lane * 512, &map_a, kb * MT_BK, src[0], src[1], src[2], src[3], &full[s]);
+                }
             }
         }
         if (!ok) tg_settle_copies(full, stages, it, &moe_error_flag, 1);
@@ -743,11 +759,11 @@ static int moe_tc_launch(const void* a, long long a_rows, long long a_stride, co
         sized[dev] = true;
     }
     const int bn = moe_tc_width(N, K, E, pairs, MODE == 1, tgo_multiprocessors());
-    CUtensorMap ma, m0, m1;
-    if (!tg_map(&ma, a, a_rows, K, a_stride, gather ? 1 : 32) || !tg_map(&m0, b0, (long long)E * N, K, K, bn) ||
+    CUtensorMap ma, mt, m0, m1;
+    if (!tg_map(&ma, a, a_rows, K, a_stride, gather ? 1 : 32) || !tg_map(&mt, a, a_rows, K, a_stride, MOE_TILE) || !tg_map(&m0, b0, (long long)E * N, K, K, bn) ||
         !tg_map(&m1, b1 ? b1 : b0, (long long)E * N, K, K, bn))
         return TGO_E_BAD_ARG;
-    return tgo_launch_pdl(moe_tc_kernel<MODE>, dim3(tgo_multiprocessors()), dim3(MT_THREADS), MT_SMEM, stream, ma, m0, m1, (bf16*)hidden, y,
+    return tgo_launch_pdl(moe_tc_kernel<MODE>, dim3(tgo_multiprocessors()), dim3(MT_THREADS), MT_SMEM, stream, ma, mt, m0, m1, (bf16*)hidden, y,
                           N, K, bn, top, act, gather ? 1 : 0, perm, tile_info, tiles);
 }
 
