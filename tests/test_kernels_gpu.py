@@ -1164,6 +1164,19 @@ def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
 
 
+@pytest.mark.parametrize("T,d", [(5, 136), (300, 72)])
+def test_routed_experts_rounded(T, d):
+    """Results in bfloat16 are the float32 ones rounded, with what is added to them."""
+    o, ff, top, E = ops(), 40, 2, 6
+    x = rnd(T, d, seed=1).to(torch.bfloat16)
+    wr = rnd(E, d, seed=2) * d ** -0.5
+    wg, wu = ((rnd(E, ff, d, seed=s) * d ** -0.5).to(torch.bfloat16) for s in (3, 4))
+    wd = (rnd(E, d, ff, seed=5) * ff ** -0.5).to(torch.bfloat16)
+    run = lambda **kw: o.moe_feed_forward(x, wr, None, wg, wu, wd, top, "silu", rnd(T, d, seed=6),       # noqa: E731
+                                          beside=rnd(T, d, seed=7).to(torch.bfloat16), **kw)
+    assert torch.equal(run(out_dtype=torch.bfloat16), run().to(torch.bfloat16))
+
+
 @pytest.mark.parametrize("T,E,identity,top", [(9, 4, 0, 2), (9, 4, 4, 3), (200, 4, 0, 2), (200, 4, 4, 3)])
 @pytest.mark.parametrize("strided", [False, True])
 def test_routed_experts_of_strided_rows_and_identities(T, E, identity, top, strided):

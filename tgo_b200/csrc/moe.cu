@@ -770,11 +770,11 @@ static int moe_tc_launch(const void* a, long long a_rows, long long a_stride, co
 // out[t][c] = sum_j wts[t][j] y[t top + j][c] + extra_gate[t] * extra[t][c]; a pair whose
 // expert is an identity expert (ids >= E_real; `ids` null: there are none) contributes
 // wts * x[t][c] instead. `beside` [T, d] (TB: float32 or bfloat16; null: none) is added too, and
-// with `accumulate` the whole is added to out: a block whose mixer and feed-forward read the
+// with `accumulate` (float32 out) the whole is added to out: a block whose mixer and feed-forward read the
 // same rows has both results put into the stream by this one pass.
-template <typename T, typename TB>
+template <typename T, typename TB, typename TO>
 __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __restrict__ wts,
-                                   const float* __restrict__ extra, float* __restrict__ out, int d,
+                                   const float* __restrict__ extra, TO* __restrict__ out, int d,
                                    int top, const int* __restrict__ ids, int E_real,
                                    const T* __restrict__ x, long long x_stride,
                                    const float* __restrict__ extra_gate,
@@ -787,7 +787,7 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
             float4 a = make_float4(0.f, 0.f, 0.f, 0.f);
             const float4 ex = extra ? *(const float4*)(extra + (size_t)t * d + c) : a;
             const float4 bs = beside ? Load4<TB>::get(beside + (size_t)t * d + c) : a;
-            const float4 o = accumulate ? *(const float4*)(out + (size_t)t * d + c) : a;
+            const float4 o = accumulate ? *(const float4*)((const float*)out + (size_t)t * d + c) : a;
 #pragma unroll 4
             for (int j = 0; j < top; ++j) {
                 const size_t pair = (size_t)t * top + j;
@@ -803,7 +803,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
             }
             if (beside) { a.x += bs.x; a.y += bs.y; a.z += bs.z; a.w += bs.w; }
             if (accumulate) { a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w; }
-            *(float4*)(out + (size_t)t * d + c) = a;
+            if constexpr (sizeof(TO) == 4) *(float4*)(out + (size_t)t * d + c) = a;
+            else *(uint2*)(out + (size_t)t * d + c) = make_uint2(tg_pack(a.x, a.y), tg_pack(a.z, a.w));
         }
         return;
     }
@@ -816,8 +817,8 @@ __global__ void moe_combine_kernel(const float* __restrict__ y, const float* __r
         }
         if (extra) a = fmaf(eg, extra[(size_t)t * d + c], a);
         if (beside) a += to_f32(beside[(size_t)t * d + c]);
-        if (accumulate) a += out[(size_t)t * d + c];
-        out[(size_t)t * d + c] = a;
+        if (accumulate) a += to_f32(out[(size_t)t * d + c]);
+        out[(size_t)t * d + c] = from_f32<TO>(a);
     }
 }
 
@@ -880,27 +881,32 @@ TGO_API int tgo_moe_route(const void* x, long long x_stride, int dtype, const fl
 }
 
 // x [T, d] rows (stride x_stride); wg, wu [E, ff, d]; wd [E, d, ff]; hidden [T top, ff] in the
-// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out float32 [T, d]. xg: null, or
+// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out [T, d], float32 or (bfloat16 x, no
+// accumulation) bfloat16. xg: null, or
 // [T top, d] in the storage type, 16-byte aligned: room for the rows of x in place order.
 TGO_API int tgo_moe_experts(const void* x, long long x_stride, int dtype, const void* wg,
                             const void* wu, const void* wd, void* hidden, float* y,
-                            const float* wts, const float* extra, float* out, int T, int d, int ff,
+                            const float* wts, const float* extra, void* out, int T, int d, int ff,
                             int top, int act, const int* perm, const int* offsets, void* xg, const int* tile_info,
                             const int* tiles, int max_tiles, const int* ids, int E_real,
                             const float* extra_gate, const void* beside, int beside_dtype,
-                            int accumulate, cudaStream_t stream) {
+                            int accumulate, int out_dtype, cudaStream_t stream) {
     if (T <= 0) return 0;
     if (d <= 0 || ff <= 0 || top <= 0 || max_tiles <= 0 || max_tiles > 65535 || act < 0 || act > 3)
         return TGO_E_BAD_ARG;
     const int comb_vec = d % 4 == 0 && x_stride % 4 == 0 && (uintptr_t)x % 16 == 0 && (uintptr_t)y % 16 == 0 &&
                          (uintptr_t)extra % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)beside % 16 == 0;
     const int comb_y = comb_vec && d > 512 ? (d / 512 < 16 ? d / 512 : 16) : 1;
-    if (beside && beside_dtype != TGO_F32 && beside_dtype != TGO_BF16) return TGO_E_BAD_ARG;
-#define MOE_COMBINE_OF(TT, TB)                                                                             \
-    tgo_launch_pdl(moe_combine_kernel<TT, TB>, dim3(T, comb_y), dim3(128), 0, stream, (const float*)y, wts, extra,  \
-                   out, d, top, ids, E_real, (const TT*)x, x_stride, extra_gate, (const TB*)beside, accumulate,     \
+    if ((beside && beside_dtype != TGO_F32 && beside_dtype != TGO_BF16) ||
+        (out_dtype != TGO_F32 && (out_dtype != TGO_BF16 || accumulate || dtype != TGO_BF16)))
+        return TGO_E_BAD_ARG;
+#define MOE_COMBINE_OF(TT, TB, TO)                                                                         \
+    tgo_launch_pdl(moe_combine_kernel<TT, TB, TO>, dim3(T, comb_y), dim3(128), 0, stream, (const float*)y, wts, extra,  \
+                   (TO*)out, d, top, ids, E_real, (const TT*)x, x_stride, extra_gate, (const TB*)beside, accumulate,     \
                    comb_vec)
-#define MOE_COMBINE(TT) (beside && beside_dtype == TGO_BF16 ? MOE_COMBINE_OF(TT, bf16) : MOE_COMBINE_OF(TT, float))
+#define MOE_COMBINE(TT)                                                                                               \
+    (out_dtype == TGO_BF16 ? (beside && beside_dtype == TGO_BF16 ? MOE_COMBINE_OF(TT, bf16, bf16) : MOE_COMBINE_OF(TT, float, bf16)) \
+                           : beside && beside_dtype == TGO_BF16 ? MOE_COMBINE_OF(TT, bf16, float) : MOE_COMBINE_OF(TT, float, float))
     const dim3 g1((ff + MOE_TN - 1) / MOE_TN, max_tiles, MOE_TILE / MOE_TM), g2((d + MOE_TN - 1) / MOE_TN, max_tiles, MOE_TILE / MOE_TM);
     int rc;
     const bool chunks = d % 8 == 0 && ff % 8 == 0 && x_stride % 8 == 0 && (uintptr_t)x % 16 == 0 &&

@@ -1299,7 +1299,7 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
                      renormalize: bool = True, route_scale: float = 1.0,
                      beside: Optional[torch.Tensor] = None,
                      residual: Optional[torch.Tensor] = None,
-                     group_best: int = 2) -> Optional[torch.Tensor]:
+                     group_best: int = 2, out_dtype: torch.dtype = torch.float32) -> Optional[torch.Tensor]:
     """A routed feed-forward: each row of x [T, d] goes to the `top` experts with the largest
     router scores (w_router float32 [E, d], b_router float32 [E]; float32 sums); expert e is
     w_down[e] (act(w_gate[e] x) * (w_up[e] x)), or, with w_gate None, w_down[e] act(w_up[e] x).
@@ -1320,7 +1320,9 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     the weights are the chosen scores as they are. `route_scale` multiplies the weights.
 
     `beside` ([T, d], float32 or bfloat16) is added to the result; with `residual` (float32
-    [T, d]) the result is added there and None is returned."""
+    [T, d]) the result is added there and None is returned. `out_dtype` bfloat16 (bfloat16 x, no
+    `residual`): the float32 sums rounded to it."""
+    assert out_dtype == torch.float32 or (out_dtype == x.dtype and residual is None)
     _need_cuda(x, w_router, b_router, w_gate, w_up, w_down, extra, correction, beside, residual)
     T, d = x.shape
     E, ff = w_up.shape[0], w_up.shape[1]
@@ -1359,7 +1361,7 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     w = {name: base + o for name, o in where.items()}
     gate, xg = w["gate"] if extra_gated else 0, w["xg"] if copies else 0
     launches = ctypes.c_int(0)
-    out = residual if residual is not None else torch.empty((T, d), dtype=torch.float32, device=dev)
+    out = residual if residual is not None else torch.empty((T, d), dtype=out_dtype, device=dev)
     lib = entry_points("moe")
     _check(lib.tgo_moe_route(
         _ptr(x), c_ll(x.stride(0)), c_int(dtype_code(x.dtype)), _ptr(w_router), _ptr(b_router),
@@ -1374,7 +1376,7 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
         c_int(ff), c_int(top), c_int(PLAIN_ACTIVATIONS[activation]), w["perm"], w["offsets"], xg, w["tile_info"],
         w["tiles"], c_int(max_tiles), w["ids"] if identity else 0, c_int(E), gate,
         _ptr(beside), c_int(dtype_code(beside.dtype) if beside is not None else 0),
-        c_int(1 if residual is not None else 0), _stream()), "moe_experts", f"(d={d}, ff={ff})")
+        c_int(1 if residual is not None else 0), c_int(dtype_code(out_dtype)), _stream()), "moe_experts", f"(d={d}, ff={ff})")
     LAUNCHES[0] += launches.value + 1            # beside the two that _check counted
     return None if residual is not None else out
 

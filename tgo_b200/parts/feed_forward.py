@@ -295,19 +295,13 @@ class RoutedExperts(Part):
     def forward(self, x, ctx, residual=None, beside=None):
         x = ops.rows_of(x)
         extra = self.shared.forward(x, ctx) if self.shared is not None else None
-        y = ops.moe_feed_forward(x, self.w_router, self.b_router, self.w_gate, self.w_up,
-                                 self.w_down, self.top, self.activation, extra, self.scores,
-                                 self.router_correction, self.identity, self.shared_gate,
-                                 self.groups, self.keep, self.renormalize, self.route_scale,
-                                 beside, residual, self.group_best)
-        if residual is not None:
-            return None
         want = self.out_dtype or ctx.act_dtype
-        if want == torch.float32:
-            return y
-        out = torch.empty(y.shape, dtype=want, device=y.device)
-        ops.cast_rows(y, out)
-        return out
+        rounded = {"out_dtype": want} if residual is None and want != torch.float32 else {}
+        return ops.moe_feed_forward(x, self.w_router, self.b_router, self.w_gate, self.w_up,
+                                    self.w_down, self.top, self.activation, extra, self.scores,
+                                    self.router_correction, self.identity, self.shared_gate,
+                                    self.groups, self.keep, self.renormalize, self.route_scale,
+                                    beside, residual, self.group_best, **rounded)
 
 
 FEED_FORWARDS.register("routed_experts", RoutedExperts)
