@@ -249,6 +249,19 @@ def test_sgemm_by_parts(M, N, K):
     assert ops().sgemm_error() == 0
 
 
+@pytest.mark.parametrize("up,wide", [(1e-38, 1.0), (1e-40, 1e3), (1e-36, 1e30), (1.0, 1e-39), (1e-22, 1e-22), (1e33, 1e-30),
+                                     (1e25, 1e10)])
+def test_sgemm_by_parts_small_and_large_numbers(up, wide):
+    """Numbers whose lower parts have no bfloat16 number of their size, and sizes past those the parts are scaled for."""
+    M, N, K = 33, 130, 512
+    x, w = (rnd(M, K, seed=5).double() * up).float(), (rnd(N, K, seed=6).double() * wide).float()
+    y = torch.empty(M, N, device=DEV)
+    ops().sgemm_tn(x, w, y)
+    want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
+    # the bound of the parts, or a chain's of K roundings; a rounding below the normal numbers is 2^-150 at most
+    assert ((y.double() - want).abs() <= K * 2.0 ** -24 * size + K * 2.0 ** -150).all()
+
+
 @pytest.mark.parametrize("T,H,G,dk,dv,rot", [(1, 1, 1, 16, 16, 16), (11, 3, 1, 48, 32, 16), (130, 2, 2, 64, 128, 0),
                                              (1203, 16, 4, 128, 128, 64)])
 def test_projection_rows_eight_channels_at_a_time(T, H, G, dk, dv, rot):

@@ -177,9 +177,12 @@ TGO_API void tgo_sgemm_force_tile(int tile) { sg_forced = tile; }
 // so a long sum there would lean towards zero; four steps at the sum's size and a rounded addition
 // per k-block err less than a chain of 64 FMA (MEASURED against 64 bits, 2-norms, normal numbers:
 // K = 2048 1.3e-7 for the chain's 8.1e-7, K = 6144 1.9e-7 for 1.4e-6).
+// Both sides are taken SP_UP times and an output SP_DOWN times: bfloat16 numbers end at 2^-133, so that the parts
+// of 1e-36 as it stands hold no more than its first 15 bits (MEASURED error 2.7e-5; at 1e-38 2.7e-3), while 24 powers
+// of two higher every float32 number has all of its parts.
 // An output's arithmetic is the same whatever tile it falls in and whatever rows are beside it. An output
-// that is not finite (an input that is not, or rounds to more than the largest bfloat16, or a sum that overflows) is made
-// again as the plain kernel makes it.
+// that is not finite (an input that is not, or is more than 2^103, or a sum past 2^80) is made again as the plain
+// kernel makes it.
 // Bound by shared memory and the tensor pipe side by side at many rows (a k-block at NT = 128: 1660 and 1540
 // cycles), by the issue of 24 products a k-block at few. With w's parts in shared memory, made by the warps that
 // sum, and the products issued by a lane that no elect.sync had chosen, a k-block took 2500 cycles at any NT.
@@ -189,6 +192,8 @@ TGO_API void tgo_sgemm_force_tile(int tile) { sg_forced = tile; }
 #include "split3.cuh"
 
 #define SP_BK 64
+#define SP_UP 0x1p24f
+#define SP_DOWN 0x1p-48f
 #define SP_MIN_K 256                                     // 256 x 256: 11.3 us for 12.3; K = 128: 11.3 for 10.2
 #define SP_THREADS 640                                   // warp 19 only fills up the last warpgroup
 #define SP_W_BYTES (128 * SP_BK * 4)                     // a k-block of w: two tiles of 32 columns
@@ -218,6 +223,8 @@ sgemm_split_kernel(const float* __restrict__ x, bf16* __restrict__ parts, int M,
 #pragma unroll
         for (int j = 0; j < 8; ++j) v[j] = k + j < K ? p[j] : 0.f;
     }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] *= SP_UP;
     uint4 part[3];
     s3_split8(v, part[0], part[1], part[2]);
 #pragma unroll
@@ -312,7 +319,7 @@ sgemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
 #pragma unroll
             for (int i = 0; i < CW; ++i)
                 if (mb + i < M) {
-                    yo[(size_t)i * N] = acc[i];
+                    yo[(size_t)i * N] = acc[i] * SP_DOWN;
                     odd = odd || !(fabsf(acc[i]) < inf);
                 }
             if (odd)                                     // as sgemm_tn_kernel makes it
@@ -342,8 +349,8 @@ sgemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
                 float4 v;
                 asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
                              : "r"(src + (uint32_t)(s * SP_W_BYTES + ((c ^ (row & 7)) << 4))) : "memory");
-                s3_split2(v.x, v.y, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
-                s3_split2(v.z, v.w, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
+                s3_split2(v.x * SP_UP, v.y * SP_UP, part[0][2 * c], part[1][2 * c], part[2][2 * c]);
+                s3_split2(v.z * SP_UP, v.w * SP_UP, part[0][2 * c + 1], part[1][2 * c + 1], part[2][2 * c + 1]);
             }
             __syncwarp();
             if (lane == 0) tg_arrive(&w_empty[s]);

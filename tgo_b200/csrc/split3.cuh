@@ -2,7 +2,8 @@
 // (hi + mid + lo, 8 bits each, every rest exact), a product of two such sums is nine products that the
 // tensor cores form exactly, and the three smallest of them (mid lo, lo mid, lo lo: below 2^-26 of
 // the whole) are left out. What is not finite has no such sum: hi is then infinite or NaN and the rests
-// NaN, so that the result is not finite either, which the callers look for.
+// NaN, so that the result is not finite either, which the callers look for. bfloat16 numbers end at 2^-133: what is
+// below 2^-110 keeps fewer bits of its own (it is off by 2^-134 at most), unless the caller scales it up before.
 #pragma once
 #include "tcgen.cuh"
 
