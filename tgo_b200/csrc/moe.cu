@@ -496,18 +496,18 @@ moe_down_kernel(const T* __restrict__ hidden, const T* __restrict__ wd, float* _
 // make one operand of 2 bn columns), the result act(gate) * up goes to hidden[place] in bfloat16.
 // MODE 2: the form without a gate, B is Wu[e] alone and the result act(up). MODE 0: A rows are
 // hidden[place], B is Wd[e], the result goes to y[pair] in float32.
-//   warp 0      TMA into a ring of stages: lanes 0 and 1 the B boxes; A in boxes of 32 rows where its
-//               rows lie in place order, else a lane four rows (gather4); rows past the tile's are
-//               not fetched, their sums are never stored;
+//   warps 0, 6  TMA into a ring of stages. Warp 6: the B boxes. Warp 0: A, a box for a whole tile
+//               or boxes of 32 rows where its rows lie in place order, else a lane four rows (gather4); rows
+//               past a part tile's are not fetched, their sums are never stored;
 //   warp 1      issues the products (a thread), 128 x n x 16 each, into two accumulators in turn;
 //   warps 2..5  accumulator -> activation -> staged, so that a store covers whole 64- or 128-byte
 //               pieces of rows, while the next item's products run.
 // Bound by the weights' way from memory for a few rows an expert (each read once; a stage is
 // 32 KB of them, four in flight an SM) and by the operands' way into the SM (about 70 bytes a
 // cycle) for full tiles. MEASURED (B200, 32 experts, top 4, ff 768 of width 2048, gated; mma.sync
-// tiles of 64 x 64 fed by cp.async before): 2048 tokens, up 91 us (250) and down 41 (135), 570 and
-// 620 TFLOP/s with the copy of x's rows before them 8 us; 64 tokens, from a flushed L2, 51 us (71) and 23
-// (25), 4.0 and 4.4 TB/s of weights.
+// tiles of 64 x 64 fed by cp.async before): 2048 tokens, up 76 us (250; 91 with one warp to ask for all) and down 40
+// (135), 680 and 640 TFLOP/s with the copy of x's rows before them 8 us; 64 tokens, from a flushed L2, 48 us (71)
+// and 24 (25), 4.2 TB/s of weights.
 #define MT_BK 64
 #define MT_A_BYTES (MOE_TILE * MT_BK * 2)
 #define MT_RING (192 * 1024)
