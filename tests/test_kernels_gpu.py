@@ -1354,7 +1354,7 @@ def test_retention_by_tiled_chunks_looks_forward_only(dk, dv, dtype):
                     assert torch.equal(got[:, others], clean[:, others]), (t, bad)
 
 
-def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
+def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True, d=None):
     """One request through the selective scan by chunks or in order (None: as the rule has it beyond the
     shortest steps): outputs and state."""
     T = xbc.shape[0]
@@ -1362,7 +1362,7 @@ def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True):
     y, state = torch.empty(T, H * P, device=DEV), torch.zeros(1, H * N * P, device=DEV)
     monkeypatch.setattr(o, "SSD_MIN_TOKENS", 1 << 30 if chunks is False else 1)
     launches = o.LAUNCHES[0]
-    o.selective_scan(xbc, dt_raw, None, a_log, None, y, 1, H, G, N, P, i32([0, T]), i32([0]), state, 0)
+    o.selective_scan(xbc, dt_raw, None, a_log, d, y, 1, H, G, N, P, i32([0, T]), i32([0]), state, 0)
     assert chunks is None or o.LAUNCHES[0] == launches + (4 if chunks else 1)
     return y, state
 
@@ -1386,6 +1386,40 @@ def test_selective_scan_by_chunks_heads_a_block(H, G, N, P, T, monkeypatch):
         want[t] = torch.einsum("hn,hnp->hp", C[t], S)
     assert (y.view(T, H, P).double() - want).norm() <= 1e-6 * want.norm()
     assert (state.view(H, N, P).double() - S).norm() <= 1e-6 * S.norm()
+    assert o.ssd_error() == 0
+
+
+@pytest.mark.parametrize("N", [64, 128])
+@pytest.mark.parametrize("P", [64, 128])
+def test_selective_scan_by_chunks_pairs_in_turn(N, P, monkeypatch):
+    """Blocks of five heads, which are three turns of 128 channels (the last half full) or five, with x beside the sums,
+    against the recurrence in 64 bits; what is not finite in a last turn stays there."""
+    o, H, G, T = ops(), 40, 2, 1500
+    # 24 chunks: five heads a block are 192 blocks, ten would be 96, fewer than the multiprocessors there are
+    assert 24 * 8 >= torch.cuda.get_device_properties(0).multi_processor_count > 24 * 4
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log, d = torch.linspace(-2.0, 1.0, H, device=DEV), rnd(H, seed=5)
+    run = lambda x: chunked_scan(o, monkeypatch, x, dt_raw, a_log, H, G, N, P, d=d)      # noqa: E731
+    y, state = run(xbc)
+    x, B, C = (z.double() for z in xbc.split([H * P, G * N, G * N], 1))
+    B, C = (z.view(T, G, N).repeat_interleave(H // G, 1) for z in (B, C))
+    dt, S = torch.nn.functional.softplus(dt_raw.double()), torch.zeros(H, N, P, dtype=torch.float64, device=DEV)
+    want = torch.empty(T, H, P, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S = torch.exp(-torch.exp(a_log.double()) * dt[t])[:, None, None] * S + \
+            (dt[t][:, None] * B[t])[:, :, None] * x[t].view(H, 1, P)
+        want[t] = torch.einsum("hn,hnp->hp", C[t], S) + d.double()[:, None] * x[t].view(H, P)
+    # for each head, so that none hides behind the others: sums of N + 64 float32 terms behind at most 24 chunks
+    assert bool(((y.view(T, H, P).double() - want).norm(dim=(0, 2)) <= 1e-6 * want.norm(dim=(0, 2))).all())
+    assert bool(((state.view(H, N, P).double() - S).norm(dim=(1, 2)) <= 1e-6 * S.norm(dim=(1, 2))).all())
+    for t, head in ((0, 4), (70, 3), (1499, 39)):
+        for bad in (float("nan"), float("inf")):
+            z = xbc.clone()
+            z[t, head * P + 9] = bad
+            got, _ = run(z)
+            others = [c for c in range(H * P) if c != head * P + 9]
+            assert torch.equal(got[:t], y[:t]) and torch.equal(got[:, others], y[:, others])
+            assert not bool(torch.isfinite(got[t, head * P + 9]))
     assert o.ssd_error() == 0
 
 

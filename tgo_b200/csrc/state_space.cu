@@ -773,10 +773,12 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
     unsigned char* sR = sB + sd_a_bytes<N, P>();         // [2]
     __shared__ double ls[SD_HEADS][SD_CHUNK];
     __shared__ float ds[SD_HEADS][SD_CHUNK], el[SD_HEADS][SD_CHUNK];
-    __shared__ __align__(8) uint64_t bars[12];
+    __shared__ __align__(8) uint64_t bars[13];
     __shared__ uint32_t tmem_slot;
-    uint64_t *cb_full = bars, *s_done = bars + 1, *r_full = bars + 2 /* [2] */, *r_done = bars + 4 /* [2] */, *y_done = bars + 6;
-    uint64_t *a_full = bars + 7, *y_free = bars + 8 /* [2] */, *settled = bars + 10, *a_done = bars + 11;
+    uint64_t *cb_full = bars, *s_done = bars + 1, *r_full = bars + 2 /* [2] */, *r_done = bars + 4 /* [2] */;
+    // y_done, one a buffer: a warp hands over A of pair q before it waits for the products of pair q - 1, so that those
+    // of q may be made first; the next phase of the same barrier, pair q + 1's, needs the warp's y_free of q - 1.
+    uint64_t *y_done = bars + 6 /* [2] */, *a_full = bars + 8, *y_free = bars + 9 /* [2] */, *settled = bars + 11, *a_done = bars + 12;
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
     const int n = ch.y, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -790,9 +792,8 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
     if (threadIdx.x == 0) {
         tg_init(cb_full, SD_THREADS / 32);
         tg_init(s_done, 1);
-        for (int i = 0; i < 2; ++i) { tg_init(&r_full[i], SD_HALF / 32); tg_init(&r_done[i], 1); tg_init(&y_free[i], SD_HALF / 32); }
+        for (int i = 0; i < 2; ++i) { tg_init(&r_full[i], SD_HALF / 32); tg_init(&r_done[i], 1); tg_init(&y_done[i], 1); tg_init(&y_free[i], SD_HALF / 32); }
         tg_init(a_full, SD_HALF / 32);
-        tg_init(y_done, 1);
         tg_init(a_done, 1);
         tg_init(settled, 1);
         tg_init_done();
@@ -841,7 +842,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                                                  tg_desc(sA + 3 * e * SD_TILE), SD_TILE >> 4, 2, tg_idesc(64, false, true), false);
                     tg_commit(&r_done[stage & 1]);
                     if (x == 1) tg_commit(a_done);
-                    if (x == STAGES - 1) tg_commit(y_done);
+                    if (x == STAGES - 1) tg_commit(&y_done[q & 1]);
                 }
                 __syncwarp();
             }
@@ -951,7 +952,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                 }
                 if (q > 0) {
                     const int d = q - 1, row = (warp & 3) * 32 + lane, l = d * HP + row / P, i0 = (warp >> 2 & 1) * 32;
-                    ok = sd_wait(y_done, d & 1, 5);
+                    ok = sd_wait(&y_done[d & 1], (d >> 1) & 1, 5);
                     if (!ok) break;
                     const uint32_t t = tmem + lanes + 256u * (d & 1) + (uint32_t)i0;
                     float* dst = y + (size_t)(ch.x + i0) * H * P + (h0 + l) * P + row % P;
