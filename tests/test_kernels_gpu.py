@@ -1354,6 +1354,38 @@ def test_retention_by_tiled_chunks_looks_forward_only(dk, dv, dtype):
                     assert torch.equal(got[:, others], clean[:, others]), (t, bad)
 
 
+def retention_of_one(z, H, dk, dv, decay, k_scale, state):
+    """One request through the chunked retention, its rows [q, k, v]: outputs [n, H, dv]; `state` [1, H, dk, dv] moves on."""
+    o, n = ops(), z.shape[0]
+    i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
+    C, out = o.retention_chunk_tokens(), torch.full((n, H * dv), float("nan"), device=DEV)
+    o.retention_chunked(z[:, :H * dk], z[:, H * dk:2 * H * dk], z[:, 2 * H * dk:], out, 1, H, dk, dv,
+                        torch.tensor(decay, device=DEV), k_scale, None, 0, i32([0, n]), i32([0]), state,
+                        i32(list(range(0, n, C))), i32([min(C, n - a) for a in range(0, n, C)]), i32([0]))
+    assert o.retention_error() == 0
+    return out.view(n, H, dv)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_retention_by_chunks_of_large_scores(dtype):
+    """A score near the end of the range whose second half of channels is past it alone: the sum over all channels is
+    finite in the order of the channels, and so is its share of the output. Rows before are as they are without it."""
+    H, dk, dv, n, key, query = 2, 128, 136, 100, 70, 75
+    z = (rnd(n, H * (2 * dk + dv), seed=4) * 0.5).to(dtype)
+    at = [0, 64, 65]
+    for t in range(n):                                   # the three channels are the two tokens' own, in head 0
+        z[t, at], z[t, [dk * H + c for c in at]] = 0.0, 0.0
+    clean = retention_of_one(z, H, dk, dv, [1.0, 0.9], 1.0, torch.zeros(1, H, dk, dv, device=DEV))
+    z[query, :dk], z[key, H * dk:H * dk + dk], z[key, 2 * H * dk:2 * H * dk + dv] = 0.0, 0.0, 1e-30
+    for i, c in enumerate(at):
+        z[query, c], z[key, H * dk + c] = 1.7e19, -1.7e19 if i == 0 else 1.7e19
+    got = retention_of_one(z, H, dk, dv, [1.0, 0.9], 1.0, torch.zeros(1, H, dk, dv, device=DEV))
+    assert torch.equal(got[:key], clean[:key]) and torch.equal(got[:, 1], clean[:, 1])
+    q, k, v = z[query, :dk].double(), z[key, H * dk:H * dk + dk].double(), z[key, 2 * H * dk:2 * H * dk + dv].double()
+    want = (q @ k) * v                                   # 2.9e8; the channels meet no other key
+    assert bool(((got[query, 0].double() - want).abs() <= 1e-6 * want).all()), (got[query, 0, :4], want[:4])
+
+
 def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True, d=None):
     """One request through the selective scan by chunks or in order (None: as the rule has it beyond the
     shortest steps): outputs and state."""
@@ -1448,6 +1480,34 @@ def test_selective_scan_by_chunks_looks_forward_only(H, G, N, P, monkeypatch):
         got, _ = chunked_scan(o, monkeypatch, xbc, y, a_log, H, G, N, P)
         assert torch.equal(got[:t], clean[:t]) and torch.equal(got[:, P:], clean[:, P:])
         assert bool(torch.isnan(got[t:, :P]).all())
+
+
+@pytest.mark.parametrize("N,P", [(64, 64), (128, 64), (64, 128), (128, 128)])
+def test_selective_scan_by_chunks_of_large_factors(N, P, monkeypatch):
+    """B, C, dt, D and x whose product is finite though C . B times dt, or with D on top, is past the range: the walk's result.
+    Rows before are as they are without it, and so is the other head."""
+    o, H, T, key, query, diag = ops(), 2, 100, 70, 73, 80
+    xbc, dt_raw = rnd(T, H * P + 2 * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log, d = torch.full((H,), -6.0, device=DEV), torch.tensor([3.3e38, 1.0], device=DEV)
+    b, c = H * P, H * P + N
+    xbc[:, b] = xbc[:, c] = xbc[:, b + 1] = xbc[:, c + 1] = 0.0
+    xbc[:, :P] = 1e-30
+    y0, _ = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, 1, N, P, d=d)
+    for t, lane, small in ((key, 0, 1e19), (query, 0, 1e19), (diag, 1, 6e18)):
+        if t != query:
+            xbc[t, b:b + N] = 0.0
+            xbc[t, b + lane] = small
+        if t != key:
+            xbc[t, c:c + N] = 0.0
+            xbc[t, c + lane] = small
+    dt_raw[key, 0], dt_raw[diag, 0] = 10.0, 0.5
+    args = (o, monkeypatch, xbc, dt_raw, a_log, H, 1, N, P)
+    got, state = chunked_scan(*args, d=d)
+    want, state2 = chunked_scan(*args, chunks=False, d=d)
+    assert bool(torch.isfinite(want).all()) and want[query, 0] > 1e9 and want[diag, 0] > 3.6e8
+    assert bool(((got - want).abs() <= 1e-5 * want.abs())[[query, diag], :P].all()), (got[query, :3], want[query, :3])
+    assert torch.equal(got[:key], y0[:key]) and (state - state2).norm() <= 6e-6 * state2.norm()
+    assert bool(((got - want)[:, P:].norm(dim=1) <= 1e-4 * want[:, P:].norm(dim=1)).all()) and o.ssd_error() == 0
 
 
 @pytest.mark.parametrize("H,G,N,P", [(6, 3, 128, 64), (3, 1, 64, 128)])

@@ -498,7 +498,10 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 //               sixteen lay the next operands down. (One slice a block, halves of Q, K and P one after the
 //               other, two blocks an SM: 167 us.)
 // Zeros of A times a value that is not finite are not zero: such a number is laid down as 0, which leaves what does
-// not depend on it as it is, bit for bit, and a block that met one makes plain sums too and writes those that are not finite.
+// not depend on it as it is, bit for bit, and a block that met one makes plain sums too (a thread a sum, out of global
+// memory) and writes those that are not finite. An A that is not finite without that, because Q K^T is too large, is 0 there too:
+// the plain sums of its row and the rows after it are written whatever they are. So are those in the place of a result
+// that the products made overflow.
 // MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
 // summaries 50 us (122), scan 40, outputs 119 us (190). The summaries are bound by the bytes of U; a block of the outputs
 // by its chain: loads 5000 cycles, parts of Q and K 3000, 168 products of 75 cycles, results 2300.
@@ -707,10 +710,13 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
                 float* dst = Uo + (size_t)(d0 + x) * dv + c;
                 if (c < dv)
 #pragma unroll
-                    for (int i = 0; i < 32; ++i, dst += dv) *dst = __uint_as_float(r[i]);
+                    for (int i = 0; i < 32; ++i, dst += dv) {
+                        odd = odd || rf_not_finite(__uint_as_float(r[i]));
+                        *dst = __uint_as_float(r[i]);
+                    }
             }
         }
-        if (odd) {
+        if (__syncthreads_or(odd)) {
             float* Kf = (float*)base;
             load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
             __syncthreads();
@@ -720,7 +726,8 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
                 float s = 0.f;
                 for (int j = 0; j < n; ++j)
                     s = fmaf(Kf[j * RF_LOOP_LD + d] * pw[n - 1 - j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
-                if (rf_not_finite(s)) Uo[(size_t)d * dv + c] = s;
+                float* to = Uo + (size_t)d * dv + c;
+                if (rf_not_finite(s) || rf_not_finite(*to)) *to = s;
             }
         }
     } else {
@@ -800,12 +807,14 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     __shared__ float pw[RC_CHUNK + 1];
     __shared__ __align__(8) uint64_t bars[9];
     __shared__ uint32_t tmem_slot;
+    __shared__ int plain_from;                           // the first row whose plain sums are written whatever they are
     uint64_t *s_done = bars, *p_done = bars + 1 /* [2] */, *v_done = bars + 3;
     uint64_t *qk_full = bars + 4, *p_full = bars + 5 /* [2] */, *a_full = bars + 7, *v_full = bars + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) tg_alloc512(&tmem_slot);
     if (threadIdx.x == 0) {
         for (int i = 0; i < 9; ++i) tg_init(&bars[i], i < 4 ? 1 : THREADS / 32);
+        plain_from = RC_CHUNK;
         tg_init_done();
     }
     pdl_wait();
@@ -942,7 +951,10 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                         const float s = __uint_as_float(s0[8 * y + x]) + (HALVES > 1 ? __uint_as_float(s1[8 * y + x]) : 0.f);
                         f[x] = gap >= 0 ? s * pw[gap >= 0 ? gap : 0] : 0.f;
                     }
-                    odd = rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f) || odd;
+                    if (rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f)) {
+                        atomicMin(&plain_from, i);
+                        odd = true;
+                    }
                 }
             }
             odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act) || odd;
@@ -972,7 +984,9 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                     for (int i = 0; i < 16; ++i, dst += (size_t)H * dv)
                         if (i0 + i < n) {
                             const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
-                            *dst = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
+                            const float sum = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
+                            odd = odd || rf_not_finite(sum);
+                            *dst = sum;
                         }
             }
         }
@@ -1003,7 +1017,8 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
             s *= pw[i + 1];
             for (int j = 0; j <= i; ++j)
                 s = fmaf(Af[i * (RC_CHUNK + 1) + j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
-            if (rf_not_finite(s)) out[((size_t)(tok0 + i) * H + h) * dv + c] = s;
+            float* to = out + ((size_t)(tok0 + i) * H + h) * dv + c;
+            if (i >= plain_from || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
         }
     }
     tg_before();

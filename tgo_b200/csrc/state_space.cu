@@ -503,7 +503,9 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
 // its diagonal, so that x goes in as it is and nothing is read for the results. Bound by the chains of conversions (about 2500
 // cycles a stage of 64 x 128 numbers for eight warps) and not by the products, 50 cycles each. Zeros of A times a value that is not finite are not
 // zero: such a number is laid down as 0, which leaves what does not depend on it as it is, bit for bit, and a
-// block that met one makes plain sums too and writes those that are not finite.
+// block that met one makes plain sums too (a thread a sum, out of global memory) and writes those that are not finite. An
+// A that is not finite without that, because C . B or its product with dt is too large, is 0 there too: the plain sums of its row
+// and the rows after it are written whatever they are. So are those in the place of a result that the products made overflow.
 #define SD_THREADS 512
 #define SD_HALF 256                   // of the outputs: one half lays the states and values down, the other A
 #define SD_HEADS 16                   // heads a block takes at most
@@ -679,7 +681,11 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
                     tg_wait_ld();
                     if (ok && l < hb)
 #pragma unroll
-                        for (int i = 0; i < 16; ++i) dst[i * P] = __uint_as_float(r0[i]) + __uint_as_float(r1[i]);
+                        for (int i = 0; i < 16; ++i) {
+                            const float sum = __uint_as_float(r0[i]) + __uint_as_float(r1[i]);
+                            odd = odd || sd_not_finite(sum);
+                            dst[i * P] = sum;
+                        }
                 }
                 tg_before();                             // before the next products into this buffer
             }
@@ -694,7 +700,8 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
             float sum = 0.f;
             for (int j = 0; j < n; ++j)
                 sum = fmaf(br[(size_t)j * C + m], rows[(size_t)j * C + (h0 + l) * P + c] * (dts[o + j] * expf((float)(cum[o + n - 1] - cum[o + j]))), sum);
-            if (sd_not_finite(sum)) U[((at + l) * N + m) * P + c] = sum;
+            float* to = U + ((at + l) * N + m) * P + c;
+            if (sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
         }
     }
     tg_before();
@@ -773,6 +780,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
     unsigned char* sR = sB + sd_a_bytes<N, P>();         // [2]
     __shared__ double ls[SD_HEADS][SD_CHUNK];
     __shared__ float ds[SD_HEADS][SD_CHUNK], el[SD_HEADS][SD_CHUNK];
+    __shared__ int plain_from[SD_HEADS];                 // a head's first row whose plain sums are written whatever they are
     __shared__ __align__(8) uint64_t bars[13];
     __shared__ uint32_t tmem_slot;
     uint64_t *cb_full = bars, *s_done = bars + 1, *r_full = bars + 2 /* [2] */, *r_done = bars + 4 /* [2] */;
@@ -798,6 +806,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
         tg_init(settled, 1);
         tg_init_done();
     }
+    if (threadIdx.x < SD_HEADS) plain_from[threadIdx.x] = SD_CHUNK;
     for (int i = threadIdx.x; i < hb * SD_CHUNK; i += SD_THREADS + 32) {
         const double l = cum[at * SD_CHUNK + i];
         (&ls[0][0])[i] = l;
@@ -946,7 +955,10 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                         }
                         const uint32_t tile = tg_smem(sA) + (uint32_t)(3 * e * SD_TILE);
                         const uint32_t dst[2] = {tile + s3_place(ai, aj / 8), tile + s3_place(ai, aj / 8 + 4)};
-                        odd = s3_put<2>(f, dst, SD_TILE) || odd;
+                        if (s3_put<2>(f, dst, SD_TILE)) {
+                            atomicMin(&plain_from[q * HP + e], ai);
+                            odd = true;
+                        }
                     }
                     sd_full(a_full);
                 }
@@ -968,7 +980,9 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                             for (int i = 0; i < 16; ++i)
                                 if (i0 + c + i < n) {
                                     const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
-                                    dst[(size_t)(c + i) * H * P] = fmaf(far, el[l][i0 + c + i], __uint_as_float(a[i]));
+                                    const float sum = fmaf(far, el[l][i0 + c + i], __uint_as_float(a[i]));
+                                    odd = odd || sd_not_finite(sum);
+                                    dst[(size_t)(c + i) * H * P] = sum;
                                 }
                     }
                     sd_full(&y_free[d & 1]);
@@ -997,7 +1011,8 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                 sum = fmaf(Sf[i * (SD_CHUNK + 1) + j] * expf((float)(cum[o + i] - cum[o + j])),
                            dts[o + j] * rows[(size_t)j * C + (h0 + l) * P + c], sum);
             sum = fmaf(D ? D[h0 + l] : 0.f, rows[(size_t)i * C + (h0 + l) * P + c], sum);
-            if (sd_not_finite(sum)) y[(size_t)(ch.x + i) * H * P + (h0 + l) * P + c] = sum;
+            float* to = y + (size_t)(ch.x + i) * H * P + (h0 + l) * P + c;
+            if (i >= plain_from[l] || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
         }
     }
     tg_before();
