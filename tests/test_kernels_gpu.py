@@ -1386,6 +1386,44 @@ def test_retention_by_chunks_of_large_scores(dtype):
     assert bool(((got[query, 0].double() - want).abs() <= 1e-6 * want).all()), (got[query, 0, :4], want[:4])
 
 
+@pytest.mark.parametrize("dk,dv", [(64, 64), (128, 136)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("qs,ks,vs,ss", [(1.0, 1.0, 1e-36, 1e-36), (1e-36, 1.0, 1.0, 1.0), (1.0, 1e-36, 1.0, 1e-36), (1e-20, 1e-16, 1.0, 1e-16),
+                                         (1e33, 1e-30, 1.0, 1e-30), (1e-30, 1e33, 1.0, 1e30), (1.0, 1e-30, 1e33, 1e5), (1e-30, 1.0, 1.0, 1e34)])
+def test_retention_by_chunks_of_small_and_large_numbers(dk, dv, dtype, qs, ks, vs, ss):
+    """Numbers whose lower parts have no bfloat16 number of their size, scores of such a size, and numbers past those that
+    the parts are scaled for, against the recurrence in 64 bits: the bound of ordinary numbers."""
+    H, n, decay = 2, 130, [0.9, 1.0]
+    z = rnd(n, H * (2 * dk + dv), seed=dk).to(dtype)
+    z[:, :H * dk] *= qs
+    z[:, H * dk:2 * H * dk] *= ks
+    z[:, 2 * H * dk:] *= vs
+    state = rnd(1, H, dk, dv, seed=1) * ss
+    S, want = state[0].double(), torch.empty(n, H, dv, dtype=torch.float64, device=DEV)
+    q, k, v = (x.double().view(n, H, -1) for x in z.split([H * dk, H * dk, H * dv], 1))
+    for t in range(n):
+        S = torch.tensor(decay, dtype=torch.float64, device=DEV)[:, None, None] * S + k[t][:, :, None] * v[t][:, None]
+        want[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    got = retention_of_one(z, H, dk, dv, decay, 1.0, state).double()
+    for h in range(H):
+        assert (got[:, h] - want[:, h]).norm() <= 1e-6 * want[:, h].norm()
+        # a state that is mostly the one before, n powers of the decay later, has a rounding of each of them on top
+        assert (state[0, h].double() - S[h]).norm() <= (1e-6 + n * 2.0 ** -24) * S[h].norm()
+
+
+def scan_in_64_bits(xbc, dt_raw, a_log, d, H, G, N, P):
+    T = xbc.shape[0]
+    x, B, C = (z.double() for z in xbc.split([H * P, G * N, G * N], 1))
+    B, C = (z.view(T, G, N).repeat_interleave(H // G, 1) for z in (B, C))
+    dt, S = torch.nn.functional.softplus(dt_raw.double()), torch.zeros(H, N, P, dtype=torch.float64, device=DEV)
+    want = torch.empty(T, H, P, dtype=torch.float64, device=DEV)
+    for t in range(T):
+        S = torch.exp(-torch.exp(a_log.double()) * dt[t])[:, None, None] * S + \
+            (dt[t][:, None] * B[t])[:, :, None] * x[t].view(H, 1, P)
+        want[t] = torch.einsum("hn,hnp->hp", C[t], S) + (0.0 if d is None else d.double()[:, None] * x[t].view(H, P))
+    return want, S
+
+
 def chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=True, d=None):
     """One request through the selective scan by chunks or in order (None: as the rule has it beyond the
     shortest steps): outputs and state."""
@@ -1433,14 +1471,7 @@ def test_selective_scan_by_chunks_pairs_in_turn(N, P, monkeypatch):
     a_log, d = torch.linspace(-2.0, 1.0, H, device=DEV), rnd(H, seed=5)
     run = lambda x: chunked_scan(o, monkeypatch, x, dt_raw, a_log, H, G, N, P, d=d)      # noqa: E731
     y, state = run(xbc)
-    x, B, C = (z.double() for z in xbc.split([H * P, G * N, G * N], 1))
-    B, C = (z.view(T, G, N).repeat_interleave(H // G, 1) for z in (B, C))
-    dt, S = torch.nn.functional.softplus(dt_raw.double()), torch.zeros(H, N, P, dtype=torch.float64, device=DEV)
-    want = torch.empty(T, H, P, dtype=torch.float64, device=DEV)
-    for t in range(T):
-        S = torch.exp(-torch.exp(a_log.double()) * dt[t])[:, None, None] * S + \
-            (dt[t][:, None] * B[t])[:, :, None] * x[t].view(H, 1, P)
-        want[t] = torch.einsum("hn,hnp->hp", C[t], S) + d.double()[:, None] * x[t].view(H, P)
+    want, S = scan_in_64_bits(xbc, dt_raw, a_log, d, H, G, N, P)
     # for each head, so that none hides behind the others: sums of N + 64 float32 terms behind at most 24 chunks
     assert bool(((y.view(T, H, P).double() - want).norm(dim=(0, 2)) <= 1e-6 * want.norm(dim=(0, 2))).all())
     assert bool(((state.view(H, N, P).double() - S).norm(dim=(1, 2)) <= 1e-6 * S.norm(dim=(1, 2))).all())
@@ -1480,6 +1511,25 @@ def test_selective_scan_by_chunks_looks_forward_only(H, G, N, P, monkeypatch):
         got, _ = chunked_scan(o, monkeypatch, xbc, y, a_log, H, G, N, P)
         assert torch.equal(got[:t], clean[:t]) and torch.equal(got[:, P:], clean[:, P:])
         assert bool(torch.isnan(got[t:, :P]).all())
+
+
+@pytest.mark.parametrize("N,P", [(64, 64), (128, 64), (64, 128), (128, 128)])
+@pytest.mark.parametrize("xs,bs,cs", [(1e-36, 1.0, 1.0), (1.0, 1e-36, 1.0), (1.0, 1.0, 1e-36), (1.0, 1e-20, 1e-16), (1e33, 1e-20, 1.0),
+                                      (1e-20, 1e33, 1.0), (1e-20, 1.0, 1e33)])
+def test_selective_scan_by_chunks_of_small_and_large_numbers(N, P, xs, bs, cs, monkeypatch):
+    """Numbers whose lower parts have no bfloat16 number of their size, and numbers past those that the parts are scaled
+    for, in x, B and C and so in the states, against the recurrence in 64 bits: the bound of ordinary numbers."""
+    H, T = 3, 150
+    xbc, dt_raw = rnd(T, H * P + 2 * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    for at, size, scale in ((0, H * P, xs), (H * P, N, bs), (H * P + N, N, cs)):
+        xbc[:, at:at + size] *= scale
+    a_log = torch.linspace(-3.0, 0.0, H, device=DEV)
+    want, S = scan_in_64_bits(xbc, dt_raw, a_log, None, H, 1, N, P)
+    y, state = chunked_scan(ops(), monkeypatch, xbc, dt_raw, a_log, H, 1, N, P)
+    assert ops().ssd_error() == 0
+    y, state = y.view(T, H, P).double(), state.view(H, N, P).double()
+    for h in range(H):
+        assert (y[:, h] - want[:, h]).norm() <= 1e-6 * want[:, h].norm() and (state[h] - S[h]).norm() <= 1e-6 * S[h].norm()
 
 
 @pytest.mark.parametrize("N,P", [(64, 64), (128, 64), (64, 128), (128, 128)])

@@ -499,9 +499,9 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 //               other, two blocks an SM: 167 us.)
 // Zeros of A times a value that is not finite are not zero: such a number is laid down as 0, which leaves what does
 // not depend on it as it is, bit for bit, and a block that met one makes plain sums too (a thread a sum, out of global
-// memory) and writes those that are not finite. An A that is not finite without that, because Q K^T is too large, is 0 there too:
-// the plain sums of its row and the rows after it are written whatever they are. So are those in the place of a result
-// that the products made overflow.
+// memory) and writes those that are not finite. A finite number too large for its parts (2^103 and more), or an A whose
+// Q K^T is (2^80), is 0 there too: the plain sums of its row and the rows after it are written whatever they are, in its slice if it
+// is one of V or P. So are those in the place of a result that the products made overflow.
 // MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
 // summaries 50 us (122), scan 40, outputs 119 us (190). The summaries are bound by the bytes of U; a block of the outputs
 // by its chain: loads 5000 cycles, parts of Q and K 3000, 168 products of 75 cycles, results 2300.
@@ -595,7 +595,7 @@ __device__ __forceinline__ void rf_ask_v(Raw8<T> (&raw)[rf_v_runs<THREADS>()], c
     }
 }
 template <typename T, int VP, int THREADS>
-__device__ __forceinline__ bool rf_put_v(uint32_t tile, const Raw8<T> (&raw)[rf_v_runs<THREADS>()], int dv, int c0, int n, int act) {
+__device__ __forceinline__ bool rf_put_v(uint32_t tile, const Raw8<T> (&raw)[rf_v_runs<THREADS>()], int dv, int c0, int n, int act, int* too_large) {
     bool odd = false;
 #pragma unroll
     for (int j = 0; j < rf_v_runs<THREADS>(); ++j) {
@@ -609,14 +609,14 @@ __device__ __forceinline__ bool rf_put_v(uint32_t tile, const Raw8<T> (&raw)[rf_
         } else {
             float f[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
             if (ok) taken8(raw[j], act, f);
-            odd = s3_put8(f, dst, 2 * RF_TILE) || odd;
+            odd = s3_put8(f, dst, 2 * RF_TILE, r, too_large) || odd;
         }
     }
     return odd;
 }
-// The parts of eight numbers to their place in three tiles `step` bytes apart.
-__device__ __forceinline__ bool rf_put8(uint32_t tile, uint32_t step, int row, int piece, const float (&f)[8]) {
-    return s3_put8(f, tile + s3_place(row, piece), step);
+// The parts of eight numbers to their place in three tiles `step` bytes apart; `from`: the first row that what is too large counts for.
+__device__ __forceinline__ bool rf_put8(uint32_t tile, uint32_t step, int row, int piece, const float (&f)[8], int from, int* too_large) {
+    return s3_put8(f, tile + s3_place(row, piece), step, from, too_large);
 }
 // The value of column c of a token, as the plain sums take it.
 template <typename T>
@@ -645,9 +645,11 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
     __shared__ float pw[RC_CHUNK + 1];
     __shared__ __align__(8) uint64_t bars[2];            // one a slice
     __shared__ uint32_t tmem_slot;
+    __shared__ int too_large[3];                         // either slice's V; K
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) tg_alloc<2 * DK>(&tmem_slot);
     if (threadIdx.x == 0) { tg_init(&bars[0], 1); tg_init(&bars[1], 1); tg_init_done(); }
+    if (threadIdx.x < 3) too_large[threadIdx.x] = RC_CHUNK;
     pdl_wait();
     const int ci = blockIdx.x, h = blockIdx.y, first = blockIdx.z * slices * RF_SLICE;
     const int n = chunk_ntok[ci], tok0 = n > 0 ? chunk_tok0[ci] : 0;      // rows past n read the first one
@@ -679,12 +681,12 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
             f[x] = r < n ? f[x] * k_scale * w : 0.f;
             g[x] = r < n ? g[x] * k_scale * w : 0.f;
         }
-        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].lo / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].lo / 8) & 7, f) || odd;
-        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].hi / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].hi / 8) & 7, g) || odd;
+        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].lo / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].lo / 8) & 7, f, r, &too_large[2]) || odd;
+        odd = rf_put8(tg_smem(base) + (uint32_t)(kr[j].hi / 64 * RF_TILE), KB * RF_TILE, r, (kr[j].hi / 8) & 7, g, r, &too_large[2]) || odd;
     }
     for (int s = 0; s < ns; ++s) {
         unsigned char* sv = sV + s * 2 * VP * RF_TILE;
-        odd = rf_put_v<T, VP, RC_THREADS>(tg_smem(sv), vr, dv, first + s * RF_SLICE, n, act) || odd;
+        odd = rf_put_v<T, VP, RC_THREADS>(tg_smem(sv), vr, dv, first + s * RF_SLICE, n, act, &too_large[s]) || odd;
         if (s + 1 < ns) rf_ask_v<T, RC_THREADS>(vr, v, v_stride, h, dv, first + (s + 1) * RF_SLICE, tok0, n);
         s3_fence();
         odd = __syncthreads_or(odd);
@@ -711,8 +713,9 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
                 if (c < dv)
 #pragma unroll
                     for (int i = 0; i < 32; ++i, dst += dv) {
-                        odd = odd || rf_not_finite(__uint_as_float(r[i]));
-                        *dst = __uint_as_float(r[i]);
+                        const float sum = __uint_as_float(r[i]) * (VP == 1 ? S3_DOWN : S3_DOWN * S3_DOWN);
+                        odd = odd || rf_not_finite(sum);
+                        *dst = sum;
                     }
             }
         }
@@ -727,7 +730,8 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
                 for (int j = 0; j < n; ++j)
                     s = fmaf(Kf[j * RF_LOOP_LD + d] * pw[n - 1 - j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
                 float* to = Uo + (size_t)d * dv + c;
-                if (rf_not_finite(s) || rf_not_finite(*to)) *to = s;
+                const bool plain = min(too_large[(c - first) / RF_SLICE], too_large[2]) < RC_CHUNK;
+                if (plain || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
             }
         }
     } else {
@@ -807,14 +811,14 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     __shared__ float pw[RC_CHUNK + 1];
     __shared__ __align__(8) uint64_t bars[9];
     __shared__ uint32_t tmem_slot;
-    __shared__ int plain_from;                           // the first row whose plain sums are written whatever they are
+    __shared__ int plain_from[3];                        // the first row whose plain sums are written whatever they are: a slice's; both
     uint64_t *s_done = bars, *p_done = bars + 1 /* [2] */, *v_done = bars + 3;
     uint64_t *qk_full = bars + 4, *p_full = bars + 5 /* [2] */, *a_full = bars + 7, *v_full = bars + 8;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (warp == 0) tg_alloc512(&tmem_slot);
     if (threadIdx.x == 0) {
         for (int i = 0; i < 9; ++i) tg_init(&bars[i], i < 4 ? 1 : THREADS / 32);
-        plain_from = RC_CHUNK;
+        plain_from[0] = plain_from[1] = plain_from[2] = RC_CHUNK;
         tg_init_done();
     }
     pdl_wait();
@@ -909,8 +913,8 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
 #pragma unroll
                 for (int x = 0; x < 8; ++x) { f[x] = r >= n ? 0.f : f[x] * w; g[x] = r >= n ? 0.f : g[x] * w; }
             const uint32_t tile = tg_smem(key ? sK : sQ);
-            odd = rf_put8(tile + (uint32_t)(run[j].lo / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].lo / 8) & 7, f) || odd;
-            odd = rf_put8(tile + (uint32_t)(run[j].hi / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].hi / 8) & 7, g) || odd;
+            odd = rf_put8(tile + (uint32_t)(run[j].lo / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].lo / 8) & 7, f, r, &plain_from[2]) || odd;
+            odd = rf_put8(tile + (uint32_t)(run[j].hi / 64 * RF_TILE), HALVES * RF_TILE, r, (run[j].hi / 8) & 7, g, r, &plain_from[2]) || odd;
         }
         full(qk_full);
         Raw8<T> vr[rf_v_runs<THREADS>()];
@@ -926,7 +930,7 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                 if (first + stage / HALVES * RF_SLICE + piece * 8 >= dv)
 #pragma unroll
                     for (int x = 0; x < 8; ++x) f[x] = 0.f;
-                odd = rf_put8(tg_smem(buf) + (uint32_t)((piece >> 3) * RF_TILE), 2 * RF_TILE, d, piece & 7, f) || odd;
+                odd = rf_put8(tg_smem(buf) + (uint32_t)((piece >> 3) * RF_TILE), 2 * RF_TILE, d, piece & 7, f, 0, &plain_from[stage / HALVES]) || odd;
             }
             if (stage + 1 < stages) ask_p(stage + 1);
             if (stage == HALVES - 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first, tok0, n);
@@ -949,22 +953,22 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                     for (int x = 0; x < 8; ++x) {
                         const int gap = i - (j0 + 8 * y + x);
                         const float s = __uint_as_float(s0[8 * y + x]) + (HALVES > 1 ? __uint_as_float(s1[8 * y + x]) : 0.f);
-                        f[x] = gap >= 0 ? s * pw[gap >= 0 ? gap : 0] : 0.f;
+                        f[x] = gap >= 0 ? s * (S3_DOWN * S3_DOWN) * pw[gap >= 0 ? gap : 0] : 0.f;
                     }
-                    if (rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f)) {
-                        atomicMin(&plain_from, i);
+                    if (rf_put8(tg_smem(sA), RF_TILE, i, (j0 >> 3) + y, f, i, &plain_from[2])) {
+                        atomicMin(&plain_from[2], i);
                         odd = true;
                     }
                 }
             }
-            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act) || odd;
+            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first, n, act, &plain_from[0]) || odd;
             if (ns > 1) rf_ask_v<T, THREADS>(vr, v, v_stride, h, dv, first + RF_SLICE, tok0, n);
             full(a_full);
         }
         if (ok) ok = __all_sync(0xffffffffu, tg_wait(v_done, 0, &retention_error_flag, 3));      // and with it all that was issued before
         tg_after();
         if (ok && ns > 1) {
-            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first + RF_SLICE, n, act) || odd;
+            odd = rf_put_v<T, VP, THREADS>(tg_smem(sV), vr, dv, first + RF_SLICE, n, act, &plain_from[1]) || odd;
             full(v_full);
         }
         if (ok) {
@@ -984,7 +988,8 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                     for (int i = 0; i < 16; ++i, dst += (size_t)H * dv)
                         if (i0 + i < n) {
                             const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
-                            const float sum = fmaf(far, pw[i0 + i + 1], __uint_as_float(a[i]));
+                            const float sum = fmaf(far * (S3_DOWN * S3_DOWN), pw[i0 + i + 1],
+                                                   __uint_as_float(a[i]) * (VP == 1 ? S3_DOWN : S3_DOWN * S3_DOWN));
                             odd = odd || rf_not_finite(sum);
                             *dst = sum;
                         }
@@ -1018,7 +1023,8 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
             for (int j = 0; j <= i; ++j)
                 s = fmaf(Af[i * (RC_CHUNK + 1) + j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
             float* to = out + ((size_t)(tok0 + i) * H + h) * dv + c;
-            if (i >= plain_from || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
+            const bool plain = i >= min(plain_from[(c - first) / RF_SLICE], plain_from[2]);
+            if (plain || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
         }
     }
     tg_before();

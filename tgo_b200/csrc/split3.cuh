@@ -2,10 +2,14 @@
 // (hi + mid + lo, 8 bits each, every rest exact), a product of two such sums is nine products that the
 // tensor cores form exactly, and the three smallest of them (mid lo, lo mid, lo lo: below 2^-26 of
 // the whole) are left out. What is not finite has no such sum: hi is then infinite or NaN and the rests
-// NaN, so that the result is not finite either, which the callers look for. bfloat16 numbers end at 2^-133: what is
-// below 2^-110 keeps fewer bits of its own (it is off by 2^-134 at most), unless the caller scales it up before.
+// NaN, so that the result is not finite either, which the callers look for. bfloat16 numbers end at 2^-133, so that
+// what is below 2^-110 would keep fewer bits: numbers are taken S3_UP times before they are cut (every float32
+// number then has all of its parts), and what they were multiplied into S3_DOWN times for each of them after.
 #pragma once
 #include "tcgen.cuh"
+
+#define S3_UP 0x1p24f
+#define S3_DOWN 0x1p-24f
 
 // The three parts of two neighbouring numbers, each part's two packed in one word. A number that rounds
 // past the largest bfloat16 gets an infinite hi.
@@ -25,15 +29,18 @@ __device__ __forceinline__ void s3_split8(const float (&v)[8], uint4& hi, uint4&
 // Whether one of two packed bfloat16 numbers is infinite or NaN.
 __device__ __forceinline__ bool s3_odd2(uint32_t w) { return (w & 0x7f80u) == 0x7f80u || (w & 0x7f800000u) == 0x7f800000u; }
 __device__ __forceinline__ bool s3_odd8(uint4 w) { return s3_odd2(w.x) || s3_odd2(w.y) || s3_odd2(w.z) || s3_odd2(w.w); }
-// The same with every part finite, for products whose masked terms must stay zero: a number that rounds past the
-// largest bfloat16 has its hi cut instead, one that is not finite is taken for 0. True: there was one of those.
-__device__ __noinline__ bool s3_mend8(const float* v, uint32_t* hi, uint32_t* mid, uint32_t* lo) {
-    bool odd = false;
+// The parts of S3_UP v, every part finite, for products whose masked terms must stay zero: what is not finite, or not S3_UP
+// times, is taken for 0, and a number that rounds past the largest bfloat16 has its hi cut instead. Bit 0 of the result:
+// there was a number that is not finite; bit 1: one that is too large.
+__device__ __noinline__ int s3_mend8(const float* v, uint32_t* hi, uint32_t* mid, uint32_t* lo) {
+    const float inf = __int_as_float(0x7f800000);
+    int odd = 0;
     for (int i = 0; i < 8; ++i) {
-        float x = v[i];
-        const bool ok = fabsf(x) < __int_as_float(0x7f800000);
-        odd = odd || !ok;
-        x = ok ? x : 0.f;
+        float x = v[i] * S3_UP;
+        if (!(fabsf(x) < inf)) {
+            odd |= fabsf(v[i]) < inf ? 2 : 1;
+            x = 0.f;
+        }
         uint32_t h = __float_as_uint(__bfloat162float(__float2bfloat16_rn(x)));
         if ((h & 0x7f800000u) == 0x7f800000u) h = __float_as_uint(x) & 0xffff0000u;
         const float r = x - __uint_as_float(h);
@@ -66,16 +73,21 @@ __device__ __forceinline__ void s3_fence() { asm volatile("fence.proxy.async.sha
 
 // A 16-byte piece's place in a tile of 128-byte rows with the 128-byte swizzle.
 __device__ __forceinline__ uint32_t s3_place(int row, int piece) { return (uint32_t)(row * 128 + ((piece ^ (row & 7)) << 4)); }
-// R eights to their places dst[r], dst[r] + step, dst[r] + 2 step with every part finite; true: a number was not. One test
-// for all of them, so that their chains of conversions run side by side.
-template <int R> __device__ __forceinline__ bool s3_put(const float (&v)[R][8], const uint32_t (&dst)[R], uint32_t step) {
+// S3_UP times R eights to their places dst[r], dst[r] + step, dst[r] + 2 step with every part finite; true: a number was not
+// finite, or too large (2^103 and more), and lies there as 0. Of the latter the smallest row goes to *too_large. One test for
+// all of them, so that their chains of conversions run side by side.
+template <int R>
+__device__ __forceinline__ bool s3_put(const float (&v)[R][8], const uint32_t (&dst)[R], uint32_t step, const int (&row)[R], int* too_large) {
     uint4 part[R][3];
     // the rest of what is not finite, or rounds to infinity, is not finite: 0 times it is not 0
     const __nv_bfloat162 zero = __floats2bfloat162_rn(0.f, 0.f);
     uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < R; ++r) {
-        s3_split8(v[r], part[r][0], part[r][1], part[r][2]);
+        float up[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) up[i] = v[r][i] * S3_UP;
+        s3_split8(up, part[r][0], part[r][1], part[r][2]);
         __nv_bfloat162 a = __hmul2(*(const __nv_bfloat162*)&part[r][1].x, zero), b = __hmul2(*(const __nv_bfloat162*)&part[r][1].y, zero);
         a = __hfma2(*(const __nv_bfloat162*)&part[r][1].z, zero, a);
         b = __hfma2(*(const __nv_bfloat162*)&part[r][1].w, zero, b);
@@ -94,9 +106,15 @@ template <int R> __device__ __forceinline__ bool s3_put(const float (&v)[R][8], 
                 for (int q = 1; q < R; ++q) f[i] = r == q ? v[q][i] : f[i];
             }
             uint32_t to = dst[0];
+            int at = row[0];
 #pragma unroll
-            for (int q = 1; q < R; ++q) to = r == q ? dst[q] : to;
-            odd = s3_mend8(f, w[0], w[1], w[2]) || odd;
+            for (int q = 1; q < R; ++q) {
+                to = r == q ? dst[q] : to;
+                at = r == q ? row[q] : at;
+            }
+            const int what = s3_mend8(f, w[0], w[1], w[2]);
+            if (what & 2) atomicMin(too_large, at);
+            odd = what != 0 || odd;
 #pragma unroll
             for (int q = 0; q < 3; ++q) s3_store16(to + q * step, make_uint4(w[q][0], w[q][1], w[q][2], w[q][3]));
         }
@@ -108,12 +126,13 @@ template <int R> __device__ __forceinline__ bool s3_put(const float (&v)[R][8], 
         for (int q = 0; q < 3; ++q) s3_store16(dst[r] + q * step, part[r][q]);
     return false;
 }
-__device__ __forceinline__ bool s3_put8(const float (&v)[8], uint32_t dst, uint32_t step) {
+__device__ __forceinline__ bool s3_put8(const float (&v)[8], uint32_t dst, uint32_t step, int row, int* too_large) {
     float f[1][8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) f[0][i] = v[i];
     const uint32_t to[1] = {dst};
-    return s3_put<1>(f, to, step);
+    const int at[1] = {row};
+    return s3_put<1>(f, to, step, at, too_large);
 }
 // D += A B^T over 16 KSTEPS of k and every kept pair of parts, the smallest first. Part p of A starts a_part * p
 // after da and a k-step a_k after the one before (descriptor units of 16 bytes); AP, BP: parts there are (1: the

@@ -503,9 +503,10 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
 // its diagonal, so that x goes in as it is and nothing is read for the results. Bound by the chains of conversions (about 2500
 // cycles a stage of 64 x 128 numbers for eight warps) and not by the products, 50 cycles each. Zeros of A times a value that is not finite are not
 // zero: such a number is laid down as 0, which leaves what does not depend on it as it is, bit for bit, and a
-// block that met one makes plain sums too (a thread a sum, out of global memory) and writes those that are not finite. An
-// A that is not finite without that, because C . B or its product with dt is too large, is 0 there too: the plain sums of its row
-// and the rows after it are written whatever they are. So are those in the place of a result that the products made overflow.
+// block that met one makes plain sums too (a thread a sum, out of global memory) and writes those that are not finite. A
+// finite number too large for its parts (2^103 and more), or an A whose C . B is (2^80), is 0 there too: the plain sums of its row
+// and the rows after it are written whatever they are, of its head if it is not one of B or C. So are those in the place of a result
+// that the products made overflow.
 #define SD_THREADS 512
 #define SD_HALF 256                   // of the outputs: one half lays the states and values down, the other A
 #define SD_HEADS 16                   // heads a block takes at most
@@ -552,16 +553,18 @@ template <int N> struct SdRows {
             v[j][1] = src[1];
         }
     }
-    __device__ __forceinline__ bool put(uint32_t tile, int n) const {
+    __device__ __forceinline__ bool put(uint32_t tile, int n, int* too_large) const {
         float f[RUNS][8];
         uint32_t dst[RUNS];
+        int row[RUNS];
 #pragma unroll
         for (int j = 0; j < RUNS; ++j) {
             const int i = threadIdx.x + j * SD_THREADS, r = i / (N / 8), piece = i % (N / 8);
             sd_eight(f[j], v[j][0], v[j][1], 1.f, r < n);
             dst[j] = tile + (piece >> 3) * SD_TILE + s3_place(r, piece & 7);
+            row[j] = r;
         }
-        return s3_put<RUNS>(f, dst, N / 64 * SD_TILE);
+        return s3_put<RUNS>(f, dst, N / 64 * SD_TILE, row, too_large);
     }
 };
 // x of a pair: 64 rows of 128 channels of neighbouring heads (channels past `width` are zeros), a row and head times
@@ -578,21 +581,24 @@ template <int THREADS> struct SdPair {
             v[j][1] = src[1];
         }
     }
-    // weights [128 / P][SD_CHUNK]; null: none
-    template <int P> __device__ __forceinline__ bool put(uint32_t tile, int n, int width, const float (*weights)[SD_CHUNK]) const {
+    // weights [128 / P][SD_CHUNK]; null: none. too_large: a place for each of the heads
+    template <int P> __device__ __forceinline__ bool put(uint32_t tile, int n, int width, const float (*weights)[SD_CHUNK], int* too_large) const {
         bool odd = false;
+        const int head = threadIdx.x % 16 * 8 / P;       // the same in every turn
 #pragma unroll
         for (int j0 = 0; j0 < RUNS; j0 += 2) {
             float f[2][8];
             uint32_t dst[2];
+            int row[2];
 #pragma unroll
             for (int j = 0; j < 2; ++j) {
                 const int i = threadIdx.x + (j0 + j) * THREADS, r = i / 16, piece = i % 16;
                 const bool in = r < n && piece * 8 < width;
-                sd_eight(f[j], v[j0 + j][0], v[j0 + j][1], in && weights ? weights[piece * 8 / P][r] : 1.f, in);
+                sd_eight(f[j], v[j0 + j][0], v[j0 + j][1], in && weights ? weights[head][r] : 1.f, in);
                 dst[j] = tile + (piece >> 3) * SD_TILE + s3_place(r, piece & 7);
+                row[j] = r;
             }
-            odd = s3_put<2>(f, dst, 2 * SD_TILE) || odd;
+            odd = s3_put<2>(f, dst, 2 * SD_TILE, row, too_large + head) || odd;
         }
         return odd;
     }
@@ -610,6 +616,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
     __shared__ float ws[2][HP][SD_CHUNK];
     __shared__ __align__(8) uint64_t bars[5];
     __shared__ uint32_t tmem_slot;
+    __shared__ int too_large[SD_HEADS + 1];              // a head's x; B
     uint64_t *v_full = bars, *v_done = bars + 2, *settled = bars + 4;
     pdl_wait();
     const int4 ch = chunks[blockIdx.x];
@@ -619,6 +626,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
     const float* rows = xbc + (size_t)ch.x * C;
     const size_t at = (size_t)blockIdx.x * nh + l0;      // the workspace holds the nh heads from `first` on
     if (warp == 0) tg_alloc<4 * N>(&tmem_slot);
+    if (threadIdx.x <= SD_HEADS) too_large[threadIdx.x] = SD_CHUNK;
     if (threadIdx.x == 0) {
         for (int i = 0; i < 2; ++i) { tg_init(&v_full[i], SD_THREADS / 32); tg_init(&v_done[i], 1); }
         tg_init(settled, 1);
@@ -650,7 +658,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
         b.load(rows + H * P + (h0 / (H / G)) * N, C, n);
         SdPair<SD_THREADS> x;
         x.load(rows + h0 * P, C, n, min(hb, HP) * P);
-        odd = b.put(tg_smem(sB), n);
+        odd = b.put(tg_smem(sB), n, &too_large[SD_HEADS]);
         for (int q = 0; q <= pairs; ++q) {
             if (q < pairs) {
                 const int heads = min(HP, hb - q * HP);
@@ -662,7 +670,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
                 }
                 ok = sd_sync<SD_THREADS>(ok);
                 if (!ok) break;
-                odd = x.put<P>(tg_smem(sV) + (q & 1) * STAGE, n, heads * P, ws[q & 1]) || odd;
+                odd = x.put<P>(tg_smem(sV) + (q & 1) * STAGE, n, heads * P, ws[q & 1], &too_large[q * HP]) || odd;
                 sd_full(&v_full[q & 1]);
                 if (q + 1 < pairs) x.load(rows + (h0 + (q + 1) * HP) * P, C, n, min(HP, hb - (q + 1) * HP) * P);
             }
@@ -682,7 +690,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
                     if (ok && l < hb)
 #pragma unroll
                         for (int i = 0; i < 16; ++i) {
-                            const float sum = __uint_as_float(r0[i]) + __uint_as_float(r1[i]);
+                            const float sum = (__uint_as_float(r0[i]) + __uint_as_float(r1[i])) * (S3_DOWN * S3_DOWN);
                             odd = odd || sd_not_finite(sum);
                             dst[i * P] = sum;
                         }
@@ -701,7 +709,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
             for (int j = 0; j < n; ++j)
                 sum = fmaf(br[(size_t)j * C + m], rows[(size_t)j * C + (h0 + l) * P + c] * (dts[o + j] * expf((float)(cum[o + n - 1] - cum[o + j]))), sum);
             float* to = U + ((at + l) * N + m) * P + c;
-            if (sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
+            if (min(too_large[l], too_large[SD_HEADS]) < SD_CHUNK || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
         }
     }
     tg_before();
@@ -780,7 +788,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
     unsigned char* sR = sB + sd_a_bytes<N, P>();         // [2]
     __shared__ double ls[SD_HEADS][SD_CHUNK];
     __shared__ float ds[SD_HEADS][SD_CHUNK], el[SD_HEADS][SD_CHUNK];
-    __shared__ int plain_from[SD_HEADS];                 // a head's first row whose plain sums are written whatever they are
+    __shared__ int plain_from[SD_HEADS + 1];             // the first row whose plain sums are written whatever they are: a head's; all heads'
     __shared__ __align__(8) uint64_t bars[13];
     __shared__ uint32_t tmem_slot;
     uint64_t *cb_full = bars, *s_done = bars + 1, *r_full = bars + 2 /* [2] */, *r_done = bars + 4 /* [2] */;
@@ -806,7 +814,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
         tg_init(settled, 1);
         tg_init_done();
     }
-    if (threadIdx.x < SD_HEADS) plain_from[threadIdx.x] = SD_CHUNK;
+    if (threadIdx.x <= SD_HEADS) plain_from[threadIdx.x] = SD_CHUNK;
     for (int i = threadIdx.x; i < hb * SD_CHUNK; i += SD_THREADS + 32) {
         const double l = cum[at * SD_CHUNK + i];
         (&ls[0][0])[i] = l;
@@ -862,8 +870,8 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
             SdRows<N> c, b;
             c.load(crow, C, n);
             b.load(brow, C, n);
-            odd = c.put(tg_smem(sC), n);
-            odd = b.put(tg_smem(sB), n) || odd;
+            odd = c.put(tg_smem(sC), n, &plain_from[SD_HEADS]);
+            odd = b.put(tg_smem(sB), n, &plain_from[SD_HEADS]) || odd;
         }
         sd_full(cb_full);
         if (warp < SD_HALF / 32) {
@@ -895,16 +903,17 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                         for (int j0 = 0; j0 < RUNS; j0 += 2) {
                             float f[2][8];
                             uint32_t dst[2];
+                            const int row[2] = {0, 0};   // every row sees the states
 #pragma unroll
                             for (int j = 0; j < 2; ++j) {
                                 const int i = threadIdx.x + (j0 + j) * SD_HALF, piece = i % 16;
                                 sd_eight(f[j], p[j0 + j][0], p[j0 + j][1], 1.f, piece * 8 < width);
                                 dst[j] = buf + (piece >> 3) * SD_TILE + s3_place(i / 16, piece & 7);
                             }
-                            odd = s3_put<2>(f, dst, 2 * SD_TILE) || odd;
+                            odd = s3_put<2>(f, dst, 2 * SD_TILE, row, &plain_from[q * HP + threadIdx.x % 16 * 8 / P]) || odd;
                         }
                     } else {
-                        odd = v.template put<P>(buf, n, width, nullptr) || odd;
+                        odd = v.template put<P>(buf, n, width, nullptr, &plain_from[q * HP]) || odd;
                     }
                     sd_full(&r_full[stage & 1]);
                     if (x == 0) v.load(rows + (h0 + q * HP) * P, C, n, width);
@@ -929,7 +938,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                         tg_wait_ld();
 #pragma unroll
                         for (int x = 0; x < 16; ++x)
-                            st[i * (SD_CHUNK + 1) + j0 + c + x] = __uint_as_float(s0[x]) + (HALVES > 1 ? __uint_as_float(s1[x]) : 0.f);
+                            st[i * (SD_CHUNK + 1) + j0 + c + x] = (__uint_as_float(s0[x]) + (HALVES > 1 ? __uint_as_float(s1[x]) : 0.f)) * (S3_DOWN * S3_DOWN);
                     }
                 }
                 sd_sync<SD_HALF>(ok);
@@ -955,7 +964,8 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                         }
                         const uint32_t tile = tg_smem(sA) + (uint32_t)(3 * e * SD_TILE);
                         const uint32_t dst[2] = {tile + s3_place(ai, aj / 8), tile + s3_place(ai, aj / 8 + 4)};
-                        if (s3_put<2>(f, dst, SD_TILE)) {
+                        const int at_row[2] = {ai, ai};
+                        if (s3_put<2>(f, dst, SD_TILE, at_row, &plain_from[q * HP + e])) {
                             atomicMin(&plain_from[q * HP + e], ai);
                             odd = true;
                         }
@@ -980,7 +990,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                             for (int i = 0; i < 16; ++i)
                                 if (i0 + c + i < n) {
                                     const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
-                                    const float sum = fmaf(far, el[l][i0 + c + i], __uint_as_float(a[i]));
+                                    const float sum = fmaf(far * (S3_DOWN * S3_DOWN), el[l][i0 + c + i], __uint_as_float(a[i]) * (S3_DOWN * S3_DOWN));
                                     odd = odd || sd_not_finite(sum);
                                     dst[(size_t)(c + i) * H * P] = sum;
                                 }
@@ -1012,7 +1022,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
                            dts[o + j] * rows[(size_t)j * C + (h0 + l) * P + c], sum);
             sum = fmaf(D ? D[h0 + l] : 0.f, rows[(size_t)i * C + (h0 + l) * P + c], sum);
             float* to = y + (size_t)(ch.x + i) * H * P + (h0 + l) * P + c;
-            if (i >= plain_from[l] || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
+            if (i >= min(plain_from[l], plain_from[SD_HEADS]) || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
         }
     }
     tg_before();
