@@ -1177,6 +1177,29 @@ def test_routed_experts_on_tensor_cores(T, d, ff, E, top, gated, activation):
     assert ((got.double() - want).abs() <= 2.0 ** -8 * size + 1e-5).all()
 
 
+@pytest.mark.parametrize("T", [1, 5, 67, 1203])
+@pytest.mark.parametrize("H,G,dk,dv,rot,biased,parts", [(16, 4, 128, 128, 64, True, 3), (3, 1, 48, 32, 16, True, 3), (2, 2, 64, 128, 64, False, 3),
+                                                        (8, 8, 96, 64, 0, True, 3), (6, 2, 80, 16, 48, True, 2), (5, 1, 256, 64, 256, False, 1)])
+def test_projection_rows_the_same_bits_by_either_form(T, H, G, dk, dv, rot, biased, parts):
+    """Rows that begin off 16 bytes go a channel a lane: the same bits, with and without keys, values, biases and a rotation."""
+    o, ps = ops(), 16
+    w, at = H * dk + G * (dk + dv), [H * dk, H * dk + G * dk]
+    x = rnd(T, w, seed=dk).to(torch.bfloat16)
+    bias = [b.contiguous() if biased else None for b in rnd(w, seed=3).split([at[0], G * dk, G * dv])]
+    rope = rnd(T, rot, seed=4) if rot else None
+    slots = torch.randperm(T + 9, generator=torch.Generator().manual_seed(1))[:T].to(torch.int32).to(DEV)
+    pages, outs = (T + 9 + ps - 1) // ps, []
+    for off in (0, 1):
+        z = torch.zeros(T, (w + 15) // 8 * 8 + off, dtype=torch.bfloat16, device=DEV)[:, off:w + off]
+        z.copy_(x)
+        kc, vc = (torch.zeros((pages, G, ps, n), dtype=torch.bfloat16, device=DEV) for n in (dk, dv))
+        q, k, v = z[:, :at[0]], z[:, at[0]:at[1]] if parts > 1 else None, z[:, at[1]:] if parts > 2 else None
+        o.qkv_bias_rope_cache(q, k, v, H, G if parts > 1 else 0, dk, dv, *bias, rope, rot, False, slots if parts > 1 else None,
+                              kc if parts > 1 else None, vc if parts > 2 else None, ps)
+        outs.append((z.clone(), kc, vc))
+    assert all(torch.equal(a, b) for a, b in zip(*outs))
+
+
 @pytest.mark.parametrize("T,d", [(5, 136), (300, 72)])
 def test_routed_experts_rounded(T, d):
     """Results in bfloat16 are the float32 ones rounded, with what is added to them."""

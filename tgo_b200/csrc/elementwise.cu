@@ -949,8 +949,9 @@ qkv_bias_rope_cache_x8_kernel(bf16* __restrict__ q, long long q_stride, const bf
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                     const float a = f[0][i + j], d = f[1][i + j];
-                    f[0][i + j] = a * c[j] - d * s[j];
-                    f[1][i + j] = d * c[j] + a * s[j];
+                    // each rounded as qkv_bias_rope_cache_kernel rounds it
+                    f[0][i + j] = fmaf(a, c[j], -__fmul_rn(d, s[j]));
+                    f[1][i + j] = fmaf(d, c[j], __fmul_rn(a, s[j]));
                 }
             }
         }
