@@ -1728,6 +1728,22 @@ def test_gated_group_norm_a_block_a_group(n, groups, act, first):
         test_gated_group_norm_in_fours(n, groups, act, first, dtype)
 
 
+@pytest.mark.parametrize("n,groups", [(516, 2), (1024, 1), (1028, 3), (1536, 1), (2044, 2)])
+@pytest.mark.parametrize("act,first", [(None, False), ("silu", True), ("sigmoid", False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_gated_group_norm_the_same_bits_by_either_form(n, groups, act, first, dtype):
+    """Gates and gains that begin off 16 bytes go a channel a lane: the same bits."""
+    T, W, outs = 37, n * groups, []
+    o, gain = rnd(T, W, seed=n), rnd(W, seed=2)
+    gate = rnd(T, W, seed=3).to(dtype)
+    for off in (0, 1):
+        at = torch.empty(W + off, device=DEV)[off:]
+        at.copy_(gain)
+        outs.append(torch.empty(T, W, dtype=dtype, device=DEV))
+        ops().gated_group_norm(o, gate if act else None, at, outs[-1], groups, 1e-5, act, first)
+    assert torch.equal(*outs)
+
+
 @pytest.mark.parametrize("H,dk,dv,ps", [(16, 576, 512, 16), (5, 576, 512, 8), (128, 264, 256, 64), (24, 200, 64, 32), (3, 448, 320, 128)])
 @pytest.mark.parametrize("window,sink", [(0, False), (130, True), (300, False)])
 def test_attention_latent_tc(H, dk, dv, ps, window, sink):

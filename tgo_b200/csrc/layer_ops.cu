@@ -459,16 +459,16 @@ __device__ __forceinline__ float gate_value(float z, int act) {
 
 // Groups of up to 512 channels that can be read four at a time (16 bytes of o and of the gain, 8 or
 // 16 of the gate): a warp a (token, group), V fours a lane in registers between the sum of squares
-// and the scaling; groups of up to 2048: the four warps of a block (WARPS) a group. Gate, gain and result as `gated_group_norm_kernel` below has them. Bound by
-// memory: every row read and written once. MEASURED (B200): 2048 tokens of 8 x 512 channels, silu,
-// 17 us (51 a channel a lane, four bytes at a time); 4096 tokens of 16 x 256 29 us (39); 2048 of
-// 1536, no gate, 6.3 us (10.5).
+// and the scaling; groups of up to 2048: the four warps of a block (WARPS) a group, which sum the squares in the order of
+// `gated_group_norm_kernel` (a channel a lane, eight warps), through shared memory. Gate, gain and result as that kernel
+// below has them. Bound by memory: every row read and written once. MEASURED (B200): 2048 tokens of 8 x 512 channels, silu,
+// 17 us (51 a channel a lane, four bytes at a time); 4096 tokens of 16 x 256 29 us (39); ten calls after each other, each of
+// 2048 of 1536, no gate: 6.3 us (8.9; 5.4 with each lane's own four summed), of 2 x 2048 10.9 (18.9).
 template <typename T, int V, int WARPS>
 __global__ void __launch_bounds__(128)
 gated_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ gate, long long gate_stride,
                             const float* __restrict__ gain, T* __restrict__ out, int n, int groups, float eps,
                             int gate_act, int gate_first, long long pairs) {
-    __shared__ float scratch[33];
     pdl_wait();
     const long long w = WARPS == 1 ? (long long)blockIdx.x * 4 + (threadIdx.x >> 5) : blockIdx.x;
     if (w >= pairs) return;
@@ -502,9 +502,32 @@ gated_group_norm_vec_kernel(const float* __restrict__ o, const T* __restrict__ g
         for (int k = 0; k < 4; ++k) {
             z[u][k] = gz ? gate_value(z[u][k], gate_act) : 1.f;
             if (gate_first) v[u][k] *= z[u][k];
-            ss += v[u][k] * v[u][k];
+            if (WARPS == 1) ss += v[u][k] * v[u][k];
         }
-    ss = WARPS == 1 ? warp_sum(ss) : block_sum(ss, scratch);
+    if constexpr (WARPS == 1) {
+        ss = warp_sum(ss);
+    } else {
+        __shared__ __align__(16) float row[128 * WARPS * V];
+        __shared__ float part[2 * WARPS];
+#pragma unroll
+        for (int u = 0; u < V; ++u) *(float4*)(row + 4 * lane + 128 * WARPS * u) = make_float4(v[u][0], v[u][1], v[u][2], v[u][3]);
+        __syncthreads();
+        float s2 = 0.f;                                  // of the warp four further on
+#pragma unroll
+        for (int i = 0; i < 128 * WARPS * V; i += 64 * WARPS) {          // past the group are zeros
+            const float a = row[i + lane], b = row[i + 32 * WARPS + lane];
+            ss += a * a;
+            s2 += b * b;
+        }
+        ss = warp_sum(ss);
+        s2 = warp_sum(s2);
+        if ((lane & 31) == 0) {
+            part[lane >> 5] = ss;
+            part[WARPS + (lane >> 5)] = s2;
+        }
+        __syncthreads();
+        ss = warp_sum((lane & 31) < 2 * WARPS ? part[lane & 31] : 0.f);
+    }
     const float r = rsqrtf(ss / (float)n + eps);
     T* y = out + (size_t)w * n;
 #pragma unroll
