@@ -262,6 +262,40 @@ def test_sgemm_by_parts_small_and_large_numbers(up, wide):
     assert ((y.double() - want).abs() <= K * 2.0 ** -24 * size + K * 2.0 ** -150).all()
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 1, 256), (40, 200, 1000), (557, 2048, 2048)])
+def test_sgemm_by_parts_past_their_range(M, N, K):
+    """Every output of numbers that the parts are not scaled for: the plain kernel's bits, at a time of its kind (an output
+    made by a thread for itself took 250 to 400 times as long as by parts; by tiles it is six to nine times)."""
+    from tgo_b200.kernels.build import load_library
+    lib, o = load_library("sgemm"), ops()
+    x, w = rnd(M, K, seed=5) * 1e33, rnd(N, K, seed=6) * 1e-5
+    x[:, 3] = 3e33                                       # every row has one past 2^103
+    outs = [torch.empty(M, N, device=DEV) for _ in range(2)]
+    assert lib.tgo_sgemm_part_bytes(ctypes.c_void_p(w.data_ptr()), K, N) > 0
+    o.sgemm_tn(x, w, outs[0])
+    try:
+        lib.tgo_sgemm_force_tile(1)
+        o.sgemm_tn(x, w, outs[1])
+    finally:
+        lib.tgo_sgemm_force_tile(0)
+    inside = (x.double() * 2.0 ** 24 @ (w.double() * 2.0 ** 24).t()).abs() < 2.0 ** 127
+    assert bool(torch.isfinite(outs[1]).all()) and not bool(inside.all())
+    assert torch.equal(*outs) and o.sgemm_error() == 0
+
+    def time(a):
+        best = float("inf")
+        for _ in range(5):
+            t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            t[0].record()
+            o.sgemm_tn(a, w, outs[0])
+            t[1].record()
+            torch.cuda.synchronize()
+            best = min(best, t[0].elapsed_time(t[1]))
+        return best
+    if M > 500:
+        assert time(x) <= 20 * time(x * 1e-33)
+
+
 @pytest.mark.parametrize("T,H,G,dk,dv,rot", [(1, 1, 1, 16, 16, 16), (11, 3, 1, 48, 32, 16), (130, 2, 2, 64, 128, 0),
                                              (1203, 16, 4, 128, 128, 64)])
 def test_projection_rows_eight_channels_at_a_time(T, H, G, dk, dv, rot):

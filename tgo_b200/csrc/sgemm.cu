@@ -182,7 +182,9 @@ TGO_API void tgo_sgemm_force_tile(int tile) { sg_forced = tile; }
 // of two higher every float32 number has all of its parts.
 // An output's arithmetic is the same whatever tile it falls in and whatever rows are beside it. An output
 // that is not finite (an input that is not, or is more than 2^103, or a sum past 2^80) is made again as the plain
-// kernel makes it.
+// kernel makes it: a block that has one makes its whole tile by FMA over tiles in shared memory (sp_plain) and writes
+// the outputs that were not finite. MEASURED, K = 2048, both launches: all of 557 x 2048 215 us (36 where all are finite; 8900
+// by a thread an output; 131 by the plain kernel), of 557 x 12288 1250 (136; 53000; 598), of one row x 2048 162 (28; 165; 60).
 // Bound by shared memory and the tensor pipe side by side at many rows (a k-block at NT = 128: 1660 and 1540
 // cycles), by the issue of 24 products a k-block at few. With w's parts in shared memory, made by the warps that
 // sum, and the products issued by a lane that no elect.sync had chosen, a k-block took 2500 cycles at any NT.
@@ -249,12 +251,77 @@ template <int N> __device__ __forceinline__ void sp_add(uint32_t t, float* acc) 
     }
 }
 
+// How many of the 256 threads that sum.
+__device__ __forceinline__ uint32_t sp_count(bool yes) {
+    uint32_t n;
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tbar.red.popc.u32 %0, 1, 256, p;\n\t}" : "=r"(n) : "r"((uint32_t)yes) : "memory");
+    return n;
+}
+
 // The registers (96 a thread at launch) go where they are used: 256 x (SP_SUM_REGS + SP_PART_REGS) + 128 x 40
 // is not more than 640 x 96.
 #define SP_SUM_REGS 128
 #define SP_PART_REGS 88
 template <int N> __device__ __forceinline__ void sp_regs_more() { asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(N)); }
 template <int N> __device__ __forceinline__ void sp_regs_less() { asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N)); }
+
+// The tile's outputs as sgemm_tn_kernel makes them, by the 256 threads that sum: NT / 16 x 8 outputs a thread, steps of 16 k
+// two ahead. Those that were finite stay.
+template <int NT>
+__device__ __forceinline__ void sp_plain(float* tile, const float* __restrict__ x, const float* __restrict__ w, float* __restrict__ y, int M, int N,
+                                         int K, int m0, int n0) {
+    constexpr int R = NT / 16, XF = SG_BK * (NT + 4), WF = SG_BK * (128 + 4);
+    static_assert(3 * (XF + WF) * (int)sizeof(float) <= SP_W_STAGES * SP_W_BYTES + SP_X_RING, "the rings' place");
+    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
+    unsigned long long acc[R][4];
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) acc[i][j] = 0ull;
+    auto load = [&](int st, int k0) {
+        if (k0 < K) {
+            float* to = tile + st * (XF + WF);
+            sg_load<NT, 256>((float (*)[NT + 4])to, x, m0, M, k0, K);
+            sg_load<128, 256>((float (*)[132])(to + XF), w, n0, N, k0, K);
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    load(0, 0);
+    load(1, SG_BK);
+    int st = 0;
+    for (int k0 = 0; k0 < K; k0 += SG_BK) {
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncwarp();
+        asm volatile("bar.sync 1, 256;" ::: "memory");   // this step's k are there, the last step's place is free
+        load(st == 0 ? 2 : st - 1, k0 + 2 * SG_BK);
+        const float* xb = tile + st * (XF + WF) + ty;
+        const float* wb = tile + st * (XF + WF) + XF + 4 * tx;
+        st = st == 2 ? 0 : st + 1;
+#pragma unroll 2
+        for (int kk = 0; kk < SG_BK; ++kk, xb += NT + 4, wb += 132) {
+            const ulonglong2 b0 = *(const ulonglong2*)wb, b1 = *(const ulonglong2*)(wb + 64);
+#pragma unroll
+            for (int i = 0; i < R; ++i) {
+                const unsigned long long aa = sg_pair(xb[16 * i], xb[16 * i]);
+                sg_fma2(acc[i][0], aa, b0.x); sg_fma2(acc[i][1], aa, b0.y);
+                sg_fma2(acc[i][2], aa, b1.x); sg_fma2(acc[i][3], aa, b1.y);
+            }
+        }
+    }
+#pragma unroll
+    for (int i = 0; i < R; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int m = m0 + ty + 16 * i, n = n0 + 64 * (j >> 1) + 4 * tx + 2 * (j & 1);
+            float v[2];
+            asm("mov.b64 {%0, %1}, %2;" : "=f"(v[0]), "=f"(v[1]) : "l"(acc[i][j]));
+#pragma unroll
+            for (int c = 0; c < 2; ++c) {
+                float* to = y + (size_t)m * N + n + c;
+                if (m < M && n + c < N && !(fabsf(*to) < __int_as_float(0x7f800000))) *to = v[c];
+            }
+        }
+}
 
 // Grid (tiles of x's rows, tiles of w's rows): the CTAs that read the same rows of w run side by side.
 // Every wait has a time limit; TMEM is freed on every path.
@@ -312,26 +379,20 @@ sgemm_tc_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant
             if (lane == 0) tg_arrive(&acc_empty[kb & 1]);
         }
         const int n = n0 + (warp & 3) * 32 + lane, mb = m0 + (warp >> 2) * CW;
+        bool odd = false;
         if (ok && n < N) {
-            const float inf = __int_as_float(0x7f800000);
             float* yo = y + (size_t)mb * N + n;
-            bool odd = false;
 #pragma unroll
             for (int i = 0; i < CW; ++i)
                 if (mb + i < M) {
                     yo[(size_t)i * N] = acc[i] * SP_DOWN;
-                    odd = odd || !(fabsf(acc[i]) < inf);
-                }
-            if (odd)                                     // as sgemm_tn_kernel makes it
-                for (int i = 0; i < CW && mb + i < M; ++i) {
-                    if (fabsf(yo[(size_t)i * N]) < inf) continue;
-                    const float* xr = x + (size_t)(mb + i) * K;
-                    const float* wn = w + (size_t)n * K;
-                    float v = 0.f;
-                    for (int k = 0; k < K; ++k) v = fmaf(xr[k], wn[k], v);
-                    yo[(size_t)i * N] = v;
+                    odd = odd || !(fabsf(acc[i]) < __int_as_float(0x7f800000));
                 }
         }
+        // every copy has landed and been read once the last products are there: the rings are free
+        __syncwarp();
+        const uint32_t waits = sp_count(!ok), odds = sp_count(odd);
+        if (!waits && odds) sp_plain<NT>((float*)wt, x, w, y, M, N, K, m0, n0);
     } else if (warp < 16) {
         sp_regs_less<SP_PART_REGS>();
         // a lane a row of w; warps 8..11 take the first 32 k of a k-block, 12..15 the others
