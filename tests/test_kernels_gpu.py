@@ -262,6 +262,26 @@ def test_sgemm_by_parts_small_and_large_numbers(up, wide):
     assert ((y.double() - want).abs() <= K * 2.0 ** -24 * size + K * 2.0 ** -150).all()
 
 
+def test_sgemm_by_parts_takes_a_bounded_workspace(monkeypatch):
+    """Rows whose parts together are past the bound go in groups: the same bits, two launches each, within it."""
+    o, M, N, K = ops(), 1001, 300, 1024
+    x, w = rnd(M, K, seed=5), rnd(N, K, seed=6)
+    want, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    o.sgemm_tn(x, w, want)
+    for rows, goes in ((400, 3), (1, 1001), (1001, 1)):
+        monkeypatch.setattr(o, "SGEMM_PARTS_BYTES", 6 * K * rows)
+        torch.cuda.synchronize()
+        torch.cuda.reset_peak_memory_stats()
+        before, launches = torch.cuda.memory_allocated(), o.LAUNCHES[0]
+        o.sgemm_tn(x, w, got.fill_(float("nan")))
+        torch.cuda.synchronize()
+        assert torch.cuda.max_memory_allocated() - before <= 6 * K * rows + 512 and o.LAUNCHES[0] - launches == 2 * goes
+        assert torch.equal(got, want)
+    monkeypatch.setattr(o, "SGEMM_PARTS_BYTES", 0)
+    o.sgemm_tn(x[:3].contiguous(), w, got[:3])
+    assert torch.equal(got[:3], want[:3])
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 1, 256), (40, 200, 1000), (557, 2048, 2048)])
 def test_sgemm_by_parts_past_their_range(M, N, K):
     """Every output of numbers that the parts are not scaled for: the plain kernel's bits, at a time of its kind (an output

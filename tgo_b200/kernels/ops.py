@@ -1579,6 +1579,11 @@ def retention_chunked(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, out: to
         LAUNCHES[0] += 2
 
 
+# What the parts of x (1.5 times x) may take: beyond it rows go in groups of about as many each, one after the other over
+# the same memory. A row's bits do not depend on the rows beside it.
+SGEMM_PARTS_BYTES = 256 << 20
+
+
 def sgemm_tn(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     """out[M,N] = x[M,K] . w[N,K]^T in true float32: on the tensor cores by parts where the sizes
     allow it (whatever M is), else by plain FMA."""
@@ -1591,10 +1596,13 @@ def sgemm_tn(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor) -> None:
     lib = entry_points("sgemm")
     row = lib.tgo_sgemm_part_bytes(_ptr(w), c_int(K), c_int(N)) if M > 0 else 0
     if row:
-        parts = torch.empty(M * row, dtype=torch.uint8, device=x.device)
-        _check(lib.tgo_sgemm_split(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), _ptr(parts), _stream()),
-               "sgemm_tn", f"(M={M}, N={N}, K={K})")
-        LAUNCHES[0] += 1
+        most = max(1, SGEMM_PARTS_BYTES // row)
+        most = -(-M // -(-M // most))
+        parts = torch.empty(min(M, most) * row, dtype=torch.uint8, device=x.device)
+        for m in range(0, M, most):
+            _check(lib.tgo_sgemm_split(x.data_ptr() + 4 * K * m, _ptr(w), out.data_ptr() + 4 * N * m, c_int(min(most, M - m)),
+                                       c_int(N), c_int(K), _ptr(parts), _stream()), "sgemm_tn", f"(M={M}, N={N}, K={K})")
+            LAUNCHES[0] += 1
         return
     _check(lib.tgo_sgemm_tn(_ptr(x), _ptr(w), _ptr(out), c_int(M), c_int(N), c_int(K), _stream()),
            "sgemm_tn", f"(M={M}, N={N}, K={K})")
