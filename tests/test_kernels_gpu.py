@@ -1713,6 +1713,31 @@ def test_selective_scan_by_chunks_in_groups_of_heads(H, G, N, P, monkeypatch):
     assert o.LAUNCHES[0] == launches + 1
 
 
+@pytest.mark.parametrize("H,G,most,at_once", [(64, 8, 22, 16), (64, 8, 40, 32), (48, 2, 30, 24), (6, 2, 4, 3)])
+def test_selective_scan_by_chunks_in_blocks_of_heads_at_a_time(H, G, most, at_once, monkeypatch):
+    """Blocks of several heads and a workspace for a part of them: whole blocks, about as many each time, in a workspace for
+    so many; the launches and the bits."""
+    from tgo_b200.kernels.build import load_library
+    o, N, P, T = ops(), 128, 64, 12000
+    lib, a_head, chunks = load_library("state_space"), N * P + 3 * 64, T // 64 + 1
+    lib.tgo_ssd_heads.restype = ctypes.c_int
+    floats = chunks * (most * a_head + 4)
+    assert lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(floats)) % 65536 == at_once
+    assert lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(chunks * (a_head + 3))) == 0
+    xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
+    a_log = torch.linspace(-3.0, 1.0, H, device=DEV)
+    monkeypatch.setattr(o, "SSD_WORKSPACE_BYTES", 1 << 40)
+    y, state = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P)
+    monkeypatch.setattr(o, "SSD_WORKSPACE_BYTES", 4 * floats)
+    torch.cuda.synchronize()
+    torch.cuda.reset_peak_memory_stats()
+    launches, before = o.LAUNCHES[0], torch.cuda.memory_allocated()
+    y2, state2 = chunked_scan(o, monkeypatch, xbc, dt_raw, a_log, H, G, N, P, chunks=None)
+    taken = torch.cuda.max_memory_allocated() - before - 4 * (T * H * P + H * N * P)
+    assert o.LAUNCHES[0] - launches == 4 * -(-H // at_once) and taken <= 4 * chunks * (at_once * a_head + 4) + 4096
+    assert torch.equal(y, y2) and torch.equal(state, state2) and bool(y.any())
+
+
 @pytest.mark.parametrize("H,G,N,P", [(4, 2, 128, 64), (2, 1, 64, 64), (3, 1, 128, 64), (3, 3, 64, 128), (2, 2, 128, 128)])
 @pytest.mark.parametrize("lens", [[128], [1, 63, 64, 65, 200, 3], [700, 129]])
 def test_selective_scan_by_chunks(H, G, N, P, lens, monkeypatch):

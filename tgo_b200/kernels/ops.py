@@ -1069,7 +1069,7 @@ def ssd_error() -> int:
 SSD_MIN_TOKENS = 160
 SSD_TOKENS_A_REQUEST = 64
 # What the workspace of a call may take: up to here all heads run at once (7700 tokens of the size above),
-# beyond it in groups of about as many heads each; a step too long for one head at a time walks.
+# beyond it in groups of about as many heads each (whole blocks of the kernels); a step too long for one head at a time walks.
 SSD_WORKSPACE_BYTES = 256 << 20
 
 
@@ -1094,26 +1094,24 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
     assert q_start.dtype == state_slots.dtype == torch.int32
     assert q_start.numel() == num_seqs + 1 and state_slots.numel() == num_seqs
     lib = entry_points("state_space")
-    chunk = lib.tgo_ssd_chunk_tokens()
-    n_chunks, a_head = max(1, T // chunk + num_seqs), state_dim * value_dim + 3 * chunk      # as tgo_ssd_scan says
-    most = min(heads, (SSD_WORKSPACE_BYTES // (4 * n_chunks) - 4) // a_head)         # heads at a time
-    if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and most > 0 and \
+    if dt_raw.dtype == torch.bfloat16 and T >= SSD_MIN_TOKENS and T >= SSD_TOKENS_A_REQUEST * num_seqs and \
             lib.tgo_ssd_takes(_ptr(xbc), _ptr(y), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(heads),
                               c_int(groups), c_int(state_dim), c_int(value_dim)):
-        goes = -(-heads // most)
-        most = -(-heads // goes)
-        if most < heads and heads // groups % 2 == 0:
-            most += most % 2                             # two heads may share a block
-            goes = -(-heads // most)
-        floats = n_chunks * (most * a_head + 4)
+        plan = lib.tgo_ssd_heads(c_int(T), c_int(num_seqs), c_int(heads), c_int(groups), c_int(state_dim), c_int(value_dim),
+                                 c_ll(SSD_WORKSPACE_BYTES // 4))
+    else:
+        plan = 0
+    if plan:
+        chunk, at_once = lib.tgo_ssd_chunk_tokens(), plan % 65536
+        floats = (T // chunk + num_seqs) * (at_once * (state_dim * value_dim + 3 * chunk) + 4)        # as tgo_ssd_heads says
         ws = torch.empty(floats, dtype=torch.float32, device=xbc.device)
         _check(lib.tgo_ssd_scan(
             _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y),
             c_int(T), c_int(num_seqs), c_int(heads), c_int(groups), c_int(state_dim), c_int(value_dim), _ptr(q_start),
-            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), _ptr(ws), c_ll(floats),
+            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(plan), _ptr(ws), c_ll(floats),
             _stream()), "ssd_scan",
             f"(heads={heads}, groups={groups}, state={state_dim}, vdim={value_dim})")
-        LAUNCHES[0] += 4 * goes - 1
+        LAUNCHES[0] += 4 * -(-heads // at_once) - 1
         return
     _check(lib.tgo_selective_scan(
         _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), c_int(dtype_code(dt_raw.dtype)),
