@@ -1327,7 +1327,7 @@ def test_routed_experts_activation_in_32_bits():
 @pytest.mark.parametrize("dk,dv,rot,act", [(64, 8, 0, 0), (64, 128, 32, 1), (128, 136, 128, 0), (128, 256, 64, 1)])
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_retention_by_tiled_chunks(dk, dv, rot, act, dtype):
-    """Heads the register-tiled kernels take, requests that end before, on and after a chunk, against
+    """Heads the tensor-core kernels take, requests that end before, on and after a chunk, against
     the recurrence in 64 bits: sums of at most dk + 64 float32 terms behind at most ten chunks."""
     o, H, lens = ops(), 3, [1, 63, 64, 65, 200, 577]
     T, B = sum(lens), len(lens)
@@ -1431,16 +1431,60 @@ def test_retention_by_tiled_chunks_looks_forward_only(dk, dv, dtype):
                     assert torch.equal(got[:, others], clean[:, others]), (t, bad)
 
 
-def retention_of_one(z, H, dk, dv, decay, k_scale, state):
+def retention_of_one(z, H, dk, dv, decay, k_scale, state, act=0):
     """One request through the chunked retention, its rows [q, k, v]: outputs [n, H, dv]; `state` [1, H, dk, dv] moves on."""
     o, n = ops(), z.shape[0]
     i32 = lambda x: torch.tensor(x, dtype=torch.int32, device=DEV)       # noqa: E731
     C, out = o.retention_chunk_tokens(), torch.full((n, H * dv), float("nan"), device=DEV)
     o.retention_chunked(z[:, :H * dk], z[:, H * dk:2 * H * dk], z[:, 2 * H * dk:], out, 1, H, dk, dv,
                         torch.tensor(decay, device=DEV), k_scale, None, 0, i32([0, n]), i32([0]), state,
-                        i32(list(range(0, n, C))), i32([min(C, n - a) for a in range(0, n, C)]), i32([0]))
+                        i32(list(range(0, n, C))), i32([min(C, n - a) for a in range(0, n, C)]), i32([0]), act=act)
     assert o.retention_error() == 0
     return out.view(n, H, dv)
+
+
+@pytest.mark.parametrize("dk,dv", [(64, 136), (64, 256), (128, 136), (128, 256), (128, 384)])
+@pytest.mark.parametrize("dtype,act", [(torch.float32, 0), (torch.bfloat16, 0), (torch.bfloat16, 1)])
+def test_retention_by_chunks_of_two_slices_a_block(dk, dv, dtype, act):
+    """Steps whose blocks take two slices of 128 value channels, the last cut or alone, against the recurrence in 64 bits; the bits
+    of a step so short that they take one. What is not finite in a second slice stays in its channel."""
+    H, n, decay = 4, 1300, [0.5, 0.9, 0.97, 1.0]
+    slices, sms = (dv + 127) // 128, torch.cuda.get_device_properties(0).multi_processor_count
+    assert (n + 63) // 64 * H * slices > sms >= 3 * H * slices           # two slices a block here, one in the short step
+    z = (rnd(n, H * (2 * dk + dv), seed=dk + dv) * 0.5).to(dtype)
+    start = rnd(1, H, dk, dv, seed=1)
+    state, short = start.clone(), start.clone()
+    got = retention_of_one(z, H, dk, dv, decay, dk ** -0.5, state, act)
+    assert torch.equal(retention_of_one(z[:150], H, dk, dv, decay, dk ** -0.5, short, act), got[:150])
+    q, k, v = (x.double().view(n, H, -1) for x in z.split([H * dk, H * dk, H * dv], 1))
+    if act:
+        q, k, v = (torch.nn.functional.silu(x) for x in (q, k, v))
+    S, want = start[0].double(), torch.empty(n, H, dv, dtype=torch.float64, device=DEV)
+    g = torch.tensor(decay, device=DEV).double()[:, None, None]
+    for t in range(n):
+        S = g * S + (k[t] * dk ** -0.5)[:, :, None] * v[t][:, None]
+        want[t] = torch.einsum("hkv,hk->hv", S, q[t])
+    # sums of dk + 64 float32 terms behind 21 chunks, and a chunk's powers of the decay by up to 64 products
+    for a in range(0, dv, 128):                          # a slice for itself, so that none hides behind another
+        b = min(dv, a + 128)
+        assert (got[:, :, a:b].double() - want[:, :, a:b]).norm() <= 3e-6 * want[:, :, a:b].norm()
+        assert (state[0, :, :, a:b].double() - S[:, :, a:b]).norm() <= 3e-6 * S[:, :, a:b].norm()
+    for t in (0, 70, 1299):
+        for bad in (float("nan"), float("inf")):
+            y = z.clone()
+            y[t, 2 * H * dk + dv + 130] = bad            # head 1
+            odd = retention_of_one(y, H, dk, dv, decay, dk ** -0.5, start.clone(), act)
+            others = torch.ones(H, dv, dtype=torch.bool, device=DEV)
+            others[1, 130] = False
+            assert torch.equal(odd[:t], got[:t]) and torch.equal(odd[:, others], got[:, others])
+            assert not bool(torch.isfinite(odd[t, 1, 130]))
+    if dtype == torch.float32:                           # too large for its parts: its slice of its head takes plain sums
+        y = z.clone()
+        y[70, 2 * H * dk + dv + 130] = 1e32
+        odd = retention_of_one(y, H, dk, dv, decay, dk ** -0.5, start.clone(), act)
+        assert torch.equal(odd[:70], got[:70]) and torch.equal(odd[:, [0, 2, 3]], got[:, [0, 2, 3]]) and torch.equal(odd[:, 1, :128], got[:, 1, :128])
+        score = (q[:, 1] @ (k[70, 1] * dk ** -0.5)) * g[1, 0, 0] ** torch.arange(-70, n - 70, device=DEV)
+        assert bool(((odd[70:, 1, 130].double() - want[70:, 1, 130] - 1e32 * score[70:]).abs() <= 1e32 * 1e-5 * score[70:].abs() + 1e26).all())
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
