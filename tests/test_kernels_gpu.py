@@ -234,6 +234,16 @@ def test_sgemm_by_parts(M, N, K):
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     assert ((outs[0].double() - want).abs() <= (K + 63) // 64 * 2.0 ** -21 * size).all()
     plain, got = torch.empty(M, N, device=DEV), torch.empty(M, N, device=DEV)
+    if M * N > 1000:
+        # that bound is one of the worst case, which two parts a number (2-norm 4e-6) stay below as well: three err by 1.3e-7
+        # (K = 2048) to 1.9e-7 (6144), and by no more than a chain of FMA
+        try:
+            lib.tgo_sgemm_force_tile(1)
+            ops().sgemm_tn(x, w, plain)
+        finally:
+            lib.tgo_sgemm_force_tile(0)
+        err = (outs[0].double() - want).norm()
+        assert err <= 4e-7 * want.norm() and err <= (plain.double() - want).norm()
     x[M // 2, 3], x[M - 1, K - 1], w[N // 2, 7] = float("inf"), float("nan"), -3.4e38
     x[0, 7] = 1e-3
     ops().sgemm_tn(x, w, got)
@@ -260,6 +270,8 @@ def test_sgemm_by_parts_small_and_large_numbers(up, wide):
     want, size = x.double() @ w.double().t(), x.double().abs() @ w.double().abs().t()
     # the bound of the parts, or a chain's of K roundings; a rounding below the normal numbers is 2^-150 at most
     assert ((y.double() - want).abs() <= K * 2.0 ** -24 * size + K * 2.0 ** -150).all()
+    if up < 1e20:                                        # by parts: all three of them, and one rounding to a number that may be no normal one
+        assert (y.double() - want).norm() <= 4e-7 * want.norm() + (M * N) ** 0.5 * 2.0 ** -149
 
 
 def test_sgemm_by_parts_takes_a_bounded_workspace(monkeypatch):
