@@ -16,7 +16,7 @@
 //               copy about every 80 cycles, and a key tile in pages of 16 takes 72 of K and 32 of V: one warp each, 138 us);
 //   warps 1, 11   issue S = Q K^T and O += P V, a thread each;
 //   warps 2..9  softmax, two threads a row, as in attention_tc.cu (lazily moved maximum).
-// Rows of V that nobody may read are zeroed by warp 10 once they have landed (P is zero there, but the
+// Rows of V that nobody may read are zeroed by warps 10 and 15, each in its slot, once they have landed (P is zero there, but the
 // cache may hold anything).
 //
 // MEASURED (B200, 2048 tokens of 16 heads, rows of 576, values of 512; mma.sync tiles of eight warps in
