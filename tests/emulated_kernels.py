@@ -536,7 +536,8 @@ def _plain_act(z, activation):
 
 def moe_feed_forward(x, w_router, b_router, w_gate, w_up, w_down, top, activation, extra=None,
                      scores="chosen", correction=None, identity=0, extra_gated=False, groups=1, keep=1,
-                     renormalize=True, route_scale=1.0, beside=None, residual=None, group_best=2):
+                     renormalize=True, route_scale=1.0, beside=None, residual=None, group_best=2,
+                     out_dtype=torch.float32):
     T, d = x.shape
     E = w_up.shape[0]
     outputs = E + identity
@@ -578,7 +579,7 @@ def moe_feed_forward(x, w_router, b_router, w_gate, w_up, w_down, top, activatio
     if residual is not None:
         residual += out
         return None
-    return out
+    return out.to(out_dtype)
 
 
 def act_rows(x, activation):

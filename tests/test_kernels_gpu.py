@@ -1267,13 +1267,14 @@ def test_projection_rows_the_same_bits_by_either_form(T, H, G, dk, dv, rot, bias
 
 
 @pytest.mark.parametrize("T,d", [(5, 136), (300, 72)])
-def test_routed_experts_rounded(T, d):
-    """Results in bfloat16 are the float32 ones rounded, with what is added to them."""
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_routed_experts_rounded(T, d, dtype):
+    """Results in bfloat16 are the float32 ones rounded, with what is added to them, of rows and matrices of either type."""
     o, ff, top, E = ops(), 40, 2, 6
-    x = rnd(T, d, seed=1).to(torch.bfloat16)
+    x = rnd(T, d, seed=1).to(dtype)
     wr = rnd(E, d, seed=2) * d ** -0.5
-    wg, wu = ((rnd(E, ff, d, seed=s) * d ** -0.5).to(torch.bfloat16) for s in (3, 4))
-    wd = (rnd(E, d, ff, seed=5) * ff ** -0.5).to(torch.bfloat16)
+    wg, wu = ((rnd(E, ff, d, seed=s) * d ** -0.5).to(dtype) for s in (3, 4))
+    wd = (rnd(E, d, ff, seed=5) * ff ** -0.5).to(dtype)
     run = lambda **kw: o.moe_feed_forward(x, wr, None, wg, wu, wd, top, "silu", rnd(T, d, seed=6),       # noqa: E731
                                           beside=rnd(T, d, seed=7).to(torch.bfloat16), **kw)
     assert torch.equal(run(out_dtype=torch.bfloat16), run().to(torch.bfloat16))

@@ -881,7 +881,7 @@ TGO_API int tgo_moe_route(const void* x, long long x_stride, int dtype, const fl
 }
 
 // x [T, d] rows (stride x_stride); wg, wu [E, ff, d]; wd [E, d, ff]; hidden [T top, ff] in the
-// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out [T, d], float32 or (bfloat16 x, no
+// storage type; y float32 [T top, d]; extra float32 [T, d] or null; out [T, d], float32 or (no
 // accumulation) bfloat16. xg: null, or
 // [T top, d] in the storage type, 16-byte aligned: room for the rows of x in place order.
 TGO_API int tgo_moe_experts(const void* x, long long x_stride, int dtype, const void* wg,
@@ -898,7 +898,7 @@ TGO_API int tgo_moe_experts(const void* x, long long x_stride, int dtype, const 
                          (uintptr_t)extra % 16 == 0 && (uintptr_t)out % 16 == 0 && (uintptr_t)beside % 16 == 0;
     const int comb_y = comb_vec && d > 512 ? (d / 512 < 16 ? d / 512 : 16) : 1;
     if ((beside && beside_dtype != TGO_F32 && beside_dtype != TGO_BF16) ||
-        (out_dtype != TGO_F32 && (out_dtype != TGO_BF16 || accumulate || dtype != TGO_BF16)))
+        (out_dtype != TGO_F32 && (out_dtype != TGO_BF16 || accumulate)))
         return TGO_E_BAD_ARG;
 #define MOE_COMBINE_OF(TT, TB, TO)                                                                         \
     tgo_launch_pdl(moe_combine_kernel<TT, TB, TO>, dim3(T, comb_y), dim3(128), 0, stream, (const float*)y, wts, extra,  \

@@ -1318,9 +1318,9 @@ def moe_feed_forward(x: torch.Tensor, w_router: torch.Tensor, b_router: Optional
     the weights are the chosen scores as they are. `route_scale` multiplies the weights.
 
     `beside` ([T, d], float32 or bfloat16) is added to the result; with `residual` (float32
-    [T, d]) the result is added there and None is returned. `out_dtype` bfloat16 (bfloat16 x, no
+    [T, d]) the result is added there and None is returned. `out_dtype` bfloat16 (no
     `residual`): the float32 sums rounded to it."""
-    assert out_dtype == torch.float32 or (out_dtype == x.dtype and residual is None)
+    assert out_dtype == torch.float32 or (out_dtype == torch.bfloat16 and residual is None)
     _need_cuda(x, w_router, b_router, w_gate, w_up, w_down, extra, correction, beside, residual)
     T, d = x.shape
     E, ff = w_up.shape[0], w_up.shape[1]

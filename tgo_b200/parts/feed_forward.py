@@ -296,12 +296,11 @@ class RoutedExperts(Part):
         x = ops.rows_of(x)
         extra = self.shared.forward(x, ctx) if self.shared is not None else None
         want = self.out_dtype or ctx.act_dtype
-        rounded = {"out_dtype": want} if residual is None and want != torch.float32 else {}
         return ops.moe_feed_forward(x, self.w_router, self.b_router, self.w_gate, self.w_up,
                                     self.w_down, self.top, self.activation, extra, self.scores,
                                     self.router_correction, self.identity, self.shared_gate,
                                     self.groups, self.keep, self.renormalize, self.route_scale,
-                                    beside, residual, self.group_best, **rounded)
+                                    beside, residual, self.group_best, want if residual is None else torch.float32)
 
 
 FEED_FORWARDS.register("routed_experts", RoutedExperts)
