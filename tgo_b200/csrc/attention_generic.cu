@@ -125,7 +125,10 @@ __global__ void attention_generic_kernel(
 // (B200, 301 + 256 tokens of 16/4 heads of 128, float32): a warp a query 772 us, this 75 (139 with each tile waited
 // for, each row's sums by themselves and the weights by shuffles); 64 tokens beside
 // fifteen single ones of 1000 keys, 16/4 heads of 128: 946 and 93 us (302; 1258 when a block walked the requests
-// that meet in it in turn), 8/8 heads of 64: 556 and 101 (178; 2691).
+// that meet in it in turn), 8/8 heads of 64: 556 and 101 (178; 2691). 32 rows a block and not 16: fewer blocks take a short
+// prompt, but keys come half as often (and groups of up to 32 heads fit): 20 calls in a row, with the 16 rows of the form before in
+// brackets, 20 tokens of 16/4 heads of 128 16.6 us (18.6), 33 of 8/8 of 64 18.6 (16.5), 128 29 (49) and 27 (35), 64 after 1000
+// 146 (329) and 115 (222); 32/1 heads of 64, a warp a query before: 4 tokens 10.4 (8.3), 8 10.9 (10.4), 20 12.4 (18).
 #define AGT_WARPS 8
 #define AGT_R 4
 #define AGT_Q (AGT_WARPS * AGT_R)

@@ -995,7 +995,10 @@ TGO_API int tgo_qkv_bias_rope_cache(void* q, long long q_stride, void* k, long l
     tgo_launch_pdl(qkv_bias_rope_cache_x8_kernel<TOK>, dim3((T + TOK - 1) / TOK, (unsigned)gy), dim3(QB8_THREADS), 0, stream, \
                    (bf16*)q, q_stride, (const bf16*)k, k_stride, (const bf16*)v, v_stride, T, H, Hkv, dk, dv, q_bias, k_bias,  \
                    v_bias, rope, rot, slots, (bf16*)k_cache, (bf16*)v_cache, page_size)
-        // four tokens a thread once that leaves four blocks a multiprocessor
+        // Four tokens a thread once that leaves four blocks a multiprocessor: about where both take as long. MEASURED, one and
+        // four, us, 20 calls in a row: 16 + 4 + 4 heads of 128, 64 turned (from 1184 tokens): 512 tokens 3.4 and 3.8, 1024 4.8 and 4.8,
+        // 2048 7.4 and 7.2, 3584 11.1 and 10.4; 32 + 8 + 8 of 128 (from 792): 512 4.3 and 4.4, 768 5.5 and 5.1, 2048 11.1 and
+        // 10.1; 8 + 2 + 2 of 64 (from 2368): 1024 2.6 and 3.2, 2048 3.9 and 3.4, 3584 5.2 and 5.5.
         if (gy <= 65535) return (T / 4) * gy >= 4LL * tgo_multiprocessors() ? QB8_GO(4) : QB8_GO(1);
 #undef QB8_GO
     }

@@ -1056,7 +1056,10 @@ static int retention_tc(const T* q, long long q_stride, const T* k, long long k_
         if ((e = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)s3)) != cudaSuccess) return (int)e;
         sized[dev] = true;
     }
-    // two slices a block, which share Q's and K's parts, unless blocks of one are fewer than the multiprocessors
+    // Two slices a block, which share Q's and K's parts, unless blocks of one are all on the chip at once. MEASURED, bfloat16,
+    // one slice and two, us: 4 heads of 128 x 256, 1024 tokens (128 blocks of one) 21.5 and 26.6, 1536 (192) 33.5 and 27.6; 16 of
+    // them, 256 tokens (128) 22.4 and 27.4, 512 (256) 35.5 and 29.3, 4096 264 and 202; 2 of 64 x 512, 1024 (128) 17.4 and 20.9,
+    // 1536 (192) 25.8 and 21.8.
     const int slices = (dv + RF_SLICE - 1) / RF_SLICE, per = (long long)chunks * H * slices > tgo_multiprocessors() ? 2 : 1;
     const int z = (slices + per - 1) / per;
     int rc = tgo_launch_pdl(k1, dim3(chunks, H, z), dim3(RC_THREADS), s1, stream, k, k_stride, v, v_stride, H, dv,

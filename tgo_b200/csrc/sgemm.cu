@@ -9,10 +9,10 @@
 // neighbouring columns go through one packed FMA (fma.rn.f32x2, each half rounded as a single
 // FMA is), which leaves issue slots for the reads (scalar FMA: 5 to 25 % slower). Steps of 16 k
 // come in by asynchronous 4-byte copies that lay them down k-major, two steps ahead.
-// MEASURED (B200, K = 2048; a 64 x 64 tile with 4 x 4 outputs a thread, loads and products in
-// turn, in brackets): 557 x 12288 outputs 597 us, 47 of 74 TFLOP/s (1272 us); 557 x 2048 134 us
-// (250); 100 x 12288 191 us (344); 3 x 32768 132 us (429); 1 x 2048 54 us (167): a single sum's
-// chain of 2048 FMA. ncu: FMA pipes 64 % busy, the rest waits for reads of shared memory.
+// MEASURED (B200, ten calls in a row), sizes that come here: K = 250, 557 x 12288 outputs 84 us, 41 of 74 TFLOP/s, 557 x
+// 2048 22, 1 x 2048 10.5; K = 128, 557 x 12288 47, 1 x 2048 6.5; K = 2050, whose rows are not whole 16 bytes, 557 x 12288 626,
+// 1 x 2048 56: a single sum's chain of 2050 FMA. At K = 2048 a 64 x 64 tile with 4 x 4 outputs a thread, loads and products in
+// turn, took 1272 for 557 x 12288 (597). ncu: FMA pipes 64 % busy, the rest waits for reads of shared memory.
 #include "common.cuh"
 
 #define SG_BK 16
@@ -560,7 +560,8 @@ TGO_API int tgo_sgemm_tn(const float* x, const float* w, float* y, int M, int N,
     // The tile: a round (as many tiles as SMs) costs `fixed` once and `round` each, in us at K = 2048,
     // fitted to the times of 15 products of 1 to 1200 rows (64 x 128: 123 us for one round, 597 for
     // six; 64 x 64: 88, 133 for two, 688 for twelve; 16 x 64: 54, 132 for four, 1450 for forty-six).
-    // 128 x 128 tiles were never the fastest (785 us where 64 x 128 took 597).
+    // 128 x 128 tiles were never the fastest (785 us where 64 x 128 took 597). For K = 64, 128, 250 and 2050, 1 to 1200 rows and
+    // 64 to 12288 outputs the choice is the fastest of the three tiles or at most 2 us behind it (1200 x 12288, K = 2050: 1304 of 1302).
     int pick = sg_forced;
     if (!pick) {
         static const struct { int bm, bn; double fixed, round; } tiles[3] = {

@@ -1062,10 +1062,12 @@ def ssd_error() -> int:
 
 
 # Steps of at least so many tokens, and so many a request on average, run the selective scan by
-# chunks in the bfloat16 engine (64 heads of 64 x 128, a call's wall time, walk against chunks: 64
-# tokens 28 against 36 us, 128 47 / 47, 256 90 / 60; 16 requests of 128 359 / 288; 256 tokens beside 31
-# single ones 198 / 226, 32 requests of 16 114 / 208: a chunk costs its two state-sized rows). The mean is
-# all the host knows without the lengths: one long portion beside many single tokens (1500 beside 31) walks.
+# chunks in the bfloat16 engine. Walk against chunks, us, 20 calls in a row: 64 heads of 64 x 128, one request of 64 tokens
+# 25 / 28, 96 35 / 29, 160 57 / 30, 256 88 / 32; 8 requests of 32 52 / 57, 16 of 40 121 / 104, 8 of 64 95 / 59, 16 of 128
+# 359 / 179, 32 of 16 112 / 207 (a chunk costs its two state-sized rows); 256 tokens beside 31 single ones 191 / 209. 24 heads:
+# 64 24 / 27, 96 35 / 27, 160 56 / 27. The walk is slower from about 80 tokens on (100 with 64 states); both lines lie where kernels
+# before these met it, and stay there because a step's bits are those of its form. The mean is all the host knows without
+# the lengths: one long portion beside many single tokens (1500 beside 31: 1004 / 296) walks.
 SSD_MIN_TOKENS = 160
 SSD_TOKENS_A_REQUEST = 64
 # What the workspace of a call may take: up to here all heads run at once (7700 tokens of the size above),
