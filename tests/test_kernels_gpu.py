@@ -314,18 +314,9 @@ def test_sgemm_by_parts_past_their_range(M, N, K):
     assert bool(torch.isfinite(outs[1]).all()) and not bool(inside.all())
     assert torch.equal(*outs) and o.sgemm_error() == 0
 
-    def time(a):
-        best = float("inf")
-        for _ in range(5):
-            t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
-            t[0].record()
-            o.sgemm_tn(a, w, outs[0])
-            t[1].record()
-            torch.cuda.synchronize()
-            best = min(best, t[0].elapsed_time(t[1]))
-        return best
     if M > 500:
-        assert time(x) <= 20 * time(x * 1e-33)
+        small = x * 1e-33
+        assert best_time(lambda: o.sgemm_tn(x, w, outs[0])) <= 20 * best_time(lambda: o.sgemm_tn(small, w, outs[0]))
 
 
 @pytest.mark.parametrize("T,H,G,dk,dv,rot", [(1, 1, 1, 16, 16, 16), (11, 3, 1, 48, 32, 16), (130, 2, 2, 64, 128, 0),
@@ -1543,6 +1534,32 @@ def test_retention_by_chunks_of_small_and_large_numbers(dk, dv, dtype, qs, ks, v
         assert (got[:, h] - want[:, h]).norm() <= 1e-6 * want[:, h].norm()
         # a state that is mostly the one before, n powers of the decay later, has a rounding of each of them on top
         assert (state[0, h].double() - S[h]).norm() <= (1e-6 + n * 2.0 ** -24) * S[h].norm()
+
+
+def best_time(run):
+    best = float("inf")
+    for _ in range(5):
+        t = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        t[0].record()
+        run()
+        t[1].record()
+        torch.cuda.synchronize()
+        best = min(best, t[0].elapsed_time(t[1]))
+    return best
+
+
+def test_chunked_kernels_of_no_numbers_at_a_time_of_their_kind(monkeypatch):
+    """Rows of NaN through retention and the selective scan by chunks: plain sums of sixteen rows a thread take seven to eight times
+    as long as a finite call, a sum a thread out of global memory took fifteen and more."""
+    z = rnd(4096, 16 * 512, seed=1).to(torch.bfloat16)
+    state = torch.zeros(1, 16, 128, 256, device=DEV)
+    run = lambda z: retention_of_one(z, 16, 128, 256, [0.9] * 16, 1.0, state.zero_())      # noqa: E731
+    bad = torch.full_like(z, float("nan"))
+    assert bool(torch.isnan(run(bad)).all()) and best_time(lambda: run(bad)) <= 11 * best_time(lambda: run(z))
+    xbc, dt_raw, a_log = rnd(2048, 64 * 64 + 16 * 128, seed=1), rnd(2048, 64, seed=3).to(torch.bfloat16), torch.zeros(64, device=DEV)
+    run = lambda x: chunked_scan(ops(), monkeypatch, x, dt_raw, a_log, 64, 8, 128, 64)[0]      # noqa: E731
+    bad = torch.full_like(xbc, float("nan"))
+    assert bool(torch.isnan(run(bad)).all()) and best_time(lambda: run(bad)) <= 11 * best_time(lambda: run(xbc))
 
 
 def scan_in_64_bits(xbc, dt_raw, a_log, d, H, G, N, P):

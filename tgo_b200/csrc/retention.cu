@@ -498,8 +498,9 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 //               sixteen lay the next operands down. (One slice a block, halves of Q, K and P one after the
 //               other, two blocks an SM: 167 us.)
 // Zeros of A times a value that is not finite are not zero: such a number is laid down as 0, which leaves what does
-// not depend on it as it is, bit for bit, and a block that met one makes plain sums too (a thread a sum, out of global
-// memory) and writes those that are not finite. A finite number too large for its parts (2^103 and more), or an A whose
+// not depend on it as it is, bit for bit, and a block that met one makes plain sums too (RF_PLAIN of a column a
+// thread; MEASURED, all three launches: 4096 tokens, 16 heads of 128 x 256, all NaN 1400 us, all finite 206; 3050 by a thread a sum) and
+// writes those that are not finite. A finite number too large for its parts (2^103 and more), or an A whose
 // Q K^T is (2^80), is 0 there too: the plain sums of its row and the rows after it are written whatever they are, in its slice if it
 // is one of V or P. So are those in the place of a result that the products made overflow.
 // MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
@@ -508,6 +509,7 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 #define RF_SLICE 128
 #define RF_TILE 8192                  // 64 rows of 64 bfloat16 numbers
 #define RF_LOOP_LD 129                // rows of the plain sums' tiles
+#define RF_PLAIN 16                   // plain sums a thread makes side by side
 
 __device__ int retention_error_flag = 0;
 
@@ -631,6 +633,32 @@ __device__ __forceinline__ bool rf_made(uint64_t* bar, uint32_t phase, int code)
     return ok;
 }
 
+// The plain sums of a block that met a number which is not finite or too large.
+template <typename T, int DK>
+__device__ __forceinline__ void rf_plain_summaries(float* Kf, const T* __restrict__ k, long long k_stride, const T* __restrict__ v, long long v_stride,
+                                                int H, int dv, float k_scale, int act, const float* __restrict__ rope, int rot, int tok0, int n,
+                                                int h, int first, int ns, const float* pw, const int* too_large, float* Uo) {
+    load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
+    __syncthreads();
+    for (int i = threadIdx.x; i < DK / RF_PLAIN * RF_SLICE * ns; i += RC_THREADS) {
+        const int d = i / (RF_SLICE * ns) * RF_PLAIN, c = first + i % (RF_SLICE * ns);
+        if (c >= dv) continue;
+        const bool plain = min(too_large[(c - first) / RF_SLICE], too_large[2]) < RC_CHUNK;
+        float s[RF_PLAIN] = {};
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+            const float x = rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act);
+#pragma unroll
+            for (int r = 0; r < RF_PLAIN; ++r) s[r] = fmaf(Kf[j * RF_LOOP_LD + d + r] * pw[n - 1 - j], x, s[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < RF_PLAIN; ++r) {
+            float* to = Uo + (size_t)(d + r) * dv + c;
+            if (plain || rf_not_finite(s[r]) || rf_not_finite(*to)) *to = s[r];
+        }
+    }
+}
+
 // VP: parts a value has (1: bfloat16 rows without an activation). A block makes the columns of up to two slices.
 template <typename T, int DK, int VP>
 __global__ void __launch_bounds__(RC_THREADS, VP == 1 ? 2 : 1)
@@ -702,6 +730,7 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
     float* Uo = U + ((size_t)ci * H + h) * DK * dv;
     if (ok) {
         const int d0 = (warp >> 2) * (DK / 2);
+        float nan = 0.f;
         for (int s = 0; s < ns; ++s) {
             const int c = first + s * RF_SLICE + (warp & 3) * 32 + lane;
 #pragma unroll
@@ -714,25 +743,13 @@ retention_summaries_tc_kernel(const T* __restrict__ k, long long k_stride, const
 #pragma unroll
                     for (int i = 0; i < 32; ++i, dst += dv) {
                         const float sum = __uint_as_float(r[i]) * (VP == 1 ? S3_DOWN : S3_DOWN * S3_DOWN);
-                        odd = odd || rf_not_finite(sum);
+                        nan = fmaf(sum, 0.f, nan);       // 0 as long as all are finite
                         *dst = sum;
                     }
             }
         }
-        if (__syncthreads_or(odd)) {
-            float* Kf = (float*)base;
-            load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
-            __syncthreads();
-            for (int i = threadIdx.x; i < DK * RF_SLICE * ns; i += RC_THREADS) {
-                const int d = i / (RF_SLICE * ns), c = first + i % (RF_SLICE * ns);
-                if (c >= dv) continue;
-                float s = 0.f;
-                for (int j = 0; j < n; ++j)
-                    s = fmaf(Kf[j * RF_LOOP_LD + d] * pw[n - 1 - j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
-                float* to = Uo + (size_t)d * dv + c;
-                const bool plain = min(too_large[(c - first) / RF_SLICE], too_large[2]) < RC_CHUNK;
-                if (plain || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
-            }
+        if (__syncthreads_or(odd || nan != 0.f)) {
+            rf_plain_summaries<T, DK>((float*)base, k, k_stride, v, v_stride, H, dv, k_scale, act, rope, rot, tok0, n, h, first, ns, pw, too_large, Uo);
         }
     } else {
         for (int s = 0; s < ns; ++s) tg_wait(&bars[s], 0, &retention_error_flag, 1);      // products that may still be under way
@@ -793,6 +810,52 @@ retention_scan4_kernel(int H, int dkdv, const float* __restrict__ decay, const i
 #define RF_OUT_THREADS 512           // and a warp that issues the products
 template <int DK> __host__ __device__ constexpr int rf_out_k() { return 3 * (DK / 64) * RF_TILE + 2 * 6 * RF_TILE; }
 template <int DK> __host__ __device__ constexpr int rf_out_bytes() { return rf_out_k<DK>() + 9 * RF_TILE; }
+
+template <typename T, int DK>
+__device__ __forceinline__ void rf_plain_outputs(float* Qf, const T* __restrict__ q, long long q_stride, const T* __restrict__ k, long long k_stride,
+                                              const T* __restrict__ v, long long v_stride, float* __restrict__ out, int H, int dv, float k_scale,
+                                              int act, const float* __restrict__ rope, int rot, int tok0, int n, int h, int first, int ns,
+                                              const float* pw, const int* plain_from, const float* __restrict__ Pc) {
+    // Qf [64][RF_LOOP_LD], then K's
+    float* Kf = Qf + RC_CHUNK * RF_LOOP_LD;
+    float* Af = Kf + RC_CHUNK * RF_LOOP_LD;          // [64][65]
+    load_rotated(Qf, RF_LOOP_LD, q, q_stride, h, DK, rope, rot, tok0, n, 1.f, act);
+    load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
+    __syncthreads();
+    for (int x = threadIdx.x; x < n * RC_CHUNK; x += RF_OUT_THREADS + 32) {
+        const int i = x / RC_CHUNK, j = x % RC_CHUNK;
+        float s = 0.f;
+        for (int d = 0; j <= i && d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Kf[j * RF_LOOP_LD + d], s);
+        Af[i * (RC_CHUNK + 1) + j] = j <= i ? s * pw[i - j] : 0.f;
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < RC_CHUNK / RF_PLAIN * RF_SLICE * ns; x += RF_OUT_THREADS + 32) {
+        const int i = x / (RF_SLICE * ns) * RF_PLAIN, c = first + x % (RF_SLICE * ns);
+        if (c >= dv || i >= n) continue;             // of rows past n the sums are made and not written
+        const int plain = min(plain_from[(c - first) / RF_SLICE], plain_from[2]);
+        float s[RF_PLAIN] = {};
+#pragma unroll 4
+        for (int d = 0; d < DK; ++d) {
+            const float p = Pc[(size_t)d * dv + c];
+#pragma unroll
+            for (int r = 0; r < RF_PLAIN; ++r) s[r] = fmaf(Qf[(i + r) * RF_LOOP_LD + d], p, s[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < RF_PLAIN; ++r) s[r] *= pw[i + r + 1];
+#pragma unroll 4
+        for (int j = 0; j < min(n, i + RF_PLAIN); ++j) {
+            const float y = rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act);
+#pragma unroll
+            for (int r = 0; r < RF_PLAIN; ++r)
+                if (j <= i + r) s[r] = fmaf(Af[(i + r) * (RC_CHUNK + 1) + j], y, s[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < RF_PLAIN; ++r) {
+            float* to = out + ((size_t)(tok0 + i + r) * H + h) * dv + c;
+            if (i + r < n && (i + r >= plain || rf_not_finite(s[r]) || rf_not_finite(*to))) *to = s[r];
+        }
+    }
+}
 
 template <typename T, int DK, int VP>
 __global__ void __launch_bounds__(RF_OUT_THREADS + 32, 1)
@@ -973,6 +1036,7 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
         }
         if (ok) {
             const int i0 = (warp >> 2) * 16;
+            float nan = 0.f;
             for (int s = 0; s < ns && ok; ++s) {
                 if (s > 0) ok = __all_sync(0xffffffffu, tg_wait(v_done, 1, &retention_error_flag, 4));
                 tg_after();
@@ -990,10 +1054,11 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
                             const float far = __uint_as_float(p0[i]) + (HALVES > 1 ? __uint_as_float(p1[i]) : 0.f);
                             const float sum = fmaf(far * (S3_DOWN * S3_DOWN), pw[i0 + i + 1],
                                                    __uint_as_float(a[i]) * (VP == 1 ? S3_DOWN : S3_DOWN * S3_DOWN));
-                            odd = odd || rf_not_finite(sum);
+                            nan = fmaf(sum, 0.f, nan);   // 0 as long as all are finite
                             *dst = sum;
                         }
             }
+            odd = odd || nan != 0.f;
         }
     }
     ok = __syncthreads_and(ok);
@@ -1001,31 +1066,8 @@ retention_outputs_tc_kernel(const T* __restrict__ q, long long q_stride, const T
     if (!ok) {                                           // products that may still be under way
         for (int x = 0; x < 8; ++x) tg_wait(&bars[x >> 1], x & 1, &retention_error_flag, 5);
     } else if (odd) {                                    // plain sums: a term past a row is not added at all
-        float* Qf = (float*)sQ;                          // [64][RF_LOOP_LD], then K's
-        float* Kf = Qf + RC_CHUNK * RF_LOOP_LD;
-        float* Af = Kf + RC_CHUNK * RF_LOOP_LD;          // [64][65]
-        load_rotated(Qf, RF_LOOP_LD, q, q_stride, h, DK, rope, rot, tok0, n, 1.f, act);
-        load_rotated(Kf, RF_LOOP_LD, k, k_stride, h, DK, rope, rot, tok0, n, k_scale, act);
-        __syncthreads();
-        for (int x = threadIdx.x; x < n * RC_CHUNK; x += THREADS + 32) {
-            const int i = x / RC_CHUNK, j = x % RC_CHUNK;
-            float s = 0.f;
-            for (int d = 0; j <= i && d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Kf[j * RF_LOOP_LD + d], s);
-            Af[i * (RC_CHUNK + 1) + j] = j <= i ? s * pw[i - j] : 0.f;
-        }
-        __syncthreads();
-        for (int x = threadIdx.x; x < n * RF_SLICE * ns; x += THREADS + 32) {
-            const int i = x / (RF_SLICE * ns), c = first + x % (RF_SLICE * ns);
-            if (c >= dv) continue;
-            float s = 0.f;
-            for (int d = 0; d < DK; ++d) s = fmaf(Qf[i * RF_LOOP_LD + d], Pc[(size_t)d * dv + c], s);
-            s *= pw[i + 1];
-            for (int j = 0; j <= i; ++j)
-                s = fmaf(Af[i * (RC_CHUNK + 1) + j], rf_value(v, v_stride, (size_t)(tok0 + j), h, dv, c, act), s);
-            float* to = out + ((size_t)(tok0 + i) * H + h) * dv + c;
-            const bool plain = i >= min(plain_from[(c - first) / RF_SLICE], plain_from[2]);
-            if (plain || rf_not_finite(s) || rf_not_finite(*to)) *to = s;
-        }
+        rf_plain_outputs<T, DK>((float*)sQ, q, q_stride, k, k_stride, v, v_stride, out, H, dv, k_scale, act, rope, rot, tok0, n, h, first, ns, pw,
+                                plain_from, Pc);
     }
     tg_before();
     __syncthreads();

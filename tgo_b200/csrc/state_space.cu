@@ -503,7 +503,8 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
 // its diagonal, so that x goes in as it is and nothing is read for the results. Bound by the chains of conversions (about 2500
 // cycles a stage of 64 x 128 numbers for eight warps) and not by the products, 50 cycles each. Zeros of A times a value that is not finite are not
 // zero: such a number is laid down as 0, which leaves what does not depend on it as it is, bit for bit, and a
-// block that met one makes plain sums too (a thread a sum, out of global memory) and writes those that are not finite. A
+// block that met one makes plain sums too (SD_PLAIN of a column a thread; MEASURED: 2048 tokens, 64 heads of 64 x 128, all NaN 1180 us, all finite 157; 2820
+// by a thread a sum) and writes those that are not finite. A
 // finite number too large for its parts (2^103 and more), or an A whose C . B is (2^80), is 0 there too: the plain sums of its row
 // and the rows after it are written whatever they are, of its head if it is not one of B or C. So are those in the place of a result
 // that the products made overflow.
@@ -511,6 +512,7 @@ ssd_steps_kernel(const T* __restrict__ dt_raw, long long dt_stride, const float*
 #define SD_HALF 256                   // of the outputs: one half lays the states and values down, the other A
 #define SD_HEADS 16                   // heads a block takes at most
 #define SD_TILE 8192                  // 64 rows of 64 bfloat16 numbers
+#define SD_PLAIN 16                   // plain sums a thread makes side by side
 
 __device__ int ssd_error_flag = 0;
 
@@ -603,6 +605,36 @@ template <int THREADS> struct SdPair {
         return odd;
     }
 };
+
+// The plain sums of a block that met a number which is not finite or too large. Not inlined: the products' chains take 2 to 4 % longer beside them.
+template <int N, int P>
+__device__ __noinline__ void sd_plain_summaries(float* Bf, const float* __restrict__ rows, const float* __restrict__ br, int C, int h0, int hb, int n,
+                                                const float* __restrict__ dts, const double* __restrict__ cum, const int* too_large, float* U) {
+    // Bf [64][N]
+    float* Wf = Bf + SD_CHUNK * N;                   // [hb][64]
+    for (int i = threadIdx.x; i < n * N; i += SD_THREADS + 32) Bf[i] = br[(size_t)(i / N) * C + i % N];
+    for (int i = threadIdx.x; i < hb * SD_CHUNK; i += SD_THREADS + 32) {
+        const int end = i / SD_CHUNK * SD_CHUNK + n - 1;
+        Wf[i] = i % SD_CHUNK < n ? dts[i] * expf((float)(cum[end] - cum[i])) : 0.f;
+    }
+    __syncthreads();
+    for (int i = threadIdx.x; i < hb * (N / SD_PLAIN) * P; i += SD_THREADS + 32) {
+        const int l = i / (N / SD_PLAIN * P), m = i / P % (N / SD_PLAIN) * SD_PLAIN, c = i % P;
+        const bool plain = min(too_large[l], too_large[SD_HEADS]) < SD_CHUNK;
+        float sum[SD_PLAIN] = {};
+#pragma unroll 4
+        for (int j = 0; j < n; ++j) {
+            const float v = rows[(size_t)j * C + (h0 + l) * P + c] * Wf[l * SD_CHUNK + j];
+#pragma unroll
+            for (int r = 0; r < SD_PLAIN; ++r) sum[r] = fmaf(Bf[j * N + m + r], v, sum[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < SD_PLAIN; ++r) {
+            float* to = U + (size_t)(l * N + m + r) * P + c;
+            if (plain || sd_not_finite(sum[r]) || sd_not_finite(*to)) *to = sum[r];
+        }
+    }
+}
 
 // Shared memory: B's parts (N / 64 tiles a part), two buffers of a pair's weighted values (two tiles a part).
 template <int N, int P>
@@ -701,16 +733,7 @@ ssd_summaries_kernel(const float* __restrict__ xbc, int C, int H, int G, int fir
     }
     ok = __syncthreads_and(ok);
     if (__syncthreads_or(odd) && ok) {                   // plain sums
-        const float* br = rows + H * P + (h0 / (H / G)) * N;
-        for (int i = threadIdx.x; i < hb * N * P; i += SD_THREADS + 32) {
-            const int l = i / (N * P), m = i / P % N, c = i % P;
-            const size_t o = (at + l) * SD_CHUNK;
-            float sum = 0.f;
-            for (int j = 0; j < n; ++j)
-                sum = fmaf(br[(size_t)j * C + m], rows[(size_t)j * C + (h0 + l) * P + c] * (dts[o + j] * expf((float)(cum[o + n - 1] - cum[o + j]))), sum);
-            float* to = U + ((at + l) * N + m) * P + c;
-            if (min(too_large[l], too_large[SD_HEADS]) < SD_CHUNK || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
-        }
+        sd_plain_summaries<N, P>((float*)sB, rows, rows + H * P + (h0 / (H / G)) * N, C, h0, hb, n, dts + at * SD_CHUNK, cum + at * SD_CHUNK, too_large, U + at * N * P);
     }
     tg_before();
     __syncthreads();
@@ -774,6 +797,58 @@ template <int N, int P> __host__ __device__ constexpr int sd_a_bytes() {
     return 3 * (N / 64 > 128 / P ? N / 64 : 128 / P) * SD_TILE;
 }
 template <int N, int P> __host__ __device__ constexpr int sd_out_bytes() { return 3 * (N / 64) * SD_TILE + sd_a_bytes<N, P>() + 2 * 6 * SD_TILE; }
+
+template <int N, int P>
+__device__ __noinline__ void sd_plain_outputs(float* Cf, const float* __restrict__ rows, const float* __restrict__ brow, const float* __restrict__ crow,
+                                              int C, int H, int h0, int hb, int n, const float* __restrict__ D, const double (*ls)[SD_CHUNK],
+                                              const float (*ds)[SD_CHUNK], const float (*el)[SD_CHUNK], const int* plain_from,
+                                              const float* __restrict__ U, float* y) {
+    // Cf [64][N]
+    float* Bf = Cf + SD_CHUNK * N;                   // [64][N + 1]
+    float* Sf = Bf + SD_CHUNK * (N + 1);             // [64][65]
+    for (int x = threadIdx.x; x < n * N; x += SD_THREADS + 32) {
+        Cf[x] = crow[(size_t)(x / N) * C + x % N];
+        Bf[x / N * (N + 1) + x % N] = brow[(size_t)(x / N) * C + x % N];
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < n * SD_CHUNK; x += SD_THREADS + 32) {
+        const int i = x / SD_CHUNK, j = x % SD_CHUNK;
+        float sum = 0.f;
+        for (int m = 0; j <= i && m < N; ++m) sum = fmaf(Cf[i * N + m], Bf[j * (N + 1) + m], sum);
+        Sf[i * (SD_CHUNK + 1) + j] = sum;
+    }
+    __syncthreads();
+    for (int x = threadIdx.x; x < hb * (SD_CHUNK / SD_PLAIN) * P; x += SD_THREADS + 32) {
+        const int l = x / (SD_CHUNK / SD_PLAIN * P), i = x / P % (SD_CHUNK / SD_PLAIN) * SD_PLAIN, c = x % P;
+        if (i >= n) continue;                        // of rows past n the sums are made and not written
+        const float* Uc = U + (size_t)l * N * P + c;
+        const float* xc = rows + (h0 + l) * P + c;
+        const int plain = min(plain_from[l], plain_from[SD_HEADS]);
+        const float Dh = D ? D[h0 + l] : 0.f;
+        float sum[SD_PLAIN] = {};
+#pragma unroll 4
+        for (int m = 0; m < N; ++m) {
+            const float u = Uc[(size_t)m * P];
+#pragma unroll
+            for (int r = 0; r < SD_PLAIN; ++r) sum[r] = fmaf(Cf[(i + r) * N + m], u, sum[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < SD_PLAIN; ++r) sum[r] *= el[l][i + r];
+        for (int j = 0; j < min(n, i + SD_PLAIN); ++j) {
+            const float v = ds[l][j] * xc[(size_t)j * C];
+#pragma unroll
+            for (int r = 0; r < SD_PLAIN; ++r)
+                if (j <= i + r) sum[r] = fmaf(Sf[(i + r) * (SD_CHUNK + 1) + j] * expf((float)(ls[l][i + r] - ls[l][j])), v, sum[r]);
+        }
+#pragma unroll
+        for (int r = 0; r < SD_PLAIN; ++r) {
+            if (i + r >= n) break;
+            const float last = fmaf(Dh, xc[(size_t)(i + r) * C], sum[r]);
+            float* to = y + (size_t)(i + r) * H * P + (h0 + l) * P + c;
+            if (i + r >= plain || sd_not_finite(last) || sd_not_finite(*to)) *to = last;
+        }
+    }
+}
 
 template <int N, int P>
 __global__ void __launch_bounds__(SD_THREADS + 32, 1)
@@ -1002,28 +1077,7 @@ ssd_outputs_kernel(const float* __restrict__ xbc, int C, int H, int G, int first
     }
     ok = __syncthreads_and(ok);
     if (__syncthreads_or(odd) && ok) {                   // plain sums: a token past a row is not added at all
-        float* Sf = (float*)sC;
-        for (int x = threadIdx.x; x < n * SD_CHUNK; x += SD_THREADS + 32) {
-            const int i = x / SD_CHUNK, j = x % SD_CHUNK;
-            float sum = 0.f;
-            for (int m = 0; j <= i && m < N; ++m) sum = fmaf(crow[(size_t)i * C + m], brow[(size_t)j * C + m], sum);
-            Sf[i * (SD_CHUNK + 1) + j] = sum;
-        }
-        __syncthreads();
-        for (int x = threadIdx.x; x < hb * n * P; x += SD_THREADS + 32) {
-            const int l = x / (n * P), i = x / P % n, c = x % P;
-            const size_t o = (at + l) * SD_CHUNK;
-            const float* Uc = U + (at + l) * N * P + c;
-            float sum = 0.f;
-            for (int m = 0; m < N; ++m) sum = fmaf(crow[(size_t)i * C + m], Uc[(size_t)m * P], sum);
-            sum *= expf((float)cum[o + i]);
-            for (int j = 0; j <= i; ++j)
-                sum = fmaf(Sf[i * (SD_CHUNK + 1) + j] * expf((float)(cum[o + i] - cum[o + j])),
-                           dts[o + j] * rows[(size_t)j * C + (h0 + l) * P + c], sum);
-            sum = fmaf(D ? D[h0 + l] : 0.f, rows[(size_t)i * C + (h0 + l) * P + c], sum);
-            float* to = y + (size_t)(ch.x + i) * H * P + (h0 + l) * P + c;
-            if (i >= min(plain_from[l], plain_from[SD_HEADS]) || sd_not_finite(sum) || sd_not_finite(*to)) *to = sum;
-        }
+        sd_plain_outputs<N, P>((float*)sC, rows, brow, crow, C, H, h0, hb, n, D, ls, ds, el, plain_from, U + at * N * P, y + (size_t)ch.x * H * P);
     }
     tg_before();
     __syncthreads();
@@ -1042,7 +1096,8 @@ static int ssd_go(const float* xbc, int C, const bf16* dt_raw, long long dt_stri
                   const float* D, float* y, int T, int B, int H, int G, const int* q_start, const int* state_slots,
                   float* state, long long state_stride, long long offset, float* ws, int each, int hb, cudaStream_t stream) {
     constexpr size_t s1 = 1024 + (3 * (N / 64) + 2 * 6) * SD_TILE, s3 = 1024 + sd_out_bytes<N, P>();
-    static_assert(s3 >= 1024 + SD_CHUNK * (SD_CHUNK + 1) * sizeof(float), "the plain sums' tile");
+    static_assert(s1 >= 1024 + SD_CHUNK * (N + SD_HEADS) * sizeof(float), "the plain sums' tiles");
+    static_assert(s3 >= 1024 + SD_CHUNK * (2 * N + 1 + SD_CHUNK + 1) * sizeof(float), "the plain sums' tiles");
     static bool sized[64] = {};                          // per device
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
