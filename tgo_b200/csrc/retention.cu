@@ -504,7 +504,7 @@ retention_outputs_kernel(const T* __restrict__ q, long long q_stride, const T* _
 // Q K^T is (2^80), is 0 there too: the plain sums of its row and the rows after it are written whatever they are, in its slice if it
 // is one of V or P. So are those in the place of a result that the products made overflow.
 // MEASURED (B200, 4096 tokens, 16 heads of 128 x 256, bfloat16 rows; register tiles of packed FMA in brackets):
-// summaries 50 us (122), scan 40, outputs 119 us (190). The summaries are bound by the bytes of U; a block of the outputs
+// summaries 51 us (122), scan 40, outputs 121 us (190). The summaries are bound by the bytes of U; a block of the outputs
 // by its chain: loads 5000 cycles, parts of Q and K 3000, 168 products of 75 cycles, results 2300.
 #define RF_SLICE 128
 #define RF_TILE 8192                  // 64 rows of 64 bfloat16 numbers

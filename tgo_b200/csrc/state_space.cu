@@ -415,7 +415,7 @@ TGO_API int tgo_selective_scan(const float* xbc, int C, const void* dt_raw, long
 // sums lose nothing), summaries (the sum of S's line), a scan over the chunks, which leaves the
 // state before each chunk in its summary's place, and outputs. MEASURED (B200, 2048 tokens, 64 heads of 64 x 128):
 // 711 us by the walk above, 224 with float32 products in register tiles of packed FMA (summaries 52, scan over the
-// chunks 32, outputs 132), 148 with their parts on the tensor cores (30, 31, 82); errors against 64 bits, means of 15
+// chunks 32, outputs 132), 151 with their parts on the tensor cores (31, 32, 84); errors against 64 bits, means of 15
 // draws: outputs 0.9e-7 (1.1e-7 by FMA), state 8.4e-8 (8.7e-8).
 // The workspace is a state's size a chunk and head; a call whose workspace does not hold all heads takes
 // them in groups, one after the other over the same memory (heads do not meet; the sums are the same).
