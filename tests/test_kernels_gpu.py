@@ -1796,7 +1796,9 @@ def test_selective_scan_by_chunks_in_blocks_of_heads_at_a_time(H, G, most, at_on
     lib, a_head, chunks = load_library("state_space"), N * P + 3 * 64, T // 64 + 1
     lib.tgo_ssd_heads.restype = ctypes.c_int
     floats = chunks * (most * a_head + 4)
-    assert lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(floats)) % 65536 == at_once
+    plan = lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(floats))
+    assert plan % 65536 == at_once
+    assert lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(chunks * (at_once * a_head + 4))) == plan
     assert lib.tgo_ssd_heads(T, 1, H, G, N, P, ctypes.c_longlong(chunks * (a_head + 3))) == 0
     xbc, dt_raw = rnd(T, H * P + 2 * G * N, seed=N + P), rnd(T, H, seed=3).to(torch.bfloat16)
     a_log = torch.linspace(-3.0, 1.0, H, device=DEV)

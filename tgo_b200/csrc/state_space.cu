@@ -1143,31 +1143,33 @@ TGO_API int tgo_ssd_takes(const void* xbc, const void* y, const void* state, lon
 // tgo_ssd_chunk_tokens() + B) times (h (N P + 3 tgo_ssd_chunk_tokens()) + 4) for h heads at a time (a summary, the steps' sizes and
 // logarithms, and what each chunk is). 0: not one head.
 // Heads a block: as many of a group as leave a block a multiprocessor, so that B and C are laid down once for them.
-// Heads at a time: about as many each time as the workspace makes needful, in whole blocks.
+// Heads at a time: about as many each time as the workspace makes needful, in whole blocks. What they take of the
+// workspace gives the same answer again.
 TGO_API int tgo_ssd_heads(int T, int B, int H, int G, int N, int P, long long ws_floats) {
     if (T <= 0 || B <= 0 || H <= 0 || H > 65535 || G <= 0 || H % G) return 0;
     const int n_chunks = T / SD_CHUNK + B, group = H / G;                // at least as many as there are
     long long most = (ws_floats / n_chunks - 4) / (N * P + 3 * SD_CHUNK);
     if (most <= 0) return 0;
     if (most > H) most = H;
-    int hb = 1;
-    for (int d = 1; d <= group && d <= most && d <= SD_HEADS; ++d)
-        if (group % d == 0 && (d <= 128 / P || (long long)n_chunks * (most / d) >= tgo_multiprocessors())) hb = d;
-    const int blocks = H / hb, at_once = (int)(most / hb), goes = (blocks + at_once - 1) / at_once;
-    return (blocks + goes - 1) / goes * hb + 65536 * hb;
+    int answer = 0;
+    for (int d = 1; d <= group && d <= most && d <= SD_HEADS; ++d) {
+        if (group % d) continue;
+        const int blocks = H / d, at_once = (int)(most / d), goes = (blocks + at_once - 1) / at_once;
+        const int each = (blocks + goes - 1) / goes;
+        if (d <= 128 / P || (long long)n_chunks * each >= tgo_multiprocessors()) answer = each * d + 65536 * d;
+    }
+    return answer;
 }
 
-// As tgo_selective_scan with dt_raw in bfloat16; heads: tgo_ssd_heads' answer; ws: the floats that h = heads % 65536
-// takes, 16-byte aligned.
+// As tgo_selective_scan with dt_raw in bfloat16; ws: ws_floats floats, 16-byte aligned, shared out as tgo_ssd_heads says.
 TGO_API int tgo_ssd_scan(const float* xbc, int C, const void* dt_raw, long long dt_stride, const float* dt_bias,
                          const float* A_log, const float* D, float* y, int T, int B, int H, int G, int N, int P,
                          const int* q_start, const int* state_slots, float* state, long long state_stride,
-                         long long ssm_offset, int heads, float* ws, long long ws_floats, cudaStream_t stream) {
+                         long long ssm_offset, float* ws, long long ws_floats, cudaStream_t stream) {
     if (B <= 0 || T <= 0) return 0;
-    const int each = heads % 65536, hb = heads / 65536;
+    const int heads = tgo_ssd_heads(T, B, H, G, N, P, ws_floats), each = heads % 65536, hb = heads / 65536;
     if (!tgo_ssd_takes(xbc, y, state, state_stride, ssm_offset, H, G, N, P) || C != H * P + 2 * G * N ||
-        state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16 || hb <= 0 || hb > SD_HEADS ||
-        H / G % hb || each <= 0 || each % hb || ws_floats < (long long)(T / SD_CHUNK + B) * ((long long)each * (N * P + 3 * SD_CHUNK) + 4))
+        state_stride < ssm_offset + (long long)H * N * P || !ws || (uintptr_t)ws % 16 || !heads)
         return TGO_E_BAD_ARG;
 #define SD_GO(N, P)                                                                                                    \
     return ssd_go<N, P>(xbc, C, (const bf16*)dt_raw, dt_stride, dt_bias, A_log, D, y, T, B, H, G, q_start, state_slots, state, \

@@ -1110,7 +1110,7 @@ def selective_scan(xbc: torch.Tensor, dt_raw: torch.Tensor, dt_bias: Optional[to
         _check(lib.tgo_ssd_scan(
             _ptr(xbc), c_int(C), _ptr(dt_raw), c_ll(dt_raw.stride(0)), _ptr(dt_bias), _ptr(a_log), _ptr(d_skip), _ptr(y),
             c_int(T), c_int(num_seqs), c_int(heads), c_int(groups), c_int(state_dim), c_int(value_dim), _ptr(q_start),
-            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), c_int(plan), _ptr(ws), c_ll(floats),
+            _ptr(state_slots), _ptr(state), c_ll(state.stride(0)), c_ll(ssm_offset), _ptr(ws), c_ll(floats),
             _stream()), "ssd_scan",
             f"(heads={heads}, groups={groups}, state={state_dim}, vdim={value_dim})")
         LAUNCHES[0] += 4 * -(-heads // at_once) - 1
